@@ -44,6 +44,12 @@ extern "C" {
 #define WG_PREC_MOD2 4
 #define WG_PREC_MOD3 5
 #define WG_PREC_MOD4 6
+/* Added to a precision: evaluate the sieve term by term.  Without it an instance's whole sum (no
+ * term range, finite-difference signs, symmetric matrix) is taken by the elimination tree, which
+ * shares the work of terms with common signs and rounds less; the per-term evaluation is the one
+ * whose term magnitudes, chunks and partials the plan reports (a plan with trees runs it when they
+ * are asked for). */
+#define WG_PREC_TERMS 64
 #define WG_MOD_PRIME_0 2147483647u
 #define WG_MOD_PRIME_1 2147483629u
 #define WG_MOD_PRIME_2 2147483587u

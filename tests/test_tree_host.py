@@ -1,0 +1,96 @@
+"""The elimination tree (tree_kernel.cuh, tree_host.h) against the oracle, on the CPU: the node
+functions compiled for the host over a scalar type whose loads and stores are checked against their
+buffers, walked as the CTA kernel walks a task and as the level launches walk blocks of nodes, over
+the forms an instance can take (simple and multiple edges, self-paired modes, loop weights, an
+unpaired vertex, batches; one photon pair up to more pairs than a block holds)."""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+import oracle
+import thewalrus_gb300 as tw
+from thewalrus_gb300 import _native as nat
+from thewalrus_gb300 import workloads as wl
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def exe(tmp_path_factory):
+    nvcc = nat._nvcc()
+    if not (os.path.exists(nvcc) or shutil.which(nvcc)):
+        pytest.skip("nvcc not available")
+    path = str(tmp_path_factory.mktemp("tree") / "tree_check")
+    build = subprocess.run([nvcc, "-std=c++17", "-O1", "-o", path, os.path.join(HERE, "tree_check.cu")],
+                           stdout=subprocess.PIPE, stderr=subprocess.STDOUT, timeout=300)
+    assert build.returncode == 0, build.stdout.decode()
+    return path
+
+
+def evaluate(exe, inst, budget, split):
+    s, n = inst.struct, inst.struct.n
+    words = [s.kind, n, s.E, s.batch_max, s.cutoff, s.has_odd, budget, split] + list(inst.reps)
+
+    def put(x, count):
+        x = np.zeros(count) if x is None else np.asarray(x).reshape(-1)
+        for z in x.astype(complex):
+            words.extend([repr(float(z.real)), repr(float(z.imag))])
+
+    put(inst.A, n * n)
+    put(inst.D, n)
+    put(inst.oddV, n)
+    words.extend([repr(s.oddloop[0]), repr(s.oddloop[1])])
+    run = subprocess.run([exe], input=" ".join(str(w) for w in words).encode(), stdout=subprocess.PIPE,
+                         stderr=subprocess.STDOUT, timeout=120)
+    assert run.returncode == 0, run.stdout.decode()
+    v = np.array([[float(x) for x in line.split()] for line in run.stdout.decode().split("\n") if line])
+    return v[:, 0] + 1j * v[:, 1], v[:, 2] + 1j * v[:, 3]
+
+
+def check(exe, inst, want):
+    # the sums of these small instances cancel by less than 1e3, so 1e-11 leaves a factor of 100
+    want = np.atleast_1d(np.asarray(want, dtype=complex))
+    for budget, split in ((1e9, 0), (3e4, 2), (2e3, 40)):
+        for got in evaluate(exe, inst, budget, split):
+            assert np.max(np.abs(got - want)) <= 1e-11 * np.max(np.abs(want)), (budget, split, got, want)
+
+
+@pytest.mark.parametrize("n", [2, 4, 6, 8, 10, 14, 18])
+def test_simple_edges(exe, n):
+    A = wl.complex_symmetric(n, seed=n)
+    check(exe, tw.prepare_hafnian(A), complex(oracle.hafnian_repeated(A, [1] * n)))
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 9, 12, 15])
+def test_loops(exe, n):
+    A = wl.complex_symmetric(n, seed=40 + n)
+    D = wl.complex_symmetric(n, seed=80 + n)[0]
+    check(exe, tw.prepare_loop_hafnian(A, D, [1] * n), complex(oracle.hafnian_repeated(A, [1] * n, mu=D, loop=True)))
+
+
+@pytest.mark.parametrize("reps", [[2], [6], [1, 1, 2], [2, 2], [4, 1, 1], [3, 3, 3, 1], [2, 2, 2, 2, 1, 1],
+                                  [5, 1, 2, 2, 1, 1, 0, 2], [12, 10], [2] * 7, [3, 1, 1, 1, 2, 1, 1]])
+@pytest.mark.parametrize("loop", [False, True])
+def test_multiple_edges(exe, reps, loop):
+    n = len(reps)
+    A = wl.complex_symmetric(n, seed=sum(reps)) * 0.4
+    D = wl.complex_symmetric(n, seed=7)[0]
+    for extra in ([0, 1] if loop else [0]):  # one photon more: an unpaired vertex
+        r = list(reps)
+        r[0] += extra
+        prep = tw.prepare_loop_hafnian(A, D, r) if loop else tw.prepare_hafnian(A, r)
+        check(exe, prep, complex(oracle.hafnian_repeated(A, r, mu=D, loop=loop)))
+
+
+@pytest.mark.parametrize("fixed", [[0, 0], [1, 0], [1, 1, 1, 1], [2, 1, 0, 2], [3, 1, 2], [1] * 7, [4, 4, 1]])
+@pytest.mark.parametrize("cutoff", [1, 4, 7])
+def test_batches(exe, fixed, cutoff):
+    n = len(fixed) + 1
+    A = wl.complex_symmetric(n, seed=n) * 0.5
+    D = wl.complex_symmetric(n, seed=9)[0]
+    want = [complex(oracle.hafnian_repeated(A, list(fixed) + [k], mu=D, loop=True)) if sum(fixed) + k else 1.0
+            for k in range(cutoff + 1)]
+    check(exe, tw.prepare_loop_hafnian_batch(A, D, list(fixed), cutoff), want)

@@ -72,9 +72,10 @@ def _integer_valued(*arrays):
 def _auto(precision, insts):
     """The precision of a call: the caller's, else exact for integer inputs (the sieve over
     residues modulo 31-bit primes, so integer hafnians come back exactly, rounded once to
-    complex128), else FP64."""
+    complex128), else FP64.  "fp64" asked for by name is the per-term evaluation, the one whose
+    rounding the term magnitudes bound and which "auto" judges."""
     if precision:
-        return precision
+        return "fp64-terms" if precision == "fp64" else precision
     if insts and all(_integral(i) for i in insts) and nat.exact_primes(insts) is not None:
         return "exact"
     return DEFAULT_PRECISION
@@ -303,6 +304,8 @@ AUTO_RTOL = 1e-10
 def run_with_magnitudes(instances, precision="fp64"):
     """Outputs of the instances with, per output, sum |prefactor x term| times the final scale
     (the size of the terms the output cancels from): (values, magnitudes)."""
+    if not precision.endswith("-terms"):
+        precision += "-terms"
     plan = nat.Plan(list(instances), precision=precision)
     try:
         plan.execute()

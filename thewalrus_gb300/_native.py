@@ -18,8 +18,8 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 SOURCES = ["sieve.cu", "noalloc.cu", "kernels_c64.cu", "kernels_cdf.cu", "kernels_f64.cu", "kernels_fdf.cu",
            "kernels_cdd.cu", "kernels_fdd.cu", "kernels_mod0.cu", "kernels_mod1.cu", "kernels_mod2.cu",
            "kernels_mod3.cu", "kernels_mod4.cu"]
-DEPS = SOURCES + ["sieve_kernel.cuh", "arith.cuh", "host_common.h", "kernels.h", "kernels_unit.cuh",
-                  "state_glue.cuh"]
+DEPS = SOURCES + ["sieve_kernel.cuh", "tree_kernel.cuh", "tree_host.h", "arith.cuh", "host_common.h", "kernels.h",
+                  "kernels_unit.cuh", "state_glue.cuh"]
 NVCC_FLAGS = ["-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared"]
 
@@ -30,6 +30,9 @@ MOD_PRIMES = (2147483647, 2147483629, 2147483587, 2147483579, 2147483563)
 WG_KIND_PLAIN, WG_KIND_LOOP, WG_KIND_BATCH_EVEN, WG_KIND_BATCH_ODD = 0, 1, 3, 4
 PRECISIONS = {"fp64": WG_PREC_FP64, "df": WG_PREC_DF, "dd": WG_PREC_DD}
 PRECISIONS.update({"mod%d" % k: v for k, v in enumerate(WG_PREC_MOD)})
+# the same, evaluated term by term (WG_PREC_TERMS): the evaluation behind the term magnitudes
+WG_PREC_TERMS = 64
+PRECISIONS.update({k + "-terms": v | WG_PREC_TERMS for k, v in list(PRECISIONS.items())})
 
 _lock = threading.Lock()
 _lib = None

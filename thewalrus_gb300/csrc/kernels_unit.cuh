@@ -24,6 +24,32 @@ int WG_CAT(sieve_occupancy_, WG_UNIT_NAME)(int wpc, int smem) {
   return nb;
 }
 
+cudaError_t WG_CAT(tree_cta_launch_, WG_UNIT_NAME)(const TreeParams& p, int ctas, int smem, cudaStream_t st) {
+  auto k = tree_cta_kernel<WG_UNIT_SCALAR>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  k<<<ctas, TREE_THREADS, smem, st>>>(p);
+  return cudaGetLastError();
+}
+
+cudaError_t WG_CAT(tree_grid_launch_, WG_UNIT_NAME)(const TreeGrid& g, int blocks, int smem, cudaStream_t st) {
+  auto k = tree_grid_kernel<WG_UNIT_SCALAR>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
+  k<<<blocks, TREE_THREADS, smem, st>>>(g);
+  return cudaGetLastError();
+}
+
+int WG_CAT(tree_occupancy_, WG_UNIT_NAME)(int smem) {
+  int nb = 0;
+  auto k = tree_cta_kernel<WG_UNIT_SCALAR>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, TREE_THREADS, smem) != cudaSuccess) return 0;
+  return nb;
+}
+
 cudaError_t WG_CAT(sieve_tables_, WG_UNIT_NAME)(const double* binom, const double* inv) {
   cudaError_t e = cudaMemcpyToSymbol(c_binom, binom, sizeof(c_binom));
   if (e != cudaSuccess) return e;

@@ -5,8 +5,11 @@
 //     converted to the kernel's scalar type,
 //   * a chunk queue: every instance's term range split into chunks whose cost is balanced
 //     against the number of resident warps, largest instances first,
-//   * one persistent sieve launch per (scalar type, resident warps per SM) group, and one reduction
-//     launch that sums chunk partials in a fixed order (bitwise reproducible results).
+//   * the elimination tree of every instance that takes one (tree_kernel.cuh): small trees as one
+//     launch per scalar type over a task queue, large ones level by level,
+//   * for the others (term ranges, inclusion/exclusion, per-term precisions, matrices that are not
+//     symmetric) one persistent sieve launch per (scalar type, resident warps per SM) group,
+//   * one reduction launch that sums the partials in a fixed order (bitwise reproducible results).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -23,6 +26,7 @@
 #include "host_common.h"
 #include "sieve_kernel.cuh"
 #include "state_glue.cuh"
+#include "tree_host.h"
 
 namespace wg {
 
@@ -127,6 +131,12 @@ static int ensure_init(int device) {
 }
 
 
+// What the choice of evaluation looks at in a matrix: symmetric to rounding (and finite), real
+// entries of both signs, indices that fall into uncoupled blocks (zero entries between them).
+struct MatrixForm {
+  bool symmetric = false, signs = false, blocks = false;
+};
+
 struct Prepared {
   InstDev d;
   int stype;
@@ -137,6 +147,9 @@ struct Prepared {
   std::vector<unsigned char> ext;  // extended matrix in the kernel's scalar type (empty: formed on device)
   size_t ext_bytes = 0;
   long long t_lo = 0, t_hi = 0;  // sieve terms [t_lo, t_hi) of this instance
+  bool tree = false;             // evaluated as an elimination tree
+  TreeInst T;
+  std::vector<double> tscales;   // output scales of the tree's sum
 };
 
 struct Group {
@@ -145,6 +158,18 @@ struct Group {
   int wpc, ctas;
   int chunk_begin, chunk_count;
 };
+
+// trees launched as one task queue, and a tree launched level by level
+struct TreeGroup {
+  int stype, first, ninst, ntasks, ctas, smem, counter;
+  long long ws_stride, off_b, off_s;
+};
+struct TreeBig {
+  int stype, index, smem, part_base;  // index: in the plan's TreeInst array
+  TreeInst T;
+  TreeGridPlan g;
+};
+constexpr int kTreeLeafBlocks = 304;
 
 }  // namespace wg
 
@@ -178,6 +203,16 @@ struct wg_plan {
   cudaEvent_t fork = nullptr;
   int device = 0;  // the device the plan's memory and tables live on
   bool serial_groups = false;
+  std::vector<wg::TreeInst> trees;
+  std::vector<wg::TreeGroup> tree_groups;
+  std::vector<wg::TreeBig> tree_bigs;
+  wg::TreeInst* d_trees = nullptr;
+  unsigned char* d_ws = nullptr;
+  // a plan with trees answers the per-term queries (magnitudes, chunks, partials) by a plan over
+  // the same device matrices that evaluates term by term, made when first asked
+  std::vector<wg::Prepared> prep;
+  wg_plan_options opt{};
+  wg_plan* terms = nullptr;
 };
 
 struct wg_state {
@@ -186,6 +221,7 @@ struct wg_state {
   wg::c64* d_gamma = nullptr;
   std::vector<wg::c64> gamma;  // host copy: self-loop weights of unpaired modes
   double alpha = 1.0;          // double-float prescale (power of two, from ||B||_inf)
+  wg::MatrixForm form;         // of B, whose blocks and symmetry every request's matrix inherits
 };
 
 namespace wg {
@@ -245,7 +281,77 @@ static inline void get_val(const void* p, int dtype, size_t idx, double& re, dou
   else { re = d[idx]; im = 0.0; }
 }
 
+// Largest |A_ij - A_ji| against the largest |A_ij| for which a matrix counts as symmetric.  The tree
+// works on the mean of the two triangles; the sieve's value differs from the given matrix's only
+// in second order of the antisymmetric part (tr(N X (S X)^(j-1)) = 0 for antisymmetric N, symmetric
+// S and X), so differences of rounding size (a product U D U^T formed by BLAS) are far below the
+// term arithmetic's roundoff: (2^-48)^2 = 2^-96 in FP64 and double-float, (2^-52)^2 in double-double.
+static inline double tree_asymmetry(int precision) {
+  return prec_mod(precision) ? 0.0 : std::ldexp(1.0, precision == WG_PREC_DD ? -52 : -48);
+}
+
+static MatrixForm matrix_form(const void* A, int dtype, size_t n, double tol) {
+  MatrixForm f;
+  double big = 0, diff = 0, re, im, re2, im2;
+  bool pos = false, neg = false;
+  std::vector<int> comp(n);
+  for (size_t i = 0; i < n; ++i) comp[i] = (int)i;
+  auto root = [&](int x) {
+    while (comp[x] != x) x = comp[x] = comp[comp[x]];
+    return x;
+  };
+  for (size_t i = 0; i < n; ++i)
+    for (size_t j = 0; j <= i; ++j) {
+      get_val(A, dtype, i * n + j, re, im);
+      get_val(A, dtype, j * n + i, re2, im2);
+      if (!(std::isfinite(re) && std::isfinite(im) && std::isfinite(re2) && std::isfinite(im2))) return f;
+      big = std::max(big, std::max(std::fabs(re), std::fabs(im)));
+      diff = std::max(diff, std::max(std::fabs(re - re2), std::fabs(im - im2)));
+      if (i != j) {
+        pos = pos || re > 0;
+        neg = neg || re < 0;
+        if (re != 0 || im != 0) comp[root((int)i)] = root((int)j);
+      }
+    }
+  f.symmetric = diff <= tol * big;
+  f.signs = pos && neg;
+  for (size_t i = 1; i < n; ++i) f.blocks = f.blocks || root((int)i) != root(0);
+  return f;
+}
+
+// Whether an instance keeps the per-term evaluation although it has a tree: where the sum cancels
+// so far that per-term results in this precision are good to little more than 1e-9, the tree's
+// (closer to the exact value by 10 to 1000 times) would move them by more than that, and results
+// stay what they were.  Share of random inputs whose results differ by more than 1e-9 relative:
+//   FP64: real matrices of both signs 0 to 0.7 % for n <= 32, 1.7 % at 36, 9 % at 40, 17 % at 44 (all
+//   positive: none); complex ones none to n = 40 (largest 1.1e-10); loop hafnians 0.5 % (real,
+//   n = 21 to 33), none (complex); Gaussian states and generic matrices with multiple edges none of
+//   200 for K <= 14, 1 % at K = 18; uncoupled blocks (a state and its conjugate, whose pairing
+//   couples what the matrix does not) 0.6 % at K = 12, 8 to 23 % at 16, 70 % at 20;
+//   double-float (roundoff 2^5 larger): complex n = 34 none of 100 (largest 8.5e-10), n = 40 15 %;
+//   real of both signs none at n = 14, 3 % at 20, 18 % at 32.
+static bool keeps_terms(int stype, int kind, int K, const MatrixForm& f) {
+  const bool real = stype == ST_REAL64 || stype == ST_REALDF, loops = kind != KIND_PLAIN;
+  if (stype == ST_REAL64 || stype == ST_CPLX64)
+    return (f.blocks && K > 12) || (real && f.signs && K > (loops ? 18 : 17));
+  if (stype == ST_REALDF || stype == ST_CPLXDF)
+    return f.blocks || K > (real && !f.signs && !loops ? TREE_MAX_K : (loops ? 10 : (real ? 8 : 17)));
+  return false;  // residues are exact, double-double results agree to the last bits
+}
+
+// takes the tree when the instance has one; `ascale`: the input prescale's share of each output
+static void take_tree(Prepared& P, int precision, const std::vector<double>& ascale, const MatrixForm& f) {
+  P.tree = f.symmetric && tree_build(P.d, P.T) && !keeps_terms(P.stype, P.d.kind, P.T.K, f);
+  if (!P.tree) return;
+  P.T.comp_off = stype_dd(P.stype) ? P.d.nout : 0;
+  P.T.pstride = (stype_dd(P.stype) ? 2 : 1) * P.d.nout;
+  P.tscales.clear();
+  for (double a : ascale) P.tscales.push_back(pow2_scale(tree_scale_exp(P.T), precision) * a);
+}
+
 static int prepare(const wg_instance& in, int precision, Prepared& P) {
+  const bool terms_only = (precision & WG_PREC_TERMS) != 0;
+  precision &= ~WG_PREC_TERMS;
   memset(&P.d, 0, sizeof(P.d));
   InstDev& d = P.d;
   if (in.dtype != WG_FLOAT64 && in.dtype != WG_COMPLEX128) return fail(WG_EINVAL, "dtype must be WG_FLOAT64 or WG_COMPLEX128");
@@ -310,6 +416,7 @@ static int prepare(const wg_instance& in, int precision, Prepared& P) {
     if (rs > 0 && std::isfinite(rs)) alpha = std::exp2(-std::round(std::log2(rs)));
   }
   const double salpha = std::sqrt(alpha);
+  std::vector<double> ascale;
   int Nf = 0;
   if (kind == KIND_PLAIN || kind == KIND_LOOP) {
     d.N = (int)(2 * sumr);
@@ -317,14 +424,16 @@ static int prepare(const wg_instance& in, int precision, Prepared& P) {
     d.Nodd = 0;
     d.half_first = d.glynn;
     const int e = d.glynn ? d.N / 2 - 1 : 0;
-    P.scales.push_back(pow2_scale(e, precision) * std::pow(alpha, -0.5 * d.N));
+    ascale.push_back(std::pow(alpha, -0.5 * d.N));
+    P.scales.push_back(pow2_scale(e, precision) * ascale.back());
   } else if (kind == KIND_LOOP_ODD) {
     d.N = (int)(2 * sumr + 1);
     d.K = d.N / 2;
     d.Nodd = d.N;
     d.half_first = 0;
     const int e = d.glynn ? d.N / 2 : 0;
-    P.scales.push_back(pow2_scale(e, precision) * std::pow(alpha, -0.5 * d.N));
+    ascale.push_back(std::pow(alpha, -0.5 * d.N));
+    P.scales.push_back(pow2_scale(e, precision) * ascale.back());
     d.oddloop = {in.oddloop[0] * salpha, in.oddloop[1] * salpha};
   } else {
     const bool odd = kind == KIND_BATCH_ODD;
@@ -348,7 +457,8 @@ static int prepare(const wg_instance& in, int precision, Prepared& P) {
     }
     for (int o = 0; o < nout; ++o) {
       const int x = Nf + o;
-      P.scales.push_back(pow2_scale(d.glynn ? x / 2 : 0, precision) * std::pow(alpha, -0.5 * x));
+      ascale.push_back(std::pow(alpha, -0.5 * x));
+      P.scales.push_back(pow2_scale(d.glynn ? x / 2 : 0, precision) * ascale.back());
     }
   }
   d.nout = nout;
@@ -449,6 +559,8 @@ static int prepare(const wg_instance& in, int precision, Prepared& P) {
         put_scalar(at(n + 2, i), P.stype, re * alpha, im * alpha);
       }
   }
+  if (!terms_only && in.term_begin == 0 && in.term_end == 0)
+    take_tree(P, precision, ascale, matrix_form(in.A, in.dtype, (size_t)n, tree_asymmetry(precision)));
   return WG_OK;
 }
 
@@ -471,7 +583,7 @@ struct GatherSpec {
 };
 
 static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_options& opt, wg_plan* pl,
-                         GatherSpec* gs);
+                         GatherSpec* gs, unsigned char* ext_pool);
 
 // One block per instance: writes [[B[x][:,x], gamma[x]], [gamma[x]^T, 0], [B[o, x], 0], [0]]
 // (alpha / sqrt(alpha) prescaled) into the instance's pool slot in its scalar type.
@@ -505,6 +617,8 @@ static __global__ void gather_kernel(const GatherDev* __restrict__ gd, const int
 // without a host copy of the matrix).
 static int prepare_request(const wg_request& r, const wg_state& st, int precision, Prepared& P, GatherDev& g,
                            std::vector<int>& idx) {
+  const bool terms_only = (precision & WG_PREC_TERMS) != 0;
+  precision &= ~WG_PREC_TERMS;
   memset(&P.d, 0, sizeof(P.d));
   InstDev& d = P.d;
   if (r.E < 1 || r.E > MAX_EDGES || !r.x || !r.edge_reps) return fail(WG_EINVAL, "request needs 1..32 edges");
@@ -536,7 +650,8 @@ static int prepare_request(const wg_request& r, const wg_state& st, int precisio
   d.half_first = odd ? 0 : 1;
   if (odd) d.oddloop = {st.gamma[r.oddmode].re * salpha, st.gamma[r.oddmode].im * salpha};
   const int e = odd ? d.N / 2 : d.N / 2 - 1;
-  P.scales.assign(1, std::ldexp(1.0, -e) * std::pow(alpha, -0.5 * d.N));
+  const double ascale = std::pow(alpha, -0.5 * d.N);
+  P.scales.assign(1, std::ldexp(1.0, -e) * ascale);
   for (int i = 0; i < r.E; ++i) {
     const int R = (i == 0 && d.half_first) ? (int)(r.edge_reps[0] + 2) / 2 : (int)r.edge_reps[i] + 1;
     d.radix[i] = R;
@@ -572,23 +687,145 @@ static int prepare_request(const wg_request& r, const wg_state& st, int precisio
   g.alpha = alpha;
   g.salpha = salpha;
   for (int i = 0; i < 2 * r.E; ++i) idx.push_back(r.x[i]);
+  if (!terms_only) take_tree(P, precision, {ascale}, st.form);
   return WG_OK;
+}
+
+static bool known_precision(int precision) {
+  const int p = precision & ~WG_PREC_TERMS;
+  return p == WG_PREC_FP64 || p == WG_PREC_DF || p == WG_PREC_DD || prec_mod(p);
 }
 
 static int build_plan(const wg_instance* v, int count, int precision, const wg_plan_options& opt, wg_plan* pl) {
   if (count < 0 || (count > 0 && !v)) return fail(WG_EINVAL, "bad instance list");
-  if (precision != WG_PREC_FP64 && precision != WG_PREC_DF && precision != WG_PREC_DD && !prec_mod(precision))
+  if (!known_precision(precision))
     return fail(WG_EINVAL, "unknown precision %d", precision);
   std::vector<Prepared> P(count);
   for (int i = 0; i < count; ++i) {
     int rc = prepare(v[i], precision, P[i]);
     if (rc) return fail(rc, "instance %d: %s", i, g_err.c_str());
   }
-  return finalize_plan(P, precision, opt, pl, nullptr);
+  return finalize_plan(P, precision, opt, pl, nullptr, nullptr);
 }
 
+// Per scalar type: SM clocks per multiply-add of a tree (measured at the grid kernel's rate)
+static double tree_mac_clocks(int stype) {
+  switch (stype) {
+    case ST_REAL64: return 0.5;
+    case ST_CPLX64: return 2.0;
+    case ST_REALDF: return 0.2;
+    case ST_CPLXDF: return 0.6;
+    case ST_REALDD: return 9.0;
+    case ST_CPLXDD: return 35.0;
+    default: return 0.15;
+  }
+}
+
+// Cuts the tree members of a plan into task-queue launches (one per scalar type) and level-launched
+// trees, and lays out their partial slots (from `nparts` on).  Returns the workspace bytes.
+// A tree goes level by level when that is estimated faster: the queue recomputes every task's
+// path, the levels cost a launch each (~4 us, 8000 clocks).
+static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) {
+  constexpr long long kMaxCtaBytes = 256 << 10;
+  constexpr double kGridBudget = 48e6, kLaunchClocks = 8000.0, kStepClocks = 2500.0;
+  const int count = (int)P.size();
+  std::vector<TreeSizes> z(count);
+  double total = 0;
+  for (int i = 0; i < count; ++i)
+    if (P[i].tree) {
+      tree_sizes(P[i].T, z[i]);
+      total += z[i].total * tree_mac_clocks(P[i].stype);
+    }
+  long long ws = 0;
+  std::vector<int> queued;
+  std::vector<double> task_cost(count, 0.0);
+  for (int i = 0; i < count; ++i) {
+    if (!P[i].tree) continue;
+    TreeInst& T = P[i].T;
+    const int sb = (int)stype_bytes(P[i].stype);
+    const double clk = tree_mac_clocks(P[i].stype);
+    int q = 0;
+    const double cta = tree_split(T, z[i], g_num_sms, std::max(z[i].total * clk / total, 0.05), kMaxCtaBytes / sb, q);
+    TreeGridPlan g;
+    tree_grid_plan(T, sb, kGridBudget, g);
+    const double t_cta = cta * clk + T.steps * kStepClocks;
+    const double t_grid = z[i].total * clk / g_num_sms + (double)g.launches * kLaunchClocks;
+    if (cta >= 0 && t_cta <= t_grid) {
+      T.q = q;
+      T.tasks = 1;
+      for (int s = 0; s < q; ++s) T.tasks *= T.radix[s];
+      task_cost[i] = z[i].total * clk / T.tasks;
+      queued.push_back(i);
+    } else {
+      TreeBig b;
+      b.stype = P[i].stype;
+      b.index = i;
+      b.g = g;
+      b.smem = tree_smem(T, sb);
+      b.part_base = nparts;
+      pl->tree_bigs.push_back(b);
+      P[i].d.part_base = T.part_base = nparts;
+      P[i].d.nchunks = (int)g.leaves * kTreeLeafBlocks;
+      nparts += P[i].d.nchunks * T.pstride;
+      ws = std::max(ws, g.bytes);
+    }
+  }
+  // the queues: costly tasks first
+  std::stable_sort(queued.begin(), queued.end(), [&](int a, int b) {
+    return P[a].stype != P[b].stype ? P[a].stype < P[b].stype : task_cost[a] > task_cost[b];
+  });
+  for (size_t k = 0; k < queued.size();) {
+    TreeGroup G;
+    memset(&G, 0, sizeof(G));
+    G.stype = P[queued[k]].stype;
+    G.first = (int)pl->trees.size();
+    const int sb = (int)stype_bytes(G.stype);
+    long long el[3] = {1, 1, 1};
+    for (; k < queued.size() && P[queued[k]].stype == G.stype; ++k) {
+      Prepared& p = P[queued[k]];
+      TreeInst& T = p.T;
+      T.task_base = G.ntasks;
+      G.ntasks += T.tasks;
+      ++G.ninst;
+      p.d.part_base = T.part_base = nparts;
+      p.d.nchunks = T.tasks;
+      nparts += T.tasks * T.pstride;
+      long long e[3];
+      tree_cta_elems(T, T.q, e);
+      for (int x = 0; x < 3; ++x) el[x] = std::max(el[x], e[x]);
+      G.smem = std::max(G.smem, tree_smem(T, sb));
+      T.a_off = p.d.a_off;
+      pl->trees.push_back(T);
+    }
+    auto al = [](long long x) { return (x + 255) & ~255ll; };
+    G.off_b = al(el[0] * sb);
+    G.off_s = G.off_b + al(el[1] * sb);
+    G.ws_stride = G.off_s + al(el[2] * sb);
+    const int occ = std::max(1, tree_occupancy(G.stype, G.smem));
+    G.ctas = std::min(G.ntasks, g_num_sms * occ);
+    ws = std::max(ws, G.ws_stride * G.ctas);
+    pl->tree_groups.push_back(G);
+  }
+  for (TreeBig& b : pl->tree_bigs) {
+    const int i = b.index;
+    b.T = P[i].T;
+    b.T.a_off = P[i].d.a_off;
+    b.index = (int)pl->trees.size();
+    pl->trees.push_back(b.T);
+  }
+  for (int i = 0; i < count; ++i)
+    if (P[i].tree) {
+      P[i].d.pstride = P[i].T.pstride;
+      P[i].d.comp_off = P[i].T.comp_off;
+      P[i].d.mag_off = 0;
+    }
+  return ws;
+}
+
+// ext_pool: the instances' matrices are on the device already, at their a_off
 static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_options& opt, wg_plan* pl,
-                         GatherSpec* gs) {
+                         GatherSpec* gs, unsigned char* ext_pool) {
+  precision &= ~WG_PREC_TERMS;
   const int count = (int)P.size();
   const double chunk_scale = opt.chunk_scale > 0 ? opt.chunk_scale : 1.0;
   const int wpc_cap = opt.max_warps_per_cta > 0 ? std::min(opt.max_warps_per_cta, 8) : kDefaultWarpsPerCta;
@@ -603,7 +840,8 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
     P[i].d.out_base = out;
     P[i].d.scale_base = (int)scales.size();
     out += P[i].d.nout;
-    scales.insert(scales.end(), P[i].scales.begin(), P[i].scales.end());
+    const std::vector<double>& sc = P[i].tree ? P[i].tscales : P[i].scales;
+    scales.insert(scales.end(), sc.begin(), sc.end());
   }
   pl->total_out = out;
   // launch shape per (scalar class, per-warp workspace), see best_shape
@@ -619,8 +857,9 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   // group per scalar type
   struct GKey { int st, res; };
   std::vector<GKey> keys;
-  std::vector<int> gid(count);
+  std::vector<int> gid(count, -1);
   for (int i = 0; i < count; ++i) {
+    if (P[i].tree) continue;
     if (!tile_rows_ok(P[i].stype, P[i].rows_max)) return fail(WG_EINVAL, "instance %d: term matrix too large", i);
     int res = 0;
     if (!opt.merge_classes) {
@@ -638,13 +877,14 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   }
   // pool
   size_t pool_bytes = 0;
-  for (int i = 0; i < count; ++i) {
+  for (int i = 0; i < count && !ext_pool; ++i) {
     P[i].d.a_off = (long long)pool_bytes;
     pool_bytes += (P[i].ext_bytes + 255) & ~(size_t)255;
   }
   if (gs)
     for (int i = 0; i < count; ++i) gs->desc[i].a_off = P[i].d.a_off;
   int nparts = 0;
+  const long long ws_bytes = plan_trees(P, pl, nparts);
   for (size_t g = 0; g < keys.size(); ++g) {
     Group G;
     G.stype = keys[g].st;
@@ -730,12 +970,16 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   const size_t b_scales = al(sizeof(double) * std::max<size_t>(scales.size(), 1));
   const size_t b_out = al(sizeof(double2) * std::max(out, 1));
   const size_t b_mag = al(sizeof(double) * std::max(out, 1));
-  const size_t b_cnt = al(sizeof(unsigned int) * std::max<size_t>(pl->groups.size(), 1));
+  const size_t ncnt = pl->groups.size() + pl->tree_groups.size();
+  for (size_t g = 0; g < pl->tree_groups.size(); ++g) pl->tree_groups[g].counter = (int)(pl->groups.size() + g);
+  const size_t b_cnt = al(sizeof(unsigned int) * std::max<size_t>(ncnt, 1));
+  const size_t b_tree = al(sizeof(TreeInst) * std::max<size_t>(pl->trees.size(), 1));
+  const size_t b_ws = al((size_t)ws_bytes);
   const size_t b_err = al(sizeof(int));
   const size_t b_gdesc = gs ? al(sizeof(GatherDev) * std::max<size_t>(gs->desc.size(), 1)) : 0;
   const size_t b_gidx = gs ? al(sizeof(int) * std::max<size_t>(gs->idx.size(), 1)) : 0;
-  const size_t total =
-      b_inst + b_chunks + b_pool + b_parts + b_scales + b_out + b_mag + b_cnt + b_err + b_gdesc + b_gidx;
+  const size_t total = b_inst + b_chunks + b_tree + b_scales + b_pool + b_parts + b_out + b_mag + b_cnt + b_err +
+                       b_gdesc + b_gidx + b_ws;
   cudaStream_t cs = (cudaStream_t)opt.stream;
   pl->alloc_stream = cs;
   pl->async_alloc = cs != nullptr;
@@ -748,45 +992,44 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   unsigned char* base = (unsigned char*)pl->dmem;
   pl->d_inst = (InstDev*)base; base += b_inst;
   pl->d_chunks = (ChunkDev*)base; base += b_chunks;
-  pl->d_pool = base; base += b_pool;
-  pl->d_partials = (double2*)base; base += b_parts;
+  pl->d_trees = (TreeInst*)base; base += b_tree;
   pl->d_scales = (double*)base; base += b_scales;
+  pl->d_pool = ext_pool ? ext_pool : base; base += b_pool;
+  pl->d_partials = (double2*)base; base += b_parts;
   pl->d_out = (double2*)base; base += b_out;
   pl->d_mag = (double*)base; base += b_mag;
   pl->d_counters = (unsigned int*)base; base += b_cnt;
   pl->d_err = (int*)base; base += b_err;
+  GatherDev* d_desc = (GatherDev*)base; base += b_gdesc;
+  int* d_idx = (int*)base; base += b_gidx;
+  pl->d_ws = base;
   pl->device_bytes = (long long)total;
   // staging: one host buffer with the same layout for the upload
-  std::vector<unsigned char> host(b_inst + b_chunks + b_pool + b_parts + b_scales, 0);
+  const size_t o_tree = b_inst + b_chunks, o_scales = o_tree + b_tree, o_pool = o_scales + b_scales;
+  std::vector<unsigned char> host(o_pool + (gs || ext_pool ? 0 : b_pool), 0);
   memcpy(host.data(), pl->inst.data(), sizeof(InstDev) * count);
   if (!pl->chunks.empty()) memcpy(host.data() + b_inst, pl->chunks.data(), sizeof(ChunkDev) * pl->chunks.size());
+  if (!pl->trees.empty()) memcpy(host.data() + o_tree, pl->trees.data(), sizeof(TreeInst) * pl->trees.size());
+  if (!scales.empty()) memcpy(host.data() + o_scales, scales.data(), sizeof(double) * scales.size());
   for (int i = 0; i < count; ++i)
-    if (!P[i].ext.empty()) memcpy(host.data() + b_inst + b_chunks + P[i].d.a_off, P[i].ext.data(), P[i].ext.size());
-  if (!scales.empty()) memcpy(host.data() + b_inst + b_chunks + b_pool + b_parts, scales.data(), sizeof(double) * scales.size());
+    if (!P[i].ext.empty() && !ext_pool) memcpy(host.data() + o_pool + P[i].d.a_off, P[i].ext.data(), P[i].ext.size());
   // uploads: stream-ordered on the creation stream when one is given (pageable sources are
   // staged before cudaMemcpyAsync returns), else synchronous
   auto up = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
     return cs ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, cs)
               : cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
   };
+  CK(up(pl->dmem, host.data(), host.size()));
+  pl->h2d_bytes = (long long)host.size();
   if (gs) {
-    // pools are formed on the device: only descriptors, chunks, scales and indices travel
-    CK(up(pl->dmem, host.data(), b_inst + b_chunks));
-    CK(up((unsigned char*)pl->dmem + b_inst + b_chunks + b_pool + b_parts,
-          host.data() + b_inst + b_chunks + b_pool + b_parts, b_scales));
-    GatherDev* d_desc = (GatherDev*)((unsigned char*)pl->d_err + b_err);
-    int* d_idx = (int*)((unsigned char*)d_desc + b_gdesc);
+    // pools are formed on the device: descriptors, chunks, scales and indices travel
     CK(up(d_desc, gs->desc.data(), sizeof(GatherDev) * gs->desc.size()));
     if (!gs->idx.empty()) CK(up(d_idx, gs->idx.data(), sizeof(int) * gs->idx.size()));
     if (count > 0) {
       gather_kernel<<<count, 256, 0, cs>>>(d_desc, d_idx, gs->B, gs->gamma, gs->M, pl->d_pool);
       CK(cudaGetLastError());
     }
-    pl->h2d_bytes = (long long)(b_inst + b_chunks + b_scales + sizeof(GatherDev) * gs->desc.size() +
-                                sizeof(int) * gs->idx.size());
-  } else {
-    CK(up(pl->dmem, host.data(), host.size()));
-    pl->h2d_bytes = (long long)host.size();
+    pl->h2d_bytes += (long long)(sizeof(GatherDev) * gs->desc.size() + sizeof(int) * gs->idx.size());
   }
   if (cs) {
     CK(cudaMemsetAsync(pl->d_counters, 0, b_cnt + b_err, cs));
@@ -794,10 +1037,100 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
     CK(cudaMemset(pl->d_counters, 0, b_cnt + b_err));
     CK(cudaStreamSynchronize(0));
   }
+  if (!pl->trees.empty()) {  // what a per-term plan of the same instances needs (terms_plan)
+    pl->prep = std::move(P);
+    for (Prepared& p : pl->prep) std::vector<unsigned char>().swap(p.ext);
+    pl->opt = opt;
+  }
+  return WG_OK;
+}
+
+// The per-term plan of a plan with trees, made on first use over the same device matrices: its
+// magnitudes, chunks and partials are those of the sieve's terms.
+static void destroy_plan(wg_plan* pl);
+static int terms_plan(wg_plan* pl, wg_plan** out) {
+  *out = pl;
+  if (pl->prep.empty()) return WG_OK;
+  if (!pl->terms) {
+    int rc = ensure_init(pl->device);
+    if (rc) return rc;
+    std::vector<Prepared> P = pl->prep;
+    for (Prepared& p : P) p.tree = false;
+    wg_plan* t = new wg_plan();
+    rc = finalize_plan(P, pl->precision, pl->opt, t, nullptr, pl->d_pool);
+    if (rc) { destroy_plan(t); return rc; }
+    pl->terms = t;
+  }
+  *out = pl->terms;
+  return WG_OK;
+}
+
+static int launch_trees(wg_plan* pl, cudaStream_t st) {
+  TreeParams p;
+  memset(&p, 0, sizeof(p));
+  p.pool = pl->d_pool;
+  p.partials = pl->d_partials;
+  p.ws = pl->d_ws;
+  for (const TreeGroup& G : pl->tree_groups) {
+    p.inst = pl->d_trees + G.first;
+    p.ninst = G.ninst;
+    p.ntasks = G.ntasks;
+    p.ws_stride = G.ws_stride;
+    p.off_b = G.off_b;
+    p.off_s = G.off_s;
+    p.counter = pl->d_counters + G.counter;
+    const cudaError_t e = tree_cta_launch(G.stype, p, G.ctas, G.smem, st);
+    if (e != cudaSuccess) return fail(WG_ECUDA, "tree launch: %s", cudaGetErrorString(e));
+  }
+  p.inst = pl->d_trees;
+  for (const TreeBig& b : pl->tree_bigs) {
+    const TreeInst& T = b.T;
+    long long part = b.part_base;
+    cudaError_t err = cudaSuccess;
+    auto launch = [&](int phase, int q, int p0, int np, int ps, int d0, int nd) {
+      if (err != cudaSuccess) return;
+      TreeGrid G;
+      G.P = p;
+      G.inst = b.index;
+      G.phase = phase;
+      G.q = q;
+      G.np = np;
+      G.p0 = p0;
+      G.pstride = ps;
+      G.d0 = d0;
+      G.nd = nd;
+      G.part = part;
+      G.par = pl->d_ws + b.g.off[q];
+      G.chi = phase == TP_ROOT ? G.par : (q < T.steps ? pl->d_ws + b.g.off[q + 1] : nullptr);
+      G.scr = pl->d_ws + b.g.scr_off;
+      const bool dd2 = b.stype == ST_CPLXDD;
+      const int TL = dd2 ? 2 : 4;
+      const long long Lp = T.deg[q] + 1, W1 = tree_width(T.X, T.E, q + 1), tp = (Lp + TL - 1) / TL;
+      const long long Lc = q < T.steps ? T.deg[q + 1] + 1 : Lp, tc = (Lc + TL - 1) / TL;
+      long long items = 1;  // threads of work
+      switch (phase) {
+        case TP_ROOT: items = tree_entries(tree_width(T.X, T.E, 0), T.diag); break;
+        case TP_M: items = tp * np; break;
+        case TP_UNIT: items = tp * tree_entries((int)W1, T.diag) * np; break;
+        case TP_PREP: case TP_GLOOP: items = 32ll * np * nd; break;
+        case TP_Y: items = tc * 2 * W1 * np * nd; break;
+        case TP_MULTI: items = tc * (tree_entries((int)W1, T.diag) - 1) * np * nd; break;
+        default: items = (long long)kTreeLeafBlocks * TREE_THREADS;
+      }
+      const int blocks = (int)std::max(1ll, (items + TREE_THREADS - 1) / TREE_THREADS);
+      err = tree_grid_launch(b.stype, G, blocks, phase == TP_LEAF ? b.smem : 0, st);
+      if (phase == TP_LEAF) part += (long long)kTreeLeafBlocks * T.pstride;
+    };
+    launch(TP_ROOT, 0, 0, 1, 1, 0, 1);
+    tree_walk(T, b.g, 0, 1, launch);
+    if (err != cudaSuccess) return fail(WG_ECUDA, "tree level launch: %s", cudaGetErrorString(err));
+  }
   return WG_OK;
 }
 
 static int launch_plan(wg_plan* pl, cudaStream_t st) {
+  const int trc = launch_trees(pl, st);
+  if (trc) return trc;
   const size_t ng = pl->groups.size();
   const bool side = ng > 1 && !pl->serial_groups;
   if (side) {
@@ -845,7 +1178,8 @@ static int launch_plan(wg_plan* pl, cudaStream_t st) {
     const int blocks = (pl->total_out * 32 + threads - 1) / threads;  // one warp per output
     const unsigned int modp = prec_mod(pl->precision) ? MOD_PRIMES[pl->precision - WG_PREC_MOD0] : 0u;
     reduce_kernel<<<std::max(blocks, 1), threads, 0, st>>>(pl->d_inst, ninst, pl->d_partials, pl->d_scales, pl->d_out,
-                                                           pl->d_counters, (int)pl->groups.size(), pl->total_out, modp,
+                                                           pl->d_counters, (int)(pl->groups.size() + pl->tree_groups.size()), pl->total_out,
+                                                           modp,
                                                            pl->d_mag);
     CK(cudaGetLastError());
   }
@@ -881,6 +1215,7 @@ static int execute_plan(wg_plan* pl, cudaStream_t st) {
 
 static void destroy_plan(wg_plan* pl) {
   if (!pl) return;
+  destroy_plan(pl->terms);
   if (pl->graph_exec) cudaGraphExecDestroy(pl->graph_exec);
   for (cudaStream_t s2 : pl->side) cudaStreamDestroy(s2);
   for (cudaEvent_t e2 : pl->side_done) cudaEventDestroy(e2);
@@ -1001,8 +1336,15 @@ int wg_plan_read(wg_plan* plan, double* out, void* stream) {
 int wg_plan_read_magnitudes(wg_plan* plan, double* out, void* stream) {
   if (!plan || (!out && plan->total_out > 0)) return fail(WG_EINVAL, "NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
+  wg_plan* terms = nullptr;
+  const int rc = terms_plan(plan, &terms);
+  if (rc) return rc;
+  if (terms != plan) {
+    const int rc2 = launch_plan(terms, st);
+    if (rc2) return rc2;
+  }
   if (plan->total_out > 0)
-    CK(cudaMemcpyAsync(out, plan->d_mag, sizeof(double) * plan->total_out, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(out, terms->d_mag, sizeof(double) * plan->total_out, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   return WG_OK;
 }
@@ -1010,27 +1352,41 @@ int wg_plan_read_magnitudes(wg_plan* plan, double* out, void* stream) {
 int wg_plan_outputs(const wg_plan* plan) { return plan ? plan->total_out : fail(WG_EINVAL, "plan is NULL"); }
 
 int wg_plan_kernel_launches(const wg_plan* plan) {
-  return plan ? (int)plan->groups.size() + (plan->inst.empty() ? 0 : 1) : fail(WG_EINVAL, "plan is NULL");
+  if (!plan) return fail(WG_EINVAL, "plan is NULL");
+  long long n = (long long)plan->groups.size() + (long long)plan->tree_groups.size() + (plan->inst.empty() ? 0 : 1);
+  for (const TreeBig& b : plan->tree_bigs) n += b.g.launches;
+  return (int)n;
 }
 
 int wg_plan_partials(wg_plan* plan, double* out, int capacity, void* stream) {
   if (!plan) return fail(WG_EINVAL, "plan is NULL");
-  if (!out || capacity < plan->nparts) return plan->nparts;
+  wg_plan* terms = nullptr;
+  const int rc = terms_plan(plan, &terms);
+  if (rc) return rc;
+  if (!out || capacity < terms->nparts) return terms->nparts;
   cudaStream_t st = (cudaStream_t)stream;
-  if (plan->nparts > 0)
-    CK(cudaMemcpyAsync(out, plan->d_partials, sizeof(double2) * plan->nparts, cudaMemcpyDeviceToHost, st));
+  if (terms != plan) {
+    const int rc2 = launch_plan(terms, st);
+    if (rc2) return rc2;
+  }
+  if (terms->nparts > 0)
+    CK(cudaMemcpyAsync(out, terms->d_partials, sizeof(double2) * terms->nparts, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  return plan->nparts;
+  return terms->nparts;
 }
 
 int wg_plan_chunk(const wg_plan* plan, int chunk, int* inst, int* part, long long* t0, long long* t1) {
-  if (!plan || chunk < 0 || chunk >= (int)plan->chunks.size()) return fail(WG_EINVAL, "bad chunk index");
-  const ChunkDev& c = plan->chunks[chunk];
+  if (!plan) return fail(WG_EINVAL, "bad chunk index");
+  wg_plan* terms = nullptr;
+  const int rc = terms_plan(const_cast<wg_plan*>(plan), &terms);
+  if (rc) return rc;
+  if (chunk < 0 || chunk >= (int)terms->chunks.size()) return fail(WG_EINVAL, "bad chunk index");
+  const ChunkDev& c = terms->chunks[chunk];
   if (inst) *inst = c.inst;
   if (part) *part = c.part;
   if (t0) *t0 = c.t0;
   if (t1) *t1 = c.t1;
-  return (int)plan->chunks.size();
+  return (int)terms->chunks.size();
 }
 
 int wg_state_create(const double* B, const double* gamma, int M, wg_state** state) {
@@ -1058,6 +1414,7 @@ int wg_state_create(const double* B, const double* gamma, int M, wg_state** stat
   }
   CK(cudaMemcpy(st->d_B, B, sizeof(c64) * (size_t)M * M, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(st->d_gamma, gamma, sizeof(c64) * M, cudaMemcpyHostToDevice));
+  st->form = matrix_form(B, WG_COMPLEX128, (size_t)M, tree_asymmetry(WG_PREC_FP64));
   *state = st;
   return WG_OK;
 }
@@ -1110,6 +1467,12 @@ int wg_state_create_from_cov(const double* cov, const double* mu, int M, double 
   if (B_out && cudaMemcpy(B_out, st->d_B, sizeof(c64) * (size_t)M * M, cudaMemcpyDeviceToHost) != cudaSuccess)
     return abandon(WG_ECUDA, "state readback failed");
   if (gamma_out) memcpy(gamma_out, st->gamma.data(), sizeof(c64) * M);
+  {
+    std::vector<c64> B((size_t)M * M);
+    if (cudaMemcpy(B.data(), st->d_B, sizeof(c64) * B.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
+      return abandon(WG_ECUDA, "state readback failed");
+    st->form = matrix_form(B.data(), WG_COMPLEX128, (size_t)M, tree_asymmetry(WG_PREC_FP64));
+  }
   release();
   const double rs = out[3];
   if (rs > 0 && std::isfinite(rs)) st->alpha = std::exp2(-std::round(std::log2(rs)));
@@ -1133,7 +1496,8 @@ int wg_plan_create_requests(const wg_state* state, const wg_request* req, int co
                             const wg_plan_options* options, wg_plan** plan) {
   if (!plan || !state || count < 0 || (count > 0 && !req)) return fail(WG_EINVAL, "bad request list");
   *plan = nullptr;
-  if (precision != WG_PREC_FP64 && precision != WG_PREC_DF) return fail(WG_EINVAL, "unknown precision %d", precision);
+  if ((precision & ~WG_PREC_TERMS) != WG_PREC_FP64 && (precision & ~WG_PREC_TERMS) != WG_PREC_DF)
+    return fail(WG_EINVAL, "unknown precision %d", precision);
   int rc = ensure_init(-1);
   if (rc) return rc;
   wg_plan_options opt;
@@ -1151,7 +1515,7 @@ int wg_plan_create_requests(const wg_state* state, const wg_request* req, int co
     if (rc) return fail(rc, "request %d: %s", i, g_err.c_str());
   }
   wg_plan* pl = new wg_plan();
-  rc = finalize_plan(P, precision, opt, pl, &gs);
+  rc = finalize_plan(P, precision, opt, pl, &gs, nullptr);
   if (rc) { destroy_plan(pl); return rc; }
   *plan = pl;
   return WG_OK;
