@@ -1,8 +1,8 @@
 """The elimination tree (tree_kernel.cuh, tree_host.h) against the oracle, on the CPU: the node
-functions compiled for the host over a scalar type whose loads and stores are checked against their
-buffers, walked as the CTA kernel walks a task and as the level launches walk blocks of nodes, over
-the forms an instance can take (simple and multiple edges, self-paired modes, loop weights, an
-unpaired vertex, batches; one photon pair up to more pairs than a block holds)."""
+functions compiled for the host over a scalar type whose loads and stores are checked against the
+levels they belong to, run through the program a launch follows, over the forms an instance can
+take (simple and multiple edges, self-paired modes, loop weights, an unpaired vertex, batches; one
+photon pair up to more nodes than a block holds) and several instances in one program."""
 import os
 import shutil
 import subprocess
@@ -30,32 +30,35 @@ def exe(tmp_path_factory):
     return path
 
 
-def evaluate(exe, inst, budget, split):
-    s, n = inst.struct, inst.struct.n
-    words = [s.kind, n, s.E, s.batch_max, s.cutoff, s.has_odd, budget, split] + list(inst.reps)
+def evaluate(exe, insts, budget, chip):
+    words = [len(insts), budget, 4, chip]
 
     def put(x, count):
         x = np.zeros(count) if x is None else np.asarray(x).reshape(-1)
         for z in x.astype(complex):
             words.extend([repr(float(z.real)), repr(float(z.imag))])
 
-    put(inst.A, n * n)
-    put(inst.D, n)
-    put(inst.oddV, n)
-    words.extend([repr(s.oddloop[0]), repr(s.oddloop[1])])
+    for inst in insts:
+        s, n = inst.struct, inst.struct.n
+        words += [s.kind, n, s.E, s.batch_max, s.cutoff, s.has_odd] + list(inst.reps)
+        put(inst.A, n * n)
+        put(inst.D, n)
+        put(inst.oddV, n)
+        words.extend([repr(s.oddloop[0]), repr(s.oddloop[1])])
     run = subprocess.run([exe], input=" ".join(str(w) for w in words).encode(), stdout=subprocess.PIPE,
                          stderr=subprocess.STDOUT, timeout=120)
     assert run.returncode == 0, run.stdout.decode()
     v = np.array([[float(x) for x in line.split()] for line in run.stdout.decode().split("\n") if line])
-    return v[:, 0] + 1j * v[:, 1], v[:, 2] + 1j * v[:, 3]
+    return v[:, 0] + 1j * v[:, 1]
 
 
 def check(exe, inst, want):
-    # the sums of these small instances cancel by less than 1e3, so 1e-11 leaves a factor of 100
+    # the sums of these small instances cancel by less than 1e3, so 1e-11 leaves a factor of 100.
+    # Whole levels; blocks of nodes; one coefficient a thread everywhere and tiles everywhere
     want = np.atleast_1d(np.asarray(want, dtype=complex))
-    for budget, split in ((1e9, 0), (3e4, 2), (2e3, 40)):
-        for got in evaluate(exe, inst, budget, split):
-            assert np.max(np.abs(got - want)) <= 1e-11 * np.max(np.abs(want)), (budget, split, got, want)
+    for budget, chip in ((1e9, 77824), (3e4, 64), (2e3, 32)):
+        got = evaluate(exe, [inst], budget, chip)
+        assert np.max(np.abs(got - want)) <= 1e-11 * np.max(np.abs(want)), (budget, chip, got, want)
 
 
 @pytest.mark.parametrize("n", [2, 4, 6, 8, 10, 14, 18])
@@ -94,3 +97,15 @@ def test_batches(exe, fixed, cutoff):
     want = [complex(oracle.hafnian_repeated(A, list(fixed) + [k], mu=D, loop=True)) if sum(fixed) + k else 1.0
             for k in range(cutoff + 1)]
     check(exe, tw.prepare_loop_hafnian_batch(A, D, list(fixed), cutoff), want)
+
+
+def test_several_instances(exe):
+    A, B = wl.complex_symmetric(9, seed=1), wl.complex_symmetric(12, seed=2)
+    D = A[0] * 0.5
+    insts = [tw.prepare_hafnian(B), tw.prepare_loop_hafnian(A, D, [1] * 9),
+             tw.prepare_loop_hafnian_batch(A, D, [1, 0, 2, 1, 0, 1, 0, 0], 5),
+             tw.prepare_loop_hafnian(A, D, [3, 1, 1, 2, 0, 1, 0, 1, 1]), tw.prepare_hafnian(B[:6, :6])]
+    for budget, chip in ((1e9, 77824), (4e3, 64)):
+        got = evaluate(exe, insts, budget, chip)
+        want = np.concatenate([evaluate(exe, [i], 1e9, 77824) for i in insts])
+        assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))

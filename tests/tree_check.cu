@@ -1,11 +1,12 @@
 // Host check of the elimination tree (tree_kernel.cuh, tree_host.h): the node functions compiled
-// for the host over a scalar type whose loads and stores are checked against their buffers, walked
-// both ways the kernels are launched (a CTA's path and subtree for every task, and level by level in
-// blocks), for one instance read from standard input.  Built and run by tests/test_tree_host.py;
-// prints each output twice, or names the first access out of range.
+// for the host over a scalar type whose loads and stores are checked against the levels they belong
+// to, run through the program that a launch of the kernel follows, for instances read from standard
+// input.  Built and run by tests/test_tree_host.py; prints the outputs, or names the first access
+// out of range.
 //
-// Input: kind n E batch_max cutoff has_odd K-budget-bytes task-split; edge_reps; A (n x n, re im);
-// D (n); oddV (n); oddloop.  kind as in walrus_gb300.h (0 plain, 1 loop, 3 / 4 batch even / odd).
+// Input: instances level-budget-bytes tile chip-threads; per instance kind n E batch_max cutoff
+// has_odd; edge_reps; A (n x n, re im); D (n); oddV (n); oddloop.  kind as in walrus_gb300.h (0 plain,
+// 1 loop, 3 / 4 batch even / odd).
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -82,121 +83,114 @@ __host__ __device__ __forceinline__ void tst<hc>(hc* p, hc v) {
 }
 }  // namespace wg
 
-struct Buf {
-  std::vector<hc> v;
-  explicit Buf(size_t n) : v(n, hc{NAN, NAN}) { g_bufs[v.data()] = n; }
-  ~Buf() { g_bufs.erase(v.data()); }
-  hc* p() { return v.data(); }
-};
-
 static double rd() {
   double x;
   if (std::scanf("%lf", &x) != 1) std::exit(2);
   return x;
 }
 
-static void leaf(const TreeInst& T, hc* par, long long ps, int np, hc* m, std::vector<hc>& out) {
-  Buf sm(5 * (T.deg[T.steps] + 1) + 32);
-  const hc s = tree_leaf<hc>(T, par, ps, np, m, sm.p(), 0, 0, 1);
-  if (T.pB < 0) out[0] = Ar<hc>::add(out[0], s);
-  else
-    for (int k = 0; k < T.nout; ++k) out[k] = Ar<hc>::add(out[k], sm.p()[5 * (T.deg[T.steps] + 1) + k]);
+template <int TL>
+static void phase(const TreeInst& T, const TreeSeg& G, const unsigned char* pool, const hc* par, hc* chi, hc* scr,
+                  hc* sm, int smn, int tid, int nthr, hc* out) {
+  hc* y = G.q < T.steps ? scr + 6ll * (T.deg[G.q + 1] + 1) * G.np * T.radix[G.q] : nullptr;
+  switch (G.phase) {
+    case TP_ROOT: tree_root<hc>(T, pool, chi, tid, nthr); break;
+    case TP_FIRST: tree_first<hc>(T, pool, chi, tid, nthr); break;
+    case TP_M: tree_m<hc, TL>(T, G.q, par, G.pstride, G.np, scr, tid, nthr); break;
+    case TP_UNIT: tree_unit<hc, TL>(T, G.q, par, G.pstride, G.np, G.fused ? nullptr : scr, chi, tid, nthr); break;
+    case TP_PREP: tree_prep<hc>(T, G.q, par, G.pstride, G.np, scr, chi, sm, smn, tid, nthr); break;
+    case TP_Y: tree_y<hc, TL>(T, G.q, par, G.pstride, G.np, scr, y, tid, nthr); break;
+    case TP_MULTI: tree_multi<hc, TL>(T, G.q, par, G.pstride, G.np, y, chi, tid, nthr); break;
+    case TP_GLOOP: tree_gloop<hc>(T, G.q, par, G.pstride, G.np, scr, y, chi, sm, smn, tid, nthr); break;
+    default: {
+      const hc s = tree_leaf<hc, TL>(T, par, G.pstride, G.np, scr, sm, smn, tid, nthr);
+      if (T.pB < 0) out[0] = Ar<hc>::add(out[0], s);
+      else
+        for (int k = 0; k < T.nout; ++k) out[k] = Ar<hc>::add(out[k], sm[k]);
+    }
+  }
 }
 
 int main() {
-  InstDev d;
-  memset(&d, 0, sizeof(d));
-  const int kind = (int)rd(), n = (int)rd(), E = (int)rd(), bm = (int)rd(), cut = (int)rd(), odd = (int)rd();
+  const int count = (int)rd();
   const double budget = rd();
-  const int split = (int)rd();
-  d.kind = kind == 1 && odd ? KIND_LOOP_ODD : kind;
-  d.n = n;
-  d.lda = n + 1;
-  d.glynn = 1;
-  d.nout = 1;
-  if (kind >= 3) {
-    d.reps[d.E++] = bm;
-    if (kind == 4) d.reps[d.E++] = 1;
-    d.nout = 2 * bm + cut + (kind == 4 ? 2 : 1);
+  const int tile = (int)rd(), chip = (int)rd();  // as tree_program's
+  std::vector<TreeInst> insts(count);
+  std::vector<TreeLevels> levels(count);
+  std::vector<std::vector<hc>> exts(count);
+  for (int k = 0; k < count; ++k) {
+    InstDev d;
+    memset(&d, 0, sizeof(d));
+    const int kind = (int)rd(), n = (int)rd(), E = (int)rd(), bm = (int)rd(), cut = (int)rd(), odd = (int)rd();
+    d.kind = kind == 1 && odd ? KIND_LOOP_ODD : kind;
+    d.n = n;
+    d.lda = n + 1;
+    d.glynn = 1;
+    d.nout = 1;
+    if (kind >= 3) {
+      d.reps[d.E++] = bm;
+      if (kind == 4) d.reps[d.E++] = 1;
+      d.nout = 2 * bm + cut + (kind == 4 ? 2 : 1);
+    }
+    for (int e = 0; e < E; ++e) d.reps[d.E++] = (int)rd();
+    exts[k].assign((size_t)(n + 3) * (n + 1), hc{0, 0});
+    auto at = [&](int r, int c) -> hc& { return exts[k][(size_t)r * (n + 1) + c]; };
+    for (int r = 0; r < n; ++r)
+      for (int c = 0; c < n; ++c) { const double re = rd(); at(r, c) = {re, rd()}; }
+    for (int i = 0; i < n; ++i) { const double re = rd(); at(i, n) = at(n, i) = {re, rd()}; }
+    for (int i = 0; i < n; ++i) { const double re = rd(); at(n + 1, i) = {re, rd()}; }
+    d.oddloop.re = rd();
+    d.oddloop.im = rd();
+    if (!tree_build(d, insts[k])) { std::printf("FAIL no tree\n"); return 1; }
+    insts[k].pstride = insts[k].nout;
+    tree_levels(insts[k], sizeof(hc), budget, levels[k]);
   }
-  for (int e = 0; e < E; ++e) d.reps[d.E++] = (int)rd();
-  Buf ext((size_t)(n + 3) * (n + 1));
-  for (auto& x : ext.v) x = {0, 0};
-  auto at = [&](int r, int c) -> hc& { return ext.v[(size_t)r * (n + 1) + c]; };
-  for (int r = 0; r < n; ++r)
-    for (int c = 0; c < n; ++c) { const double re = rd(); at(r, c) = {re, rd()}; }
-  for (int i = 0; i < n; ++i) { const double re = rd(); at(i, n) = at(n, i) = {re, rd()}; }
-  for (int i = 0; i < n; ++i) { const double re = rd(); at(n + 1, i) = {re, rd()}; }
-  d.oddloop.re = rd();
-  d.oddloop.im = rd();
-
-  TreeInst T;
-  if (!tree_build(d, T)) { std::printf("FAIL no tree\n"); return 1; }
-  const unsigned char* pool = reinterpret_cast<const unsigned char*>(ext.p());
-  const double scale = std::ldexp(1.0, -tree_scale_exp(T));
-  std::vector<hc> a(T.nout, hc{0, 0}), b = a;
-
-  // every task of the CTA kernel: its path, then its subtree
-  T.q = std::min(split, T.steps);
-  long long el[3], tasks = 1;
-  for (int q = 0; q < T.q; ++q) tasks *= T.radix[q];
-  tree_cta_elems(T, T.q, el);
-  for (long long t = 0; t < tasks; ++t) {
-    Buf b0(el[0]), b1(std::max<long long>(el[1], 1)), sc(std::max<long long>(el[2], 1));
-    hc* buf[2] = {b0.p(), b1.p()};
-    long long code = t;
-    tree_root<hc>(T, pool, buf[0], 0, 1);
-    int cur = 0, np = 1;
-    for (int q = 0; q < T.steps; ++q) {
-      const int R = T.radix[q];
-      int d0 = 0, nd = R;
-      if (q < T.q) { d0 = (int)(code % R); code /= R; nd = 1; }
-      hc *par = buf[cur], *chi = buf[cur ^ 1];
-      if (T.reps[q] == 1) {
-        if (T.pL >= 0) tree_m<hc>(T, q, par, np, np, sc.p(), 0, 1);
-        tree_unit<hc>(T, q, par, np, np, sc.p(), chi, d0, nd, 0, 1);
-      } else {
-        hc* y = sc.p() + 6ll * (T.deg[q + 1] + 1) * np * nd;
-        tree_prep<hc>(T, q, par, np, np, sc.p(), chi, d0, nd, 0, 1);
-        if (tree_width(T.X, T.E, q + 1) > 0) {
-          tree_y<hc>(T, q, par, np, np, sc.p(), y, nd, 0, 1);
-          tree_multi<hc>(T, q, par, np, np, y, chi, nd, 0, 1);
-          if (T.pL >= 0) tree_gloop<hc>(T, q, par, np, np, sc.p(), y, chi, d0, nd, 0, 1);
-        }
+  TreeProgram P;
+  std::vector<int> base, cnt;
+  int nparts = 0;
+  tree_program(insts, levels, sizeof(hc), tile, chip, nparts, base, cnt, P);
+  std::vector<hc> ws((size_t)P.ws_bytes / sizeof(hc), hc{NAN, NAN}), sm(P.smem);
+  std::vector<int> slots(nparts, 0);
+  std::vector<std::vector<hc>> out(count);
+  for (int k = 0; k < count; ++k) out[k].assign(P.insts[k].nout, hc{0, 0});
+  unsigned char* w = reinterpret_cast<unsigned char*>(ws.data());
+  for (const TreeRound& R : P.rounds)
+    for (int g = R.seg0; g < R.seg0 + R.nseg; ++g) {
+      const TreeSeg& G = P.segs[g];
+      const TreeInst& T = P.insts[G.inst];
+      const TreeLevels& L = levels[G.inst];
+      const int end = g + 1 < R.seg0 + R.nseg ? P.segs[g + 1].warp0 : R.nwarps, warps = end - G.warp0;
+      if (warps < 1) { std::printf("FAIL segment without warps\n"); return 1; }
+      // what the segment may touch: its two levels, its scratch
+      const long long l0 = T.scr_off - L.scr_off;
+      auto range = [&](long long off, long long elems) { g_bufs[reinterpret_cast<hc*>(w + off)] = (size_t)elems; };
+      g_bufs.clear();
+      g_bufs[sm.data()] = sm.size();
+      range(l0 + L.off[G.q], L.cap[G.q] * tree_node_elems(T, G.q));
+      if (G.q < T.steps) range(l0 + L.off[G.q + 1], L.cap[G.q + 1] * tree_node_elems(T, G.q + 1));
+      range(T.scr_off, (L.bytes - L.scr_off) / (long long)sizeof(hc));
+      const hc* par = reinterpret_cast<const hc*>(w + G.par) + G.p0;
+      hc *chi = reinterpret_cast<hc*>(w + G.chi), *scr = reinterpret_cast<hc*>(w + T.scr_off);
+      const unsigned char* pool = reinterpret_cast<const unsigned char*>(exts[G.inst].data());
+      // chip 32: the phases that do not stage their series in shared memory
+      const int smn = chip > 32 ? P.smem : (T.pB >= 0 ? 5 * (T.deg[T.steps] + 1) + 32 : 0);
+      // every lane of the segment's warps as one thread (warp-wide phases: a warp of one lane)
+      const bool wide = G.phase == TP_PREP || G.phase == TP_GLOOP || (G.phase == TP_LEAF && T.pB >= 0);
+      const int nthr = wide ? warps : warps * 32;
+      for (int t = 0; t < nthr; ++t) {
+        if (G.tile == 0) phase<0>(T, G, pool, par, chi, scr, sm.data(), smn, t, nthr, out[G.inst].data());
+        else if (G.tile == 1) phase<1>(T, G, pool, par, chi, scr, sm.data(), smn, t, nthr, out[G.inst].data());
+        else phase<4>(T, G, pool, par, chi, scr, sm.data(), smn, t, nthr, out[G.inst].data());
       }
-      np *= nd;
-      cur ^= 1;
+      if (G.phase == TP_LEAF && count > 1)
+        for (int x = 0; x < warps * T.pstride; ++x)
+          if (slots.at(G.part + x)++) { std::printf("FAIL partial slot used twice\n"); return 1; }
     }
-    if (T.steps < T.E && T.pO >= 0) tree_m<hc>(T, T.steps, buf[cur], np, np, sc.p(), 0, 1);
-    leaf(T, buf[cur], np, np, sc.p(), a);
+  for (int x : slots)
+    if (!x && count > 1) { std::printf("FAIL partial slot never written\n"); return 1; }
+  for (int k = 0; k < count; ++k) {
+    const double scale = std::ldexp(1.0, -tree_scale_exp(P.insts[k]));
+    for (const hc& z : out[k]) std::printf("%.17g %.17g\n", z.re * scale, z.im * scale);
   }
-
-  // level by level
-  TreeGridPlan g;
-  tree_grid_plan(T, sizeof(hc), budget, g);
-  std::vector<Buf*> lev;
-  for (int q = 0; q <= T.steps; ++q) lev.push_back(new Buf((size_t)(g.cap[q] * tree_node_elems(T, q))));
-  Buf sc((size_t)(g.bytes - g.scr_off) / sizeof(hc));
-  long long launches = 1;
-  auto launch = [&](int phase, int q, int p0, int np, int ps, int d0, int nd) {
-    ++launches;
-    hc *par = lev[q]->p() + p0, *chi = q < T.steps ? lev[q + 1]->p() : nullptr;
-    hc* y = q < T.steps ? sc.p() + 6ll * (T.deg[q] + 1 + T.reps[q]) * np * nd : nullptr;
-    switch (phase) {
-      case TP_M: tree_m<hc>(T, q, par, ps, np, sc.p(), 0, 1); break;
-      case TP_UNIT: tree_unit<hc>(T, q, par, ps, np, sc.p(), chi, d0, nd, 0, 1); break;
-      case TP_PREP: tree_prep<hc>(T, q, par, ps, np, sc.p(), chi, d0, nd, 0, 1); break;
-      case TP_Y: tree_y<hc>(T, q, par, ps, np, sc.p(), y, nd, 0, 1); break;
-      case TP_MULTI: tree_multi<hc>(T, q, par, ps, np, y, chi, nd, 0, 1); break;
-      case TP_GLOOP: tree_gloop<hc>(T, q, par, ps, np, sc.p(), y, chi, d0, nd, 0, 1); break;
-      default: leaf(T, par, ps, np, sc.p(), b);
-    }
-  };
-  tree_root<hc>(T, pool, lev[0]->p(), 0, 1);
-  tree_walk(T, g, 0, 1, launch);
-  if (launches != g.launches) { std::printf("FAIL launch count\n"); return 1; }
-  for (int k = 0; k < T.nout; ++k)
-    std::printf("%.17g %.17g %.17g %.17g\n", a[k].re * scale, a[k].im * scale, b[k].re * scale, b[k].im * scale);
-  for (auto* x : lev) delete x;
   return 0;
 }

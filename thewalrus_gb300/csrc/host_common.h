@@ -66,51 +66,19 @@ static inline int sieve_occupancy(int stype, int wpc, int smem) {
   }
 }
 
-static inline cudaError_t tree_cta_launch(int stype, const TreeParams& p, int ctas, int smem, cudaStream_t st) {
+static inline cudaError_t tree_launch(int stype, const TreeParams& p, int ctas, int smem, cudaStream_t st) {
   switch (stype) {
-    case ST_CPLX64: return tree_cta_launch_c64(p, ctas, smem, st);
-    case ST_CPLXDF: return tree_cta_launch_cdf(p, ctas, smem, st);
-    case ST_REAL64: return tree_cta_launch_f64(p, ctas, smem, st);
-    case ST_REALDF: return tree_cta_launch_fdf(p, ctas, smem, st);
-    case ST_MOD0: return tree_cta_launch_mod0(p, ctas, smem, st);
-    case ST_MOD1: return tree_cta_launch_mod1(p, ctas, smem, st);
-    case ST_MOD2: return tree_cta_launch_mod2(p, ctas, smem, st);
-    case ST_MOD3: return tree_cta_launch_mod3(p, ctas, smem, st);
-    case ST_REALDD: return tree_cta_launch_fdd(p, ctas, smem, st);
-    case ST_CPLXDD: return tree_cta_launch_cdd(p, ctas, smem, st);
-    default: return tree_cta_launch_mod4(p, ctas, smem, st);
-  }
-}
-
-static inline cudaError_t tree_grid_launch(int stype, const TreeGrid& g, int blocks, int smem, cudaStream_t st) {
-  switch (stype) {
-    case ST_CPLX64: return tree_grid_launch_c64(g, blocks, smem, st);
-    case ST_CPLXDF: return tree_grid_launch_cdf(g, blocks, smem, st);
-    case ST_REAL64: return tree_grid_launch_f64(g, blocks, smem, st);
-    case ST_REALDF: return tree_grid_launch_fdf(g, blocks, smem, st);
-    case ST_MOD0: return tree_grid_launch_mod0(g, blocks, smem, st);
-    case ST_MOD1: return tree_grid_launch_mod1(g, blocks, smem, st);
-    case ST_MOD2: return tree_grid_launch_mod2(g, blocks, smem, st);
-    case ST_MOD3: return tree_grid_launch_mod3(g, blocks, smem, st);
-    case ST_REALDD: return tree_grid_launch_fdd(g, blocks, smem, st);
-    case ST_CPLXDD: return tree_grid_launch_cdd(g, blocks, smem, st);
-    default: return tree_grid_launch_mod4(g, blocks, smem, st);
-  }
-}
-
-static inline int tree_occupancy(int stype, int smem) {
-  switch (stype) {
-    case ST_CPLX64: return tree_occupancy_c64(smem);
-    case ST_CPLXDF: return tree_occupancy_cdf(smem);
-    case ST_REAL64: return tree_occupancy_f64(smem);
-    case ST_REALDF: return tree_occupancy_fdf(smem);
-    case ST_MOD0: return tree_occupancy_mod0(smem);
-    case ST_MOD1: return tree_occupancy_mod1(smem);
-    case ST_MOD2: return tree_occupancy_mod2(smem);
-    case ST_MOD3: return tree_occupancy_mod3(smem);
-    case ST_REALDD: return tree_occupancy_fdd(smem);
-    case ST_CPLXDD: return tree_occupancy_cdd(smem);
-    default: return tree_occupancy_mod4(smem);
+    case ST_CPLX64: return tree_launch_c64(p, ctas, smem, st);
+    case ST_CPLXDF: return tree_launch_cdf(p, ctas, smem, st);
+    case ST_REAL64: return tree_launch_f64(p, ctas, smem, st);
+    case ST_REALDF: return tree_launch_fdf(p, ctas, smem, st);
+    case ST_MOD0: return tree_launch_mod0(p, ctas, smem, st);
+    case ST_MOD1: return tree_launch_mod1(p, ctas, smem, st);
+    case ST_MOD2: return tree_launch_mod2(p, ctas, smem, st);
+    case ST_MOD3: return tree_launch_mod3(p, ctas, smem, st);
+    case ST_REALDD: return tree_launch_fdd(p, ctas, smem, st);
+    case ST_CPLXDD: return tree_launch_cdd(p, ctas, smem, st);
+    default: return tree_launch_mod4(p, ctas, smem, st);
   }
 }
 

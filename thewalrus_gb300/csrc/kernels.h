@@ -14,9 +14,7 @@ namespace wg {
 #define WG_KERNEL_UNIT_DECL(T)                                                                      \
   cudaError_t sieve_launch_##T(const SieveParams& p, int ctas, int wpc, cudaStream_t st); \
   int sieve_occupancy_##T(int wpc, int smem);                                             \
-  cudaError_t tree_cta_launch_##T(const TreeParams& p, int ctas, int smem, cudaStream_t st);   \
-  cudaError_t tree_grid_launch_##T(const TreeGrid& g, int blocks, int smem, cudaStream_t st);  \
-  int tree_occupancy_##T(int smem);                                                       \
+  cudaError_t tree_launch_##T(const TreeParams& p, int ctas, int smem, cudaStream_t st);  \
   cudaError_t sieve_tables_##T(const double* binom, const double* inv);
 
 WG_KERNEL_UNIT_DECL(c64)

@@ -24,30 +24,20 @@ int WG_CAT(sieve_occupancy_, WG_UNIT_NAME)(int wpc, int smem) {
   return nb;
 }
 
-cudaError_t WG_CAT(tree_cta_launch_, WG_UNIT_NAME)(const TreeParams& p, int ctas, int smem, cudaStream_t st) {
-  auto k = tree_cta_kernel<WG_UNIT_SCALAR>;
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  k<<<ctas, TREE_THREADS, smem, st>>>(p);
-  return cudaGetLastError();
-}
-
-cudaError_t WG_CAT(tree_grid_launch_, WG_UNIT_NAME)(const TreeGrid& g, int blocks, int smem, cudaStream_t st) {
-  auto k = tree_grid_kernel<WG_UNIT_SCALAR>;
+// several CTAs wait for one another, so they are launched cooperatively
+cudaError_t WG_CAT(tree_launch_, WG_UNIT_NAME)(const TreeParams& p, int ctas, int smem, cudaStream_t st) {
+  auto k = tree_kernel<typename TreeScalar<WG_UNIT_SCALAR>::T>;
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
-  k<<<blocks, TREE_THREADS, smem, st>>>(g);
-  return cudaGetLastError();
-}
-
-int WG_CAT(tree_occupancy_, WG_UNIT_NAME)(int smem) {
-  int nb = 0;
-  auto k = tree_cta_kernel<WG_UNIT_SCALAR>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, TREE_THREADS, smem) != cudaSuccess) return 0;
-  return nb;
+  if (ctas == 1) {
+    k<<<1, TREE_THREADS, smem, st>>>(p);
+    return cudaGetLastError();
+  }
+  TreeParams arg = p;
+  void* args[] = {&arg};
+  return cudaLaunchCooperativeKernel((const void*)k, dim3(ctas), dim3(TREE_THREADS), args, (size_t)smem, st);
 }
 
 cudaError_t WG_CAT(sieve_tables_, WG_UNIT_NAME)(const double* binom, const double* inv) {

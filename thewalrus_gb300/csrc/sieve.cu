@@ -88,11 +88,11 @@ static int ensure_init(int device) {
   }
   CK(cudaDeviceGetAttribute(&T.sms, cudaDevAttrMultiProcessorCount, dev));
   // stream-ordered plans (one-shot calls, serving batches) allocate from this process's default
-  // pool of the device: keep up to 256 MiB of freed memory there instead of releasing it to the
+  // pool of the device: keep up to 1.5 GiB of freed memory (a large tree's levels) there instead of releasing it to the
   // CUDA driver at every synchronisation, so a repeated call reuses it
   cudaMemPool_t pool;
   CK(cudaDeviceGetDefaultMemPool(&pool, dev));
-  unsigned long long keep = 256ull << 20;
+  unsigned long long keep = 1536ull << 20;
   CK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
   // constant tables: binomials and reciprocals
   static double binom[BINOM_N][BINOM_N];
@@ -159,17 +159,12 @@ struct Group {
   int chunk_begin, chunk_count;
 };
 
-// trees launched as one task queue, and a tree launched level by level
-struct TreeGroup {
-  int stype, first, ninst, ntasks, ctas, smem, counter;
-  long long ws_stride, off_b, off_s;
+// One launch of the tree kernel: trees of one scalar type and the program that walks them.
+struct TreeLaunch {
+  int stype, ctas, smem, sm_warp, sm_cache, sm_ws, cached, counter;
+  int ninst, nrounds, nsegs;
+  size_t prog_off;  // of the instances, rounds and segments in the plan's program bytes
 };
-struct TreeBig {
-  int stype, index, smem, part_base;  // index: in the plan's TreeInst array
-  TreeInst T;
-  TreeGridPlan g;
-};
-constexpr int kTreeLeafBlocks = 304;
 
 }  // namespace wg
 
@@ -203,10 +198,10 @@ struct wg_plan {
   cudaEvent_t fork = nullptr;
   int device = 0;  // the device the plan's memory and tables live on
   bool serial_groups = false;
-  std::vector<wg::TreeInst> trees;
-  std::vector<wg::TreeGroup> tree_groups;
-  std::vector<wg::TreeBig> tree_bigs;
-  wg::TreeInst* d_trees = nullptr;
+  std::vector<wg::TreeLaunch> trees;
+  std::vector<unsigned char> tree_prog;
+  int tree_parts = 0;  // most partials of a tree's output
+  unsigned char* d_prog = nullptr;
   unsigned char* d_ws = nullptr;
   // a plan with trees answers the per-term queries (magnitudes, chunks, partials) by a plan over
   // the same device matrices that evaluates term by term, made when first asked
@@ -721,105 +716,107 @@ static double tree_mac_clocks(int stype) {
   }
 }
 
-// Cuts the tree members of a plan into task-queue launches (one per scalar type) and level-launched
-// trees, and lays out their partial slots (from `nparts` on).  Returns the workspace bytes.
-// A tree goes level by level when that is estimated faster: the queue recomputes every task's
-// path, the levels cost a launch each (~4 us, 8000 clocks).
+// Groups the tree members of a plan into launches (one scalar type each, as many instances as share
+// a workspace budget), makes their programs and lays out their partial slots.  Returns the
+// workspace bytes; the launches run one after another and share it.
 static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) {
-  constexpr long long kMaxCtaBytes = 256 << 10;
-  constexpr double kGridBudget = 48e6, kLaunchClocks = 8000.0, kStepClocks = 2500.0;
+  // A level's byte budget: larger levels are walked in blocks.  A launch's: beyond it the
+  // instances go to the next launch.  Both keep the workspace within what the device's pool keeps.
+  constexpr double kLevelBytes = 200e6, kLaunchBytes = 600e6;
+  constexpr long long kSharedBytes = 200 << 10;
   const int count = (int)P.size();
-  std::vector<TreeSizes> z(count);
-  double total = 0;
+  auto al = [](long long x) { return (x + 255) & ~255ll; };
+  std::vector<TreeLevels> lev(count);
+  std::vector<int> order;
   for (int i = 0; i < count; ++i)
     if (P[i].tree) {
-      tree_sizes(P[i].T, z[i]);
-      total += z[i].total * tree_mac_clocks(P[i].stype);
+      tree_levels(P[i].T, tree_bytes(P[i].stype), kLevelBytes, lev[i]);
+      order.push_back(i);
     }
-  long long ws = 0;
-  std::vector<int> queued;
-  std::vector<double> task_cost(count, 0.0);
-  for (int i = 0; i < count; ++i) {
-    if (!P[i].tree) continue;
-    TreeInst& T = P[i].T;
-    const int sb = (int)stype_bytes(P[i].stype);
-    const double clk = tree_mac_clocks(P[i].stype);
-    int q = 0;
-    const double cta = tree_split(T, z[i], g_num_sms, std::max(z[i].total * clk / total, 0.05), kMaxCtaBytes / sb, q);
-    TreeGridPlan g;
-    tree_grid_plan(T, sb, kGridBudget, g);
-    const double t_cta = cta * clk + T.steps * kStepClocks;
-    const double t_grid = z[i].total * clk / g_num_sms + (double)g.launches * kLaunchClocks;
-    if (cta >= 0 && t_cta <= t_grid) {
-      T.q = q;
-      T.tasks = 1;
-      for (int s = 0; s < q; ++s) T.tasks *= T.radix[s];
-      task_cost[i] = z[i].total * clk / T.tasks;
-      queued.push_back(i);
-    } else {
-      TreeBig b;
-      b.stype = P[i].stype;
-      b.index = i;
-      b.g = g;
-      b.smem = tree_smem(T, sb);
-      b.part_base = nparts;
-      pl->tree_bigs.push_back(b);
-      P[i].d.part_base = T.part_base = nparts;
-      P[i].d.nchunks = (int)g.leaves * kTreeLeafBlocks;
-      nparts += P[i].d.nchunks * T.pstride;
-      ws = std::max(ws, g.bytes);
-    }
-  }
-  // the queues: costly tasks first
-  std::stable_sort(queued.begin(), queued.end(), [&](int a, int b) {
-    return P[a].stype != P[b].stype ? P[a].stype < P[b].stype : task_cost[a] > task_cost[b];
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return P[a].stype != P[b].stype ? P[a].stype < P[b].stype : lev[a].bytes > lev[b].bytes;
   });
-  for (size_t k = 0; k < queued.size();) {
-    TreeGroup G;
+  long long ws = 0;
+  for (size_t k = 0; k < order.size();) {
+    TreeLaunch G;
     memset(&G, 0, sizeof(G));
-    G.stype = P[queued[k]].stype;
-    G.first = (int)pl->trees.size();
-    const int sb = (int)stype_bytes(G.stype);
-    long long el[3] = {1, 1, 1};
-    for (; k < queued.size() && P[queued[k]].stype == G.stype; ++k) {
-      Prepared& p = P[queued[k]];
-      TreeInst& T = p.T;
-      T.task_base = G.ntasks;
-      G.ntasks += T.tasks;
-      ++G.ninst;
-      p.d.part_base = T.part_base = nparts;
-      p.d.nchunks = T.tasks;
-      nparts += T.tasks * T.pstride;
-      long long e[3];
-      tree_cta_elems(T, T.q, e);
-      for (int x = 0; x < 3; ++x) el[x] = std::max(el[x], e[x]);
-      G.smem = std::max(G.smem, tree_smem(T, sb));
-      T.a_off = p.d.a_off;
-      pl->trees.push_back(T);
+    G.stype = P[order[k]].stype;
+    const int sb = tree_bytes(G.stype), tile = G.stype == ST_CPLXDD ? tree_tile<cdd>() : tree_tile<c64>();
+    std::vector<TreeInst> insts;
+    std::vector<TreeLevels> levels;
+    const size_t k0 = k;
+    long long bytes = 0;
+    for (; k < order.size() && P[order[k]].stype == G.stype; ++k) {
+      if (k > k0 && (double)(bytes + lev[order[k]].bytes) > kLaunchBytes) break;
+      bytes += lev[order[k]].bytes;
+      insts.push_back(P[order[k]].T);
+      insts.back().a_off = P[order[k]].d.a_off;
+      levels.push_back(lev[order[k]]);
     }
-    auto al = [](long long x) { return (x + 255) & ~255ll; };
-    G.off_b = al(el[0] * sb);
-    G.off_s = G.off_b + al(el[1] * sb);
-    G.ws_stride = G.off_s + al(el[2] * sb);
-    const int occ = std::max(1, tree_occupancy(G.stype, G.smem));
-    G.ctas = std::min(G.ntasks, g_num_sms * occ);
-    ws = std::max(ws, G.ws_stride * G.ctas);
-    pl->tree_groups.push_back(G);
-  }
-  for (TreeBig& b : pl->tree_bigs) {
-    const int i = b.index;
-    b.T = P[i].T;
-    b.T.a_off = P[i].d.a_off;
-    b.index = (int)pl->trees.size();
-    pl->trees.push_back(b.T);
-  }
-  for (int i = 0; i < count; ++i)
-    if (P[i].tree) {
-      P[i].d.pstride = P[i].T.pstride;
-      P[i].d.comp_off = P[i].T.comp_off;
-      P[i].d.mag_off = 0;
+    TreeProgram prog;
+    std::vector<int> base, cnt;
+    const double clk = tree_mac_clocks(G.stype);
+    const int np0 = nparts;
+    G.ctas = g_num_sms;
+    tree_program(insts, levels, sb, tile, g_num_sms * TREE_THREADS, nparts, base, cnt, prog);
+    if (tree_one_cta(prog, clk) <= tree_whole_chip(prog, clk, g_num_sms)) {
+      G.ctas = 1;
+      nparts = np0;
+      prog = TreeProgram();
+      tree_program(insts, levels, sb, tile, TREE_THREADS, nparts, base, cnt, prog);
     }
+    for (size_t j = 0; j < insts.size(); ++j) {
+      InstDev& d = P[order[k0 + j]].d;
+      d.part_base = base[j];
+      d.nchunks = cnt[j];
+      d.pstride = insts[j].pstride;
+      d.comp_off = insts[j].comp_off;
+      d.mag_off = 0;
+      pl->tree_parts = std::max(pl->tree_parts, cnt[j]);
+    }
+    G.ninst = (int)prog.insts.size();
+    G.nrounds = (int)prog.rounds.size();
+    G.nsegs = (int)prog.segs.size();
+    const size_t b_inst = sizeof(TreeInst) * prog.insts.size(), b_rounds = sizeof(TreeRound) * prog.rounds.size(),
+                 b_segs = sizeof(TreeSeg) * prog.segs.size();
+    G.prog_off = pl->tree_prog.size();
+    pl->tree_prog.resize(G.prog_off + al((long long)(b_inst + b_rounds + b_segs)));
+    memcpy(pl->tree_prog.data() + G.prog_off, prog.insts.data(), b_inst);
+    memcpy(pl->tree_prog.data() + G.prog_off + b_inst, prog.rounds.data(), b_rounds);
+    memcpy(pl->tree_prog.data() + G.prog_off + b_inst + b_rounds, prog.segs.data(), b_segs);
+    G.sm_warp = prog.smem;
+    G.sm_cache = (int)al((long long)prog.smem * (TREE_THREADS / 32) * sb);
+    G.smem = G.sm_cache;
+    G.cached = G.smem + al((long long)(b_inst + b_rounds + b_segs)) <= kSharedBytes;
+    if (G.cached) G.smem += (int)al((long long)(b_inst + b_rounds + b_segs));
+    if (G.ctas == 1 && G.smem + prog.ws_bytes <= kSharedBytes) {
+      G.sm_ws = G.smem;
+      G.smem += (int)prog.ws_bytes;
+    } else {
+      ws = std::max(ws, prog.ws_bytes);
+    }
+    pl->trees.push_back(G);
+  }
   return ws;
+}
+
+// whether the plan is one tree launch, which then also reduces (tree_finish): few enough outputs
+// for one CTA
+static bool plan_single(const wg_plan* pl) {
+  return pl->groups.empty() && pl->trees.size() == 1 && pl->total_out <= 64;
+}
+static int plan_counters(const wg_plan* pl) {
+  return (int)(pl->groups.size() + pl->trees.size()) + 1;  // and tree_finish's
+}
+static unsigned int plan_prime(const wg_plan* pl) {
+  return prec_mod(pl->precision) ? MOD_PRIMES[pl->precision - WG_PREC_MOD0] : 0u;
+}
+// warps that sum an output's partials, of the `nw` of a block: one, as the per-term launches
+// always had, unless a tree left several hundred
+static int plan_wpo(const wg_plan* pl, int nw) {
+  int w = 1;
+  while (w < nw && w * 64 < pl->tree_parts && w * pl->total_out < nw) w *= 2;
+  return w;
 }
 
 // ext_pool: the instances' matrices are on the device already, at their a_off
@@ -970,10 +967,11 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   const size_t b_scales = al(sizeof(double) * std::max<size_t>(scales.size(), 1));
   const size_t b_out = al(sizeof(double2) * std::max(out, 1));
   const size_t b_mag = al(sizeof(double) * std::max(out, 1));
-  const size_t ncnt = pl->groups.size() + pl->tree_groups.size();
-  for (size_t g = 0; g < pl->tree_groups.size(); ++g) pl->tree_groups[g].counter = (int)(pl->groups.size() + g);
+  const size_t ncnt = (size_t)plan_counters(pl);
+  int counter = (int)pl->groups.size();
+  for (TreeLaunch& g : pl->trees) g.counter = counter++;
   const size_t b_cnt = al(sizeof(unsigned int) * std::max<size_t>(ncnt, 1));
-  const size_t b_tree = al(sizeof(TreeInst) * std::max<size_t>(pl->trees.size(), 1));
+  const size_t b_tree = al(std::max<size_t>(pl->tree_prog.size(), 1));
   const size_t b_ws = al((size_t)ws_bytes);
   const size_t b_err = al(sizeof(int));
   const size_t b_gdesc = gs ? al(sizeof(GatherDev) * std::max<size_t>(gs->desc.size(), 1)) : 0;
@@ -992,7 +990,7 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   unsigned char* base = (unsigned char*)pl->dmem;
   pl->d_inst = (InstDev*)base; base += b_inst;
   pl->d_chunks = (ChunkDev*)base; base += b_chunks;
-  pl->d_trees = (TreeInst*)base; base += b_tree;
+  pl->d_prog = base; base += b_tree;
   pl->d_scales = (double*)base; base += b_scales;
   pl->d_pool = ext_pool ? ext_pool : base; base += b_pool;
   pl->d_partials = (double2*)base; base += b_parts;
@@ -1009,7 +1007,7 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   std::vector<unsigned char> host(o_pool + (gs || ext_pool ? 0 : b_pool), 0);
   memcpy(host.data(), pl->inst.data(), sizeof(InstDev) * count);
   if (!pl->chunks.empty()) memcpy(host.data() + b_inst, pl->chunks.data(), sizeof(ChunkDev) * pl->chunks.size());
-  if (!pl->trees.empty()) memcpy(host.data() + o_tree, pl->trees.data(), sizeof(TreeInst) * pl->trees.size());
+  if (!pl->tree_prog.empty()) memcpy(host.data() + o_tree, pl->tree_prog.data(), pl->tree_prog.size());
   if (!scales.empty()) memcpy(host.data() + o_scales, scales.data(), sizeof(double) * scales.size());
   for (int i = 0; i < count; ++i)
     if (!P[i].ext.empty() && !ext_pool) memcpy(host.data() + o_pool + P[i].d.a_off, P[i].ext.data(), P[i].ext.size());
@@ -1071,59 +1069,36 @@ static int launch_trees(wg_plan* pl, cudaStream_t st) {
   p.pool = pl->d_pool;
   p.partials = pl->d_partials;
   p.ws = pl->d_ws;
-  for (const TreeGroup& G : pl->tree_groups) {
-    p.inst = pl->d_trees + G.first;
-    p.ninst = G.ninst;
-    p.ntasks = G.ntasks;
-    p.ws_stride = G.ws_stride;
-    p.off_b = G.off_b;
-    p.off_s = G.off_s;
-    p.counter = pl->d_counters + G.counter;
-    const cudaError_t e = tree_cta_launch(G.stype, p, G.ctas, G.smem, st);
-    if (e != cudaSuccess) return fail(WG_ECUDA, "tree launch: %s", cudaGetErrorString(e));
+  p.err = pl->d_err;
+  if (plan_single(pl)) {
+    p.fin.inst = pl->d_inst;
+    p.fin.ninst = (int)pl->inst.size();
+    p.fin.partials = pl->d_partials;
+    p.fin.scales = pl->d_scales;
+    p.fin.out = pl->d_out;
+    p.fin.mags = pl->d_mag;
+    p.fin.err = pl->d_err;
+    p.fin.counters = pl->d_counters;
+    p.fin.ncounters = plan_counters(pl);
+    p.fin.done = pl->d_counters + plan_counters(pl) - 1;
+    p.fin.total_out = pl->total_out;
+    p.fin.wpo = plan_wpo(pl, TREE_THREADS / 32);
+    p.fin.modp = plan_prime(pl);
   }
-  p.inst = pl->d_trees;
-  for (const TreeBig& b : pl->tree_bigs) {
-    const TreeInst& T = b.T;
-    long long part = b.part_base;
-    cudaError_t err = cudaSuccess;
-    auto launch = [&](int phase, int q, int p0, int np, int ps, int d0, int nd) {
-      if (err != cudaSuccess) return;
-      TreeGrid G;
-      G.P = p;
-      G.inst = b.index;
-      G.phase = phase;
-      G.q = q;
-      G.np = np;
-      G.p0 = p0;
-      G.pstride = ps;
-      G.d0 = d0;
-      G.nd = nd;
-      G.part = part;
-      G.par = pl->d_ws + b.g.off[q];
-      G.chi = phase == TP_ROOT ? G.par : (q < T.steps ? pl->d_ws + b.g.off[q + 1] : nullptr);
-      G.scr = pl->d_ws + b.g.scr_off;
-      const bool dd2 = b.stype == ST_CPLXDD;
-      const int TL = dd2 ? 2 : 4;
-      const long long Lp = T.deg[q] + 1, W1 = tree_width(T.X, T.E, q + 1), tp = (Lp + TL - 1) / TL;
-      const long long Lc = q < T.steps ? T.deg[q + 1] + 1 : Lp, tc = (Lc + TL - 1) / TL;
-      long long items = 1;  // threads of work
-      switch (phase) {
-        case TP_ROOT: items = tree_entries(tree_width(T.X, T.E, 0), T.diag); break;
-        case TP_M: items = tp * np; break;
-        case TP_UNIT: items = tp * tree_entries((int)W1, T.diag) * np; break;
-        case TP_PREP: case TP_GLOOP: items = 32ll * np * nd; break;
-        case TP_Y: items = tc * 2 * W1 * np * nd; break;
-        case TP_MULTI: items = tc * (tree_entries((int)W1, T.diag) - 1) * np * nd; break;
-        default: items = (long long)kTreeLeafBlocks * TREE_THREADS;
-      }
-      const int blocks = (int)std::max(1ll, (items + TREE_THREADS - 1) / TREE_THREADS);
-      err = tree_grid_launch(b.stype, G, blocks, phase == TP_LEAF ? b.smem : 0, st);
-      if (phase == TP_LEAF) part += (long long)kTreeLeafBlocks * T.pstride;
-    };
-    launch(TP_ROOT, 0, 0, 1, 1, 0, 1);
-    tree_walk(T, b.g, 0, 1, launch);
-    if (err != cudaSuccess) return fail(WG_ECUDA, "tree level launch: %s", cudaGetErrorString(err));
+  for (const TreeLaunch& G : pl->trees) {
+    p.ninst = G.ninst;
+    p.nrounds = G.nrounds;
+    p.nsegs = G.nsegs;
+    p.inst = (const TreeInst*)(pl->d_prog + G.prog_off);
+    p.rounds = (const TreeRound*)(p.inst + G.ninst);
+    p.segs = (const TreeSeg*)(p.rounds + G.nrounds);
+    p.cached = G.cached;
+    p.sm_warp = G.sm_warp;
+    p.sm_cache = G.sm_cache;
+    p.sm_ws = G.sm_ws;
+    p.bar = pl->d_counters + G.counter;
+    const cudaError_t e = tree_launch(G.stype, p, G.ctas, G.smem, st);
+    if (e != cudaSuccess) return fail(WG_ECUDA, "tree launch: %s", cudaGetErrorString(e));
   }
   return WG_OK;
 }
@@ -1173,14 +1148,12 @@ static int launch_plan(wg_plan* pl, cudaStream_t st) {
     }
   }
   const int ninst = (int)pl->inst.size();
-  if (ninst > 0) {
-    const int threads = 128;
-    const int blocks = (pl->total_out * 32 + threads - 1) / threads;  // one warp per output
-    const unsigned int modp = prec_mod(pl->precision) ? MOD_PRIMES[pl->precision - WG_PREC_MOD0] : 0u;
+  if (ninst > 0 && !plan_single(pl)) {
+    const int threads = 256, wpo = plan_wpo(pl, threads / 32);
+    const int per = threads / 32 / wpo, blocks = (pl->total_out + per - 1) / per;
     reduce_kernel<<<std::max(blocks, 1), threads, 0, st>>>(pl->d_inst, ninst, pl->d_partials, pl->d_scales, pl->d_out,
-                                                           pl->d_counters, (int)(pl->groups.size() + pl->tree_groups.size()), pl->total_out,
-                                                           modp,
-                                                           pl->d_mag);
+                                                           pl->d_counters, plan_counters(pl), pl->total_out, wpo,
+                                                           plan_prime(pl), pl->d_mag, pl->d_err);
     CK(cudaGetLastError());
   }
   return WG_OK;
@@ -1353,9 +1326,7 @@ int wg_plan_outputs(const wg_plan* plan) { return plan ? plan->total_out : fail(
 
 int wg_plan_kernel_launches(const wg_plan* plan) {
   if (!plan) return fail(WG_EINVAL, "plan is NULL");
-  long long n = (long long)plan->groups.size() + (long long)plan->tree_groups.size() + (plan->inst.empty() ? 0 : 1);
-  for (const TreeBig& b : plan->tree_bigs) n += b.g.launches;
-  return (int)n;
+  return (int)(plan->groups.size() + plan->trees.size()) + (plan->inst.empty() || plan_single(plan) ? 0 : 1);
 }
 
 int wg_plan_partials(wg_plan* plan, double* out, int capacity, void* stream) {

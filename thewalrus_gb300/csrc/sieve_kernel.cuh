@@ -1175,66 +1175,120 @@ __device__ __forceinline__ void two_sum_merge(double& s, double& c, double s2, d
   c = c + c2 + e;
 }
 
-// One warp per output: lane l Neumaier-sums the chunk partials l, l+32, ... in order, then the
-// lanes merge in a fixed butterfly (bitwise reproducible), and the final scale (0.5^(N/2-1)
-// etc., and the undoing of any input prescaling) is applied.  Thread 0 re-arms the work
-// counters for the next execution.
-static __global__ void reduce_kernel(const InstDev* __restrict__ inst, int ninst, const double2* __restrict__ partials,
-                              const double* __restrict__ scales, double2* __restrict__ out, unsigned int* counters,
-                              int ncounters, int total_out, unsigned int modp, double* __restrict__ mags = nullptr) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw < total_out) {
-    // locate the instance (outputs are laid out instance by instance)
-    int lo = 0, hi = ninst - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (inst[mid].out_base <= gw) lo = mid; else hi = mid - 1;
+// A sum of partials: value and compensation of both components, and the magnitudes.
+struct RSum {
+  double sr, cr, si, ci, ms;
+};
+__device__ __forceinline__ void rsum_merge(RSum& a, const RSum& b) {
+  two_sum_merge(a.sr, a.cr, b.sr, b.cr);
+  two_sum_merge(a.si, a.ci, b.si, b.ci);
+  a.ms += b.ms;
+}
+
+// One warp: lane l Neumaier-sums the partials c0 + l, c0 + l + stride, ... of output o in order, then
+// the lanes merge in a fixed butterfly (bitwise reproducible); every lane returns the sum.
+__device__ __forceinline__ RSum reduce_warp(const InstDev& I, const double2* partials, int o, int c0, int stride) {
+  const int nch = I.nchunks, comp_off = I.comp_off, mag_off = I.mag_off;
+  const int ps = I.pstride > I.nout ? I.pstride : I.nout;  // slots per chunk
+  const double2* part = partials + I.part_base + o;
+  RSum s = {0, 0, 0, 0, 0};
+#pragma unroll 4
+  for (int c = c0 + (threadIdx.x & 31); c < nch; c += stride) {
+    const double2 v = __ldcg(part + (long long)c * ps);
+    neumaier(s.sr, s.cr, v.x);
+    neumaier(s.si, s.ci, v.y);
+    if (comp_off) {  // double-double kinds: the chunk's compensation
+      const double2 w = __ldcg(part + (long long)c * ps + comp_off);
+      s.cr += w.x;
+      s.ci += w.y;
     }
-    const InstDev& I = inst[lo];
-    const int o = gw - I.out_base;
-    double sr = 0, si = 0, cr = 0, ci = 0, ms = 0;
-    const int ps = I.pstride > I.nout ? I.pstride : I.nout;  // slots per chunk
-    for (int c = lane; c < I.nchunks; c += 32) {
-      const double2 v = partials[I.part_base + c * ps + o];
-      neumaier(sr, cr, v.x);
-      neumaier(si, ci, v.y);
-      if (I.comp_off) {  // double-double kinds: the chunk's compensation
-        const double2 w = partials[I.part_base + c * ps + I.comp_off + o];
-        cr += w.x;
-        ci += w.y;
-      }
-      if (I.mag_off) ms += partials[I.part_base + c * ps + I.mag_off + o].x;
-    }
-#pragma unroll
-    for (int off = 16; off; off >>= 1) ms += __shfl_xor_sync(0xffffffffu, ms, off);
-#pragma unroll
-    for (int off = 16; off; off >>= 1) {
-      const double osr = __shfl_xor_sync(0xffffffffu, sr, off), ocr = __shfl_xor_sync(0xffffffffu, cr, off);
-      const double osi = __shfl_xor_sync(0xffffffffu, si, off), oci = __shfl_xor_sync(0xffffffffu, ci, off);
-      if (lane & off) {  // the upper lane adds into the lower lane's sum: same order on both sides
-        double a = osr, b = ocr;
-        two_sum_merge(a, b, sr, cr);
-        sr = a; cr = b;
-        a = osi; b = oci;
-        two_sum_merge(a, b, si, ci);
-        si = a; ci = b;
-      } else {
-        two_sum_merge(sr, cr, osr, ocr);
-        two_sum_merge(si, ci, osi, oci);
-      }
-    }
-    if (lane == 0) {
-      const double sc = scales[I.scale_base + o];
-      if (modp) {  // residues (< 2^31) summed exactly in FP64 (fewer than 2^22 chunks), then mod p
-        const unsigned long long r = (unsigned long long)(sr + cr) % modp;
-        out[gw] = make_double2((double)(r * (unsigned long long)sc % modp), 0.0);
-      } else {
-        out[gw] = make_double2((sr + cr) * sc, (si + ci) * sc);
-      }
-      if (mags) mags[gw] = I.mag_off ? ms * fabs(sc) : 0.0;
-    }
+    if (mag_off) s.ms += __ldcg(part + (long long)c * ps + mag_off).x;
   }
+  if (c0 + 1 >= nch) {  // one partial: lane 0's
+    s.sr = __shfl_sync(0xffffffffu, s.sr, 0);
+    s.cr = __shfl_sync(0xffffffffu, s.cr, 0);
+    s.si = __shfl_sync(0xffffffffu, s.si, 0);
+    s.ci = __shfl_sync(0xffffffffu, s.ci, 0);
+    s.ms = __shfl_sync(0xffffffffu, s.ms, 0);
+    return s;
+  }
+#pragma unroll
+  for (int off = 16; off; off >>= 1) {
+    RSum x;
+    x.sr = __shfl_xor_sync(0xffffffffu, s.sr, off);
+    x.cr = __shfl_xor_sync(0xffffffffu, s.cr, off);
+    x.si = __shfl_xor_sync(0xffffffffu, s.si, off);
+    x.ci = __shfl_xor_sync(0xffffffffu, s.ci, off);
+    x.ms = __shfl_xor_sync(0xffffffffu, s.ms, off);
+    if (threadIdx.x & off) {  // the upper lane adds into the lower lane's sum: same order on both sides
+      const RSum t = s;
+      s = x;
+      x = t;
+    }
+    rsum_merge(s, x);
+  }
+  return s;
+}
+
+// the instance that output gw belongs to (outputs are laid out instance by instance)
+__device__ __forceinline__ const InstDev& reduce_instance(const InstDev* inst, int ninst, int gw) {
+  int lo = 0, hi = ninst - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (inst[mid].out_base <= gw) lo = mid; else hi = mid - 1;
+  }
+  return inst[lo];
+}
+
+// The final scale (0.5^(N/2-1) etc., and the undoing of any input prescaling); NaN when a launch gave
+// up waiting for its own blocks (*err).
+__device__ __forceinline__ void reduce_write(const InstDev& I, int gw, const RSum& s, const double* scales, double2* out,
+                                             unsigned int modp, double* mags, const int* err) {
+  const double sc = scales[I.scale_base + gw - I.out_base];
+  if (err && *err) {
+    out[gw] = make_double2(nan(""), nan(""));
+  } else if (modp) {  // residues (< 2^31) summed exactly in FP64 (fewer than 2^22 chunks), then mod p
+    const unsigned long long r = (unsigned long long)(s.sr + s.cr) % modp;
+    out[gw] = make_double2((double)(r * (unsigned long long)sc % modp), 0.0);
+  } else {
+    out[gw] = make_double2((s.sr + s.cr) * sc, (s.si + s.ci) * sc);
+  }
+  if (mags) mags[gw] = I.mag_off ? s.ms * fabs(sc) : 0.0;
+}
+
+// Outputs first, first + step, ... of a block: `wpo` of its warps to an output (their sums merged in
+// warp order), so that one output of many partials is not one warp's serial sum.
+__device__ __forceinline__ void reduce_block(const InstDev* inst, int ninst, const double2* partials,
+                                             const double* scales, double2* out, int first, int step, int total_out,
+                                             int wpo, unsigned int modp, double* mags, const int* err) {
+  __shared__ RSum s_part[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = warp % wpo, per = (blockDim.x >> 5) / wpo;
+  for (int g0 = first; g0 < total_out; g0 += step) {
+    const int gw = g0 + warp / wpo;
+    const bool live = warp / wpo < per && gw < total_out;
+    RSum s = {0, 0, 0, 0, 0};
+    if (live) {
+      const InstDev& I = reduce_instance(inst, ninst, gw);
+      s = reduce_warp(I, partials, gw - I.out_base, sub * 32, wpo * 32);
+      if (lane == 0) s_part[warp] = s;
+    }
+    __syncthreads();
+    if (live && sub == 0 && lane == 0) {
+      for (int w = 1; w < wpo; ++w) rsum_merge(s, s_part[warp + w]);
+      reduce_write(reduce_instance(inst, ninst, gw), gw, s, scales, out, modp, mags, err);
+    }
+    __syncthreads();
+  }
+}
+
+// Blocks of `wpo` warps per output over all outputs; thread 0 re-arms the work counters for the next
+// execution.
+static __global__ void reduce_kernel(const InstDev* __restrict__ inst, int ninst, const double2* __restrict__ partials,
+                                     const double* __restrict__ scales, double2* __restrict__ out,
+                                     unsigned int* counters, int ncounters, int total_out, int wpo, unsigned int modp,
+                                     double* __restrict__ mags, const int* __restrict__ err) {
+  const int per = (blockDim.x >> 5) / wpo;
+  reduce_block(inst, ninst, partials, scales, out, blockIdx.x * per, gridDim.x * per, total_out, wpo, modp, mags, err);
   if (blockIdx.x == 0 && threadIdx.x == 0)
     for (int i = 0; i < ncounters; ++i) counters[i] = 0u;
 }

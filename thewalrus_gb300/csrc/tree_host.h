@@ -1,5 +1,5 @@
-// Host side of the elimination tree: an instance's edge order and positions, the sizes and costs
-// of its levels, and how its tree is cut into tasks or launches.
+// Host side of the elimination tree: an instance's edge order and positions, the sizes of its levels,
+// and the program (rounds of segments) that a launch of the tree kernel runs.
 #pragma once
 #include <algorithm>
 #include <cstring>
@@ -11,7 +11,7 @@
 namespace wg {
 
 // The tree of a prepared instance (whole sum, finite-difference signs); false when it does not
-// take one: more than TREE_MAX_K photons pairs, or inclusion/exclusion signs.
+// take one: more than TREE_MAX_K photon pairs, or inclusion/exclusion signs.
 static inline bool tree_build(const InstDev& d, TreeInst& T) {
   memset(&T, 0, sizeof(T));
   const bool batch = d.kind >= KIND_BATCH_EVEN;
@@ -51,7 +51,7 @@ static inline bool tree_build(const InstDev& d, TreeInst& T) {
   order.insert(order.end(), multi.begin(), multi.end());
   order.insert(order.end(), simple.begin() + s0, simple.end());
   T.E = (int)order.size();
-  // closed forms of the last simple edges (the root edge is eliminated when it is the only one)
+  // closed forms of the last simple edges
   int rem = 0;
   if (!batch)
     while (rem < (T.pL < 0 ? 2 : 1) && rem < T.E && d.reps[order[T.E - 1 - rem]] == 1) ++rem;
@@ -74,104 +74,47 @@ static inline bool tree_build(const InstDev& d, TreeInst& T) {
 // binary exponent of the outputs' scale: 2^-r of every eliminated edge, twice the half of the first
 static inline int tree_scale_exp(const TreeInst& T) { return T.deg[T.steps] - (T.steps > 0 ? 1 : 0); }
 
-struct TreeSizes {
-  double nodes[MAX_EDGES + 2];  // of the whole tree, after q steps
-  double cost[MAX_EDGES + 2];   // multiply-adds of step q per parent with all children; [steps]: the leaf's
-  double one[MAX_EDGES + 2];    // of step q per parent with one child
-  double total = 0;
-};
+// bytes of a node element
+static inline int tree_bytes(int stype) { return stype == ST_CPLX64 ? (int)sizeof(c3) : (int)stype_bytes(stype); }
 
-static inline void tree_sizes(const TreeInst& T, TreeSizes& z) {
-  z.nodes[0] = 1;
-  z.total = 0;
-  for (int q = 0; q < T.steps; ++q) {
-    const double L = T.deg[q] + 1, Lc = T.deg[q + 1] + 1, W = tree_width(T.X, T.E, q + 1);
-    const double ne = tree_entries((int)W, T.diag), R = T.radix[q];
-    if (T.reps[q] == 1) {
-      z.one[q] = z.cost[q] = (ne * 2 + (T.pL >= 0)) * L * (L + 1) / 2;
-    } else {
-      z.one[q] = (ne * 2 + 4 * W + 45) * Lc * (Lc + 1) / 2;
-      z.cost[q] = R * z.one[q];
-    }
-    z.nodes[q + 1] = z.nodes[q] * R;
-    z.total += z.nodes[q] * z.cost[q];
-  }
-  const double L = T.deg[T.steps] + 1;
-  z.cost[T.steps] = (T.pB >= 0 ? 12.0 * T.nout : 4.0) * L * (L + 1) / 2;
-  z.total += z.nodes[T.steps] * z.cost[T.steps];
-}
-
-// elements of a node, and of the scratch of step q (np parents, nd children each)
+// elements of a node, and of the scratch of step q (np parents)
 static inline long long tree_node_elems(const TreeInst& T, int q) {
   return (long long)tree_entries(tree_width(T.X, T.E, q), T.diag) * (T.deg[q] + 1);
 }
-static inline long long tree_scratch_elems(const TreeInst& T, int q, long long np, int nd) {
+static inline long long tree_scratch_elems(const TreeInst& T, int q, long long np) {
   if (q == T.steps) return T.pO >= 0 && T.steps < T.E ? np * (T.deg[q] + 1) : 0;
   if (T.reps[q] == 1) return T.pL >= 0 ? np * (T.deg[q] + 1) : 0;
-  return np * nd * (T.deg[q + 1] + 1) * (6 + 2ll * tree_width(T.X, T.E, q + 1));
+  return np * T.radix[q] * (T.deg[q + 1] + 1) * (6 + 2ll * tree_width(T.X, T.E, q + 1));
 }
 
-// CTA kernel: elements of the two node buffers and the scratch when q edges are on the path
-static inline void tree_cta_elems(const TreeInst& T, int q, long long out[3]) {
-  out[0] = out[1] = out[2] = 0;
-  long long np = 1;
-  for (int s = 0; s <= T.steps; ++s) {
-    out[s & 1] = std::max(out[s & 1], np * tree_node_elems(T, s));
-    const int nd = s < T.steps ? (s < q ? 1 : T.radix[s]) : 1;
-    out[2] = std::max(out[2], tree_scratch_elems(T, s, np, nd));
-    if (s < T.steps) np *= nd;
-  }
-}
-
-// Grid mode: one buffer per level, as many nodes as the level has or its byte budget allows (the
-// levels below are then walked in blocks of parents, depth first), and the scratch of a step.
-struct TreeGridPlan {
+// Levels of one instance in the workspace: one buffer per level, as many nodes as the level has or a
+// byte budget allows (the levels below are then walked in blocks of parents, depth first).
+struct TreeLevels {
   long long cap[MAX_EDGES + 2] = {0};    // nodes of level q's buffer
   long long chunk[MAX_EDGES + 2] = {0};  // parents of step q per block
   long long off[MAX_EDGES + 2] = {0};    // byte offsets
   long long scr_off = 0, bytes = 0;
-  long long launches = 0, leaves = 0;    // of one execution
+  double phases = 0;                     // about, of one execution
 };
 
-template <class F>
-static void tree_walk(const TreeInst& T, const TreeGridPlan& g, int q, int np, F& launch) {
-  if (q == T.steps) {
-    if (T.pO >= 0 && T.steps < T.E) launch(TP_M, q, 0, np, np, 0, 0);
-    launch(TP_LEAF, q, 0, np, np, 0, 0);
-    return;
-  }
-  const int R = T.radix[q], blocks = (int)((np + g.chunk[q] - 1) / g.chunk[q]), per = (np + blocks - 1) / blocks;
-  for (int p0 = 0; p0 < np; p0 += per) {
-    const int c = std::min(per, np - p0);
-    if (T.reps[q] == 1) {
-      if (T.pL >= 0) launch(TP_M, q, p0, c, np, 0, R);
-      launch(TP_UNIT, q, p0, c, np, 0, R);
-    } else {
-      launch(TP_PREP, q, p0, c, np, 0, R);
-      if (tree_width(T.X, T.E, q + 1) > 0) {
-        launch(TP_Y, q, p0, c, np, 0, R);
-        launch(TP_MULTI, q, p0, c, np, 0, R);
-        if (T.pL >= 0) launch(TP_GLOOP, q, p0, c, np, 0, R);
-      }
-    }
-    tree_walk(T, g, q + 1, c * R, launch);
-  }
-}
-
-static inline void tree_grid_plan(const TreeInst& T, int sb, double budget, TreeGridPlan& g) {
-  double nodes = 1;
+static inline void tree_levels(const TreeInst& T, int sb, double budget, TreeLevels& g) {
+  double nodes = 1, walks = 1;
   long long off = 0, scr = 0;
   auto al = [](long long x) { return (x + 255) & ~255ll; };
+  g.phases = 1;
   for (int q = 0; q <= T.steps; ++q) {
     const long long nb = tree_node_elems(T, q) * sb;
     const int R = q ? T.radix[q - 1] : 1;
     long long cap = std::max<long long>((long long)(budget / (double)nb), std::max(R, 64));
     if (q) {  // a block's children and its scratch
-      const long long se = std::max<long long>(tree_scratch_elems(T, q - 1, 1, R) * sb, 1);
-      g.chunk[q - 1] = std::min(std::max<long long>(cap / R, 1), std::max<long long>((long long)(budget / (double)se), 1));
-      g.chunk[q - 1] = std::min(g.chunk[q - 1], g.cap[q - 1]);
-      cap = g.chunk[q - 1] * R;
-      scr = std::max(scr, tree_scratch_elems(T, q - 1, g.chunk[q - 1], R) * sb);
+      const long long se = std::max<long long>(tree_scratch_elems(T, q - 1, 1) * sb, 1);
+      long long c = std::min(std::max<long long>(cap / R, 1), std::max<long long>((long long)(budget / (double)se), 1));
+      c = std::min(c, g.cap[q - 1]);
+      g.chunk[q - 1] = c;
+      cap = c * R;
+      scr = std::max(scr, tree_scratch_elems(T, q - 1, c) * sb);
+      walks *= (double)((g.cap[q - 1] + c - 1) / c);
+      g.phases += walks * (T.reps[q - 1] == 1 ? (T.pL >= 0 ? 2 : 1) : 4);
     }
     if (nodes < (double)cap) cap = (long long)nodes;
     g.cap[q] = cap;
@@ -179,46 +122,191 @@ static inline void tree_grid_plan(const TreeInst& T, int sb, double budget, Tree
     off += al(cap * nb);
     if (q < T.steps) nodes *= T.radix[q];
   }
-  scr = std::max(scr, tree_scratch_elems(T, T.steps, g.cap[T.steps], 1) * sb);
+  g.phases += walks * (T.pO >= 0 ? 2 : 1);
+  scr = std::max(scr, tree_scratch_elems(T, T.steps, g.cap[T.steps]) * sb);
   g.scr_off = off;
   g.bytes = off + al(std::max<long long>(scr, 16));
-  g.launches = 1;  // the root
-  g.leaves = 0;
-  auto count = [&](int phase, int, int, int, int, int, int) {
-    ++g.launches;
-    g.leaves += phase == TP_LEAF;
-  };
-  tree_walk(T, g, 0, 1, count);
 }
 
-// shared memory of the leaf and of the block sums
-static inline int tree_smem(const TreeInst& T, int sb) {
-  const int nw = TREE_THREADS / 32;
-  return nw * (T.pB >= 0 ? 5 * (T.deg[T.steps] + 1) + 32 : 1) * sb;
+// A loop kind's simple edge needs m = C_ij + v_i v_j as a series first (TP_M); a level of so few
+// coefficients that four threads each do not fill `threads` sums it inside the step instead.
+static inline bool tree_fused(const TreeInst& T, int q, double np, double threads) {
+  return 4.0 * np * (T.deg[q] + 1) * tree_entries(tree_width(T.X, T.E, q + 1), T.diag) <= threads;
 }
 
-// Where the path of a CTA's task ends: the split that minimises the whole work, each path
-// recomputed by every task below it, over the chip's SMs plus one task's time as the tail
-// (weighted by the instance's share of the launch's work).  Returns that time in multiply-adds
-// of one SM; the workspace bound keeps a subtree's widest levels within max_elems.
-static inline double tree_split(const TreeInst& T, const TreeSizes& z, int sms, double share, long long max_elems,
-                                int& q_best) {
-  double best = -1, path = 0;
-  q_best = 0;
-  for (int q = 0; q <= T.steps; ++q) {
-    double sub = 0;
-    for (int s = q; s <= T.steps; ++s) sub += z.nodes[s] / z.nodes[q] * z.cost[s];
-    const double tasks = z.nodes[q], task = path + sub, f = tasks * task / sms + share * task;
-    long long el[3];
-    tree_cta_elems(T, q, el);
-    const bool fits = el[0] + el[1] + el[2] <= max_elems && tasks <= 65536.0;
-    if (fits && (best < 0 || f < best)) {
-      best = f;
-      q_best = q;
-    }
-    if (q < T.steps) path += z.one[q];
+// the phases of an instance in order, each once for every block: f(phase, q, p0, np, level's nodes)
+template <class F>
+static void tree_walk(const TreeInst& T, const TreeLevels& g, int q, int np, double threads, F& f) {
+  if (q == T.steps) {
+    if (T.pO >= 0 && T.steps < T.E) f(TP_M, q, 0, np, np);
+    f(TP_LEAF, q, 0, np, np);
+    return;
   }
-  return best;
+  const int R = T.radix[q], blocks = (int)((np + g.chunk[q] - 1) / g.chunk[q]), per = (np + blocks - 1) / blocks;
+  for (int p0 = 0; p0 < np; p0 += per) {
+    const int c = std::min(per, np - p0);
+    if (T.reps[q] == 1) {
+      if (T.pL >= 0 && !tree_fused(T, q, c, threads)) f(TP_M, q, p0, c, np);
+      f(TP_UNIT, q, p0, c, np);
+    } else {
+      f(TP_PREP, q, p0, c, np);
+      if (tree_width(T.X, T.E, q + 1) > 0) {
+        f(TP_Y, q, p0, c, np);
+        f(TP_MULTI, q, p0, c, np);
+        if (T.pL >= 0) f(TP_GLOOP, q, p0, c, np);
+      }
+    }
+    tree_walk(T, g, q + 1, c * R, threads, f);
+  }
+}
+
+// threads of a phase with `tile` coefficients a thread (0: four threads a coefficient), and its
+// multiply-adds
+static inline double tree_items(const TreeInst& T, int phase, int q, double np, int tile) {
+  if (tile == 0) {
+    const bool whole = phase == TP_ROOT || phase == TP_FIRST || phase == TP_PREP || phase == TP_GLOOP ||
+                       (phase == TP_LEAF && (T.pB >= 0 || T.steps == T.E));
+    return tree_items(T, phase, q, np, 1) * (whole ? 1 : 4);
+  }
+  const int Lp = T.deg[q] + 1, Lc = q < T.steps ? T.deg[q + 1] + 1 : Lp, W = tree_width(T.X, T.E, q + 1);
+  const double nc = q < T.steps ? np * T.radix[q] : np;
+  switch (phase) {
+    case TP_ROOT: return tree_entries(tree_width(T.X, T.E, 0), T.diag);
+    case TP_FIRST: return tree_entries(W, T.diag);
+    case TP_M: return np * tree_tiles(Lp, tile);
+    case TP_UNIT: return np * tree_tiles(Lp, tile) * tree_entries(W, T.diag);
+    case TP_PREP: case TP_GLOOP: return 32 * nc;
+    case TP_Y: return nc * 2 * W * tree_tiles(Lc, tile);
+    case TP_MULTI: return nc * (tree_entries(W, T.diag) - 1) * tree_tiles(Lc, tile);
+    default: return T.pB >= 0 ? 32 * np : np * (T.steps < T.E ? tree_tiles(Lp, tile) : 1);
+  }
+}
+static inline double tree_macs(const TreeInst& T, int phase, int q, double np) {
+  const double Lp = T.deg[q] + 1, Lc = q < T.steps ? T.deg[q + 1] + 1 : Lp, W = tree_width(T.X, T.E, q + 1);
+  const double nc = q < T.steps ? np * T.radix[q] : np, tp = Lp * (Lp + 1) / 2, tc = Lc * (Lc + 1) / 2;
+  switch (phase) {
+    case TP_ROOT: return 0;
+    case TP_FIRST: return 2 * tree_entries((int)W, T.diag);
+    case TP_M: return np * tp;
+    case TP_UNIT: return np * tp * (2 * tree_entries((int)W, T.diag) - 1);
+    case TP_PREP: return nc * 12 * tc * std::max(1.0, 32 / Lc);
+    case TP_GLOOP: return nc * 5 * tc * std::max(1.0, 32 / Lc);
+    case TP_Y: return nc * 4 * W * tc;
+    case TP_MULTI: return nc * 2 * (tree_entries((int)W, T.diag) - 1) * tc;
+    default: return np * (T.pB >= 0 ? 3.0 * T.nout : 3.0) * tp;
+  }
+}
+
+// elements of a warp's shared memory: the output sums, a batch's work series (with copies of two of
+// the node's), a multiple edge's; `most` when those would take too much (the phases then work in L2,
+// a batch without the copies)
+static inline int tree_smem(const TreeInst& T, int most) {
+  const int L = T.deg[T.steps] + 1;
+  int need = 1, lc = 0;
+  for (int q = 0; q < T.steps; ++q)
+    if (T.reps[q] > 1) lc = std::max(lc, T.deg[q + 1] + 1);
+  if (9 * lc <= most) need = std::max(need, 9 * lc);
+  if (T.pB >= 0) need = std::max(need, 7 * L + 32 <= most ? 7 * L + 32 : 5 * L + 32);
+  return need;
+}
+
+// The program of one launch over `insts` (their levels placed one after another in the workspace):
+// round r holds phase r of every instance, so that the narrow levels of one run beside others'.
+// `nparts` advances by the leaves' partial slots; part_base[i] and part_count[i] are instance i's.
+struct TreeProgram {
+  std::vector<TreeInst> insts;
+  std::vector<TreeRound> rounds;
+  std::vector<TreeSeg> segs;
+  long long ws_bytes = 0;
+  int smem = 1;  // elements of a warp's shared memory
+  double macs = 0;
+};
+
+static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<TreeLevels>& levels, int sb, int tile,
+                                int chip_threads, int& nparts, std::vector<int>& part_base,
+                                std::vector<int>& part_count, TreeProgram& P) {
+  std::vector<std::vector<TreeSeg>> rounds;
+  part_base.assign(insts.size(), 0);
+  part_count.assign(insts.size(), 0);
+  for (size_t k = 0; k < insts.size(); ++k) {
+    TreeInst& T = insts[k];
+    const TreeLevels& g = levels[k];
+    T.scr_off = P.ws_bytes + g.scr_off;
+    P.smem = std::max(P.smem, tree_smem(T, (64 << 10) / (TREE_THREADS / 32) / sb));
+    const double fuse_threads = chip_threads / (double)insts.size();
+    size_t r = 0;
+    auto add = [&](int phase, int q, int p0, int np, int ps) {
+      TreeSeg s;
+      memset(&s, 0, sizeof(s));
+      s.par = P.ws_bytes + g.off[q];
+      s.chi = phase == TP_ROOT ? s.par : P.ws_bytes + g.off[std::min(q + 1, T.steps)];
+      s.inst = (int)k;
+      s.np = np;
+      s.p0 = p0;
+      s.pstride = ps;
+      s.phase = (unsigned char)phase;
+      s.q = (unsigned char)q;
+      s.fused = phase == TP_UNIT && T.pL >= 0 && tree_fused(T, q, np, fuse_threads);
+      if (rounds.size() <= r) rounds.emplace_back();
+      rounds[r++].push_back(s);
+      P.macs += tree_macs(T, phase, q, np);
+    };
+    if (T.steps > 0 && T.reps[0] == 1) {
+      add(TP_FIRST, 0, 0, 1, 1);
+      tree_walk(T, g, 1, 1, fuse_threads, add);
+    } else {
+      add(TP_ROOT, 0, 0, 1, 1);
+      tree_walk(T, g, 0, 1, fuse_threads, add);
+    }
+    P.ws_bytes += g.bytes;
+  }
+  // partial slots instance by instance, so that an instance's are contiguous
+  for (auto& R : rounds) {
+    // whole tiles when those fill the chip, else one coefficient a thread, else four threads each
+    double whole = 0, split = 0;
+    for (const TreeSeg& s : R) {
+      whole += tree_items(insts[s.inst], s.phase, s.q, s.np, tile);
+      split += tree_items(insts[s.inst], s.phase, s.q, s.np, 0);
+    }
+    const int use = whole >= chip_threads ? tile : (split > chip_threads ? 1 : 0);
+    TreeRound rr;
+    memset(&rr, 0, sizeof(rr));
+    rr.seg0 = (int)P.segs.size();
+    rr.nseg = (int)R.size();
+    // the costly segments' warps first
+    std::stable_sort(R.begin(), R.end(), [&](const TreeSeg& a, const TreeSeg& b) {
+      return tree_macs(insts[a.inst], a.phase, a.q, a.np) > tree_macs(insts[b.inst], b.phase, b.q, b.np);
+    });
+    for (TreeSeg& s : R) {
+      const TreeInst& T = insts[s.inst];
+      s.tile = (unsigned char)(s.fused ? 0 : use);
+      long long warps = (long long)((tree_items(T, s.phase, s.q, s.np, s.tile) + 31) / 32);
+      // leaves: at most the chip's warps, each with a partial for the reduction; the CTAs of a
+      // single instance keep their sums over all leaf rounds and leave one partial each
+      if (s.phase == TP_LEAF) {
+        warps = std::max<long long>(std::min<long long>(warps, chip_threads / 32), 1);
+        s.part = insts.size() > 1 ? part_count[s.inst] : 0;
+        part_count[s.inst] = insts.size() > 1 ? part_count[s.inst] + (int)warps : chip_threads / TREE_THREADS;
+      }
+      s.warp0 = rr.nwarps;
+      rr.nwarps += (int)std::max<long long>(warps, 1);
+      P.segs.push_back(s);
+    }
+    P.rounds.push_back(rr);
+  }
+  for (size_t k = 0; k < insts.size(); ++k) {
+    part_base[k] = nparts;
+    nparts += part_count[k] * insts[k].pstride;
+  }
+  for (TreeSeg& s : P.segs)
+    if (s.phase == TP_LEAF) s.part = part_base[s.inst] + s.part * insts[s.inst].pstride;
+  P.insts = insts;
+}
+
+// one CTA's time for a program, in SM clocks: its multiply-adds and a barrier with its latencies a round
+static inline double tree_one_cta(const TreeProgram& P, double clk) { return 1.5 * P.macs * clk + 2500.0 * P.rounds.size(); }
+static inline double tree_whole_chip(const TreeProgram& P, double clk, int sms) {
+  return P.macs * clk / sms + 8000.0 * P.rounds.size();
 }
 
 }  // namespace wg

@@ -39,27 +39,34 @@ namespace wg {
 
 constexpr int TREE_MAX_K = 63;
 constexpr int TREE_MAX_POS = 3 + 2 * MAX_EDGES;
-constexpr int TREE_THREADS = 256;
+constexpr int TREE_THREADS = 512;  // one CTA per SM
 
 // The node functions also compile for the host, one thread as a warp of one lane: a CPU check runs
 // them over a checked scalar type (tests/tree_check.cu).
 #ifdef __CUDA_ARCH__
 #define WG_TREE_LANES 32
+#define WG_TREE_SPLIT 4
 #define WG_TREE_SYNCWARP() __syncwarp()
 #else
 #define WG_TREE_LANES 1
+#define WG_TREE_SPLIT 1
 #define WG_TREE_SYNCWARP() ((void)0)
 #endif
 
-// coefficients a thread forms in registers
+// Coefficients a thread forms in registers (TL below): more of them share a load, but a level with
+// fewer tiles than threads leaves the chip idle, so narrower levels take one coefficient a thread and
+// the narrowest four threads a coefficient (TL = 0), whose chain of loads and FP64 instructions is the
+// level's time.
 template <class S>
-constexpr int tree_tile() { return Ar<S>::dd && Ar<S>::cplx ? 2 : 4; }
+__host__ __device__ constexpr int tree_tile() { return Ar<S>::dd && Ar<S>::cplx ? 2 : 3; }
+__host__ __device__ __forceinline__ int tree_tiles(int L, int TL) { return (L + TL - 1) / TL; }
 
 // One instance's tree.  Positions 0 .. X-1 are the rows that are never eliminated (pL: the loop
 // weights, pO: an unpaired vertex, pB: the batch mode), then the edges' vertices, the last edge
 // first: step q eliminates positions X + 2 (E-1-q) and the next, the highest two left.
-struct TreeInst {
+struct alignas(16) TreeInst {
   long long a_off;           // byte offset of the extended matrix in the pool
+  long long scr_off;         // of the instance's scratch in the workspace
   int lda;
   int E, K, X;
   int pL, pO, pB;            // -1: none
@@ -67,35 +74,60 @@ struct TreeInst {
   int dpos;                  // diagonal entries of positions >= dpos are kept (pending multiple edges)
   int steps;                 // edges eliminated by steps: E, E - 1 or E - 2 (tree_leaf's closed forms)
   int nout;
-  int part_base, pstride, comp_off;  // partial slots of a task or leaf block (as InstDev's)
-  int q;                     // CTA kernel: edges whose sign a task fixes
-  int tasks, task_base;      // CTA kernel
+  int pstride, comp_off;     // partial slots of a leaf warp (as InstDev's)
   c64 oddloop;               // entry (pO, pL) when the unpaired vertex is not a vertex of A
   short row[TREE_MAX_POS], col[TREE_MAX_POS];  // position -> row and column of the extended matrix
   unsigned char reps[MAX_EDGES], radix[MAX_EDGES];
   unsigned char deg[MAX_EDGES + 4];  // degree of the series after q steps
 };
 
-struct TreeParams {
-  const TreeInst* inst;
-  int ninst, ntasks;
-  const unsigned char* pool;
-  unsigned char* ws;         // CTA kernel: per-CTA workspace
-  long long ws_stride;
-  long long off_b, off_s;    // second node buffer, scratch
-  double2* partials;
-  unsigned int* counter;
+// The program of a launch: rounds of segments, with a barrier of the whole launch after each round.
+// A segment is one phase of one step of one instance over a block of parents [p0, p0 + np) of a
+// level of pstride nodes, by the round's warps [warp0, next segment's warp0).
+enum TreePhase : int { TP_ROOT = 0, TP_FIRST, TP_M, TP_UNIT, TP_PREP, TP_Y, TP_MULTI, TP_GLOOP, TP_LEAF };
+struct alignas(16) TreeSeg {
+  long long par, chi;        // workspace byte offsets of the parents' and the children's level
+  int inst, warp0;
+  int np, p0, pstride;
+  int part;                  // leaf: the first warp's partial slot (one instance: the first CTA's)
+  unsigned char phase, q, tile;  // tile: coefficients a thread, 0: four threads a coefficient
+  unsigned char fused;       // TP_UNIT without a TP_M before it
+  unsigned char pad[4];
+};
+struct alignas(16) TreeRound {
+  int seg0, nseg, nwarps, pad;
 };
 
-// grid mode: one launch per phase of a step
-enum TreePhase : int { TP_ROOT = 0, TP_M, TP_UNIT, TP_PREP, TP_Y, TP_MULTI, TP_GLOOP, TP_LEAF };
-struct TreeGrid {
-  TreeParams P;
-  int inst, phase, q;
-  int np, p0, pstride;       // parents [p0, p0 + np) of a buffer of pstride nodes
-  int d0, nd;                // digits d0 .. d0 + nd - 1
-  long long part;            // leaf: first partial slot of the launch
-  unsigned char *par, *chi, *scr;
+static_assert(sizeof(TreeInst) % 16 == 0 && sizeof(TreeSeg) % 16 == 0 && sizeof(TreeRound) % 16 == 0,
+              "programs are copied in 16-byte words");
+
+// the final reduction's arguments, when a plan's only launch does it (done != nullptr)
+struct TreeFinish {
+  const InstDev* inst;
+  const double2* partials;
+  const double* scales;
+  double2* out;
+  double* mags;
+  int* err;
+  unsigned int *done, *counters;
+  int ninst, total_out, ncounters, wpo;  // wpo: warps per output
+  unsigned int modp;
+};
+
+struct TreeParams {
+  const TreeInst* inst;
+  const TreeRound* rounds;
+  const TreeSeg* segs;
+  int ninst, nrounds, nsegs;
+  int cached;                // instances, rounds and segments are copied to shared memory first
+  int sm_warp, sm_cache;     // shared memory: elements of a warp's work, byte offset of the cache
+  int sm_ws;                 // shared memory: offset of the workspace (one CTA; 0: ws)
+  const unsigned char* pool;
+  unsigned char* ws;
+  double2* partials;
+  unsigned int* bar;
+  int* err;
+  TreeFinish fin;
 };
 
 __host__ __device__ __forceinline__ int tree_width(int X, int E, int q) { return X + 2 * (E - q); }
@@ -118,20 +150,93 @@ __host__ __device__ __forceinline__ void tree_decode(int e, int diag, int& a, in
   b = x - r * (r + 1) / 2;
 }
 
-// one scalar in one access: the buffers are 16-byte aligned
+// Node scalars: complex FP64 nodes carry re + im beside the parts (c3), so that a product of series
+// takes three real products a term instead of four (re = P1 - P2, im = P3 - P1 - P2 with P1 = sum
+// re re, P2 = sum im im, P3 = sum (re + im)(re + im)); its rounding is relative to |a| |b|, as
+// the four products' is.  Complex n = 40: 5,836 -> 5,405 us, n = 36: 1,212 -> 1,147 us.
+struct c3 {
+  double re, im, s;
+};
+template <>
+struct Ar<c3> {
+  using S = c3;
+  using Comp = double;
+  static constexpr int NC = 2;
+  static constexpr bool cplx = true, fp64 = true, modular = false, dd = false;
+  __device__ static __forceinline__ S of(double re, double im) { return {re, im, re + im}; }
+  __device__ static __forceinline__ S zero() { return {0.0, 0.0, 0.0}; }
+  __device__ static __forceinline__ S one() { return {1.0, 0.0, 1.0}; }
+  __device__ static __forceinline__ S add(S a, S b) { return of(a.re + b.re, a.im + b.im); }
+  __device__ static __forceinline__ S sub(S a, S b) { return of(a.re - b.re, a.im - b.im); }
+  __device__ static __forceinline__ S neg(S a) { return {neg_d(a.re), neg_d(a.im), neg_d(a.s)}; }
+  __device__ static __forceinline__ S mul(S a, S b) {
+    const c64 z = Ar<c64>::mul({a.re, a.im}, {b.re, b.im});
+    return of(z.re, z.im);
+  }
+  __device__ static __forceinline__ S fma(S a, S b, S c) {
+    const c64 z = Ar<c64>::fma({a.re, a.im}, {b.re, b.im}, {c.re, c.im});
+    return of(z.re, z.im);
+  }
+  __device__ static __forceinline__ S scale(S a, double s) { return of(a.re * s, a.im * s); }
+  __device__ static __forceinline__ S scale_f(S a, float s) { return scale(a, (double)s); }
+  __device__ static __forceinline__ S from_c64(c64 v) { return of(v.re, v.im); }
+  __device__ static __forceinline__ c64 to_c64(S a) { return {a.re, a.im}; }
+  __device__ static __forceinline__ Comp comp(const S& a, int i) { return i ? a.im : a.re; }
+  __device__ static __forceinline__ void set_comp(S& a, int i, Comp v) {
+    if (i) a.im = v; else a.re = v;
+    a.s = a.re + a.im;
+  }
+  __device__ static __forceinline__ Comp cadd(Comp a, Comp b) { return a + b; }
+  __device__ static __forceinline__ Comp shfl_xor(Comp v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
+};
+// the node scalar of a matrix scalar, and back
+template <class M>
+struct TreeScalar {
+  using T = M;
+};
+template <>
+struct TreeScalar<c64> {
+  using T = c3;
+};
+template <class S>
+struct TreeMatrix {
+  using T = S;
+  __host__ __device__ static __forceinline__ S load(const S* p) { return *p; }
+};
+template <>
+struct TreeMatrix<c3> {
+  using T = c64;
+  __device__ static __forceinline__ c3 load(const c64* p) { return Ar<c3>::of(p->re, p->im); }
+};
+
+// the running sum of a series product
+template <class S>
+struct ConvAcc {
+  S v;
 #pragma nv_exec_check_disable
+  __host__ __device__ static __forceinline__ ConvAcc of(S x) { return {x}; }
+#pragma nv_exec_check_disable
+  __host__ __device__ __forceinline__ void fma(S a, S b) { v = Ar<S>::fma(a, b, v); }
+#pragma nv_exec_check_disable
+  __host__ __device__ __forceinline__ S sum() const { return v; }
+};
+template <>
+struct ConvAcc<c3> {
+  double p1, p2, p3;
+  __device__ static __forceinline__ ConvAcc of(c3 x) { return {x.re, 0.0, x.s}; }
+  __device__ __forceinline__ void fma(c3 a, c3 b) {
+    p1 = ::fma(a.re, b.re, p1);
+    p2 = ::fma(a.im, b.im, p2);
+    p3 = ::fma(a.s, b.s, p3);
+  }
+  __device__ __forceinline__ c3 sum() const { return Ar<c3>::of(p1 - p2, p3 - p1 - p2); }
+};
+
+// loads and stores of node elements (the host check counts them)
 template <class S>
 __host__ __device__ __forceinline__ S tld(const S* p) { return *p; }
-template <>
-__host__ __device__ __forceinline__ c64 tld<c64>(const c64* p) {
-  const double2 v = *reinterpret_cast<const double2*>(p);
-  return {v.x, v.y};
-}
-#pragma nv_exec_check_disable
 template <class S>
 __host__ __device__ __forceinline__ void tst(S* p, S v) { *p = v; }
-template <>
-__host__ __device__ __forceinline__ void tst<c64>(c64* p, c64 v) { *reinterpret_cast<double2*>(p) = make_double2(v.re, v.im); }
 
 // acc[k] += sum_s a_s b_(t0+k-s), k < T, s < la: coefficients t0 .. t0+T-1 of a product of two
 // series (element stride sa, sb).  A window of T coefficients of b slides through registers, so a
@@ -139,43 +244,42 @@ __host__ __device__ __forceinline__ void tst<c64>(c64* p, c64 v) { *reinterpret_
 // runs out.  t0 < 0: only the coefficients t0 + k >= 0.
 #pragma nv_exec_check_disable
 template <class S, int T>
-__host__ __device__ __forceinline__ void conv_tile(S (&acc)[T], const S* a, long long sa, int la, const S* b,
+__host__ __device__ __forceinline__ void conv_tile(ConvAcc<S> (&acc)[T], const S* a, long long sa, int la, const S* b,
                                           long long sb, int t0) {
-  using A = Ar<S>;
   if (t0 < 0) {
 #pragma unroll
     for (int k = 1; k < T; ++k) {
       const int t = t0 + k;
       if (t >= 0)
-        for (int s = 0; s <= t && s < la; ++s) acc[k] = A::fma(tld(a + s * sa), tld(b + (t - s) * sb), acc[k]);
+        for (int s = 0; s <= t && s < la; ++s) acc[k].fma(tld(a + s * sa), tld(b + (t - s) * sb));
     }
     return;
   }
   S w[T];
 #pragma unroll
   for (int k = 0; k < T; ++k) w[k] = tld(b + (t0 + k) * sb);
-  const int sm = t0 < la - 1 ? t0 : la - 1;
+  const int n = t0 < la ? t0 : la;  // steps that slide the window
   const S* pa = a;
   const S* pb = b + (t0 - 1) * sb;
 #pragma unroll 4
-  for (int s = 0; s <= sm; ++s) {
-    const S x = tld(pa);
+  for (int s = 0; s < n; ++s) {
+    const S x = tld(pa), y = tld(pb);
     pa += sa;
+    pb -= sb;
 #pragma unroll
-    for (int k = 0; k < T; ++k) acc[k] = A::fma(x, w[k], acc[k]);
+    for (int k = 0; k < T; ++k) acc[k].fma(x, w[k]);
 #pragma unroll
     for (int k = T - 1; k > 0; --k) w[k] = w[k - 1];
-    if (s < t0) w[0] = tld(pb);
-    pb -= sb;
+    w[0] = y;
   }
-  // s = t0 + kk: w[k] = b_(k-1) here
+  // s = t0 + kk: w[k] = b_k here
 #pragma unroll
-  for (int kk = 1; kk < T; ++kk) {
+  for (int kk = 0; kk < T; ++kk) {
     if (t0 + kk < la) {
       const S x = tld(pa);
       pa += sa;
 #pragma unroll
-      for (int k = kk; k < T; ++k) acc[k] = A::fma(x, w[k - kk + 1], acc[k]);
+      for (int k = kk; k < T; ++k) acc[k].fma(x, w[k - kk]);
     }
   }
 }
@@ -211,111 +315,241 @@ __host__ __device__ __forceinline__ S tree_times(S x, int k) {
 template <class S>
 __host__ __device__ __forceinline__ S conv_one(const S* a, long long sa, int la, const S* b, long long sb, int lb, int t) {
   using A = Ar<S>;
-  S r = A::zero();
+  ConvAcc<S> r = ConvAcc<S>::of(Ar<S>::zero());
   const int s0 = t - lb + 1 > 0 ? t - lb + 1 : 0;
-  for (int s = s0; s <= t && s < la; ++s) r = A::fma(tld(a + s * sa), tld(b + (t - s) * sb), r);
-  return r;
+  const int n = t < la - 1 ? t : la - 1;
+#pragma unroll 4
+  for (int s = s0; s <= n; ++s) r.fma(tld(a + s * sa), tld(b + (t - s) * sb));
+  return r.sum();
+}
+
+// the terms s = sub, sub + WG_TREE_SPLIT, ... of coefficient t of a product
+#pragma nv_exec_check_disable
+template <class S>
+__host__ __device__ __forceinline__ void conv_part(ConvAcc<S>& acc, const S* a, long long sa, int la, const S* b, long long sb,
+                                                   int t, int sub) {
+  const int n = t < la - 1 ? t : la - 1;
+#pragma unroll 4
+  for (int s = sub; s <= n; s += WG_TREE_SPLIT) acc.fma(tld(a + s * sa), tld(b + (t - s) * sb));
+}
+// the same of two products at once: their loads overlap
+#pragma nv_exec_check_disable
+template <class S>
+__host__ __device__ __forceinline__ void conv_part2(ConvAcc<S>& acc, const S* a, const S* b, const S* c, const S* d, long long sa,
+                                                    int la, long long sb, int t, int sub) {
+  const int n = t < la - 1 ? t : la - 1;
+#pragma unroll 2
+  for (int s = sub; s <= n; s += WG_TREE_SPLIT) {
+    const S x = tld(a + s * sa), y = tld(b + (t - s) * sb), z = tld(c + s * sa), w = tld(d + (t - s) * sb);
+    acc.fma(x, y);
+    acc.fma(z, w);
+  }
+}
+// the sum over the four threads of a coefficient, in each of them
+#pragma nv_exec_check_disable
+template <class S>
+__host__ __device__ __forceinline__ S split_sum(S v) {
+#ifdef __CUDA_ARCH__
+  using A = Ar<S>;
+#pragma unroll
+  for (int off = 1; off < WG_TREE_SPLIT; off *= 2) {
+#pragma unroll
+    for (int c = 0; c < A::NC; ++c) {
+      const typename A::Comp x = A::comp(v, c);
+      A::set_comp(v, c, A::cadd(x, A::shfl_xor(x, off)));
+    }
+  }
+#endif
+  return v;
 }
 
 __host__ __device__ __forceinline__ bool tree_need(const TreeInst& T, int a, int b) {
   return a != b || a == T.pB || a >= T.dpos;
 }
 
+// entry (a, b) of the root: the mean of the matrix's two triangles (equal to either when they
+// agree); the unpaired vertex of an odd loop hafnian has a row only, and its loop weight apart
+#pragma nv_exec_check_disable
+template <class S>
+__host__ __device__ __forceinline__ S tree_root_entry(const TreeInst& T, const typename TreeMatrix<S>::T* ext, int a,
+                                                           int b) {
+  using A = Ar<S>;
+  using M = TreeMatrix<S>;
+  const int ca = T.col[a], cb = T.col[b];
+  if (ca < 0 || cb < 0) {
+    const int o = ca < 0 ? a : b, x = ca < 0 ? b : a;
+    return x == o ? A::zero() : (x == T.pL ? A::from_c64(T.oddloop) : M::load(ext + (size_t)T.row[o] * T.lda + T.col[x]));
+  }
+  const S x = M::load(ext + (size_t)T.row[a] * T.lda + cb), y = M::load(ext + (size_t)T.row[b] * T.lda + ca);
+  return A::add(x, tree_half(A::sub(y, x)));
+}
+
 // ---- root: one node, one coefficient per entry
 #pragma nv_exec_check_disable
 template <class S>
-__host__ __device__ void tree_root(const TreeInst& T, const unsigned char* __restrict__ pool, S* out, int tid,
-                          int nthr) {
-  using A = Ar<S>;
-  const S* __restrict__ ext = reinterpret_cast<const S*>(pool + T.a_off);
-  const int W = tree_width(T.X, T.E, 0), ne = tree_entries(W, T.diag);
+__host__ __device__ void tree_root(const TreeInst& T, const unsigned char* __restrict__ pool, S* out, int tid, int nthr) {
+  using M = typename TreeMatrix<S>::T;
+  const M* __restrict__ ext = reinterpret_cast<const M*>(pool + T.a_off);
+  const int ne = tree_entries(tree_width(T.X, T.E, 0), T.diag);
   for (int e = tid; e < ne; e += nthr) {
-    S v = A::one();
-    if (e > 0) {
-      int a, b;
+    int a = 0, b = 0;
+    if (e) tree_decode(e, T.diag, a, b);
+    tst(out + e, e ? tree_root_entry<S>(T, ext, a, b) : Ar<S>::one());
+  }
+}
+
+// ---- the root and its simple edge in one: the +1 child, two coefficients an entry
+#pragma nv_exec_check_disable
+template <class S>
+__host__ __device__ void tree_first(const TreeInst& T, const unsigned char* __restrict__ pool, S* chi, int tid,
+                                    int nthr) {
+  using A = Ar<S>;
+  using M = typename TreeMatrix<S>::T;
+  const M* __restrict__ ext = reinterpret_cast<const M*>(pool + T.a_off);
+  const int i = T.X + 2 * (T.E - 1), j = i + 1, ne = tree_entries(i, T.diag);
+  for (int e = tid; e < ne; e += nthr) {
+    int a = 0, b = 0;
+    S c = A::one(), u;
+    if (e) {
       tree_decode(e, T.diag, a, b);
-      const int ca = T.col[a], cb = T.col[b];
-      if (ca < 0 || cb < 0) {  // the unpaired vertex has a row only, and its loop weight apart
-        const int o = ca < 0 ? a : b, x = ca < 0 ? b : a;
-        v = x == o ? A::zero() : (x == T.pL ? A::from_c64(T.oddloop) : ext[(size_t)T.row[o] * T.lda + T.col[x]]);
-      } else {
-        // the mean of the two triangles: equal to either when they agree
-        const S x = ext[(size_t)T.row[a] * T.lda + cb], y = ext[(size_t)T.row[b] * T.lda + ca];
-        v = A::add(x, tree_half(A::sub(y, x)));
-      }
+      if (!tree_need(T, a, b)) continue;
+      c = tree_root_entry<S>(T, ext, a, b);
+      u = A::fma(tree_root_entry<S>(T, ext, i, a), tree_root_entry<S>(T, ext, j, b),
+                 A::mul(tree_root_entry<S>(T, ext, j, a), tree_root_entry<S>(T, ext, i, b)));
+    } else {
+      u = tree_root_entry<S>(T, ext, j, i);
+      if (T.pL >= 0) u = A::fma(tree_root_entry<S>(T, ext, i, T.pL), tree_root_entry<S>(T, ext, j, T.pL), u);
     }
-    tst(out + e, v);
+    tst(chi + 2 * e, c);
+    tst(chi + 2 * e + 1, u);
   }
 }
 
 // ---- m = C_ij + v_i v_j of the edge of step q (loop kinds): scr[t np + p]
 #pragma nv_exec_check_disable
-template <class S>
+template <class S, int TL>
 __host__ __device__ void tree_m(const TreeInst& T, int q, const S* par, long long ps, int np, S* scr,
                        int tid, int nthr) {
   using A = Ar<S>;
-  constexpr int TL = tree_tile<S>();
   const int i = T.X + 2 * (T.E - 1 - q), j = i + 1;
-  const int Lp = T.deg[q] + 1, nt = (Lp + TL - 1) / TL;
+  const int Lp = T.deg[q] + 1;
+  if constexpr (TL == 0) {
+    const int total = Lp * np, sub = tid % WG_TREE_SPLIT, step = nthr / WG_TREE_SPLIT;
+    for (int x0 = 0; x0 < total; x0 += step) {
+      const int x = x0 + tid / WG_TREE_SPLIT, p = x % np, t = Lp - 1 - x / np;
+      const long long st = (long long)Lp * ps;
+      ConvAcc<S> acc = ConvAcc<S>::of(A::zero());
+      if (x < total)
+        conv_part(acc, par + tree_ent(i, T.pL, T.diag) * st + p, ps, Lp, par + tree_ent(j, T.pL, T.diag) * st + p, ps,
+                  t, sub);
+      const S v = split_sum(acc.sum());
+      if (x < total && sub == 0)
+        tst(scr + (long long)t * np + p, A::add(tld(par + tree_ent(j, i, T.diag) * st + t * ps + p), v));
+    }
+    return;
+  }
+  constexpr int TT = TL ? TL : 1;
+  const int nt = (Lp + TT - 1) / TT;
   for (int x = tid; x < nt * np; x += nthr) {
-    const int p = x % np, t0 = Lp - TL * (x / np + 1);
-    S acc[TL];
+    const int p = x % np, t0 = Lp - TT * (x / np + 1);
+    ConvAcc<S> acc[TT];
 #pragma unroll
-    for (int k = 0; k < TL; ++k)
-      acc[k] = t0 + k >= 0 ? tld(par + ((long long)tree_ent(j, i, T.diag) * Lp + t0 + k) * ps + p) : A::zero();
-    conv_tile<S, TL>(acc, par + (long long)tree_ent(i, T.pL, T.diag) * Lp * ps + p, ps, Lp,
+    for (int k = 0; k < TT; ++k)
+      acc[k] = ConvAcc<S>::of(
+          t0 + k >= 0 ? tld(par + ((long long)tree_ent(j, i, T.diag) * Lp + t0 + k) * ps + p) : A::zero());
+    conv_tile<S, TT>(acc, par + (long long)tree_ent(i, T.pL, T.diag) * Lp * ps + p, ps, Lp,
                      par + (long long)tree_ent(j, T.pL, T.diag) * Lp * ps + p, ps, t0);
 #pragma unroll
-    for (int k = 0; k < TL; ++k)
-      if (t0 + k >= 0) tst(scr + (long long)(t0 + k) * np + p, acc[k]);
+    for (int k = 0; k < TT; ++k)
+      if (t0 + k >= 0) tst(scr + (long long)(t0 + k) * np + p, acc[k].sum());
   }
 }
 
 // ---- a simple edge: children delta = +1 (nodes 0 .. np-1) and -1 (np .. 2 np - 1) from the same
-// products; digits d0 .. d0 + nd - 1 are made (0: +1, 1: -1).  The weight -1 of the second joins g.
+// products.  The weight -1 of the second joins g.
 #pragma nv_exec_check_disable
-template <class S>
+template <class S, int TL>
 __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long long ps, int np,
-                          const S* m, S* chi, int d0, int nd, int tid, int nthr) {
+                          const S* m, S* chi, int tid, int nthr) {
   using A = Ar<S>;
-  constexpr int TL = tree_tile<S>();
   const int i = T.X + 2 * (T.E - 1 - q), j = i + 1, dg = T.diag;
-  const int ne = tree_entries(i, dg), Lp = T.deg[q] + 1, Lc = Lp + 1, nt = (Lp + TL - 1) / TL;
+  const int ne = tree_entries(i, dg), Lp = T.deg[q] + 1, Lc = Lp + 1;
+  const int nd = T.radix[q];  // 1: the root, which takes +1 only
   const long long cs = (long long)np * nd;
+  if constexpr (TL == 0) {
+    const unsigned total = (unsigned)Lp * ne * np, step = nthr / WG_TREE_SPLIT;
+    const int sub = tid % WG_TREE_SPLIT;
+    for (unsigned x0 = 0; x0 < total; x0 += step) {
+      const unsigned x = x0 + tid / WG_TREE_SPLIT, r = x / np;
+      const int p = x - r * np, e = r % ne, t = Lp - 1 - (int)(r / ne);
+      int a = 0, b = 0;
+      if (e) tree_decode(e, dg, a, b);
+      const bool live = x < total && (e == 0 || tree_need(T, a, b));
+      const S* pp = par + p;
+      const long long st = (long long)Lp * ps;
+      const S* base = pp + e * st;
+      ConvAcc<S> acc = ConvAcc<S>::of(A::zero());
+      S c = A::zero(), c0 = A::zero();
+      if (live) {
+        if (sub < 2 && t + 1 < Lp) c = tld(base + (t + 1) * ps);
+        if (sub < 2 && t == 0) c0 = tld(base);
+        if (e) {
+          conv_part2(acc, pp + tree_ent(i, a, dg) * st, pp + tree_ent(j, b, dg) * st, pp + tree_ent(j, a, dg) * st,
+                     pp + tree_ent(i, b, dg) * st, ps, Lp, ps, t, sub);
+        } else if (T.pL >= 0 && m) {
+          conv_part(acc, pp, ps, Lp, m + p, (long long)np, t, sub);
+        } else {
+          conv_part(acc, pp, ps, Lp, pp + tree_ent(j, i, dg) * st, ps, t, sub);
+          if (T.pL >= 0)  // m not formed beforehand: a round less, where rounds are the time
+            for (int s = sub; s <= t; s += WG_TREE_SPLIT)
+              acc.fma(tld(pp + s * ps), conv_one(pp + tree_ent(i, T.pL, dg) * st, ps, Lp,
+                                                 pp + tree_ent(j, T.pL, dg) * st, ps, Lp, t - s));
+        }
+      }
+      const S u = split_sum(acc.sum());
+      if (live && sub < 2) {  // thread 0 stores the +1 child, thread 1 the -1 child
+        S* o = chi + (long long)e * Lc * cs + p;
+        for (int h = sub; h < (WG_TREE_SPLIT > 1 ? sub + 1 : 2) && h < nd; ++h) {
+          tst(o + h * np + (t + 1) * cs, h == 0 ? A::add(c, u) : (e == 0 ? A::sub(u, c) : A::sub(c, u)));
+          if (t == 0) tst(o + h * np, h == 1 && e == 0 ? A::neg(c0) : c0);
+        }
+      }
+    }
+    return;
+  }
+  constexpr int TT = TL ? TL : 1;
+  const int nt = (Lp + TT - 1) / TT;
   const unsigned total = (unsigned)nt * ne * np;
   for (unsigned x = tid; x < total; x += nthr) {
     const unsigned r = x / np;
-    const int p = x - r * np, e = r % ne, t0 = Lp - TL * ((int)(r / ne) + 1);
+    const int p = x - r * np, e = r % ne, t0 = Lp - TT * ((int)(r / ne) + 1);
     const S* pp = par + p;
-    S acc[TL];
+    ConvAcc<S> acc[TT];
 #pragma unroll
-    for (int k = 0; k < TL; ++k) acc[k] = A::zero();
+    for (int k = 0; k < TT; ++k) acc[k] = ConvAcc<S>::of(A::zero());
     if (e == 0) {
-      if (T.pL >= 0) conv_tile<S, TL>(acc, pp, ps, Lp, m + p, np, t0);
-      else conv_tile<S, TL>(acc, pp, ps, Lp, pp + (long long)tree_ent(j, i, dg) * Lp * ps, ps, t0);
+      if (T.pL >= 0) conv_tile<S, TT>(acc, pp, ps, Lp, m + p, np, t0);
+      else conv_tile<S, TT>(acc, pp, ps, Lp, pp + (long long)tree_ent(j, i, dg) * Lp * ps, ps, t0);
     } else {
       int a, b;
       tree_decode(e, dg, a, b);
       if (!tree_need(T, a, b)) continue;
       const long long st = (long long)Lp * ps;
-      conv_tile<S, TL>(acc, pp + tree_ent(i, a, dg) * st, ps, Lp, pp + tree_ent(j, b, dg) * st, ps, t0);
-      conv_tile<S, TL>(acc, pp + tree_ent(j, a, dg) * st, ps, Lp, pp + tree_ent(i, b, dg) * st, ps, t0);
+      conv_tile<S, TT>(acc, pp + tree_ent(i, a, dg) * st, ps, Lp, pp + tree_ent(j, b, dg) * st, ps, t0);
+      conv_tile<S, TT>(acc, pp + tree_ent(j, a, dg) * st, ps, Lp, pp + tree_ent(i, b, dg) * st, ps, t0);
     }
     const S* base = pp + (long long)e * Lp * ps;
     S* o = chi + (long long)e * Lc * cs + p;
 #pragma unroll
-    for (int k = -1; k < TL; ++k) {  // coefficient t + 1 of the children; k = -1: coefficient 0
+    for (int k = -1; k < TT; ++k) {  // coefficient t + 1 of the children; k = -1: coefficient 0
       const int t = t0 + k;
       if (k < 0 ? t0 <= 0 : t >= 0) {
         const int tc = k < 0 ? 0 : t + 1;
         const S c = tc < Lp ? tld(base + tc * ps) : A::zero();
-        const S u = k < 0 ? A::zero() : acc[k < 0 ? 0 : k];
+        const S u = k < 0 ? A::zero() : acc[k < 0 ? 0 : k].sum();
         S* w = o + tc * cs;
-        if (d0 == 0) {
-          tst(w, A::add(c, u));
-          w += np;
-        }
-        if (d0 + nd > 1) tst(w, e == 0 ? A::sub(u, c) : A::sub(c, u));
+        tst(w, A::add(c, u));
+        if (nd > 1) tst(w + np, e == 0 ? A::sub(u, c) : A::sub(c, u));
       }
     }
   }
@@ -335,75 +569,105 @@ __host__ __device__ __forceinline__ double tree_weight(const TreeInst& T, int q,
   return w;
 }
 
+// A series in memory: elements `st` apart.
+template <class S>
+struct TreeSer {
+  S* p;
+  long long st;
+  __host__ __device__ __forceinline__ S& operator[](int t) const { return p[t * st]; }
+};
+#pragma nv_exec_check_disable
+template <class S>
+__host__ __device__ __forceinline__ S conv_ser(TreeSer<S> a, int la, TreeSer<S> b, int lb, int t) {
+  return conv_one((const S*)a.p, a.st, la, (const S*)b.p, b.st, lb, t);
+}
+// a copy of n elements of src (in global memory) into the warp's shared memory at dst
+#pragma nv_exec_check_disable
+template <class S>
+__host__ __device__ __forceinline__ TreeSer<S> ser_stage(const S* src, long long st, int n, S* dst, int lane) {
+  for (int t = lane; t < n; t += WG_TREE_LANES) dst[t] = tld(src + t * st);
+  return {dst, 1};
+}
+
 // Series of the edge's 2 x 2 block, one warp per child: scr[(f Lc + t) nc + x], f = 0..2 the entries
 // P_ii, P_ij, P_jj, f = 3 the factor h = Delta^(-1/2) (Delta = (1 - z c)^2 - z^2 a b, z = delta eta,
-// a, b, c = C_ii, C_jj, C_ij), f = 4.. work; without loop weights also the child's g = w g h.
+// a, b, c = C_ii, C_jj, C_ij), f = 4.. work; without loop weights also the child's g = w g h.  The
+// recurrences are chains of short steps, so they run on copies in the warp's shared memory (smn
+// elements at sm) when those fit: a step costs 30 clocks of latency there and 700 in L2.
 #pragma nv_exec_check_disable
 template <class S>
 __host__ __device__ void tree_prep(const TreeInst& T, int q, const S* par, long long ps, int np, S* scr,
-                          S* chi, int d0, int nd, int tid, int nthr) {
+                          S* chi, S* sm, int smn, int tid, int nthr) {
   using A = Ar<S>;
   const int i = T.X + 2 * (T.E - 1 - q), j = i + 1, r = T.reps[q];
-  const int Lp = T.deg[q] + 1, Lc = Lp + r, nc = np * nd;
+  const int Lp = T.deg[q] + 1, Lc = Lp + r, nc = np * T.radix[q];
   const int lane = tid & (WG_TREE_LANES - 1);
+  const bool staged = smn >= 7 * Lc;
   for (int x = tid / WG_TREE_LANES; x < nc; x += nthr / WG_TREE_LANES) {
-    const int p = x % np, d = d0 + x / np;
+    const int p = x % np, d = x / np;
     const double z = (double)(r - 2 * d);
     const S* pp = par + p;
-    const S* ca = pp + (long long)tree_ent(i, i, 1) * Lp * ps;
-    const S* cb = pp + (long long)tree_ent(j, j, 1) * Lp * ps;
-    const S* cc = pp + (long long)tree_ent(j, i, 1) * Lp * ps;
-    auto at = [&](int f, int t) -> S& { return scr[((long long)f * Lc + t) * nc + x]; };
-    const long long fs = (long long)Lc * nc;
-    // Delta = 1 - 2 z c + z^2 (c c - a b), f = 4
+    const long long st = (long long)Lp * ps;
+    auto work = [&](int f) -> TreeSer<S> { return {scr + (long long)f * Lc * nc + x, nc}; };
+    const TreeSer<S> P0 = work(0), P1 = work(1), P2 = work(2), H = work(3);
+    TreeSer<S> ca = {const_cast<S*>(pp + tree_ent(i, i, 1) * st), ps}, cb = {const_cast<S*>(pp + tree_ent(j, j, 1) * st), ps};
+    TreeSer<S> cc = {const_cast<S*>(pp + tree_ent(j, i, 1) * st), ps}, g = {const_cast<S*>(pp), ps};
+    TreeSer<S> h = H, dl = work(4), hh = work(5);
+    if (staged) {
+      ca = ser_stage<S>(ca.p, ps, Lp, sm, lane);
+      cb = ser_stage<S>(cb.p, ps, Lp, sm + Lc, lane);
+      cc = ser_stage<S>(cc.p, ps, Lp, sm + 2 * Lc, lane);
+      g = ser_stage<S>(g.p, ps, Lp, sm + 3 * Lc, lane);
+      h = {sm + 4 * Lc, 1};
+      dl = {sm + 5 * Lc, 1};
+      hh = {sm + 6 * Lc, 1};
+      WG_TREE_SYNCWARP();
+    }
+    // Delta = 1 - 2 z c + z^2 (c c - a b)
     for (int t = lane; t < Lc; t += WG_TREE_LANES) {
       S v = t == 0 ? A::one() : A::zero();
-      if (t >= 1 && t - 1 < Lp) v = A::sub(v, A::scale(tld(cc + (t - 1) * ps), 2.0 * z));
+      if (t >= 1 && t - 1 < Lp) v = A::sub(v, A::scale(cc[t - 1], 2.0 * z));
       if (t >= 2) {
-        const S k = A::sub(conv_one(cc, ps, Lp, cc, ps, Lp, t - 2), conv_one(ca, ps, Lp, cb, ps, Lp, t - 2));
+        const S k = A::sub(conv_ser(cc, Lp, cc, Lp, t - 2), conv_ser(ca, Lp, cb, Lp, t - 2));
         v = A::add(v, A::scale(k, z * z));
       }
-      at(4, t) = v;
-      at(3, t) = t == 0 ? A::one() : A::zero();
+      dl[t] = v;
+      h[t] = t == 0 ? A::one() : A::zero();
     }
     WG_TREE_SYNCWARP();
     // h = Delta^(-1/2), right-looking as in inv_sqrt_series
     for (int k = 0; k + 1 < Lc; ++k) {
-      const S gk = at(3, k);
+      const S gk = h[k];
       for (int t = k + 1 + lane; t < Lc; t += WG_TREE_LANES) {
         S acc;
-        if constexpr (A::modular) {
-          acc = A::fma(at(4, t - k), A::mul(gk, A::mul(A::of_int(t + k), A::half())), at(3, t));
-          if (t == k + 1) acc = A::neg(tree_div(acc, t));
-        } else {
-          acc = A::fma(at(4, t - k), A::scale_f(gk, 0.5f * (float)(t + k)), at(3, t));
-          if (t == k + 1) acc = A::neg(tree_div(acc, t));
-        }
-        at(3, t) = acc;
+        if constexpr (A::modular) acc = A::fma(dl[t - k], A::mul(gk, A::mul(A::of_int(t + k), A::half())), h[t]);
+        else acc = A::fma(dl[t - k], A::scale_f(gk, 0.5f * (float)(t + k)), h[t]);
+        if (t == k + 1) acc = A::neg(tree_div(acc, t));
+        h[t] = acc;
       }
       WG_TREE_SYNCWARP();
     }
-    const S* h = scr + 3 * fs + x;
-    S* hh = scr + 5 * fs + x;  // 1 / Delta
-    for (int t = lane; t < Lc; t += WG_TREE_LANES) hh[(long long)t * nc] = conv_one(h, nc, Lc, h, nc, Lc, t);
+    // 1 / Delta
+    for (int t = lane; t < Lc; t += WG_TREE_LANES) hh[t] = conv_ser(h, Lc, h, Lc, t);
     WG_TREE_SYNCWARP();
     // P = z / Delta [[z b, 1 - z c], [1 - z c, z a]]
     for (int t = lane; t < Lc; t += WG_TREE_LANES) {
       S pi = A::zero(), pj = A::zero(), pc = A::zero();
-      if (t >= 1) pc = A::scale(hh[(long long)(t - 1) * nc], z);
+      if (t >= 1) pc = A::scale(hh[t - 1], z);
       if (t >= 2) {
-        pi = A::scale(conv_one((const S*)hh, nc, Lc, cb, ps, Lp, t - 2), z * z);
-        pj = A::scale(conv_one((const S*)hh, nc, Lc, ca, ps, Lp, t - 2), z * z);
-        pc = A::sub(pc, A::scale(conv_one((const S*)hh, nc, Lc, cc, ps, Lp, t - 2), z * z));
+        pi = A::scale(conv_ser(hh, Lc, cb, Lp, t - 2), z * z);
+        pj = A::scale(conv_ser(hh, Lc, ca, Lp, t - 2), z * z);
+        pc = A::sub(pc, A::scale(conv_ser(hh, Lc, cc, Lp, t - 2), z * z));
       }
-      at(0, t) = pi;
-      at(1, t) = pc;
-      at(2, t) = pj;
+      tst(&P0[t], pi);
+      tst(&P1[t], pc);
+      tst(&P2[t], pj);
+      if (staged && T.pL >= 0) tst(&H[t], h[t]);  // for tree_gloop
     }
     if (T.pL < 0) {
       const double w = tree_weight(T, q, d);
       for (int t = lane; t < Lc; t += WG_TREE_LANES)
-        tst(chi + (long long)t * nc + x, A::scale(conv_one(h, nc, Lc, pp, ps, Lp, t), w));
+        tst(chi + (long long)t * nc + x, A::scale(conv_ser(h, Lc, g, Lp, t), w));
     }
     WG_TREE_SYNCWARP();
   }
@@ -411,119 +675,162 @@ __host__ __device__ void tree_prep(const TreeInst& T, int q, const S* par, long 
 
 // Y = P C_e,b for every remaining row b: scr_y[((2 b + s) Lc + t) nc + x]
 #pragma nv_exec_check_disable
-template <class S>
+template <class S, int TL>
 __host__ __device__ void tree_y(const TreeInst& T, int q, const S* par, long long ps, int np,
-                       const S* scr, S* y, int nd, int tid, int nthr) {
+                       const S* scr, S* y, int tid, int nthr) {
   using A = Ar<S>;
-  constexpr int TL = tree_tile<S>();
   const int i = T.X + 2 * (T.E - 1 - q), j = i + 1, W = i;
-  const int Lp = T.deg[q] + 1, Lc = Lp + T.reps[q], nc = np * nd, nt = (Lc + TL - 1) / TL;
+  const int Lp = T.deg[q] + 1, Lc = Lp + T.reps[q], nc = np * T.radix[q];
   const long long fs = (long long)Lc * nc;
+  if constexpr (TL == 0) {
+    const int total = Lc * 2 * W * nc, sub = tid % WG_TREE_SPLIT, step = nthr / WG_TREE_SPLIT;
+    for (int x0 = 0; x0 < total; x0 += step) {
+      const int x = x0 + tid / WG_TREE_SPLIT, r = x / nc, c = x - r * nc, bs = r % (2 * W), t = Lc - 1 - r / (2 * W);
+      const int b = bs >> 1, s = bs & 1, p = c % np;
+      ConvAcc<S> acc = ConvAcc<S>::of(A::zero());
+      if (x < total) {
+        conv_part2(acc, par + (long long)tree_ent(i, b, T.diag) * Lp * ps + p, scr + s * fs + c,
+                   par + (long long)tree_ent(j, b, T.diag) * Lp * ps + p, scr + (s + 1) * fs + c, ps, Lp, (long long)nc,
+                   t, sub);
+      }
+      const S v = split_sum(acc.sum());
+      if (x < total && sub == 0) tst(y + (long long)bs * fs + (long long)t * nc + c, v);
+    }
+    return;
+  }
+  constexpr int TT = TL ? TL : 1;
+  const int nt = (Lc + TT - 1) / TT;
   for (int x = tid; x < nt * 2 * W * nc; x += nthr) {
-    const int r = x / nc, c = x - r * nc, bs = r % (2 * W), t0 = Lc - TL * (r / (2 * W) + 1);
+    const int r = x / nc, c = x - r * nc, bs = r % (2 * W), t0 = Lc - TT * (r / (2 * W) + 1);
     const int b = bs >> 1, s = bs & 1, p = c % np;
-    S acc[TL];
+    ConvAcc<S> acc[TT];
 #pragma unroll
-    for (int k = 0; k < TL; ++k) acc[k] = A::zero();
-    conv_tile<S, TL>(acc, par + (long long)tree_ent(i, b, T.diag) * Lp * ps + p, ps, Lp, scr + s * fs + c, nc, t0);
-    conv_tile<S, TL>(acc, par + (long long)tree_ent(j, b, T.diag) * Lp * ps + p, ps, Lp, scr + (s + 1) * fs + c, nc,
+    for (int k = 0; k < TT; ++k) acc[k] = ConvAcc<S>::of(A::zero());
+    conv_tile<S, TT>(acc, par + (long long)tree_ent(i, b, T.diag) * Lp * ps + p, ps, Lp, scr + s * fs + c, nc, t0);
+    conv_tile<S, TT>(acc, par + (long long)tree_ent(j, b, T.diag) * Lp * ps + p, ps, Lp, scr + (s + 1) * fs + c, nc,
                      t0);
 #pragma unroll
-    for (int k = 0; k < TL; ++k)
-      if (t0 + k >= 0) tst(y + (long long)bs * fs + (long long)(t0 + k) * nc + c, acc[k]);
+    for (int k = 0; k < TT; ++k)
+      if (t0 + k >= 0) tst(y + (long long)bs * fs + (long long)(t0 + k) * nc + c, acc[k].sum());
   }
 }
 
 // C' = C + C_ae Y(b)
 #pragma nv_exec_check_disable
-template <class S>
+template <class S, int TL>
 __host__ __device__ void tree_multi(const TreeInst& T, int q, const S* par, long long ps, int np,
-                           const S* y, S* chi, int nd, int tid, int nthr) {
+                           const S* y, S* chi, int tid, int nthr) {
   using A = Ar<S>;
-  constexpr int TL = tree_tile<S>();
   const int i = T.X + 2 * (T.E - 1 - q), j = i + 1, dg = T.diag;
   const int ne = tree_entries(i, dg) - 1;
-  const int Lp = T.deg[q] + 1, Lc = Lp + T.reps[q], nc = np * nd, nt = (Lc + TL - 1) / TL;
+  const int Lp = T.deg[q] + 1, Lc = Lp + T.reps[q], nc = np * T.radix[q];
   const long long fs = (long long)Lc * nc, st = (long long)Lp * ps;
+  if constexpr (TL == 0) {
+    const unsigned total = (unsigned)Lc * ne * nc, step = nthr / WG_TREE_SPLIT;
+    const int sub = tid % WG_TREE_SPLIT;
+    for (unsigned x0 = 0; x0 < total; x0 += step) {
+      const unsigned x = x0 + tid / WG_TREE_SPLIT, r = x / nc;
+      const int c = x - r * nc, e = 1 + r % ne, t = Lc - 1 - (int)(r / ne), p = c % np;
+      int a, b;
+      tree_decode(e, dg, a, b);
+      const bool live = x < total && tree_need(T, a, b);
+      ConvAcc<S> acc = ConvAcc<S>::of(A::zero());
+      if (live) {
+        conv_part2(acc, par + p + tree_ent(i, a, dg) * st, y + (long long)(2 * b) * fs + c,
+                   par + p + tree_ent(j, a, dg) * st, y + (long long)(2 * b + 1) * fs + c, ps, Lp, (long long)nc, t, sub);
+      }
+      S v = split_sum(acc.sum());
+      if (live && sub == 0) {
+        if (t < Lp) v = A::add(v, tld(par + p + e * st + t * ps));
+        tst(chi + (long long)e * fs + (long long)t * nc + c, v);
+      }
+    }
+    return;
+  }
+  constexpr int TT = TL ? TL : 1;
+  const int nt = (Lc + TT - 1) / TT;
   const unsigned total = (unsigned)nt * ne * nc;
   for (unsigned x = tid; x < total; x += nthr) {
     const unsigned r = x / nc;
-    const int c = x - r * nc, e = 1 + r % ne, t0 = Lc - TL * ((int)(r / ne) + 1), p = c % np;
+    const int c = x - r * nc, e = 1 + r % ne, t0 = Lc - TT * ((int)(r / ne) + 1), p = c % np;
     int a, b;
     tree_decode(e, dg, a, b);
     if (!tree_need(T, a, b)) continue;
     const S* base = par + p + (long long)e * st;
-    S acc[TL];
+    ConvAcc<S> acc[TT];
 #pragma unroll
-    for (int k = 0; k < TL; ++k) {
+    for (int k = 0; k < TT; ++k) {
       const int t = t0 + k;
-      acc[k] = t >= 0 && t < Lp ? tld(base + t * ps) : A::zero();
+      acc[k] = ConvAcc<S>::of(t >= 0 && t < Lp ? tld(base + t * ps) : A::zero());
     }
-    conv_tile<S, TL>(acc, par + p + tree_ent(i, a, dg) * st, ps, Lp, y + (long long)(2 * b) * fs + c, nc, t0);
-    conv_tile<S, TL>(acc, par + p + tree_ent(j, a, dg) * st, ps, Lp, y + (long long)(2 * b + 1) * fs + c, nc, t0);
+    conv_tile<S, TT>(acc, par + p + tree_ent(i, a, dg) * st, ps, Lp, y + (long long)(2 * b) * fs + c, nc, t0);
+    conv_tile<S, TT>(acc, par + p + tree_ent(j, a, dg) * st, ps, Lp, y + (long long)(2 * b + 1) * fs + c, nc, t0);
 #pragma unroll
-    for (int k = 0; k < TL; ++k)
-      if (t0 + k >= 0) tst(chi + (long long)e * fs + (long long)(t0 + k) * nc + c, acc[k]);
+    for (int k = 0; k < TT; ++k)
+      if (t0 + k >= 0) tst(chi + (long long)e * fs + (long long)(t0 + k) * nc + c, acc[k].sum());
   }
 }
 
-// loop kinds: g' = w g h exp(v_e Y(L) / 2), one warp per child
+// loop kinds: g' = w g h exp(v_e Y(L) / 2), one warp per child; shared memory as in tree_prep
 #pragma nv_exec_check_disable
 template <class S>
 __host__ __device__ void tree_gloop(const TreeInst& T, int q, const S* par, long long ps, int np, S* scr,
-                           const S* y, S* chi, int d0, int nd, int tid, int nthr) {
+                           const S* y, S* chi, S* sm, int smn, int tid, int nthr) {
   using A = Ar<S>;
   const int i = T.X + 2 * (T.E - 1 - q), j = i + 1;
-  const int Lp = T.deg[q] + 1, Lc = Lp + T.reps[q], nc = np * nd;
+  const int Lp = T.deg[q] + 1, Lc = Lp + T.reps[q], nc = np * T.radix[q];
   const long long fs = (long long)Lc * nc, st = (long long)Lp * ps;
   const int lane = tid & (WG_TREE_LANES - 1);
+  const bool staged = smn >= 9 * Lc;
   for (int x = tid / WG_TREE_LANES; x < nc; x += nthr / WG_TREE_LANES) {
-    const int p = x % np, d = d0 + x / np;
-    const S* vi = par + p + tree_ent(i, T.pL, T.diag) * st;
-    const S* vj = par + p + tree_ent(j, T.pL, T.diag) * st;
-    const S* yi = y + (long long)(2 * T.pL) * fs + x;
-    const S* yj = y + (long long)(2 * T.pL + 1) * fs + x;
-    S* u = scr + 4 * fs + x;
-    S* ex = scr + 5 * fs + x;
-    S* gh = scr + x;  // P is no longer needed here
+    const int p = x % np, d = x / np;
+    TreeSer<S> vi = {const_cast<S*>(par + p + tree_ent(i, T.pL, T.diag) * st), ps};
+    TreeSer<S> vj = {const_cast<S*>(par + p + tree_ent(j, T.pL, T.diag) * st), ps};
+    TreeSer<S> g = {const_cast<S*>(par + p), ps}, h = {scr + 3 * fs + x, nc};
+    TreeSer<S> yi = {const_cast<S*>(y + (long long)(2 * T.pL) * fs + x), nc}, yj = {yi.p + fs, nc};
+    TreeSer<S> u = {scr + 4 * fs + x, nc}, ex = {scr + 5 * fs + x, nc}, gh = {scr + x, nc};  // P is not needed any more
+    if (staged) {
+      vi = ser_stage<S>(vi.p, ps, Lp, sm, lane);
+      vj = ser_stage<S>(vj.p, ps, Lp, sm + Lc, lane);
+      g = ser_stage<S>(g.p, ps, Lp, sm + 2 * Lc, lane);
+      yi = ser_stage<S>(yi.p, nc, Lc, sm + 3 * Lc, lane);
+      yj = ser_stage<S>(yj.p, nc, Lc, sm + 4 * Lc, lane);
+      h = ser_stage<S>(h.p, nc, Lc, sm + 5 * Lc, lane);
+      u = {sm + 6 * Lc, 1};
+      ex = {sm + 7 * Lc, 1};
+      gh = {sm + 8 * Lc, 1};
+      WG_TREE_SYNCWARP();
+    }
     for (int t = lane; t < Lc; t += WG_TREE_LANES) {
-      u[(long long)t * nc] = tree_half(A::add(conv_one(vi, ps, Lp, yi, nc, Lc, t), conv_one(vj, ps, Lp, yj, nc, Lc, t)));
-      ex[(long long)t * nc] = t == 0 ? A::one() : A::zero();
+      u[t] = tree_half(A::add(conv_ser(vi, Lp, yi, Lc, t), conv_ser(vj, Lp, yj, Lc, t)));
+      ex[t] = t == 0 ? A::one() : A::zero();
+      gh[t] = conv_ser(h, Lc, g, Lp, t);
     }
     WG_TREE_SYNCWARP();
     for (int k = 0; k + 1 < Lc; ++k) {  // exp, right-looking as in exp_series
-      const S ek = ex[(long long)k * nc];
+      const S ek = ex[k];
       for (int t = k + 1 + lane; t < Lc; t += WG_TREE_LANES) {
         S acc;
-        const S ut = u[(long long)(t - k) * nc];
-        if constexpr (A::modular) {
-          acc = A::fma(A::mul(ut, A::of_int(t - k)), ek, ex[(long long)t * nc]);
-          if (t == k + 1) acc = tree_div(acc, t);
-        } else {
-          acc = A::fma(A::scale_f(ut, (float)(t - k)), ek, ex[(long long)t * nc]);
-          if (t == k + 1) acc = tree_div(acc, t);
-        }
-        ex[(long long)t * nc] = acc;
+        if constexpr (A::modular) acc = A::fma(A::mul(u[t - k], A::of_int(t - k)), ek, ex[t]);
+        else acc = A::fma(A::scale_f(u[t - k], (float)(t - k)), ek, ex[t]);
+        if (t == k + 1) acc = tree_div(acc, t);
+        ex[t] = acc;
       }
       WG_TREE_SYNCWARP();
     }
-    const S* h = scr + 3 * fs + x;
-    for (int t = lane; t < Lc; t += WG_TREE_LANES) gh[(long long)t * nc] = conv_one(h, nc, Lc, par + p, ps, Lp, t);
-    WG_TREE_SYNCWARP();
     const double w = tree_weight(T, q, d);
     for (int t = lane; t < Lc; t += WG_TREE_LANES)
-      tst(chi + (long long)t * nc + x, A::scale(conv_one((const S*)ex, nc, Lc, (const S*)gh, nc, Lc, t), w));
+      tst(chi + (long long)t * nc + x, A::scale(conv_ser(ex, Lc, gh, Lc, t), w));
     WG_TREE_SYNCWARP();
   }
 }
 
 // ---- leaves: this thread's share of the output (batch: the sums of the warp, left in sm) over nodes [0, np) of a buffer of stride ps
 #pragma nv_exec_check_disable
-template <class S>
-__host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, int np, const S* m, S* sm, int wb,
+template <class S, int TL>
+__host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, int np, const S* m, S* sm, int smn,
                                 int tid, int nthr) {
   using A = Ar<S>;
-  constexpr int TL = tree_tile<S>();
   const int L = T.deg[T.steps] + 1, D = L - 1, dg = T.diag;
   const long long st = (long long)L * ps;
   S sum = A::zero();
@@ -532,18 +839,21 @@ __host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, i
     // and tile of h.  Two edges on X .. X+3 (no loop weights): h = haf(4 x 4).  One edge on X, X+1:
     // h = C_ij + v_i v_j; with an unpaired vertex o, h = v_o (C_ij + v_i v_j) + C_io v_j + C_jo v_i
     // (m = C_ij + v_i v_j from tree_m).
-    const int nt = (L + TL - 1) / TL, X = T.X;
+    constexpr int TT = TL ? TL : 1;
+    const int nt = TL ? (L + TT - 1) / TT : L * WG_TREE_SPLIT, X = T.X;
     const bool two = T.E - T.steps == 2;
     for (int x = tid; x < nt * np; x += nthr) {
-      const int p = x % np, t0 = L - TL * (x / np + 1);
+      // four threads a coefficient: neighbours share the node and coefficient, and split its products
+      const int sub = TL ? 0 : x % WG_TREE_SPLIT, xx = TL ? x : x / WG_TREE_SPLIT;
+      const int p = xx % np, t0 = L - TT * (xx / np + 1);
       const S* pp = par + p;
-      S acc[TL];
+      ConvAcc<S> acc[TT];
 #pragma unroll
-      for (int k = 0; k < TL; ++k) acc[k] = A::zero();
-      if (!two && T.pO < 0) {
+      for (int k = 0; k < TT; ++k) acc[k] = ConvAcc<S>::of(A::zero());
+      if (!two && T.pO < 0 && sub == 0) {
 #pragma unroll
-        for (int k = 0; k < TL; ++k)
-          if (t0 + k >= 0) acc[k] = tld(pp + tree_ent(X + 1, X, dg) * st + (t0 + k) * ps);
+        for (int k = 0; k < TT; ++k)
+          if (t0 + k >= 0) acc[k] = ConvAcc<S>::of(tld(pp + tree_ent(X + 1, X, dg) * st + (t0 + k) * ps));
       }
       const int nw = two ? 3 : (T.pO >= 0 ? 3 : (T.pL >= 0 ? 1 : 0));
 #pragma unroll 1
@@ -564,11 +874,12 @@ __host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, i
           u = pp + st * tree_ent(X + w, T.pO, dg);
           v = pp + st * tree_ent(X + 1 - w, T.pL, dg);
         }
-        conv_tile<S, TL>(acc, u, su, L, v, ps, t0);
+        if constexpr (TL == 0) conv_part(acc[0], u, su, L, v, ps, t0, sub);
+        else conv_tile<S, TT>(acc, u, su, L, v, ps, t0);
       }
 #pragma unroll
-      for (int k = 0; k < TL; ++k)
-        if (t0 + k >= 0) sum = A::fma(tld(pp + (D - t0 - k) * ps), acc[k], sum);
+      for (int k = 0; k < TT; ++k)
+        if (t0 + k >= 0) sum = A::fma(tld(pp + (D - t0 - k) * ps), acc[k].sum(), sum);
     }
   } else if (T.pB < 0) {
     for (int p = tid; p < np; p += nthr) {
@@ -582,16 +893,20 @@ __host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, i
   } else {
     // batch mode b with loop series v and pair series c: k photons give H_k = v H_(k-1) +
     // (k-1) c H_(k-2); with an unpaired vertex o: v_o H_k + k c_ob H_(k-1).  One warp per node, its
-    // work series and the output sums in the warp's part of sm.
+    // output sums and work series (and, when they fit, v and c) in the warp's shared memory.
     const int lane = tid & (WG_TREE_LANES - 1), nw = nthr / WG_TREE_LANES;
-    S* const base = sm + wb * (5 * L + 32);
-    S *gv = base + 3 * L, *gc = base + 4 * L, *o = base + 5 * L;
+    const bool staged = smn >= 7 * L + 32;
+    S *const o = sm, *const base = sm + 32, *gv = base + 3 * L, *gc = base + 4 * L;
     for (int k = lane; k < T.nout; k += WG_TREE_LANES) o[k] = A::zero();
     WG_TREE_SYNCWARP();
     for (int p = tid / WG_TREE_LANES; p < np; p += nw) {
       const S* pp = par + p;
-      const S* v = pp + (long long)tree_ent2(T.pB, T.pL, dg) * st;
-      const S* c = pp + (long long)tree_ent(T.pB, T.pB, 1) * st;
+      TreeSer<S> v = {const_cast<S*>(pp + (long long)tree_ent2(T.pB, T.pL, dg) * st), ps};
+      TreeSer<S> c = {const_cast<S*>(pp + (long long)tree_ent(T.pB, T.pB, 1) * st), ps};
+      if (staged) {
+        v = ser_stage<S>(v.p, ps, L, base + 5 * L, lane);
+        c = ser_stage<S>(c.p, ps, L, base + 6 * L, lane);
+      }
       S *h0 = base, *h1 = base + L, *h2 = base + 2 * L;
       for (int t = lane; t < L; t += WG_TREE_LANES) {
         h0[t] = A::zero();
@@ -611,8 +926,8 @@ __host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, i
           part = A::fma(gv[D - t], h1[t], part);
           if (k && T.pO >= 0) part = A::fma(tree_times(gc[D - t], k), h0[t], part);
           if (k + 1 < T.nout) {
-            S n = conv_one(v, ps, L, (const S*)h1, 1, L, t);
-            if (k) n = A::add(n, tree_times(conv_one(c, ps, L, (const S*)h0, 1, L, t), k));
+            S n = conv_ser(v, L, TreeSer<S>{h1, 1}, L, t);
+            if (k) n = A::add(n, tree_times(conv_ser(c, L, TreeSer<S>{h0, 1}, L, t), k));
             h2[t] = n;
           }
         }
@@ -631,136 +946,182 @@ __host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, i
   return sum;
 }
 
-// block sum of the leaf shares in a fixed order, into the partial slots
+// a warp's leaf share: lane k < nout returns output k's (batch: from the warp's part of sm)
 template <class S>
-__device__ void tree_store(const TreeInst& T, S sum, long long slot, double2* __restrict__ partials, S* red) {
+__device__ __forceinline__ S tree_warp_share(const TreeInst& T, S sum, const S* sm) {
+  const int lane = threadIdx.x & 31;
+  if (T.pB < 0) return warp_sum(sum);
+  __syncwarp();
+  if (lane < T.nout) sum = sm[lane];
+  __syncwarp();
+  return sum;
+}
+template <class S>
+__device__ __forceinline__ void tree_store(const TreeInst& T, S sum, long long slot, double2* partials) {
   using A = Ar<S>;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const bool batch = T.pB >= 0;
-  const int L = T.deg[T.steps] + 1;
-  if (!batch) {
-    sum = warp_sum(sum);
-    if (lane == 0) red[warp] = sum;
-  }
-  __syncthreads();
-  if (warp == 0 && lane < T.nout) {
-    S s = A::zero();
-    for (int w = 0; w < nw; ++w) s = A::add(s, batch ? red[w * (5 * L + 32) + 5 * L + lane] : red[w]);
-    const c64 z = A::to_c64(s);
+  const int lane = threadIdx.x & 31;
+  if (lane < T.nout) {
+    const c64 z = A::to_c64(sum);
     partials[slot + lane] = make_double2(z.re, z.im);
     if constexpr (A::dd) {
-      const c64 zl = A::lo_c64(s);
+      const c64 zl = A::lo_c64(sum);
       partials[slot + T.comp_off + lane] = make_double2(zl.re, zl.im);
     }
   }
-  __syncthreads();
 }
 
-// ---- one CTA per task: the path of the task's first q signs, then the whole subtree below it,
-// level by level in the CTA's own workspace (two node buffers and scratch, L2 resident)
+// Barrier of all CTAs of a cooperative launch (one CTA: a block barrier).  The wait is bounded: after
+// about 3 s of polling a CTA gives up, its later barriers do not wait, and the error flag makes the
+// outputs NaN.
+struct TreeSync {
+  unsigned int* bar;
+  int* err;
+  unsigned int target = 0;
+  bool ok = true;  // thread 0's
+  __device__ __forceinline__ void operator()() {
+    __syncthreads();
+    if (gridDim.x == 1) return;
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(bar, 1u);
+      if (ok) {
+        unsigned int v, n = 0;
+        do {
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+        } while (v < target && ++n < (1u << 22));
+        ok = v >= target;
+        if (!ok) atomicExch(err, 1);
+      }
+      __threadfence();
+    }
+    __syncthreads();
+  }
+};
+
+// The plan's only launch also reduces: the CTA that finishes last sums the partials of every
+// output, as reduce_kernel does, and re-arms the counters.
+__device__ __forceinline__ void tree_finish(const TreeFinish& F) {
+  if (!F.done) return;
+  __shared__ int s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = gridDim.x == 1 || atomicAdd(F.done, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last) return;
+  const int nw = blockDim.x >> 5;
+  reduce_block(F.inst, F.ninst, F.partials, F.scales, F.out, 0, nw / F.wpo, F.total_out, F.wpo, F.modp, F.mags, F.err);
+  for (int i = threadIdx.x; i < F.ncounters; i += blockDim.x) F.counters[i] = 0u;
+}
+
+// ---- trees by the whole chip in one cooperative launch: every round over all warps, one barrier of
+// the launch after it.  Consecutive warps of a round lie on different SMs, so that a narrow level
+// still uses every FP64 pipe.  Levels live in the workspace (L2 resident; a single CTA's in shared
+// memory).
 template <class S>
-static __global__ void __launch_bounds__(TREE_THREADS, 2) tree_cta_kernel(const TreeParams P) {
+static __global__ void __launch_bounds__(TREE_THREADS, 1) tree_kernel(const TreeParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ TreeInst T;
-  __shared__ int s_task;
+  using A = Ar<S>;
+  constexpr int TL = tree_tile<S>();
   S* sm = reinterpret_cast<S*>(smem);
-  unsigned char* ws = P.ws + (long long)blockIdx.x * P.ws_stride;
-  S* buf[2] = {reinterpret_cast<S*>(ws), reinterpret_cast<S*>(ws + P.off_b)};
-  S* scr = reinterpret_cast<S*>(ws + P.off_s);
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  for (;;) {
-    if (tid == 0) s_task = (int)atomicAdd(P.counter, 1u);
+  S* smw = sm + (threadIdx.x >> 5) * P.sm_warp;
+  S total = A::zero();
+  const TreeInst* insts = P.inst;
+  const TreeRound* rounds = P.rounds;
+  const TreeSeg* segs = P.segs;
+  if (P.cached) {  // the host laid the three arrays out one after another
+    const int words = (int)((P.ninst * sizeof(TreeInst) + P.nrounds * sizeof(TreeRound) + P.nsegs * sizeof(TreeSeg)) / 16);
+    const int4* src = reinterpret_cast<const int4*>(P.inst);
+    int4* dst = reinterpret_cast<int4*>(smem + P.sm_cache);
+    for (int w = threadIdx.x; w < words; w += blockDim.x) dst[w] = src[w];
+    insts = reinterpret_cast<const TreeInst*>(dst);
+    rounds = reinterpret_cast<const TreeRound*>(insts + P.ninst);
+    segs = reinterpret_cast<const TreeSeg*>(rounds + P.nrounds);
     __syncthreads();
-    const int task = s_task;
-    if (task >= P.ntasks) break;
-    int lo = 0, hi = P.ninst - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (P.inst[mid].task_base <= task) lo = mid; else hi = mid - 1;
-    }
-    {
-      const int* src = reinterpret_cast<const int*>(P.inst + lo);
-      int* dst = reinterpret_cast<int*>(&T);
-      for (int w = tid; w < (int)(sizeof(TreeInst) / 4); w += nthr) dst[w] = src[w];
-    }
-    __syncthreads();
-    int code = task - T.task_base;
-    tree_root<S>(T, P.pool, buf[0], tid, nthr);
-    __syncthreads();
-    int cur = 0, np = 1;
-    for (int q = 0; q < T.steps; ++q) {
-      const int R = T.radix[q];
-      int d0 = 0, nd = R;
-      if (q < T.q) {
-        d0 = code % R;
-        code /= R;
-        nd = 1;
+  }
+  unsigned char* ws = P.sm_ws ? smem + P.sm_ws : P.ws;
+  const int lane = threadIdx.x & 31;
+  const int gw = ((int)threadIdx.x >> 5) * gridDim.x + blockIdx.x, gn = gridDim.x * (blockDim.x >> 5);
+  TreeSync sync{P.bar, P.err};
+  for (int r = 0; r < P.nrounds; ++r) {
+    const TreeRound R = rounds[r];
+    // (warps that take their next item from a counter as they come free measured 4 % slower here at
+    // n = 40 than this fixed stride)
+    for (int vw = gw; vw < R.nwarps; vw += gn) {
+      int lo = R.seg0, hi = R.seg0 + R.nseg - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (segs[mid].warp0 <= vw) lo = mid; else hi = mid - 1;
       }
-      const S* par = buf[cur];
-      S* chi = buf[cur ^ 1];
-      if (T.reps[q] == 1) {
-        if (T.pL >= 0) {
-          tree_m<S>(T, q, par, np, np, scr, tid, nthr);
-          __syncthreads();
+      const TreeSeg G = segs[lo];
+      const int end = lo + 1 < R.seg0 + R.nseg ? segs[lo + 1].warp0 : R.nwarps;
+      const TreeInst& T = insts[G.inst];
+      const int tid = (vw - G.warp0) * 32 + lane, nthr = (end - G.warp0) * 32;
+      const S* par = reinterpret_cast<const S*>(ws + G.par) + G.p0;
+      S* chi = reinterpret_cast<S*>(ws + G.chi);
+      S* scr = reinterpret_cast<S*>(ws + T.scr_off);
+      switch (G.phase) {
+        case TP_ROOT: tree_root<S>(T, P.pool, chi, tid, nthr); break;
+        case TP_FIRST: tree_first<S>(T, P.pool, chi, tid, nthr); break;
+        case TP_M:
+          if (G.tile == 0) tree_m<S, 0>(T, G.q, par, G.pstride, G.np, scr, tid, nthr);
+          else if (G.tile == 1) tree_m<S, 1>(T, G.q, par, G.pstride, G.np, scr, tid, nthr);
+          else tree_m<S, TL>(T, G.q, par, G.pstride, G.np, scr, tid, nthr);
+          break;
+        case TP_UNIT:
+          if (G.tile == 0) tree_unit<S, 0>(T, G.q, par, G.pstride, G.np, G.fused ? nullptr : scr, chi, tid, nthr);
+          else if (G.tile == 1) tree_unit<S, 1>(T, G.q, par, G.pstride, G.np, scr, chi, tid, nthr);
+          else tree_unit<S, TL>(T, G.q, par, G.pstride, G.np, scr, chi, tid, nthr);
+          break;
+        case TP_PREP: tree_prep<S>(T, G.q, par, G.pstride, G.np, scr, chi, smw, P.sm_warp, tid, nthr); break;
+        case TP_LEAF: {
+          const S sum = G.tile == 0   ? tree_leaf<S, 0>(T, par, G.pstride, G.np, scr, smw, P.sm_warp, tid, nthr)
+                        : G.tile == 1 ? tree_leaf<S, 1>(T, par, G.pstride, G.np, scr, smw, P.sm_warp, tid, nthr)
+                                      : tree_leaf<S, TL>(T, par, G.pstride, G.np, scr, smw, P.sm_warp, tid, nthr);
+          if (P.ninst == 1) {  // all leaves are one instance's: one partial per CTA, below
+            total = A::add(total, T.pB < 0 ? sum : tree_warp_share<S>(T, sum, smw));
+          } else {
+            tree_store<S>(T, tree_warp_share<S>(T, sum, smw), G.part + (long long)(vw - G.warp0) * T.pstride, P.partials);
+          }
+          break;
         }
-        tree_unit<S>(T, q, par, np, np, scr, chi, d0, nd, tid, nthr);
-      } else {
-        const int Lc = T.deg[q] + 1 + T.reps[q];
-        S* y = scr + 6ll * Lc * np * nd;
-        tree_prep<S>(T, q, par, np, np, scr, chi, d0, nd, tid, nthr);
-        __syncthreads();
-        if (tree_width(T.X, T.E, q + 1) > 0) {
-          tree_y<S>(T, q, par, np, np, scr, y, nd, tid, nthr);
-          __syncthreads();
-          tree_multi<S>(T, q, par, np, np, y, chi, nd, tid, nthr);
-          if (T.pL >= 0) tree_gloop<S>(T, q, par, np, np, scr, y, chi, d0, nd, tid, nthr);
+        default: {
+          S* y = scr + 6ll * (T.deg[G.q + 1] + 1) * G.np * T.radix[G.q];
+          if (G.phase == TP_GLOOP) {
+            tree_gloop<S>(T, G.q, par, G.pstride, G.np, scr, y, chi, smw, P.sm_warp, tid, nthr);
+          } else if (G.phase == TP_Y) {
+            if (G.tile == 0) tree_y<S, 0>(T, G.q, par, G.pstride, G.np, scr, y, tid, nthr);
+            else if (G.tile == 1) tree_y<S, 1>(T, G.q, par, G.pstride, G.np, scr, y, tid, nthr);
+            else tree_y<S, TL>(T, G.q, par, G.pstride, G.np, scr, y, tid, nthr);
+          } else {
+            if (G.tile == 0) tree_multi<S, 0>(T, G.q, par, G.pstride, G.np, y, chi, tid, nthr);
+            else if (G.tile == 1) tree_multi<S, 1>(T, G.q, par, G.pstride, G.np, y, chi, tid, nthr);
+            else tree_multi<S, TL>(T, G.q, par, G.pstride, G.np, y, chi, tid, nthr);
+          }
         }
       }
-      np *= nd;
-      cur ^= 1;
-      __syncthreads();
     }
-    if (T.steps < T.E && T.pO >= 0) {
-      tree_m<S>(T, T.steps, buf[cur], np, np, scr, tid, nthr);
-      __syncthreads();
-    }
-    const S sum = tree_leaf<S>(T, buf[cur], np, np, scr, sm, tid >> 5, tid, nthr);
-    tree_store<S>(T, sum, T.part_base + (long long)(task - T.task_base) * T.pstride, P.partials, sm);
+    if (r + 1 < P.nrounds) sync();
   }
-}
-
-// ---- one phase of one step over a whole block of nodes
-template <class S>
-static __global__ void __launch_bounds__(TREE_THREADS, 2) tree_grid_kernel(const TreeGrid G) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ TreeInst T;
-  {
-    const int* src = reinterpret_cast<const int*>(G.P.inst + G.inst);
-    int* dst = reinterpret_cast<int*>(&T);
-    for (int w = threadIdx.x; w < (int)(sizeof(TreeInst) / 4); w += blockDim.x) dst[w] = src[w];
-  }
-  __syncthreads();
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
-  const S* par = reinterpret_cast<const S*>(G.par) + G.p0;
-  S* chi = reinterpret_cast<S*>(G.chi);
-  S* scr = reinterpret_cast<S*>(G.scr);
-  switch (G.phase) {
-    case TP_ROOT: tree_root<S>(T, G.P.pool, chi, tid, nthr); break;
-    case TP_M: tree_m<S>(T, G.q, par, G.pstride, G.np, scr, tid, nthr); break;
-    case TP_UNIT: tree_unit<S>(T, G.q, par, G.pstride, G.np, scr, chi, G.d0, G.nd, tid, nthr); break;
-    case TP_PREP: tree_prep<S>(T, G.q, par, G.pstride, G.np, scr, chi, G.d0, G.nd, tid, nthr); break;
-    case TP_LEAF: {
-      const S sum = tree_leaf<S>(T, par, G.pstride, G.np, scr, reinterpret_cast<S*>(smem), threadIdx.x >> 5, tid, nthr);
-      tree_store<S>(T, sum, G.part + (long long)blockIdx.x * T.pstride, G.P.partials, reinterpret_cast<S*>(smem));
-      break;
-    }
-    default: {
-      S* y = scr + 6ll * (T.deg[G.q] + 1 + T.reps[G.q]) * G.np * G.nd;
-      if (G.phase == TP_Y) tree_y<S>(T, G.q, par, G.pstride, G.np, scr, y, G.nd, tid, nthr);
-      else if (G.phase == TP_MULTI) tree_multi<S>(T, G.q, par, G.pstride, G.np, y, chi, G.nd, tid, nthr);
-      else tree_gloop<S>(T, G.q, par, G.pstride, G.np, scr, y, chi, G.d0, G.nd, tid, nthr);
+  if (P.ninst == 1) {
+    const TreeInst& T = insts[0];
+    if (T.pB < 0) total = warp_sum(total);
+    __syncthreads();  // sm's leaf part is free now
+    if (lane < T.nout) sm[(threadIdx.x >> 5) * T.nout + lane] = total;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const int nw = blockDim.x >> 5;
+      S s = A::zero();
+      if (T.nout == 1) s = warp_sum(lane < nw ? sm[lane] : s);
+      else if (lane < T.nout)
+        for (int w = 0; w < nw; ++w) s = A::add(s, sm[w * T.nout + lane]);
+      tree_store<S>(T, s, segs[P.nsegs - 1].part + (long long)blockIdx.x * T.pstride, P.partials);
     }
   }
+  tree_finish(P.fin);
 }
 
 }  // namespace wg
