@@ -75,7 +75,14 @@ static inline bool tree_build(const InstDev& d, TreeInst& T) {
 static inline int tree_scale_exp(const TreeInst& T) { return T.deg[T.steps] - (T.steps > 0 ? 1 : 0); }
 
 // bytes of a node element
-static inline int tree_bytes(int stype) { return stype == ST_CPLX64 ? (int)sizeof(c3) : (int)stype_bytes(stype); }
+static inline int tree_bytes(int stype) {
+  switch (stype) {
+    case ST_CPLX64: return (int)sizeof(TreeScalar<c64>::T);
+    case ST_CPLXDF: return (int)sizeof(TreeScalar<cdf>::T);
+    case ST_CPLXDD: return (int)sizeof(TreeScalar<cdd>::T);
+    default: return (int)stype_bytes(stype);
+  }
+}
 
 // elements of a node, and of the scratch of step q (np parents)
 static inline long long tree_node_elems(const TreeInst& T, int q) {

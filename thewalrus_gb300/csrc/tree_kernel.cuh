@@ -150,44 +150,87 @@ __host__ __device__ __forceinline__ void tree_decode(int e, int diag, int& a, in
   b = x - r * (r + 1) / 2;
 }
 
-// Node scalars: complex FP64 nodes carry re + im beside the parts (c3), so that a product of series
-// takes three real products a term instead of four (re = P1 - P2, im = P3 - P1 - P2 with P1 = sum
-// re re, P2 = sum im im, P3 = sum (re + im)(re + im)); its rounding is relative to |a| |b|, as
-// the four products' is.  Complex n = 40: 5,836 -> 5,405 us, n = 36: 1,212 -> 1,147 us.
-struct c3 {
-  double re, im, s;
+// The running sum of real products.  Double-float and double-double sums stay unnormalised until
+// they are read: a product's error terms and the two-sum's join the low part, which takes 12
+// instructions a product where the scalar types' fma, which renormalises every time, takes 15.
+template <class R>
+struct RealAcc {
+  R v;
+#pragma nv_exec_check_disable
+  __host__ __device__ static __forceinline__ RealAcc of(R x) { return {x}; }
+#pragma nv_exec_check_disable
+  __host__ __device__ __forceinline__ void fma(R a, R b) { v = Ar<R>::fma(a, b, v); }
+#pragma nv_exec_check_disable
+  __host__ __device__ __forceinline__ R sum() const { return v; }
 };
 template <>
-struct Ar<c3> {
-  using S = c3;
-  using Comp = double;
+struct RealAcc<dfr> {
+  float hi, lo;
+  __device__ static __forceinline__ RealAcc of(dfr x) { return {x.hi, x.lo}; }
+  __device__ __forceinline__ void fma(dfr a, dfr b) {
+    const float p = a.hi * b.hi;
+    float e = fmaf(a.hi, b.hi, -p);
+    e = fmaf(a.hi, b.lo, e);
+    e = fmaf(a.lo, b.hi, e);
+    const dfr s = df_two_sum(hi, p);
+    hi = s.hi;
+    lo += s.lo + e;
+  }
+  __device__ __forceinline__ dfr sum() const { return df_two_sum(hi, lo); }
+};
+template <>
+struct RealAcc<ddr> {
+  double hi, lo;
+  __device__ static __forceinline__ RealAcc of(ddr x) { return {x.hi, x.lo}; }
+  __device__ __forceinline__ void fma(ddr a, ddr b) {
+    const double p = a.hi * b.hi;
+    double e = ::fma(a.hi, b.hi, -p);
+    e = ::fma(a.hi, b.lo, e);
+    e = ::fma(a.lo, b.hi, e);
+    const ddr s = dd_two_sum(hi, p);
+    hi = s.hi;
+    lo += s.lo + e;
+  }
+  __device__ __forceinline__ ddr sum() const { return dd_two_sum(hi, lo); }
+};
+
+// Complex nodes carry re + im beside the parts, so that a product of series takes three real products
+// a term instead of four (re = P1 - P2, im = P3 - P1 - P2 with P1 = sum re re, P2 = sum im im, P3 = sum
+// (re + im)(re + im)); its rounding is relative to |a| |b|, as the four products' is.  C: the matrix
+// scalar, R: its real one.  FP64 n = 40: 5,836 -> 5,405 us, n = 36: 1,212 -> 1,147 us.
+template <class R, class C>
+struct c3 {
+  R re, im, s;
+};
+template <class R, class C>
+struct Ar<c3<R, C>> {
+  using S = c3<R, C>;
+  using B = Ar<R>;
+  using Comp = typename Ar<C>::Comp;
   static constexpr int NC = 2;
-  static constexpr bool cplx = true, fp64 = true, modular = false, dd = false;
-  __device__ static __forceinline__ S of(double re, double im) { return {re, im, re + im}; }
-  __device__ static __forceinline__ S zero() { return {0.0, 0.0, 0.0}; }
-  __device__ static __forceinline__ S one() { return {1.0, 0.0, 1.0}; }
-  __device__ static __forceinline__ S add(S a, S b) { return of(a.re + b.re, a.im + b.im); }
-  __device__ static __forceinline__ S sub(S a, S b) { return of(a.re - b.re, a.im - b.im); }
-  __device__ static __forceinline__ S neg(S a) { return {neg_d(a.re), neg_d(a.im), neg_d(a.s)}; }
-  __device__ static __forceinline__ S mul(S a, S b) {
-    const c64 z = Ar<c64>::mul({a.re, a.im}, {b.re, b.im});
-    return of(z.re, z.im);
-  }
-  __device__ static __forceinline__ S fma(S a, S b, S c) {
-    const c64 z = Ar<c64>::fma({a.re, a.im}, {b.re, b.im}, {c.re, c.im});
-    return of(z.re, z.im);
-  }
-  __device__ static __forceinline__ S scale(S a, double s) { return of(a.re * s, a.im * s); }
-  __device__ static __forceinline__ S scale_f(S a, float s) { return scale(a, (double)s); }
-  __device__ static __forceinline__ S from_c64(c64 v) { return of(v.re, v.im); }
-  __device__ static __forceinline__ c64 to_c64(S a) { return {a.re, a.im}; }
+  static constexpr bool cplx = true, fp64 = B::fp64, modular = false, dd = B::dd;
+  __device__ static __forceinline__ S of(R re, R im) { return {re, im, B::add(re, im)}; }
+  __device__ static __forceinline__ S of(C z) { return of(z.re, z.im); }
+  __device__ static __forceinline__ C to(S a) { return {a.re, a.im}; }
+  __device__ static __forceinline__ S zero() { return {B::zero(), B::zero(), B::zero()}; }
+  __device__ static __forceinline__ S one() { return {B::one(), B::zero(), B::one()}; }
+  __device__ static __forceinline__ S add(S a, S b) { return of(B::add(a.re, b.re), B::add(a.im, b.im)); }
+  __device__ static __forceinline__ S sub(S a, S b) { return of(B::sub(a.re, b.re), B::sub(a.im, b.im)); }
+  __device__ static __forceinline__ S neg(S a) { return {B::neg(a.re), B::neg(a.im), B::neg(a.s)}; }
+  __device__ static __forceinline__ S mul(S a, S b) { return of(Ar<C>::mul(to(a), to(b))); }
+  __device__ static __forceinline__ S fma(S a, S b, S c) { return of(Ar<C>::fma(to(a), to(b), to(c))); }
+  __device__ static __forceinline__ S scale(S a, double s) { return of(B::scale(a.re, s), B::scale(a.im, s)); }
+  __device__ static __forceinline__ S scale_f(S a, float s) { return of(B::scale_f(a.re, s), B::scale_f(a.im, s)); }
+  __device__ static __forceinline__ S div_int(S a, int k) { return of(B::div_int(a.re, k), B::div_int(a.im, k)); }
+  __device__ static __forceinline__ S from_c64(c64 v) { return of(Ar<C>::from_c64(v)); }
+  __device__ static __forceinline__ c64 to_c64(S a) { return Ar<C>::to_c64(to(a)); }
+  __device__ static __forceinline__ c64 lo_c64(S a) { return Ar<C>::lo_c64(to(a)); }
   __device__ static __forceinline__ Comp comp(const S& a, int i) { return i ? a.im : a.re; }
-  __device__ static __forceinline__ void set_comp(S& a, int i, Comp v) {
-    if (i) a.im = v; else a.re = v;
-    a.s = a.re + a.im;
+  __device__ static __forceinline__ void set_comp(S& a, int i, Comp v) {  // parts in order
+    if (i) a = of(a.re, v); else a.re = v;
   }
-  __device__ static __forceinline__ Comp cadd(Comp a, Comp b) { return a + b; }
-  __device__ static __forceinline__ Comp shfl_xor(Comp v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
+  __device__ static __forceinline__ Comp cadd(Comp a, Comp b) { return Ar<C>::cadd(a, b); }
+  __device__ static __forceinline__ Comp shfl_xor(Comp v, int m) { return Ar<C>::shfl_xor(v, m); }
 };
 // the node scalar of a matrix scalar, and back
 template <class M>
@@ -196,40 +239,48 @@ struct TreeScalar {
 };
 template <>
 struct TreeScalar<c64> {
-  using T = c3;
+  using T = c3<double, c64>;
+};
+template <>
+struct TreeScalar<cdf> {
+  using T = c3<dfr, cdf>;
+};
+template <>
+struct TreeScalar<cdd> {
+  using T = c3<ddr, cdd>;
 };
 template <class S>
 struct TreeMatrix {
   using T = S;
   __host__ __device__ static __forceinline__ S load(const S* p) { return *p; }
 };
-template <>
-struct TreeMatrix<c3> {
-  using T = c64;
-  __device__ static __forceinline__ c3 load(const c64* p) { return Ar<c3>::of(p->re, p->im); }
+template <class R, class C>
+struct TreeMatrix<c3<R, C>> {
+  using T = C;
+  __device__ static __forceinline__ c3<R, C> load(const C* p) { return Ar<c3<R, C>>::of(*p); }
 };
 
 // the running sum of a series product
 template <class S>
-struct ConvAcc {
-  S v;
+struct ConvAcc : RealAcc<S> {
 #pragma nv_exec_check_disable
-  __host__ __device__ static __forceinline__ ConvAcc of(S x) { return {x}; }
-#pragma nv_exec_check_disable
-  __host__ __device__ __forceinline__ void fma(S a, S b) { v = Ar<S>::fma(a, b, v); }
-#pragma nv_exec_check_disable
-  __host__ __device__ __forceinline__ S sum() const { return v; }
+  __host__ __device__ static __forceinline__ ConvAcc of(S x) { return {RealAcc<S>::of(x)}; }
 };
-template <>
-struct ConvAcc<c3> {
-  double p1, p2, p3;
-  __device__ static __forceinline__ ConvAcc of(c3 x) { return {x.re, 0.0, x.s}; }
-  __device__ __forceinline__ void fma(c3 a, c3 b) {
-    p1 = ::fma(a.re, b.re, p1);
-    p2 = ::fma(a.im, b.im, p2);
-    p3 = ::fma(a.s, b.s, p3);
+template <class R, class C>
+struct ConvAcc<c3<R, C>> {
+  RealAcc<R> p1, p2, p3;
+  __device__ static __forceinline__ ConvAcc of(c3<R, C> x) {
+    return {RealAcc<R>::of(x.re), RealAcc<R>::of(Ar<R>::zero()), RealAcc<R>::of(x.s)};
   }
-  __device__ __forceinline__ c3 sum() const { return Ar<c3>::of(p1 - p2, p3 - p1 - p2); }
+  __device__ __forceinline__ void fma(c3<R, C> a, c3<R, C> b) {
+    p1.fma(a.re, b.re);
+    p2.fma(a.im, b.im);
+    p3.fma(a.s, b.s);
+  }
+  __device__ __forceinline__ c3<R, C> sum() const {
+    const R x = p1.sum(), y = p2.sum();
+    return Ar<c3<R, C>>::of(Ar<R>::sub(x, y), Ar<R>::sub(Ar<R>::sub(p3.sum(), x), y));
+  }
 };
 
 // loads and stores of node elements (the host check counts them)
@@ -1044,13 +1095,26 @@ static __global__ void __launch_bounds__(TREE_THREADS, 1) tree_kernel(const Tree
   }
   unsigned char* ws = P.sm_ws ? smem + P.sm_ws : P.ws;
   const int lane = threadIdx.x & 31;
-  const int gw = ((int)threadIdx.x >> 5) * gridDim.x + blockIdx.x, gn = gridDim.x * (blockDim.x >> 5);
+  const int gn = gridDim.x * (blockDim.x >> 5);
+  __shared__ int s_next[2];
+  if (threadIdx.x == 0) s_next[0] = 0;
+  __syncthreads();
   TreeSync sync{P.bar, P.err};
   for (int r = 0; r < P.nrounds; ++r) {
     const TreeRound R = rounds[r];
-    // (warps that take their next item from a counter as they come free measured 4 % slower here at
-    // n = 40 than this fixed stride)
-    for (int vw = gw; vw < R.nwarps; vw += gn) {
+    // A round's warps go to the CTAs in turn.  Where that is more than one a warp, the CTA's warps take
+    // its next one as they come free (from a counter in shared memory; one in global memory for all CTAs
+    // measured 4 % slower at n = 40 than fixed turns).  Fixed turns otherwise, so that a single
+    // instance's leaf sums, at most one a warp, add up in the same order every time.
+    if (threadIdx.x == 0) s_next[(r + 1) & 1] = 0;
+    const bool taken = R.nwarps > gn;
+    for (int turn = threadIdx.x >> 5;; turn += blockDim.x >> 5) {
+      if (taken) {
+        if (lane == 0) turn = atomicAdd(&s_next[r & 1], 1);
+        turn = __shfl_sync(0xffffffffu, turn, 0);
+      }
+      const int vw = turn * (int)gridDim.x + (int)blockIdx.x;
+      if (vw >= R.nwarps) break;
       int lo = R.seg0, hi = R.seg0 + R.nseg - 1;
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
