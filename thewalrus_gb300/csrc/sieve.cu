@@ -68,6 +68,43 @@ static int fail(int code, const char* fmt, ...) {
                                        __FILE__, __LINE__);                                     \
   } while (0)
 
+// Pinned blocks for the one-shot calls: a call stages its upload in one and its kernels write the
+// results there, so neither passes through pageable memory (a small call's result took 9 us to
+// come back by a copy).  A call takes a block and returns it when it has waited for its stream; at
+// most kMaxPinned are kept for the next calls of any thread, more are freed.
+constexpr size_t kPinnedBytes = 256 << 10;
+constexpr size_t kMaxPinned = 16;
+static std::mutex g_pinned_mu;
+static std::vector<unsigned char*> g_pinned;
+
+static unsigned char* pinned_take() {
+  {
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    if (!g_pinned.empty()) {
+      unsigned char* p = g_pinned.back();
+      g_pinned.pop_back();
+      return p;
+    }
+  }
+  void* p = nullptr;
+  if (cudaHostAlloc(&p, kPinnedBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return (unsigned char*)p;
+}
+static void pinned_give(unsigned char* p) {
+  if (!p) return;
+  {
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    if (g_pinned.size() < kMaxPinned) {
+      g_pinned.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
 static int ensure_init(int device) {
   std::lock_guard<std::mutex> lk(g_init_mu);
   if (g_device >= 0 && (device < 0 || device == g_device)) {
@@ -196,6 +233,8 @@ struct wg_plan {
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> side_done;
   cudaEvent_t fork = nullptr;
+  unsigned char* pinned = nullptr;  // one-shot plans: a pinned block (pinned_take)
+  double2* h_out = nullptr;         // the outputs in it, written by the kernels
   int device = 0;  // the device the plan's memory and tables live on
   bool serial_groups = false;
   std::vector<wg::TreeLaunch> trees;
@@ -756,15 +795,8 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
     TreeProgram prog;
     std::vector<int> base, cnt;
     const double clk = tree_mac_clocks(G.stype);
-    const int np0 = nparts;
-    G.ctas = g_num_sms;
-    tree_program(insts, levels, sb, tile, g_num_sms * TREE_THREADS, nparts, base, cnt, prog);
-    if (tree_one_cta(prog, clk) <= tree_whole_chip(prog, clk, g_num_sms)) {
-      G.ctas = 1;
-      nparts = np0;
-      prog = TreeProgram();
-      tree_program(insts, levels, sb, tile, TREE_THREADS, nparts, base, cnt, prog);
-    }
+    G.ctas = tree_one_cta(insts, levels, clk, g_num_sms) ? 1 : g_num_sms;
+    tree_program(insts, levels, sb, tile, G.ctas * TREE_THREADS, nparts, base, cnt, prog);
     for (size_t j = 0; j < insts.size(); ++j) {
       InstDev& d = P[order[k0 + j]].d;
       d.part_base = base[j];
@@ -976,8 +1008,11 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   const size_t b_err = al(sizeof(int));
   const size_t b_gdesc = gs ? al(sizeof(GatherDev) * std::max<size_t>(gs->desc.size(), 1)) : 0;
   const size_t b_gidx = gs ? al(sizeof(int) * std::max<size_t>(gs->idx.size(), 1)) : 0;
-  const size_t total = b_inst + b_chunks + b_tree + b_scales + b_pool + b_parts + b_out + b_mag + b_cnt + b_err +
-                       b_gdesc + b_gidx + b_ws;
+  // what is uploaded (zeroed counters included) first, in one copy; the matrices last of it, since
+  // serving forms them on the device
+  const size_t o_tree = b_inst + b_chunks, o_scales = o_tree + b_tree, o_cnt = o_scales + b_scales;
+  const size_t o_gdesc = o_cnt + b_cnt + b_err, o_pool = o_gdesc + b_gdesc + b_gidx;
+  const size_t total = o_pool + b_pool + b_parts + b_out + b_mag + b_ws;
   cudaStream_t cs = (cudaStream_t)opt.stream;
   pl->alloc_stream = cs;
   pl->async_alloc = cs != nullptr;
@@ -992,49 +1027,53 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   pl->d_chunks = (ChunkDev*)base; base += b_chunks;
   pl->d_prog = base; base += b_tree;
   pl->d_scales = (double*)base; base += b_scales;
-  pl->d_pool = ext_pool ? ext_pool : base; base += b_pool;
-  pl->d_partials = (double2*)base; base += b_parts;
-  pl->d_out = (double2*)base; base += b_out;
-  pl->d_mag = (double*)base; base += b_mag;
   pl->d_counters = (unsigned int*)base; base += b_cnt;
   pl->d_err = (int*)base; base += b_err;
   GatherDev* d_desc = (GatherDev*)base; base += b_gdesc;
   int* d_idx = (int*)base; base += b_gidx;
+  pl->d_pool = ext_pool ? ext_pool : base; base += b_pool;
+  pl->d_partials = (double2*)base; base += b_parts;
+  pl->d_out = (double2*)base; base += b_out;
+  pl->d_mag = (double*)base; base += b_mag;
   pl->d_ws = base;
   pl->device_bytes = (long long)total;
-  // staging: one host buffer with the same layout for the upload
-  const size_t o_tree = b_inst + b_chunks, o_scales = o_tree + b_tree, o_pool = o_scales + b_scales;
-  std::vector<unsigned char> host(o_pool + (gs || ext_pool ? 0 : b_pool), 0);
-  memcpy(host.data(), pl->inst.data(), sizeof(InstDev) * count);
-  if (!pl->chunks.empty()) memcpy(host.data() + b_inst, pl->chunks.data(), sizeof(ChunkDev) * pl->chunks.size());
-  if (!pl->tree_prog.empty()) memcpy(host.data() + o_tree, pl->tree_prog.data(), pl->tree_prog.size());
-  if (!scales.empty()) memcpy(host.data() + o_scales, scales.data(), sizeof(double) * scales.size());
+  // staging: one host buffer with the same layout for the upload, in the pinned block when it fits
+  // there beside the outputs
+  const size_t staged = o_pool + (gs || ext_pool ? 0 : b_pool);
+  std::vector<unsigned char> pageable;
+  unsigned char* host;
+  if (pl->pinned && b_out + staged <= kPinnedBytes) {
+    pl->h_out = (double2*)pl->pinned;
+    pl->d_out = pl->h_out;
+    host = pl->pinned + b_out;
+    memset(host, 0, staged);
+  } else {
+    pageable.assign(staged, 0);
+    host = pageable.data();
+  }
+  memcpy(host, pl->inst.data(), sizeof(InstDev) * count);
+  if (!pl->chunks.empty()) memcpy(host + b_inst, pl->chunks.data(), sizeof(ChunkDev) * pl->chunks.size());
+  if (!pl->tree_prog.empty()) memcpy(host + o_tree, pl->tree_prog.data(), pl->tree_prog.size());
+  if (!scales.empty()) memcpy(host + o_scales, scales.data(), sizeof(double) * scales.size());
+  if (gs) {
+    memcpy(host + o_gdesc, gs->desc.data(), sizeof(GatherDev) * gs->desc.size());
+    if (!gs->idx.empty()) memcpy(host + o_gdesc + b_gdesc, gs->idx.data(), sizeof(int) * gs->idx.size());
+  }
   for (int i = 0; i < count; ++i)
-    if (!P[i].ext.empty() && !ext_pool) memcpy(host.data() + o_pool + P[i].d.a_off, P[i].ext.data(), P[i].ext.size());
+    if (!P[i].ext.empty() && !ext_pool) memcpy(host + o_pool + P[i].d.a_off, P[i].ext.data(), P[i].ext.size());
   // uploads: stream-ordered on the creation stream when one is given (pageable sources are
   // staged before cudaMemcpyAsync returns), else synchronous
   auto up = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
     return cs ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, cs)
               : cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
   };
-  CK(up(pl->dmem, host.data(), host.size()));
-  pl->h2d_bytes = (long long)host.size();
-  if (gs) {
-    // pools are formed on the device: descriptors, chunks, scales and indices travel
-    CK(up(d_desc, gs->desc.data(), sizeof(GatherDev) * gs->desc.size()));
-    if (!gs->idx.empty()) CK(up(d_idx, gs->idx.data(), sizeof(int) * gs->idx.size()));
-    if (count > 0) {
-      gather_kernel<<<count, 256, 0, cs>>>(d_desc, d_idx, gs->B, gs->gamma, gs->M, pl->d_pool);
-      CK(cudaGetLastError());
-    }
-    pl->h2d_bytes += (long long)(sizeof(GatherDev) * gs->desc.size() + sizeof(int) * gs->idx.size());
+  CK(up(pl->dmem, host, staged));
+  pl->h2d_bytes = (long long)staged;
+  if (gs && count > 0) {  // pools are formed on the device
+    gather_kernel<<<count, 256, 0, cs>>>(d_desc, d_idx, gs->B, gs->gamma, gs->M, pl->d_pool);
+    CK(cudaGetLastError());
   }
-  if (cs) {
-    CK(cudaMemsetAsync(pl->d_counters, 0, b_cnt + b_err, cs));
-  } else {
-    CK(cudaMemset(pl->d_counters, 0, b_cnt + b_err));
-    CK(cudaStreamSynchronize(0));
-  }
+  if (!cs) CK(cudaStreamSynchronize(0));
   if (!pl->trees.empty()) {  // what a per-term plan of the same instances needs (terms_plan)
     pl->prep = std::move(P);
     for (Prepared& p : pl->prep) std::vector<unsigned char>().swap(p.ext);
@@ -1508,19 +1547,31 @@ int wg_plan_destroy(wg_plan* plan) {
 
 // One-shot plans run stream-ordered on the caller's stream, or on the calling thread's default
 // stream: their memory comes from the stream-ordered pool and goes back to it without a
-// device-wide synchronisation, and the uploads need none either (a small hafnian costs ~85 us
-// with a cudaMalloc / cudaFree pair per call).
+// device-wide synchronisation, and the uploads need none either; upload and results go through a
+// pinned block.
 int wg_run(const wg_instance* inst, int count, int precision, double* out, void* stream) {
-  wg_plan* pl = nullptr;
   const cudaStream_t st = stream ? (cudaStream_t)stream : cudaStreamPerThread;
   wg_plan_options opt;
   memset(&opt, 0, sizeof(opt));
   opt.chunk_scale = 1.0;
   opt.stream = st;
-  int rc = wg_plan_create_ex(inst, count, precision, &opt, &pl);
+  int rc = ensure_init(-1);
   if (rc) return rc;
-  rc = wg_plan_execute(pl, st);
-  if (!rc) rc = wg_plan_read(pl, out, st);
+  wg_plan* pl = new wg_plan();
+  pl->pinned = pinned_take();
+  rc = build_plan(inst, count, precision, opt, pl);
+  if (!rc) rc = execute_plan(pl, st);
+  if (!rc && !out && pl->total_out > 0) rc = fail(WG_EINVAL, "NULL argument");
+  if (!rc && pl->h_out) {
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) rc = fail(WG_ECUDA, "one-shot run: %s", cudaGetErrorString(e));
+    else memcpy(out, pl->h_out, sizeof(double2) * pl->total_out);
+  } else if (!rc) {
+    rc = wg_plan_read(pl, out, st);
+  }
+  // nothing in flight may still read or write the block that the next call takes
+  if (rc) cudaStreamSynchronize(st);
+  pinned_give(pl->pinned);
   destroy_plan(pl);
   return rc;
 }

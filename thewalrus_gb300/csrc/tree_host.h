@@ -226,7 +226,6 @@ struct TreeProgram {
   std::vector<TreeSeg> segs;
   long long ws_bytes = 0;
   int smem = 1;  // elements of a warp's shared memory
-  double macs = 0;
 };
 
 static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<TreeLevels>& levels, int sb, int tile,
@@ -256,7 +255,6 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
       s.fused = phase == TP_UNIT && T.pL >= 0 && tree_fused(T, q, np, fuse_threads);
       if (rounds.size() <= r) rounds.emplace_back();
       rounds[r++].push_back(s);
-      P.macs += tree_macs(T, phase, q, np);
     };
     if (T.steps > 0 && T.reps[0] == 1) {
       add(TP_FIRST, 0, 0, 1, 1);
@@ -310,10 +308,23 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
   P.insts = insts;
 }
 
-// one CTA's time for a program, in SM clocks: its multiply-adds and a barrier with its latencies a round
-static inline double tree_one_cta(const TreeProgram& P, double clk) { return 1.5 * P.macs * clk + 2500.0 * P.rounds.size(); }
-static inline double tree_whole_chip(const TreeProgram& P, double clk, int sms) {
-  return P.macs * clk / sms + 8000.0 * P.rounds.size();
+// Whether one CTA does a launch's work sooner than the whole chip: the multiply-adds against the
+// rounds, whose grid barrier and L2 latencies cost ~8000 clocks and one CTA's ~2500.
+static inline bool tree_one_cta(const std::vector<TreeInst>& insts, const std::vector<TreeLevels>& levels, double clk,
+                                int sms) {
+  double macs = 0, rounds = 0;
+  for (size_t k = 0; k < insts.size(); ++k) {
+    const TreeInst& T = insts[k];
+    double n = 0;
+    auto add = [&](int phase, int q, int, int np, int) {
+      macs += tree_macs(T, phase, q, np);
+      n += 1;
+    };
+    if (levels[k].phases > 200) return false;
+    tree_walk(T, levels[k], 0, 1, 1e30, add);
+    rounds = std::max(rounds, n);
+  }
+  return 1.5 * macs * clk + 2500.0 * rounds <= macs * clk / sms + 8000.0 * rounds;
 }
 
 }  // namespace wg
