@@ -171,6 +171,14 @@ int wg_plan_destroy(wg_plan* plan);
  * stream-ordered pool, which keeps up to 1.5 GiB of freed memory for the next call. */
 int wg_run(const wg_instance* inst, int count, int precision, double* out, void* stream);
 
+/* hafnian(A, loop) of an n x n matrix as the public function takes it (row-major, WG_FLOAT64 or
+ * WG_COMPLEX128), checks and pairing included; *done = 0 when the input is not an ordinary one
+ * (not finite, not symmetric, diagonal, integer-valued, badly scaled, n < 5 or too large) and the
+ * caller has to take the general route. */
+int wg_hafnian_direct(const void* A, int n, int dtype, int loop, double rtol, double atol, double out[2], int* done);
+/* Pairing of repeated indices (matched_reps): x has room for 4 n entries, mult for 2 n. */
+int wg_matched_reps(const int64_t* reps, int n, int64_t* x, int64_t* mult, int* E, int* odd);
+
 /* Serving: a Gaussian state resident on the device and plans whose loop-hafnian matrices are
  * formed on the device from it.  No single counterpart in the reference: it replaces the host
  * work of thewalrus/quantum/fock_tensors.py:74-92 (reduction of B and gamma by the photon

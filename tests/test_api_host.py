@@ -10,6 +10,7 @@ import pytest
 
 import thewalrus_gb300 as tw
 from thewalrus_gb300 import _hafnian as H
+from thewalrus_gb300 import _native as nat
 
 
 @pytest.mark.filterwarnings("ignore:overflow encountered")  # numpy.allclose(1e308, -1e308) warns too
@@ -142,3 +143,71 @@ def test_prepared_instances_match_a_direct_construction():
         assert np.array_equal(bi.A, typed(A[np.ix_(nz, nz)][np.ix_(edges, edges)], cplx))
         assert np.array_equal(bi.D, typed(np.asarray(D)[nz][edges], cplx))
         assert np.array_equal(bi.reps, fm)
+
+
+def test_native_pairing_matches_the_heap_rule():
+    """matched_reps (native) against the rule written out with a Python heap, ties, zeros, large and
+    non-integer-typed counts included."""
+    import heapq
+
+    def rule(reps):
+        reps = [int(r) for r in reps]
+        if sum(reps) == 0:
+            return [], [], None
+        pool = [(-r, -i) for i, r in enumerate(reps) if r > 0]
+        heapq.heapify(pool)
+        left, right, mult = [], [], []
+        while len(pool) > 1 or (pool and -pool[0][0] > 1):
+            r, i = heapq.heappop(pool)
+            r, i = -r, -i
+            if not pool or r > 2 * -pool[0][0]:
+                left.append(i)
+                right.append(i)
+                mult.append(r // 2)
+                if r % 2:
+                    heapq.heappush(pool, (-1, -i))
+            else:
+                s, j = heapq.heappop(pool)
+                s, j = -s, -j
+                left.append(i)
+                right.append(j)
+                mult.append(s)
+                if r > s:
+                    heapq.heappush(pool, (-(r - s), -i))
+        return left + right, mult, -pool[0][1] if len(pool) == 1 else None
+
+    rng = np.random.default_rng(5)
+    cases = [rng.integers(0, hi, size=n) for n in (1, 2, 3, 7, 20, 64) for hi in (1, 2, 3, 9) for _ in range(20)]
+    cases += [[], [0], [1], [2.0, 3.0, 1.0], (1, 1, 1, 1), [100000, 1, 1], np.ones(31, dtype=np.uint8)]
+    for reps in cases:
+        x, m, odd = tw.matched_reps(reps)
+        wx, wm, wodd = rule(reps)
+        assert list(x) == wx and list(m) == wm and odd == wodd, reps
+        assert x.dtype == m.dtype == np.int64
+
+
+def test_direct_route_takes_ordinary_matrices_only(monkeypatch):
+    """hafnian's native route says no to every input whose answer or error the general route defines."""
+    seen = []
+    monkeypatch.setattr(nat, "run", lambda insts, precision="fp64", stream=0: seen.append(precision) or np.zeros(1))
+    rng = np.random.default_rng(3)
+    S = rng.normal(size=(6, 6))
+    S = S + S.T
+    bad = S.copy()
+    bad[0, 1] = np.nan
+    asym = S.copy()
+    asym[0, 1] += 1e-3
+    inf = S.copy()
+    inf[0, 1] = inf[1, 0] = np.inf
+    scaled = S * np.outer([1, 1, 1, 1, 1, 1e6], [1, 1, 1, 1, 1, 1e6])
+    for A in (np.ones((6, 6)), np.diag(rng.normal(size=6)), bad, asym, inf, scaled, np.eye(5), np.round(S)):
+        for loop in (False, True):
+            assert nat.hafnian_direct(np.ascontiguousarray(A), loop, 1e-5, 1e-8) is None
+    with pytest.raises(ValueError):
+        tw.hafnian(bad)
+    with pytest.raises(ValueError):
+        tw.hafnian(asym)
+    assert tw.hafnian(np.diag(np.arange(6.0) + 0.5)) == 0
+    assert tw.hafnian(S[:5, :5].copy()) == 0.0  # odd
+    tw.hafnian(scaled)
+    assert seen == ["fp64"]

@@ -112,3 +112,14 @@ def test_plan_of_every_kind(options):
     assert np.array_equal(plan.read_magnitudes(), terms.read_magnitudes())
     a, b = plan.partials(), terms.partials()
     assert a[1] == b[1] and np.array_equal(a[0], b[0])
+
+
+@pytest.mark.parametrize("n", [5, 6, 7, 9, 12, 21, 26])
+def test_direct_route_is_the_general_one(n):
+    """hafnian's single native call against the checks, pairing and preparation in Python: the same
+    instance, so the same bits; complex, real, and complex with real values."""
+    A = wl.complex_symmetric(n, seed=n)
+    for M in (A, A.real.copy(), A.real.astype(complex)):
+        for loop in ((False, True) if n % 2 == 0 else (True,)):
+            prep = tw.prepare_loop_hafnian(M) if loop else tw.prepare_hafnian(M)
+            assert tw.hafnian(M, loop=loop) == nat.run([prep])[0]

@@ -18,8 +18,6 @@ that cancel beyond FP64's reach), "auto" (FP64, and double-double again for the 
 term magnitudes say FP64 may miss 1e-10) or "exact" (integer inputs).  Sieve results come back as
 ``numpy.complex128`` also for real input, as in the reference.
 """
-import heapq
-
 import numpy as np
 
 from . import _native as nat
@@ -122,32 +120,10 @@ def matched_reps(reps):
     itself ``r // 2`` times, otherwise it is paired with the second as often as the second
     allows.  Returns ``(x, edge_reps, oddmode)`` with vertex ``x[i]`` matched to ``x[i + E]``.
     """
-    reps = [int(r) for r in reps]
-    if sum(reps) == 0:
-        return np.array([], dtype=int), np.array([], dtype=int), None
-    # a heap of (-count, -index): the largest count first, ties broken by the larger index first
-    pool = [(-r, -i) for i, r in enumerate(reps) if r > 0]
-    heapq.heapify(pool)
-    left, right, mult = [], [], []
-    while len(pool) > 1 or (pool and -pool[0][0] > 1):
-        top_r, top_i = heapq.heappop(pool)
-        top_r, top_i = -top_r, -top_i
-        if not pool or top_r > 2 * -pool[0][0]:
-            left.append(top_i)
-            right.append(top_i)
-            mult.append(top_r // 2)
-            if top_r % 2:
-                heapq.heappush(pool, (-1, -top_i))
-        else:
-            sec_r, sec_i = heapq.heappop(pool)
-            sec_r, sec_i = -sec_r, -sec_i
-            left.append(top_i)
-            right.append(sec_i)
-            mult.append(sec_r)
-            if top_r > sec_r:
-                heapq.heappush(pool, (-(top_r - sec_r), -top_i))
-    oddmode = -pool[0][1] if len(pool) == 1 else None
-    return np.asarray(left + right, dtype=np.int64), np.asarray(mult, dtype=np.int64), oddmode
+    arr = np.asarray(reps)
+    if arr.ndim != 1 or arr.dtype.kind not in "iu":
+        arr = np.array([int(r) for r in reps], dtype=np.int64)
+    return nat.matched_reps(np.ascontiguousarray(arr, dtype=np.int64))
 
 
 def _cast(x, dt):
@@ -426,6 +402,12 @@ def hafnian(A, loop=False, rtol=1e-05, atol=1e-08, approx=False, num_samples=100
     (FP64, re-run in double-double when the sum of the terms' magnitudes says FP64 may miss
     1e-10) or "exact" (integer inputs only).
     """
+    if (precision is None and not approx and (loop or method == "glynn") and type(A) is np.ndarray
+            and A.ndim == 2 and A.shape[0] == A.shape[1] >= 5 and A.dtype.char in "dD" and A.dtype.isnative
+            and A.flags.c_contiguous and isinstance(rtol, float) and isinstance(atol, float)):
+        value = nat.hafnian_direct(A, loop, rtol, atol)  # the usual input: one native call
+        if value is not None:
+            return value
     input_validation(A, rtol=rtol, atol=atol)
     glynn = _method_glynn(method) if not loop else True
     done, value = _closed_form(A, loop, rtol, atol)

@@ -123,7 +123,7 @@ EXPORTS = [
     "wg_plan_destroy", "wg_run",
     "wg_measure_fp_peaks", "wg_hafnian_noalloc", "wg_state_create", "wg_state_destroy",
     "wg_plan_create_requests", "wg_plan_device_bytes", "wg_instance_terms", "wg_state_create_from_cov",
-    "wg_check_arith", "wg_plan_read_magnitudes",
+    "wg_check_arith", "wg_plan_read_magnitudes", "wg_hafnian_direct", "wg_matched_reps",
 ]
 
 
@@ -158,6 +158,8 @@ def load(build_if_needed=True):
     lib.wg_hafnian.argtypes = [vp, i32, i32, ip, i32, i32, i32, dp, vp]
     lib.wg_loop_hafnian.argtypes = [vp, vp, i32, i32, ip, i32, i32, dp, vp, i32, i32, dp, vp]
     lib.wg_loop_hafnian_batch.argtypes = [vp, vp, i32, i32, ip, i32, i32, i32, i32, i32, i32, dp, vp]
+    lib.wg_hafnian_direct.argtypes = [vp, i32, i32, i32, ctypes.c_double, ctypes.c_double, dp, ctypes.POINTER(i32)]
+    lib.wg_matched_reps.argtypes = [vp, i32, vp, vp, ctypes.POINTER(i32), ctypes.POINTER(i32)]
     lib.wg_plan_create.argtypes = [ctypes.POINTER(WgInstance), i32, i32, ctypes.c_double,
                                    ctypes.POINTER(vp)]
     lib.wg_plan_create_ex.argtypes = [ctypes.POINTER(WgInstance), i32, i32, ctypes.POINTER(WgPlanOptions),
@@ -318,14 +320,16 @@ class Plan:
         self = cls.__new__(cls)
         self.lib = load()
         self.instances = []
-        keep = []
         arr = (WgRequest * max(len(requests), 1))()
+        # every request's indices and multiplicities in one array each
+        xa = np.concatenate([r[0] for r in requests] or [np.zeros(0)]).astype(np.int32)
+        ra = np.concatenate([r[1] for r in requests] or [np.zeros(0)]).astype(np.int64)
+        px, pr = xa.ctypes.data, ra.ctypes.data
         for i, (x, reps, odd) in enumerate(requests):
-            xa = np.ascontiguousarray(x, dtype=np.int32)
-            ra = np.ascontiguousarray(reps, dtype=np.int64)
-            keep.append((xa, ra))
-            arr[i] = WgRequest(xa.ctypes.data, ra.ctypes.data, len(ra), -1 if odd is None else int(odd))
-        self._keep, self._arr = keep, arr
+            arr[i] = WgRequest(px, pr, len(reps), -1 if odd is None else int(odd))
+            px += 4 * len(x)
+            pr += 8 * len(reps)
+        self._keep, self._arr = (xa, ra), arr
         opt = WgPlanOptions(float(options.get("chunk_scale", 1.0)), int(options.get("max_warps_per_cta", 0)),
                             int(bool(options.get("merge_classes", False))), int(bool(options.get("use_graph", False))),
                             int(bool(options.get("serial_groups", False))), options.get("stream"))
@@ -442,6 +446,29 @@ def run(instances, precision="fp64", stream=0):
     check(lib.wg_run(arr, len(insts), PRECISIONS[precision],
                      out.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), ctypes.c_void_p(stream)))
     return (out[0::2] + 1j * out[1::2])[:total]
+
+
+def hafnian_direct(A, loop, rtol, atol):
+    """``hafnian(A, loop)`` of a float64 or complex128 C-contiguous square array by one native call
+    (``wg_hafnian_direct``), or None when the input needs the general route."""
+    lib = load()
+    out = (ctypes.c_double * 2)()
+    done = ctypes.c_int()
+    check(lib.wg_hafnian_direct(A.__array_interface__["data"][0], A.shape[0],
+                                WG_COMPLEX128 if A.dtype.kind == "c" else WG_FLOAT64, int(bool(loop)), float(rtol),
+                                float(atol), out, ctypes.byref(done)))
+    return np.complex128(complex(out[0], out[1])) if done.value else None
+
+
+def matched_reps(reps):
+    """Pairing of the repetition counts (an int64 array): (x, edge_reps, oddmode or None)."""
+    n = len(reps)
+    buf = np.empty(6 * n + 1, dtype=np.int64)
+    p = buf.__array_interface__["data"][0]
+    E, odd = ctypes.c_int(), ctypes.c_int()
+    check(load().wg_matched_reps(reps.__array_interface__["data"][0], n, p, p + 32 * n, ctypes.byref(E),
+                                 ctypes.byref(odd)))
+    return buf[:2 * E.value], buf[4 * n:4 * n + E.value], None if odd.value < 0 else odd.value
 
 
 def check_arith(op, x, x_lo=None, y=None, y_lo=None):

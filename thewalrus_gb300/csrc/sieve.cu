@@ -1576,6 +1576,147 @@ int wg_run(const wg_instance* inst, int count, int precision, double* out, void*
   return rc;
 }
 
+// An ordinary (loop) hafnian straight from the caller's matrix: the checks of the public function
+// (finite, symmetric and not diagonal in numpy.allclose's sense, not integer-valued, paired rows of
+// comparable sums), the pairing of single indices (n-1 with n-2, n-3 with n-4, ...; 0 is left over
+// when n is odd), and the run.  *done = 0, with nothing computed, whenever a check says that
+// the general route has to answer.
+int wg_hafnian_direct(const void* A, int n, int dtype, int loop, double rtol, double atol, double out[2], int* done) {
+  if (!done || !out || !A) return fail(WG_EINVAL, "NULL argument");
+  *done = 0;
+  if (n < 5 || (n % 2 && !loop) || n / 2 > MAX_EDGES || !(rtol >= 0) || !(atol >= 0)) return WG_OK;
+  if (dtype != WG_FLOAT64 && dtype != WG_COMPLEX128) return WG_OK;
+  const double* a = (const double*)A;
+  const size_t nn = (size_t)n * n;
+  const bool cx = dtype == WG_COMPLEX128;
+  bool imag = false, integral = true;
+  for (size_t k = 0; k < nn; ++k) {
+    const double re = cx ? a[2 * k] : a[k], im = cx ? a[2 * k + 1] : 0.0;
+    if (!(std::isfinite(re) && std::isfinite(im))) return WG_OK;
+    imag = imag || im != 0;
+    integral = integral && re == std::nearbyint(re);
+  }
+  if (!imag && integral) return WG_OK;
+  // real values of a complex matrix run the real tree
+  std::vector<double> real;
+  if (cx && !imag) {
+    real.resize(nn);
+    for (size_t k = 0; k < nn; ++k) real[k] = a[2 * k];
+    a = real.data();
+  }
+  auto mod = [&](int i, int j) {
+    const size_t k = (size_t)i * n + j;
+    return imag ? std::hypot(a[2 * k], a[2 * k + 1]) : std::fabs(a[k]);
+  };
+  bool diagonal = true;
+  std::vector<double> rows(n, 0.0);
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j < n; ++j) {
+      const double m = mod(i, j);
+      rows[i] += m;
+      if (i == j) {
+        if (loop) rows[i] += m;
+        continue;
+      }
+      diagonal = diagonal && m <= atol + rtol * m;
+      const size_t x = (size_t)i * n + j, y = (size_t)j * n + i;  // |A_ji - A_ij| against |A_ij|
+      const double d = imag ? (a[2 * x] == a[2 * y] && a[2 * x + 1] == a[2 * y + 1]
+                                   ? 0.0
+                                   : std::hypot(a[2 * y] - a[2 * x], a[2 * y + 1] - a[2 * x + 1]))
+                            : std::fabs(a[y] - a[x]);
+      if (!(d <= atol + rtol * m)) return WG_OK;
+    }
+  if (diagonal) return WG_OK;
+  const int E = n / 2;
+  std::vector<int> x(2 * E);
+  for (int e = 0; e < E; ++e) {
+    x[e] = n - 1 - 2 * e;
+    x[E + e] = n - 2 - 2 * e;
+    const double ra = rows[x[e]], rb = rows[x[E + e]];
+    if (ra > 0 && rb > 0 && !(ra <= 16.0 * rb && rb <= 16.0 * ra)) return WG_OK;  // _pair_balance's spread
+  }
+  const int w = imag ? 2 : 1, m = 2 * E;
+  std::vector<double> Ax((size_t)m * m * w), D, V;
+  for (int i = 0; i < m; ++i)
+    for (int j = 0; j < m; ++j) memcpy(&Ax[((size_t)i * m + j) * w], a + ((size_t)x[i] * n + x[j]) * w, sizeof(double) * w);
+  std::vector<int64_t> reps(E, 1);
+  wg_instance in;
+  memset(&in, 0, sizeof(in));
+  in.kind = loop ? WG_KIND_LOOP : WG_KIND_PLAIN;
+  in.n = m;
+  in.E = E;
+  in.dtype = imag ? WG_COMPLEX128 : WG_FLOAT64;
+  in.glynn = 1;
+  in.edge_reps = reps.data();
+  in.A = Ax.data();
+  if (loop) {
+    D.resize((size_t)m * w);
+    for (int i = 0; i < m; ++i) memcpy(&D[(size_t)i * w], a + ((size_t)x[i] * n + x[i]) * w, sizeof(double) * w);
+    in.D = D.data();
+    if (n % 2) {
+      V.resize((size_t)m * w);
+      for (int i = 0; i < m; ++i) memcpy(&V[(size_t)i * w], a + (size_t)x[i] * w, sizeof(double) * w);
+      in.has_odd = 1;
+      in.oddV = V.data();
+      memcpy(in.oddloop, a, sizeof(double) * w);
+    }
+  }
+  const int rc = wg_run(&in, 1, WG_PREC_FP64, out, nullptr);
+  if (!rc) *done = 1;
+  return rc;
+}
+
+// Pairing of repeated indices into edges with multiplicities (thewalrus/_hafnian.py:80-159): the two
+// largest remaining counts (ties: the larger index first) pair as often as the second allows; one
+// that exceeds twice the second, or is alone, pairs with itself.  x: the edges' first ends, then
+// their second ends (2 * *E entries, room for 4 n: an index pairs with itself at most once, which
+// leaves it 1 or 0, and every other edge uses an index up, so there are at most 2 n edges); mult: *E
+// entries (room for 2 n); *odd: the index left over, or -1.
+int wg_matched_reps(const int64_t* reps, int n, int64_t* x, int64_t* mult, int* E, int* odd) {
+  if ((n > 0 && (!reps || !x || !mult)) || n < 0 || !E || !odd) return fail(WG_EINVAL, "bad pairing arguments");
+  *E = 0;
+  *odd = -1;
+  int64_t sum = 0;
+  std::vector<std::pair<int64_t, int>> pool;  // a heap by count, then index
+  for (int i = 0; i < n; ++i) {
+    sum += reps[i];
+    if (reps[i] > 0) pool.emplace_back(reps[i], i);
+  }
+  if (sum == 0) return WG_OK;
+  std::make_heap(pool.begin(), pool.end());
+  auto pop = [&] {
+    std::pop_heap(pool.begin(), pool.end());
+    const auto t = pool.back();
+    pool.pop_back();
+    return t;
+  };
+  auto push = [&](int64_t r, int i) {
+    pool.emplace_back(r, i);
+    std::push_heap(pool.begin(), pool.end());
+  };
+  std::vector<int64_t> right;
+  int e = 0;
+  while (pool.size() > 1 || (pool.size() == 1 && pool.front().first > 1)) {
+    const auto top = pop();
+    if (pool.empty() || top.first > 2 * pool.front().first) {
+      x[e] = top.second;
+      right.push_back(top.second);
+      mult[e++] = top.first / 2;
+      if (top.first % 2) push(1, top.second);
+    } else {
+      const auto sec = pop();
+      x[e] = top.second;
+      right.push_back(sec.second);
+      mult[e++] = sec.first;
+      if (top.first > sec.first) push(top.first - sec.first, top.second);
+    }
+  }
+  std::copy(right.begin(), right.end(), x + e);
+  *E = e;
+  if (pool.size() == 1) *odd = pool.front().second;
+  return WG_OK;
+}
+
 int wg_hafnian(const void* A, int n, int dtype, const int64_t* edge_reps, int E, int glynn, int precision,
                double out[2], void* stream) {
   wg_instance in;

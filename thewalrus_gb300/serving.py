@@ -103,7 +103,8 @@ class GaussianState:
 
     def norm(self, pattern):
         """<0|psi> / sqrt(prod n_i!) for the pattern."""
-        return self.vacuum / math.sqrt(float(np.prod([math.factorial(int(k)) for k in pattern])))
+        counts = pattern.tolist() if isinstance(pattern, np.ndarray) else pattern
+        return self.vacuum / math.sqrt(float(math.prod([math.factorial(int(k)) for k in counts if k > 1])))
 
     def trivial_loop_hafnian(self, pattern):
         """The loop hafnian for patterns with at most one photon (no sieve needed), else None."""
@@ -169,7 +170,7 @@ class ProbabilityServer:
         (loop kind: the first radix halved unless there is an unpaired mode) times (m + 1)^3 for
         the largest bordered term matrix, m = 2 * (edges with a nonzero repetition)."""
         _, reps, odd = triple
-        reps = [int(r) for r in reps]
+        reps = np.asarray(reps).tolist()
         if not reps:
             return 0.0
         steps = float((reps[0] + 2) // 2 if odd is None else reps[0] + 1)
@@ -212,13 +213,14 @@ class ProbabilityServer:
                 nxt += 1
                 progressed = True
                 _, sidx, pat = requests[j]
-                triv = self.states[sidx].trivial_loop_hafnian(pat)
+                photons = int(np.asarray(pat).sum())
+                triv = self.states[sidx].trivial_loop_hafnian(pat) if photons < 2 else None
                 if triv is not None:  # no photons or one: answered without the sieve
                     self._finish(results, requests, j, triv, time.perf_counter() - t0, -1, time_scale)
                     done += 1
                     continue
                 triple = matched_reps(pat)
-                info[j] = (self.request_cost(triple), triple, int(np.sum(pat)))
+                info[j] = (self.request_cost(triple), triple, photons)
                 pending.append(j)
             # completions
             for fl in list(inflight):
@@ -282,7 +284,7 @@ class ProbabilityServer:
         arr = arr * time_scale
         amp = lhaf * self.states[sidx].norm(pat)
         results[j] = {"amplitude": amp, "probability": abs(amp) ** 2, "arrival": arr, "done": tdone,
-                      "latency": tdone - arr, "batch": bid, "photons": int(np.sum(pat))}
+                      "latency": tdone - arr, "batch": bid, "photons": int(np.asarray(pat).sum())}
 
 
 def summary(results, makespan=None):
