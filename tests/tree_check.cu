@@ -98,6 +98,12 @@ static void phase(const TreeInst& T, const TreeSeg& G, const unsigned char* pool
     case TP_FIRST: tree_first<hc>(T, pool, chi, tid, nthr); break;
     case TP_M: tree_m<hc, TL>(T, G.q, par, G.pstride, G.np, scr, tid, nthr); break;
     case TP_UNIT: tree_unit<hc, TL>(T, G.q, par, G.pstride, G.np, G.fused ? nullptr : scr, chi, tid, nthr); break;
+    case TP_G2:
+      tree_g2<hc>(T, G.q, par, G.pstride, G.np, scr + (2ll * tree_width(T.X, T.E, G.q + 1)) * (T.deg[G.q] + 1) * G.np, chi,
+                  sm, smn, tid, nthr);
+      break;
+    case TP_W2: tree_w2<hc, TL>(T, G.q, par, G.pstride, G.np, scr, tid, nthr); break;
+    case TP_MULTI2: tree_multi2<hc, TL>(T, G.q, par, G.pstride, G.np, scr, chi, tid, nthr); break;
     case TP_PREP: tree_prep<hc>(T, G.q, par, G.pstride, G.np, scr, chi, sm, smn, tid, nthr); break;
     case TP_Y: tree_y<hc, TL>(T, G.q, par, G.pstride, G.np, scr, y, tid, nthr); break;
     case TP_MULTI: tree_multi<hc, TL>(T, G.q, par, G.pstride, G.np, y, chi, tid, nthr); break;
@@ -175,7 +181,7 @@ int main() {
       // chip 32: the phases that do not stage their series in shared memory
       const int smn = chip > 32 ? P.smem : (T.pB >= 0 ? 5 * (T.deg[T.steps] + 1) + 32 : 0);
       // every lane of the segment's warps as one thread (warp-wide phases: a warp of one lane)
-      const bool wide = G.phase == TP_PREP || G.phase == TP_GLOOP || (G.phase == TP_LEAF && T.pB >= 0);
+      const bool wide = G.phase == TP_PREP || G.phase == TP_GLOOP || G.phase == TP_G2 || (G.phase == TP_LEAF && T.pB >= 0);
       const int nthr = wide ? warps : warps * 32;
       for (int t = 0; t < nthr; ++t) {
         if (G.tile == 0) phase<0>(T, G, pool, par, chi, scr, sm.data(), smn, t, nthr, out[G.inst].data());

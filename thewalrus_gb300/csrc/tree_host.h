@@ -91,6 +91,7 @@ static inline long long tree_node_elems(const TreeInst& T, int q) {
 static inline long long tree_scratch_elems(const TreeInst& T, int q, long long np) {
   if (q == T.steps) return T.pO >= 0 && T.steps < T.E ? np * (T.deg[q] + 1) : 0;
   if (T.reps[q] == 1) return T.pL >= 0 ? np * (T.deg[q] + 1) : 0;
+  if (T.reps[q] == 2) return np * (T.deg[q] + 1) * (8 + 2ll * tree_width(T.X, T.E, q + 1));
   return np * T.radix[q] * (T.deg[q + 1] + 1) * (6 + 2ll * tree_width(T.X, T.E, q + 1));
 }
 
@@ -121,7 +122,7 @@ static inline void tree_levels(const TreeInst& T, int sb, double budget, TreeLev
       cap = c * R;
       scr = std::max(scr, tree_scratch_elems(T, q - 1, c) * sb);
       walks *= (double)((g.cap[q - 1] + c - 1) / c);
-      g.phases += walks * (T.reps[q - 1] == 1 ? (T.pL >= 0 ? 2 : 1) : 4);
+      g.phases += walks * (T.reps[q - 1] == 1 ? (T.pL >= 0 ? 2 : 1) : (T.reps[q - 1] == 2 ? 2 : 4));
     }
     if (nodes < (double)cap) cap = (long long)nodes;
     g.cap[q] = cap;
@@ -155,6 +156,11 @@ static void tree_walk(const TreeInst& T, const TreeLevels& g, int q, int np, dou
     if (T.reps[q] == 1) {
       if (T.pL >= 0 && !tree_fused(T, q, c, threads)) f(TP_M, q, p0, c, np);
       f(TP_UNIT, q, p0, c, np);
+    } else if (T.reps[q] == 2) {
+      const bool rows = tree_width(T.X, T.E, q + 1) > 0;
+      if (rows) f(TP_W2, q, p0, c, np);
+      f(TP_G2, q, p0, c, np);  // beside TP_W2, in the same round
+      if (rows) f(TP_MULTI2, q, p0, c, np);
     } else {
       f(TP_PREP, q, p0, c, np);
       if (tree_width(T.X, T.E, q + 1) > 0) {
@@ -171,7 +177,7 @@ static void tree_walk(const TreeInst& T, const TreeLevels& g, int q, int np, dou
 // multiply-adds
 static inline double tree_items(const TreeInst& T, int phase, int q, double np, int tile) {
   if (tile == 0) {
-    const bool whole = phase == TP_ROOT || phase == TP_FIRST || phase == TP_PREP || phase == TP_GLOOP ||
+    const bool whole = phase == TP_ROOT || phase == TP_FIRST || phase == TP_PREP || phase == TP_GLOOP || phase == TP_G2 ||
                        (phase == TP_LEAF && (T.pB >= 0 || T.steps == T.E));
     return tree_items(T, phase, q, np, 1) * (whole ? 1 : 4);
   }
@@ -183,6 +189,9 @@ static inline double tree_items(const TreeInst& T, int phase, int q, double np, 
     case TP_M: return np * tree_tiles(Lp, tile);
     case TP_UNIT: return np * tree_tiles(Lp, tile) * tree_entries(W, T.diag);
     case TP_PREP: case TP_GLOOP: return 32 * nc;
+    case TP_G2: return 32 * np;
+    case TP_W2: return np * 2 * W * tree_tiles(Lp, tile);
+    case TP_MULTI2: return np * (tree_entries(W, T.diag) - 1) * tree_tiles(Lp + 1, tile);
     case TP_Y: return nc * 2 * W * tree_tiles(Lc, tile);
     case TP_MULTI: return nc * (tree_entries(W, T.diag) - 1) * tree_tiles(Lc, tile);
     default: return T.pB >= 0 ? 32 * np : np * (T.steps < T.E ? tree_tiles(Lp, tile) : 1);
@@ -198,6 +207,9 @@ static inline double tree_macs(const TreeInst& T, int phase, int q, double np) {
     case TP_UNIT: return np * tp * (2 * tree_entries((int)W, T.diag) - 1);
     case TP_PREP: return nc * 12 * tc * std::max(1.0, 32 / Lc);
     case TP_GLOOP: return nc * 5 * tc * std::max(1.0, 32 / Lc);
+    case TP_G2: return np * 8 * tp * std::max(1.0, 10 / Lp);
+    case TP_W2: return np * 4 * W * tp;
+    case TP_MULTI2: return np * 4 * (tree_entries((int)W, T.diag) - 1) * tp;
     case TP_Y: return nc * 4 * W * tc;
     case TP_MULTI: return nc * 2 * (tree_entries((int)W, T.diag) - 1) * tc;
     default: return np * (T.pB >= 0 ? 3.0 * T.nout : 3.0) * tp;
@@ -211,9 +223,10 @@ static inline int tree_smem(const TreeInst& T, int most) {
   const int L = T.deg[T.steps] + 1;
   int need = 1, lc = 0;
   for (int q = 0; q < T.steps; ++q)
-    if (T.reps[q] > 1) lc = std::max(lc, T.deg[q + 1] + 1);
+    if (T.reps[q] > 1) lc = std::max(lc, T.deg[q + 1] + 1);  // 8 series of a double edge, 9 of the others
   if (9 * lc <= most) need = std::max(need, 9 * lc);
-  if (T.pB >= 0) need = std::max(need, 7 * L + 32 <= most ? 7 * L + 32 : 5 * L + 32);
+  const int all = 32 + (T.nout + 4) * L;
+  if (T.pB >= 0) need = std::max(need, all <= most ? all : 5 * L + 32);
   return need;
 }
 
@@ -241,6 +254,7 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
     P.smem = std::max(P.smem, tree_smem(T, (64 << 10) / (TREE_THREADS / 32) / sb));
     const double fuse_threads = chip_threads / (double)insts.size();
     size_t r = 0;
+    int last = -1;
     auto add = [&](int phase, int q, int p0, int np, int ps) {
       TreeSeg s;
       memset(&s, 0, sizeof(s));
@@ -253,6 +267,8 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
       s.phase = (unsigned char)phase;
       s.q = (unsigned char)q;
       s.fused = phase == TP_UNIT && T.pL >= 0 && tree_fused(T, q, np, fuse_threads);
+      if (phase == TP_G2 && last == TP_W2) --r;
+      last = phase;
       if (rounds.size() <= r) rounds.emplace_back();
       rounds[r++].push_back(s);
     };
@@ -284,7 +300,7 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
     });
     for (TreeSeg& s : R) {
       const TreeInst& T = insts[s.inst];
-      s.tile = (unsigned char)(s.fused ? 0 : use);
+      s.tile = (unsigned char)(s.fused ? 0 : (use == 1 && (s.phase == TP_W2 || s.phase == TP_MULTI2) ? tile : use));
       long long warps = (long long)((tree_items(T, s.phase, s.q, s.np, s.tile) + 31) / 32);
       // leaves: at most the chip's warps, each with a partial for the reduction; the CTAs of a
       // single instance keep their sums over all leaf rounds and leave one partial each

@@ -15,7 +15,8 @@
 // its signs cancel.  The step is
 //   C_ab' = C_ab + delta eta (C_ia C_jb + C_ja C_ib),   g' = g (1 + delta eta (C_ij + v_i v_j)),
 // with v as one more row of C (position pL), and both signs share the products.  No divisions and
-// no pivots.  Multiple edges take the whole 2 x 2 block, P = (X_e^-1 - C_ee)^-1:
+// no pivots.  Double edges go to second order likewise (tree_w2); higher multiplicities take the
+// whole 2 x 2 block, P = (X_e^-1 - C_ee)^-1:
 //   C' = C + C_re P C_er,   g' = g det(I - X_e C_ee)^(-1/2) exp(v_e^T P v_e / 2).
 // delta -> -delta leaves a term's share unchanged (degree K in the deltas, as the weights), so
 // the first edge takes half of its signs.  The last simple edges close: two of them in the hafnian
@@ -84,7 +85,7 @@ struct alignas(16) TreeInst {
 // The program of a launch: rounds of segments, with a barrier of the whole launch after each round.
 // A segment is one phase of one step of one instance over a block of parents [p0, p0 + np) of a
 // level of pstride nodes, by the round's warps [warp0, next segment's warp0).
-enum TreePhase : int { TP_ROOT = 0, TP_FIRST, TP_M, TP_UNIT, TP_PREP, TP_Y, TP_MULTI, TP_GLOOP, TP_LEAF };
+enum TreePhase : int { TP_ROOT = 0, TP_FIRST, TP_M, TP_UNIT, TP_PREP, TP_Y, TP_MULTI, TP_GLOOP, TP_W2, TP_G2, TP_MULTI2, TP_LEAF };
 struct alignas(16) TreeSeg {
   long long par, chi;        // workspace byte offsets of the parents' and the children's level
   int inst, warp0;
@@ -263,8 +264,13 @@ struct TreeMatrix<c3<R, C>> {
 // the running sum of a series product
 template <class S>
 struct ConvAcc : RealAcc<S> {
+  using U = S;  // the sum as an addend
 #pragma nv_exec_check_disable
   __host__ __device__ static __forceinline__ ConvAcc of(S x) { return {RealAcc<S>::of(x)}; }
+#pragma nv_exec_check_disable
+  __host__ __device__ __forceinline__ U parts() const { return this->sum(); }
+#pragma nv_exec_check_disable
+  __host__ __device__ static __forceinline__ S plus(S c, U u) { return Ar<S>::add(c, u); }
 };
 template <class R, class C>
 struct ConvAcc<c3<R, C>> {
@@ -277,9 +283,14 @@ struct ConvAcc<c3<R, C>> {
     p2.fma(a.im, b.im);
     p3.fma(a.s, b.s);
   }
-  __device__ __forceinline__ c3<R, C> sum() const {
+  using U = C;  // without re + im, which an addend does not need (an FP64 instruction a sum)
+  __device__ __forceinline__ U parts() const {
     const R x = p1.sum(), y = p2.sum();
-    return Ar<c3<R, C>>::of(Ar<R>::sub(x, y), Ar<R>::sub(Ar<R>::sub(p3.sum(), x), y));
+    return {Ar<R>::sub(x, y), Ar<R>::sub(Ar<R>::sub(p3.sum(), x), y)};
+  }
+  __device__ __forceinline__ c3<R, C> sum() const { return Ar<c3<R, C>>::of(parts()); }
+  __device__ static __forceinline__ c3<R, C> plus(c3<R, C> c, U u) {
+    return Ar<c3<R, C>>::of(Ar<R>::add(c.re, u.re), Ar<R>::add(c.im, u.im));
   }
 };
 
@@ -292,23 +303,23 @@ __host__ __device__ __forceinline__ void tst(S* p, S v) { *p = v; }
 // acc[k] += sum_s a_s b_(t0+k-s), k < T, s < la: coefficients t0 .. t0+T-1 of a product of two
 // series (element stride sa, sb).  A window of T coefficients of b slides through registers, so a
 // step is one load of each series and T multiply-adds; the last T-1 steps are the triangle where b
-// runs out.  t0 < 0: only the coefficients t0 + k >= 0.
+// runs out.  t0 < 0: only the coefficients t0 + k >= 0.  b has lb coefficients.
 #pragma nv_exec_check_disable
 template <class S, int T>
 __host__ __device__ __forceinline__ void conv_tile(ConvAcc<S> (&acc)[T], const S* a, long long sa, int la, const S* b,
-                                          long long sb, int t0) {
+                                          long long sb, int t0, int lb = 1 << 30) {
   if (t0 < 0) {
 #pragma unroll
     for (int k = 1; k < T; ++k) {
       const int t = t0 + k;
       if (t >= 0)
-        for (int s = 0; s <= t && s < la; ++s) acc[k].fma(tld(a + s * sa), tld(b + (t - s) * sb));
+        for (int s = t < lb ? 0 : t - lb + 1; s <= t && s < la; ++s) acc[k].fma(tld(a + s * sa), tld(b + (t - s) * sb));
     }
     return;
   }
   S w[T];
 #pragma unroll
-  for (int k = 0; k < T; ++k) w[k] = tld(b + (t0 + k) * sb);
+  for (int k = 0; k < T; ++k) w[k] = t0 + k < lb ? tld(b + (t0 + k) * sb) : Ar<S>::zero();
   const int n = t0 < la ? t0 : la;  // steps that slide the window
   const S* pa = a;
   const S* pb = b + (t0 - 1) * sb;
@@ -557,12 +568,15 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
                                                  pp + tree_ent(j, T.pL, dg) * st, ps, Lp, t - s));
         }
       }
-      const S u = split_sum(acc.sum());
-      if (live && sub < 2) {  // thread 0 stores the +1 child, thread 1 the -1 child
+      using CA = ConvAcc<S>;
+      const typename CA::U u = split_sum(acc.parts());
+      if (live && sub < 2) {  // thread 0 stores the +1 child, thread 1 the -1 child, in the same instructions
         S* o = chi + (long long)e * Lc * cs + p;
         for (int h = sub; h < (WG_TREE_SPLIT > 1 ? sub + 1 : 2) && h < nd; ++h) {
-          tst(o + h * np + (t + 1) * cs, h == 0 ? A::add(c, u) : (e == 0 ? A::sub(u, c) : A::sub(c, u)));
-          if (t == 0) tst(o + h * np, h == 1 && e == 0 ? A::neg(c0) : c0);
+          const S v = CA::plus(c, h ? Ar<typename CA::U>::neg(u) : u);
+          const bool flip = h == 1 && e == 0;
+          tst(o + h * np + (t + 1) * cs, flip ? A::neg(v) : v);
+          if (t == 0) tst(o + h * np, flip ? A::neg(c0) : c0);
         }
       }
     }
@@ -597,10 +611,18 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
       if (k < 0 ? t0 <= 0 : t >= 0) {
         const int tc = k < 0 ? 0 : t + 1;
         const S c = tc < Lp ? tld(base + tc * ps) : A::zero();
-        const S u = k < 0 ? A::zero() : acc[k < 0 ? 0 : k].sum();
         S* w = o + tc * cs;
-        tst(w, A::add(c, u));
-        if (nd > 1) tst(w + np, e == 0 ? A::sub(u, c) : A::sub(c, u));
+        if (k < 0) {
+          tst(w, c);
+          if (nd > 1) tst(w + np, e == 0 ? A::neg(c) : c);
+        } else {
+          const typename ConvAcc<S>::U u = acc[k < 0 ? 0 : k].parts();
+          tst(w, ConvAcc<S>::plus(c, u));
+          if (nd > 1) {
+            const S v = ConvAcc<S>::plus(c, Ar<typename ConvAcc<S>::U>::neg(u));
+            tst(w + np, e == 0 ? A::neg(v) : v);
+          }
+        }
       }
     }
   }
@@ -822,6 +844,175 @@ __host__ __device__ void tree_multi(const TreeInst& T, int q, const S* par, long
   }
 }
 
+// ---- a double edge.  To second order in z = delta eta (higher orders use the edge three times),
+//   C' = C + z (c_i c_j^T + c_j c_i^T) + z^2 (c_i w_i^T + c_j w_j^T),  w_i = C_jj c_i + C_ij c_j,  w_j = C_ij c_i + C_ii c_j,
+//   g' = g (1 + z M + z^2 (M^2 - w^2 + A B / 2)),  w = v_i v_j, M = C_ij + w, A = C_ii + v_i^2, B = C_jj + v_j^2,
+// for z = 2, 0, -2 times eta: no recurrences, and the products serve all three children.
+// w_i, w_j of every remaining row: y[((2 b + s) Lp + t) np + p]
+#pragma nv_exec_check_disable
+template <class S, int TL>
+__host__ __device__ void tree_w2(const TreeInst& T, int q, const S* par, long long ps, int np, S* y, int tid, int nthr) {
+  using A = Ar<S>;
+  const int i = T.X + 2 * (T.E - 1 - q), j = i + 1, W = i, Lp = T.deg[q] + 1;
+  const long long st = (long long)Lp * ps;
+  constexpr int TT = TL ? TL : 1, SP = TL ? 1 : WG_TREE_SPLIT;
+  const int nt = (Lp + TT - 1) / TT, total = nt * 2 * W * np, sub = tid % SP;
+  for (int x0 = 0; x0 < total; x0 += nthr / SP) {
+    const int x = x0 + tid / SP, r = x / np, p = x - r * np, bs = r % (2 * W), t0 = Lp - TT * (r / (2 * W) + 1);
+    const int b = bs >> 1, s = bs & 1;
+    const S* pp = par + p;
+    const S *ci = pp + tree_ent(i, b, T.diag) * st, *cj = pp + tree_ent(j, b, T.diag) * st;
+    const S *m0 = pp + (s ? tree_ent(j, i, 1) : tree_ent(j, j, 1)) * st;
+    const S *m1 = pp + (s ? tree_ent(i, i, 1) : tree_ent(j, i, 1)) * st;
+    ConvAcc<S> acc[TT];
+#pragma unroll
+    for (int k = 0; k < TT; ++k) acc[k] = ConvAcc<S>::of(A::zero());
+    if constexpr (TL == 0) {
+      if (x < total) conv_part2(acc[0], ci, m0, cj, m1, ps, Lp, ps, t0, sub);
+      const S v = split_sum(acc[0].sum());
+      if (x < total && sub == 0) tst(y + ((long long)bs * Lp + t0) * np + p, v);
+    } else if (x < total) {
+      conv_tile<S, TT>(acc, ci, ps, Lp, m0, ps, t0);
+      conv_tile<S, TT>(acc, cj, ps, Lp, m1, ps, t0);
+#pragma unroll
+      for (int k = 0; k < TT; ++k)
+        if (t0 + k >= 0) tst(y + ((long long)bs * Lp + t0 + k) * np + p, acc[k].sum());
+    }
+  }
+}
+
+// the children's entries: child coefficient t = U1_(t-1) z + U2_(t-2) z^2 + C_t, a tile over t - 1
+#pragma nv_exec_check_disable
+template <class S, int TL>
+__host__ __device__ void tree_multi2(const TreeInst& T, int q, const S* par, long long ps, int np, const S* y, S* chi,
+                                     int tid, int nthr) {
+  using A = Ar<S>;
+  using CA = ConvAcc<S>;
+  const int i = T.X + 2 * (T.E - 1 - q), j = i + 1, dg = T.diag, nd = T.radix[q];
+  const int ne = tree_entries(i, dg) - 1, Lp = T.deg[q] + 1, Lc = Lp + 2, Lt = Lp + 1;
+  const long long st = (long long)Lp * ps, yt = (long long)Lp * np, cs = (long long)np * nd;
+  constexpr int TT = TL ? TL : 1, SP = TL ? 1 : WG_TREE_SPLIT;
+  const unsigned nt = (Lt + TT - 1) / TT, total = nt * ne * np;
+  const int sub = tid % SP;
+  for (unsigned x0 = 0; x0 < total; x0 += nthr / SP) {
+    const unsigned x = x0 + tid / SP, r = x / np;
+    const int p = x - r * np, e = 1 + r % ne, t0 = Lt - TT * ((int)(r / ne) + 1);
+    int a, b;
+    tree_decode(e, dg, a, b);
+    const bool live = x < total && tree_need(T, a, b);
+    const S* pp = par + p;
+    const S *ia = pp + tree_ent(i, a, dg) * st, *ja = pp + tree_ent(j, a, dg) * st;
+    const S *wi = y + 2 * b * yt + p, *wj = wi + yt;
+    CA u1[TT], u2[TT];
+#pragma unroll
+    for (int k = 0; k < TT; ++k) u1[k] = u2[k] = CA::of(A::zero());
+    if (live) {
+      const S *ib = pp + tree_ent(i, b, dg) * st, *jb = pp + tree_ent(j, b, dg) * st;
+      if constexpr (TL == 0) {
+        if (t0 < Lp) conv_part2(u1[0], ia, jb, ja, ib, ps, Lp, ps, t0, sub);
+        if (t0 > 0) conv_part2(u2[0], ia, wi, ja, wj, ps, Lp, (long long)np, t0 - 1, sub);
+      } else {
+        conv_tile<S, TT>(u1, ia, ps, Lp, jb, ps, t0, Lp);
+        conv_tile<S, TT>(u1, ja, ps, Lp, ib, ps, t0, Lp);
+        conv_tile<S, TT>(u2, ia, ps, Lp, wi, np, t0 - 1, Lp);
+        conv_tile<S, TT>(u2, ja, ps, Lp, wj, np, t0 - 1, Lp);
+      }
+    }
+    const S* base = pp + e * st;
+    S* o = chi + (long long)e * Lc * cs + p;
+#pragma unroll
+    for (int k = -1; k < TT; ++k) {  // child coefficient t0 + k + 1; k = -1: coefficient 0
+      const int t = t0 + k + 1;
+      if (k < 0) {
+        if (live && t0 <= 0 && sub == 0)
+          for (int d = 0; d < nd; ++d) tst(o + d * np, tld(base));
+        continue;
+      }
+      S v1 = u1[k < 0 ? 0 : k].sum(), v2 = u2[k < 0 ? 0 : k].sum();
+      if constexpr (TL == 0) {
+        v1 = split_sum(v1);
+        v2 = split_sum(v2);
+      }
+      if (!live || t < 1 || sub != 0) continue;
+      const S c = t < Lp ? tld(base + t * ps) : A::zero();
+      const S even = A::add(c, tree_times(v2, 4)), odd = tree_times(v1, 2);
+      S* w = o + t * cs;
+      tst(w, A::add(even, odd));
+      if (nd > 1) tst(w + np, c);
+      if (nd > 2) tst(w + 2 * np, A::sub(even, odd));
+    }
+  }
+}
+
+// the children's g, one warp per parent; series in the warp's shared memory, or in `wk` (8 Lp np)
+#pragma nv_exec_check_disable
+template <class S>
+__host__ __device__ void tree_g2(const TreeInst& T, int q, const S* par, long long ps, int np, S* wk, S* chi, S* sm,
+                                 int smn, int tid, int nthr) {
+  using A = Ar<S>;
+  const int i = T.X + 2 * (T.E - 1 - q), j = i + 1, nd = T.radix[q], Lp = T.deg[q] + 1;
+  const long long st = (long long)Lp * ps, cs = (long long)np * nd;
+  const int lane = tid & (WG_TREE_LANES - 1);
+  const bool loops = T.pL >= 0;
+  for (int p = tid / WG_TREE_LANES; p < np; p += nthr / WG_TREE_LANES) {
+    S* w0 = smn >= 8 * Lp ? sm : wk + 8ll * Lp * p;
+    auto ser = [&](int f, int t) -> S& { return w0[f * Lp + t]; };  // g, M, A, B, w, v_i, v_j, second order
+    const S* pp = par + p;
+    for (int t = lane; t < Lp; t += WG_TREE_LANES) {
+      ser(0, t) = tld(pp + t * ps);
+      ser(1, t) = tld(pp + tree_ent(j, i, 1) * st + t * ps);
+      ser(2, t) = tld(pp + tree_ent(i, i, 1) * st + t * ps);
+      ser(3, t) = tld(pp + tree_ent(j, j, 1) * st + t * ps);
+      if (loops) {
+        ser(5, t) = tld(pp + tree_ent(i, T.pL, 1) * st + t * ps);
+        ser(6, t) = tld(pp + tree_ent(j, T.pL, 1) * st + t * ps);
+      }
+    }
+    WG_TREE_SYNCWARP();
+    if (loops) {  // w, v_i^2, v_j^2 side by side over the lanes
+      for (int x = lane; x < 3 * Lp; x += WG_TREE_LANES) {
+        const int f = x / Lp, t = x - f * Lp;
+        const S *u = w0 + (f == 2 ? 6 : 5) * Lp, *v = w0 + (f == 1 ? 5 : 6) * Lp;
+        const S r = conv_one(u, 1, Lp, v, 1, Lp, t);
+        if (f == 0) {
+          ser(4, t) = r;
+          ser(1, t) = A::add(ser(1, t), r);
+        } else {
+          ser(f + 1, t) = A::add(ser(f + 1, t), r);
+        }
+      }
+      WG_TREE_SYNCWARP();
+    }
+    for (int t = lane; t < Lp; t += WG_TREE_LANES) {
+      ConvAcc<S> x = ConvAcc<S>::of(A::zero()), y = x, z = x;
+      for (int s = 0; s <= t; ++s) {
+        x.fma(ser(1, s), ser(1, t - s));
+        y.fma(ser(2, s), ser(3, t - s));
+        if (loops) z.fma(ser(4, s), ser(4, t - s));
+      }
+      S r = A::add(x.sum(), tree_half(y.sum()));
+      if (loops) r = A::sub(r, z.sum());
+      ser(7, t) = r;
+    }
+    WG_TREE_SYNCWARP();
+    for (int x = lane; x < 2 * Lp; x += WG_TREE_LANES) {  // g M and g times the second order
+      const int f = x / Lp, t = x - f * Lp;
+      ser(5 + f, t) = conv_one((const S*)w0, 1, Lp, (const S*)(w0 + (f ? 7 : 1) * Lp), 1, Lp, t);
+    }
+    WG_TREE_SYNCWARP();
+    for (int x = lane; x < nd * (Lp + 2); x += WG_TREE_LANES) {
+      const int d = x / (Lp + 2), t = x - d * (Lp + 2);
+      S r = t < Lp ? ser(0, t) : A::zero();
+      if (d != 1) {
+        if (t >= 1 && t - 1 < Lp) r = A::add(r, tree_times(ser(5, t - 1), 2 - 2 * d));
+        if (t >= 2) r = A::add(r, tree_times(ser(6, t - 2), 4));
+      }
+      tst(chi + t * cs + d * np + p, A::scale(r, tree_weight(T, q, d)));
+    }
+    WG_TREE_SYNCWARP();
+  }
+}
+
 // loop kinds: g' = w g h exp(v_e Y(L) / 2), one warp per child; shared memory as in tree_prep
 #pragma nv_exec_check_disable
 template <class S>
@@ -943,11 +1134,16 @@ __host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, i
     }
   } else {
     // batch mode b with loop series v and pair series c: k photons give H_k = v H_(k-1) +
-    // (k-1) c H_(k-2); with an unpaired vertex o: v_o H_k + k c_ob H_(k-1).  One warp per node, its
-    // output sums and work series (and, when they fit, v and c) in the warp's shared memory.
+    // (k-1) c H_(k-2); with an unpaired vertex o: v_o H_k + k c_ob H_(k-1).  One warp per node, the
+    // series and the output sums in its shared memory.  An FP64 instruction takes its 64 clocks
+    // however few lanes it has, so the lanes split: four to a coefficient, then four to an output
+    // (12 modes, cutoff 6: 53,000 clocks with a lane per coefficient and a warp sum per output).
     const int lane = tid & (WG_TREE_LANES - 1), nw = nthr / WG_TREE_LANES;
-    const bool staged = smn >= 7 * L + 32;
-    S *const o = sm, *const base = sm + 32, *gv = base + 3 * L, *gc = base + 4 * L;
+    const int sub = lane % WG_TREE_SPLIT, grp = lane / WG_TREE_SPLIT;
+    constexpr int NG = WG_TREE_LANES / WG_TREE_SPLIT;
+    const bool staged = smn >= 32 + (T.nout + 4) * L;  // every H_k kept, and copies of v and c
+    const int rows = staged ? T.nout : 3;
+    S *const o = sm, *const h = sm + 32, *gv = h + rows * L, *gc = gv + L;
     for (int k = lane; k < T.nout; k += WG_TREE_LANES) o[k] = A::zero();
     WG_TREE_SYNCWARP();
     for (int p = tid / WG_TREE_LANES; p < np; p += nw) {
@@ -955,43 +1151,57 @@ __host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, i
       TreeSer<S> v = {const_cast<S*>(pp + (long long)tree_ent2(T.pB, T.pL, dg) * st), ps};
       TreeSer<S> c = {const_cast<S*>(pp + (long long)tree_ent(T.pB, T.pB, 1) * st), ps};
       if (staged) {
-        v = ser_stage<S>(v.p, ps, L, base + 5 * L, lane);
-        c = ser_stage<S>(c.p, ps, L, base + 6 * L, lane);
+        v = ser_stage<S>(v.p, ps, L, gc + L, lane);
+        c = ser_stage<S>(c.p, ps, L, gc + 2 * L, lane);
       }
-      S *h0 = base, *h1 = base + L, *h2 = base + 2 * L;
       for (int t = lane; t < L; t += WG_TREE_LANES) {
-        h0[t] = A::zero();
-        h1[t] = t == 0 ? A::one() : A::zero();
+        h[t] = t == 0 ? A::one() : A::zero();
         if (T.pO >= 0) {
           gv[t] = conv_one(pp, ps, L, pp + (long long)tree_ent2(T.pO, T.pL, dg) * st, ps, L, t);
           gc[t] = conv_one(pp, ps, L, pp + (long long)tree_ent2(T.pO, T.pB, dg) * st, ps, L, t);
         } else {
           gv[t] = tld(pp + t * ps);
-          gc[t] = A::zero();
         }
       }
       WG_TREE_SYNCWARP();
-      for (int k = 0; k < T.nout; ++k) {  // h1 = H_k, h0 = H_(k-1)
-        S part = A::zero();
-        for (int t = lane; t < L; t += WG_TREE_LANES) {
-          part = A::fma(gv[D - t], h1[t], part);
-          if (k && T.pO >= 0) part = A::fma(tree_times(gc[D - t], k), h0[t], part);
-          if (k + 1 < T.nout) {
-            S n = conv_ser(v, L, TreeSer<S>{h1, 1}, L, t);
-            if (k) n = A::add(n, tree_times(conv_ser(c, L, TreeSer<S>{h0, 1}, L, t), k));
-            h2[t] = n;
+      // the dots of outputs k0 .. k1 - 1
+      auto dots = [&](int k0, int k1) {
+        for (int kb = k0; kb < k1; kb += NG) {
+          const int k = kb + grp;
+          ConvAcc<S> x = ConvAcc<S>::of(A::zero()), y = x;
+          if (k < k1) {
+            const S *hk = h + (k % rows) * L, *hl = h + ((k + rows - 1) % rows) * L;
+            for (int t = sub; t < L; t += WG_TREE_SPLIT) {
+              x.fma(gv[D - t], hk[t]);
+              if (k && T.pO >= 0) y.fma(gc[D - t], hl[t]);
+            }
           }
+          S r = x.sum();
+          if (T.pO >= 0) r = A::add(r, tree_times(y.sum(), k));
+          r = split_sum(r);
+          if (k < k1 && sub == 0) o[k] = A::add(o[k], r);
         }
-#ifdef __CUDA_ARCH__
-        part = warp_sum(part);
-#endif
-        if (lane == 0) o[k] = A::add(o[k], part);
         WG_TREE_SYNCWARP();
-        S* u = h0;
-        h0 = h1;
-        h1 = h2;
-        h2 = u;
+      };
+      for (int k = 1; k < T.nout; ++k) {
+        S* hn = h + (k % rows) * L;
+        const S *h1 = h + ((k - 1) % rows) * L, *h2 = h + ((k + rows - 2) % rows) * L;
+        if (!staged) dots(k - 1, k);
+        for (int tb = 0; tb < L; tb += NG) {
+          const int t = tb + grp;
+          ConvAcc<S> x = ConvAcc<S>::of(A::zero()), y = x;
+          if (t < L) {
+            conv_part(x, (const S*)v.p, v.st, L, h1, 1ll, t, sub);
+            if (k > 1) conv_part(y, (const S*)c.p, c.st, L, h2, 1ll, t, sub);
+          }
+          S n = x.sum();
+          if (k > 1) n = A::add(n, tree_times(y.sum(), k - 1));
+          n = split_sum(n);
+          if (t < L && sub == 0) hn[t] = n;
+        }
+        WG_TREE_SYNCWARP();
       }
+      dots(staged ? 0 : T.nout - 1, T.nout);
     }
   }
   return sum;
@@ -1152,6 +1362,19 @@ static __global__ void __launch_bounds__(TREE_THREADS, 1) tree_kernel(const Tree
           }
           break;
         }
+        case TP_G2: {
+          S* wk = scr + (2ll * tree_width(T.X, T.E, G.q + 1)) * (T.deg[G.q] + 1) * G.np;
+          tree_g2<S>(T, G.q, par, G.pstride, G.np, wk, chi, smw, P.sm_warp, tid, nthr);
+          break;
+        }
+        case TP_W2:
+          if (G.tile == 0) tree_w2<S, 0>(T, G.q, par, G.pstride, G.np, scr, tid, nthr);
+          else tree_w2<S, TL>(T, G.q, par, G.pstride, G.np, scr, tid, nthr);
+          break;
+        case TP_MULTI2:
+          if (G.tile == 0) tree_multi2<S, 0>(T, G.q, par, G.pstride, G.np, scr, chi, tid, nthr);
+          else tree_multi2<S, TL>(T, G.q, par, G.pstride, G.np, scr, chi, tid, nthr);
+          break;
         default: {
           S* y = scr + 6ll * (T.deg[G.q + 1] + 1) * G.np * T.radix[G.q];
           if (G.phase == TP_GLOOP) {
