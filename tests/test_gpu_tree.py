@@ -80,6 +80,19 @@ def test_batches(modes, cutoff, top, precision):
         both(tw.prepare_loop_hafnian_batch(B, D, list(fixed), cut), precision)
 
 
+@pytest.mark.parametrize("fixed", [[3] * 4, [2] * 6, [1] * 8, [25, 25, 24, 24]])
+def test_batches_of_any_shared_memory(fixed):
+    """A CTA's shared memory grows with the outputs and the photon pairs: below, about and above the
+    48 KB that a launch may use unasked, and (double-double) above what an SM has."""
+    n = len(fixed) + 1
+    A, D = wl.complex_symmetric(n, seed=n), wl.complex_symmetric(n, seed=5)[0] * 0.5
+    for cutoff in range(1, 16):
+        inst = tw.prepare_loop_hafnian_batch(A, D, fixed, cutoff)
+        if max(fixed) < 10:
+            both(inst, "fp64")
+        both(inst, "dd")
+
+
 @pytest.mark.parametrize("photons,max_rep", [(16, 4), (28, 3), (36, 2)])
 def test_multiple_edges_by_levels(photons, max_rep):
     A, gamma, rpt = wl.gaussian_state_loop(modes=14, seed=2, photons=photons, max_rep=max_rep)

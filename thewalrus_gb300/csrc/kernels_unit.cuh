@@ -27,7 +27,7 @@ int WG_CAT(sieve_occupancy_, WG_UNIT_NAME)(int wpc, int smem) {
 // several CTAs wait for one another, so they are launched cooperatively
 cudaError_t WG_CAT(tree_launch_, WG_UNIT_NAME)(const TreeParams& p, int ctas, int smem, cudaStream_t st) {
   auto k = tree_kernel<typename TreeScalar<WG_UNIT_SCALAR>::T>;
-  if (smem > 48 * 1024) {
+  if (smem > 32 * 1024) {  // with the kernel's static shared memory it may pass 48 KB, which needs the attribute
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }

@@ -375,7 +375,8 @@ static bool keeps_terms(int stype, int kind, int K, const MatrixForm& f) {
 
 // takes the tree when the instance has one; `ascale`: the input prescale's share of each output
 static void take_tree(Prepared& P, int precision, const std::vector<double>& ascale, const MatrixForm& f) {
-  P.tree = f.symmetric && tree_build(P.d, P.T) && !keeps_terms(P.stype, P.d.kind, P.T.K, f);
+  P.tree = f.symmetric && tree_build(P.d, P.T) && tree_fits(P.T, tree_bytes(P.stype)) &&
+           !keeps_terms(P.stype, P.d.kind, P.T.K, f);
   if (!P.tree) return;
   P.T.comp_off = stype_dd(P.stype) ? P.d.nout : 0;
   P.T.pstride = (stype_dd(P.stype) ? 2 : 1) * P.d.nout;
@@ -762,7 +763,6 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
   // A level's byte budget: larger levels are walked in blocks.  A launch's: beyond it the
   // instances go to the next launch.  Both keep the workspace within what the device's pool keeps.
   constexpr double kLevelBytes = 200e6, kLaunchBytes = 600e6;
-  constexpr long long kSharedBytes = 200 << 10;
   const int count = (int)P.size();
   auto al = [](long long x) { return (x + 255) & ~255ll; };
   std::vector<TreeLevels> lev(count);
@@ -819,9 +819,9 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
     G.sm_warp = prog.smem;
     G.sm_cache = (int)al((long long)prog.smem * (TREE_THREADS / 32) * sb);
     G.smem = G.sm_cache;
-    G.cached = G.smem + al((long long)(b_inst + b_rounds + b_segs)) <= kSharedBytes;
+    G.cached = G.smem + al((long long)(b_inst + b_rounds + b_segs)) <= TREE_SMEM_BYTES;
     if (G.cached) G.smem += (int)al((long long)(b_inst + b_rounds + b_segs));
-    if (G.ctas == 1 && G.smem + prog.ws_bytes <= kSharedBytes) {
+    if (G.ctas == 1 && G.smem + prog.ws_bytes <= TREE_SMEM_BYTES) {
       G.sm_ws = G.smem;
       G.smem += (int)prog.ws_bytes;
     } else {

@@ -10,6 +10,8 @@
 
 namespace wg {
 
+constexpr long long TREE_SMEM_BYTES = 200 << 10;  // dynamic shared memory of a CTA, at most
+
 // The tree of a prepared instance (whole sum, finite-difference signs); false when it does not
 // take one: more than TREE_MAX_K photon pairs, or inclusion/exclusion signs.
 static inline bool tree_build(const InstDev& d, TreeInst& T) {
@@ -230,6 +232,15 @@ static inline int tree_smem(const TreeInst& T, int most) {
   return need;
 }
 
+// elements of a warp's shared memory in a launch of node elements of `sb` bytes, and whether a CTA has
+// that much: not for double-double batches of more than ~45 photon pairs, which have no tree
+static inline int tree_warp_elems(const TreeInst& T, int sb) {
+  return tree_smem(T, (64 << 10) / (TREE_THREADS / 32) / sb);
+}
+static inline bool tree_fits(const TreeInst& T, int sb) {
+  return (long long)tree_warp_elems(T, sb) * (TREE_THREADS / 32) * sb <= TREE_SMEM_BYTES;
+}
+
 // The program of one launch over `insts` (their levels placed one after another in the workspace):
 // round r holds phase r of every instance, so that the narrow levels of one run beside others'.
 // `nparts` advances by the leaves' partial slots; part_base[i] and part_count[i] are instance i's.
@@ -251,7 +262,7 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
     TreeInst& T = insts[k];
     const TreeLevels& g = levels[k];
     T.scr_off = P.ws_bytes + g.scr_off;
-    P.smem = std::max(P.smem, tree_smem(T, (64 << 10) / (TREE_THREADS / 32) / sb));
+    P.smem = std::max(P.smem, tree_warp_elems(T, sb));
     const double fuse_threads = chip_threads / (double)insts.size();
     size_t r = 0;
     int last = -1;
