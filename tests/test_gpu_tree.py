@@ -64,8 +64,14 @@ def test_loops(n, precision):
 
 @pytest.mark.parametrize("precision", ["fp64", "df", "dd"])
 @pytest.mark.parametrize("reps", [[4], [7], [3, 3], [2] * 6, [1, 1, 1, 1, 2, 2, 3], [6, 5, 1, 1, 2], [9, 1, 4, 4],
-                                  [3, 3, 2, 2, 2, 1, 1, 1, 1, 1, 1, 1]])
+                                  [3, 3, 2, 2, 2, 1, 1, 1, 1, 1, 1, 1], [1] * 12 + [3] * 4, [1] * 16 + [6, 6],
+                                  [1] * 8 + [2] * 4 + [4] * 4, [1] * 12 + [5, 5, 9, 9]])
 def test_multiple_edges(reps, precision):
+    """FP64 against double-double terms: FP64 terms of many photons in one edge cancel by 10^5 and more."""
+    def both(inst, precision):
+        oracle = "dd" if precision == "fp64" else precision
+        close(nat.run([inst], precision), nat.run([inst], oracle + "-terms"), precision)
+
     A = wl.complex_symmetric(len(reps), seed=sum(reps)) * 0.3
     D = wl.complex_symmetric(len(reps), seed=3)[0] * 0.5
     if sum(reps) % 2 == 0:

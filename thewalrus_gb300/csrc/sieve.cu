@@ -851,6 +851,38 @@ static int plan_wpo(const wg_plan* pl, int nw) {
   return w;
 }
 
+// Whether the terms of a plan's trees are summed sooner one by one.  The terms run side by side, so
+// that their latency grows with the edges alone, and a tree's with its rounds: 0.7 of a term's edge for
+// a simple one, 2 for a double edge, 4 for one of three photons or more (its root and exponential
+// recurrences are chains of FP64 latencies).  What more terms than fit side by side cost grows with
+// their number, a tree's time hardly.  One unit is 6.5 to 12.5 us (FP64 plain to batches; double-double
+// 17 to 108); the weights are fitted to 2261 measured calls of 1 to 12 edges, multiplicities 1 to 12,
+// 1 to 10^4 terms, all scalar types.  us by tree and by terms (complex FP64, plain): [1 x 8] 57 and 97,
+// [3, 3, 3, 3] 136 and 76, [1, 2, 3] 68 and 57, [1 x 4, 2, 2, 3] 105 and 107, [1 x 6, 2, 2, 3] 118 and 203;
+// the rule takes the slower side by more than 10 % in 9 calls (1.27 at most) for the tree.
+static bool terms_sooner(const std::vector<Prepared>& P) {
+  double tree = 0, terms = 0, work = 0;
+  for (const Prepared& p : P) {
+    if (!p.tree) continue;
+    if (!tile_rows_ok(p.stype, p.rows_max)) return false;
+    const TreeInst& T = p.T;
+    double rounds = 0, t = 1;
+    int big = 0;
+    for (int q = 0; q < T.E; ++q) {
+      rounds += T.reps[q] == 1 ? 0.7 : (T.reps[q] == 2 ? 2.0 : 4.0);
+      big += T.reps[q] > 2;
+      t *= T.radix[q];
+    }
+    const bool dd = stype_dd(p.stype);
+    // per-term work against a tree's: no less of it where all edges are multiple, a batch has its outputs'
+    const double share = p.d.nout > 1 ? 1.2 * p.d.nout : (T.E - big) / (double)std::max(T.E, 1);
+    tree = std::max(tree, rounds);
+    terms = std::max(terms, (dd ? 0.9 : 2.0) + T.E);
+    work += (dd ? 3.75e-5 : 1.5e-5) * share * t * ((double)T.E * T.E * T.E + (double)T.K * T.K);
+  }
+  return tree > terms + work;
+}
+
 // ext_pool: the instances' matrices are on the device already, at their a_off
 static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_options& opt, wg_plan* pl,
                          GatherSpec* gs, unsigned char* ext_pool) {
@@ -862,6 +894,8 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   pl->serial_groups = opt.serial_groups != 0;
   pl->precision = precision;
   pl->device = g_device;
+  if (terms_sooner(P))
+    for (Prepared& p : P) p.tree = false;
   // outputs and scales in instance order
   int out = 0;
   std::vector<double> scales;
