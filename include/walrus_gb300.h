@@ -44,6 +44,9 @@ extern "C" {
 #define WG_PREC_MOD2 4
 #define WG_PREC_MOD3 5
 #define WG_PREC_MOD4 6
+/* wg_run: modulo each of the first k primes (k = 1 .. 5); the outputs of one prime follow those of
+ * the one before, so that `out` holds k times as many. */
+#define WG_PREC_PRIMES(k) (16 + (k))
 /* Added to a precision: evaluate the sieve term by term.  Without it an instance's whole sum (no
  * term range, finite-difference signs, symmetric matrix) is taken by the elimination tree, which
  * shares the work of terms with common signs and rounds less; the per-term evaluation is the one

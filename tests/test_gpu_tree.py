@@ -54,6 +54,22 @@ def test_residues(n):
         both(tw.prepare_loop_hafnian_batch(A, np.arange(1.0, 8.0), reps[:6], 4), "mod2")
 
 
+@pytest.mark.parametrize("copies", [1, 40])
+@pytest.mark.parametrize("sizes", [(4,), (24,), (30, 12), (38,)])
+@pytest.mark.parametrize("primes", [1, 2, 3, 5])
+def test_primes_of_one_call(primes, sizes, copies):
+    """Side by side, one after another (n = 38), beside per-term groups and with outputs for a
+    reduction of their own."""
+    insts = [tw.prepare_hafnian(wl.adjacency01(n, seed=n, p=0.6)) for n in sizes]
+    if copies > 1:
+        A = wl.adjacency01(6, seed=1, p=0.7) + np.diag(np.arange(6.0))
+        insts += [tw.prepare_hafnian(wl.adjacency01(10, seed=3), glynn=False)]
+        insts += [tw.prepare_loop_hafnian_batch(A, np.arange(1.0, 7.0), [2, 1, 3, 1, 1], 4)] * copies
+    got = nat._run(insts, nat.WG_PREC_PRIMES + primes, 0, primes).real.reshape(primes, -1)
+    for k in range(primes):
+        assert np.array_equal(got[k], nat.run(insts, "mod%d-terms" % k).real)
+
+
 @pytest.mark.parametrize("precision", ["fp64", "df", "dd"])
 @pytest.mark.parametrize("n", [3, 5, 8, 13, 20, 23, 27])
 def test_loops(n, precision):

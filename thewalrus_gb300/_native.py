@@ -17,7 +17,7 @@ LIB = os.path.join(BUILD, "libwalrus_gb300.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 SOURCES = ["sieve.cu", "noalloc.cu", "kernels_c64.cu", "kernels_cdf.cu", "kernels_f64.cu", "kernels_fdf.cu",
            "kernels_cdd.cu", "kernels_fdd.cu", "kernels_mod0.cu", "kernels_mod1.cu", "kernels_mod2.cu",
-           "kernels_mod3.cu", "kernels_mod4.cu"]
+           "kernels_mod3.cu", "kernels_mod4.cu", "kernels_mods.cu"]
 DEPS = SOURCES + ["sieve_kernel.cuh", "tree_kernel.cuh", "tree_host.h", "arith.cuh", "host_common.h", "kernels.h",
                   "kernels_unit.cuh", "state_glue.cuh"]
 NVCC_FLAGS = ["-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-lineinfo", "-std=c++17",
@@ -32,6 +32,7 @@ PRECISIONS = {"fp64": WG_PREC_FP64, "df": WG_PREC_DF, "dd": WG_PREC_DD}
 PRECISIONS.update({"mod%d" % k: v for k, v in enumerate(WG_PREC_MOD)})
 # the same, evaluated term by term (WG_PREC_TERMS): the evaluation behind the term magnitudes
 WG_PREC_TERMS = 64
+WG_PREC_PRIMES = 16  # + k: modulo each of the first k primes
 PRECISIONS.update({k + "-terms": v | WG_PREC_TERMS for k, v in list(PRECISIONS.items())})
 
 _lock = threading.Lock()
@@ -426,8 +427,8 @@ def run_exact(instances, stream=0, nprimes=None):
     k = nprimes or exact_primes(instances)
     if k is None:
         raise ValueError("exact precision: the outputs may exceed 2^153, beyond five primes")
-    per_prime = [run(instances, "mod%d" % j, stream).real for j in range(k)]
-    return [crt([round(float(r[i])) for r in per_prime], MOD_PRIMES[:k]) for i in range(len(per_prime[0]))]
+    per_prime = _run(instances, WG_PREC_PRIMES + k, stream, k).real.reshape(k, -1).astype(np.int64)
+    return [crt(r, MOD_PRIMES[:k]) for r in per_prime.T.tolist()]
 
 
 def run(instances, precision="fp64", stream=0):
@@ -435,15 +436,19 @@ def run(instances, precision="fp64", stream=0):
     ``precision="exact"`` the exact integers, rounded to complex128."""
     if precision == "exact":
         return np.array([complex(float(v), 0.0) for v in run_exact(instances, stream)], dtype=np.complex128)
+    return _run(instances, PRECISIONS[precision], stream)
+
+
+def _run(instances, code, stream, sets=1):
     lib = load()
     insts = list(instances)
     arr = (WgInstance * max(len(insts), 1))()
     total = 0
     for i, inst in enumerate(insts):
         arr[i] = inst.struct
-        total += inst.outputs()
+        total += sets * inst.outputs()
     out = np.zeros(2 * max(total, 1))
-    check(lib.wg_run(arr, len(insts), PRECISIONS[precision],
+    check(lib.wg_run(arr, len(insts), code,
                      out.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), ctypes.c_void_p(stream)))
     return (out[0::2] + 1j * out[1::2])[:total]
 

@@ -552,6 +552,8 @@ template <uint32_t P>
 struct modp {
   uint32_t v;  // Montgomery form
 };
+constexpr int MOD_N = 5;
+constexpr uint32_t MOD_PRIMES[MOD_N] = {2147483647u, 2147483629u, 2147483587u, 2147483579u, 2147483563u};
 
 template <uint32_t P>
 struct Montgomery {

@@ -26,7 +26,6 @@ static size_t stype_bytes(int st) {
   if (stype_dd(st)) return st == ST_REALDD ? 16 : 32;
   return (st == ST_REAL64 || st == ST_REALDF) ? 8 : 16;
 }
-static const uint32_t MOD_PRIMES[5] = {2147483647u, 2147483629u, 2147483587u, 2147483579u, 2147483563u};
 
 // the largest term tile a warp works on: 80 rows of complex scalars, 96 of real ones (the packed
 // pivot keys hold row indices below 128)
@@ -72,13 +71,15 @@ static inline cudaError_t tree_launch(int stype, const TreeParams& p, int ctas, 
     case ST_CPLXDF: return tree_launch_cdf(p, ctas, smem, st);
     case ST_REAL64: return tree_launch_f64(p, ctas, smem, st);
     case ST_REALDF: return tree_launch_fdf(p, ctas, smem, st);
-    case ST_MOD0: return tree_launch_mod0(p, ctas, smem, st);
-    case ST_MOD1: return tree_launch_mod1(p, ctas, smem, st);
-    case ST_MOD2: return tree_launch_mod2(p, ctas, smem, st);
-    case ST_MOD3: return tree_launch_mod3(p, ctas, smem, st);
     case ST_REALDD: return tree_launch_fdd(p, ctas, smem, st);
     case ST_CPLXDD: return tree_launch_cdd(p, ctas, smem, st);
-    default: return tree_launch_mod4(p, ctas, smem, st);
+    default: {
+      TreeMods m;
+      m.n = 1;
+      m.prime[0] = stype - ST_MOD0;
+      m.p[0] = p;
+      return tree_launch_mods(m, ctas, smem, st);
+    }
   }
 }
 
@@ -92,6 +93,7 @@ static inline cudaError_t sieve_tables_all(const double* binom, const double* in
   if (e == cudaSuccess) e = sieve_tables_mod2(binom, inv);
   if (e == cudaSuccess) e = sieve_tables_mod3(binom, inv);
   if (e == cudaSuccess) e = sieve_tables_mod4(binom, inv);
+  if (e == cudaSuccess) e = sieve_tables_mods(binom, inv);
   if (e == cudaSuccess) e = sieve_tables_fdd(binom, inv);
   if (e == cudaSuccess) e = sieve_tables_cdd(binom, inv);
   return e;

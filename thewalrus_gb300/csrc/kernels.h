@@ -1,8 +1,9 @@
 // Sieve-kernel instantiations live in one translation unit per scalar class (kernels_c64.cu,
 // kernels_cdf.cu, kernels_f64.cu, kernels_fdf.cu, kernels_cdd.cu, kernels_fdd.cu,
 // kernels_mod{0..4}.cu: residues modulo one prime each) so that they compile in parallel.  Each unit
-// instantiates sieve_kernel<S> and the tree kernels and holds its own copy of the constant tables (binomials,
-// reciprocals), which the host fills through sieve_tables_*.
+// instantiates sieve_kernel<S> and the tree kernel (the residues' is kernels_mods.cu, for all primes) and
+// holds its own copy of the constant tables (binomials, reciprocals), which the host fills through
+// sieve_tables_*.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -14,7 +15,6 @@ namespace wg {
 #define WG_KERNEL_UNIT_DECL(T)                                                                      \
   cudaError_t sieve_launch_##T(const SieveParams& p, int ctas, int wpc, cudaStream_t st); \
   int sieve_occupancy_##T(int wpc, int smem);                                             \
-  cudaError_t tree_launch_##T(const TreeParams& p, int ctas, int smem, cudaStream_t st);  \
   cudaError_t sieve_tables_##T(const double* binom, const double* inv);
 
 WG_KERNEL_UNIT_DECL(c64)
@@ -29,5 +29,40 @@ WG_KERNEL_UNIT_DECL(mod2)
 WG_KERNEL_UNIT_DECL(mod3)
 WG_KERNEL_UNIT_DECL(mod4)
 #undef WG_KERNEL_UNIT_DECL
+#define WG_TREE_UNIT_DECL(T) cudaError_t tree_launch_##T(const TreeParams& p, int ctas, int smem, cudaStream_t st);
+WG_TREE_UNIT_DECL(c64)
+WG_TREE_UNIT_DECL(cdf)
+WG_TREE_UNIT_DECL(f64)
+WG_TREE_UNIT_DECL(fdf)
+WG_TREE_UNIT_DECL(cdd)
+WG_TREE_UNIT_DECL(fdd)
+#undef WG_TREE_UNIT_DECL
+cudaError_t tree_launch_mods(const TreeMods& m, int ctas, int smem, cudaStream_t st);
+cudaError_t sieve_tables_mods(const double* binom, const double* inv);
+
+// A launch of `ctas` CTAs whose trees are shared by `group` of them: these wait for one another, so
+// that more than one are launched cooperatively.
+template <class Params>
+static inline cudaError_t tree_launch_kernel(void (*k)(Params), const Params& p, int ctas, int group, int smem,
+                                             cudaStream_t st) {
+  if (smem > 32 * 1024) {  // with the kernel's static shared memory it may pass 48 KB, which needs the attribute
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
+  if (group == 1) {
+    k<<<ctas, TREE_THREADS, smem, st>>>(p);
+    return cudaGetLastError();
+  }
+  Params arg = p;
+  void* args[] = {&arg};
+  return cudaLaunchCooperativeKernel((const void*)k, dim3(ctas), dim3(TREE_THREADS), args, (size_t)smem, st);
+}
+
+// 1/k modulo a prime in Montgomery form, k < 256, by k * inv(k) = 1: inv(k) = -(p / k) inv(p mod k)
+static inline void mod_inverses(uint64_t p, uint32_t* inv) {
+  uint32_t plain[256] = {0, 1};
+  for (uint64_t k = 2; k < 256; ++k) plain[k] = (uint32_t)((p - (p / k) * plain[p % k] % p) % p);
+  for (int k = 0; k < 256; ++k) inv[k] = (uint32_t)(((uint64_t)plain[k] << 32) % p);
+}
 
 }  // namespace wg

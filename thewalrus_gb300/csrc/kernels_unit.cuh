@@ -24,21 +24,11 @@ int WG_CAT(sieve_occupancy_, WG_UNIT_NAME)(int wpc, int smem) {
   return nb;
 }
 
-// several CTAs wait for one another, so they are launched cooperatively
+#ifndef WG_UNIT_PRIME  // (residues: kernels_mods.cu)
 cudaError_t WG_CAT(tree_launch_, WG_UNIT_NAME)(const TreeParams& p, int ctas, int smem, cudaStream_t st) {
-  auto k = tree_kernel<typename TreeScalar<WG_UNIT_SCALAR>::T>;
-  if (smem > 32 * 1024) {  // with the kernel's static shared memory it may pass 48 KB, which needs the attribute
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
-  if (ctas == 1) {
-    k<<<1, TREE_THREADS, smem, st>>>(p);
-    return cudaGetLastError();
-  }
-  TreeParams arg = p;
-  void* args[] = {&arg};
-  return cudaLaunchCooperativeKernel((const void*)k, dim3(ctas), dim3(TREE_THREADS), args, (size_t)smem, st);
+  return tree_launch_kernel(tree_kernel<typename TreeScalar<WG_UNIT_SCALAR>::T>, p, ctas, ctas, smem, st);
 }
+#endif
 
 cudaError_t WG_CAT(sieve_tables_, WG_UNIT_NAME)(const double* binom, const double* inv) {
   cudaError_t e = cudaMemcpyToSymbol(c_binom, binom, sizeof(c_binom));
@@ -46,12 +36,8 @@ cudaError_t WG_CAT(sieve_tables_, WG_UNIT_NAME)(const double* binom, const doubl
   e = cudaMemcpyToSymbol(c_inv, inv, sizeof(c_inv));
 #ifdef WG_UNIT_PRIME
   if (e != cudaSuccess) return e;
-  uint32_t invmod[256];  // 1/k mod p by k * inv(k) = 1: inv(k) = -(p / k) inv(p mod k)
-  invmod[0] = 0;
-  invmod[1] = 1;
-  const uint64_t P = WG_UNIT_PRIME;
-  for (uint64_t k = 2; k < 256; ++k) invmod[k] = (uint32_t)((P - (P / k) * invmod[P % k] % P) % P);
-  for (int k = 0; k < 256; ++k) invmod[k] = Montgomery<WG_UNIT_PRIME>::to_mont(invmod[k]);
+  uint32_t invmod[256];
+  mod_inverses(WG_UNIT_PRIME, invmod);
   e = cudaMemcpyToSymbol(c_invmod, invmod, sizeof(invmod));
 #endif
   return e;

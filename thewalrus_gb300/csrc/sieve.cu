@@ -201,6 +201,7 @@ struct TreeLaunch {
   int stype, ctas, smem, sm_warp, sm_cache, sm_ws, cached, counter;
   int ninst, nrounds, nsegs;
   size_t prog_off;  // of the instances, rounds and segments in the plan's program bytes
+  long long ws_off;
 };
 
 }  // namespace wg
@@ -213,6 +214,8 @@ struct wg_plan {
   int nparts = 0;
   long long h2d_bytes = 0;
   int precision = 0;
+  int primes = 1;           // > 1: every instance modulo so many primes, all instances of one first
+  bool side_trees = false;  // the primes' trees run side by side in one launch
   void* dmem = nullptr;
   wg::InstDev* d_inst = nullptr;
   wg::ChunkDev* d_chunks = nullptr;
@@ -553,6 +556,7 @@ static int prepare(const wg_instance& in, int precision, Prepared& P) {
     if (kind == KIND_LOOP_ODD && !integral(in.oddloop[0])) return fail(WG_EINVAL, "exact precision needs an integer self-loop weight");
     if (maxr > 50) return fail(WG_EINVAL, "exact precision supports edge repetitions up to 50");
     P.stype = ST_MOD0 + (precision - WG_PREC_MOD0);
+    d.modp = MOD_PRIMES[precision - WG_PREC_MOD0];
   } else {
     P.stype = precision == WG_PREC_DF   ? (cplx ? ST_CPLXDF : ST_REALDF)
               : precision == WG_PREC_DD ? (cplx ? ST_CPLXDD : ST_REALDD)
@@ -730,16 +734,24 @@ static bool known_precision(int precision) {
   const int p = precision & ~WG_PREC_TERMS;
   return p == WG_PREC_FP64 || p == WG_PREC_DF || p == WG_PREC_DD || prec_mod(p);
 }
+// the primes of WG_PREC_PRIMES(k) (0: another precision)
+static int prec_primes(int precision) {
+  const int k = (precision & ~WG_PREC_TERMS) - WG_PREC_PRIMES(0);
+  return k >= 1 && k <= MOD_N ? k : 0;
+}
 
 static int build_plan(const wg_instance* v, int count, int precision, const wg_plan_options& opt, wg_plan* pl) {
   if (count < 0 || (count > 0 && !v)) return fail(WG_EINVAL, "bad instance list");
-  if (!known_precision(precision))
-    return fail(WG_EINVAL, "unknown precision %d", precision);
-  std::vector<Prepared> P(count);
-  for (int i = 0; i < count; ++i) {
-    int rc = prepare(v[i], precision, P[i]);
-    if (rc) return fail(rc, "instance %d: %s", i, g_err.c_str());
+  const int primes = prec_primes(precision);
+  if (!known_precision(precision) && !primes) return fail(WG_EINVAL, "unknown precision %d", precision);
+  pl->primes = std::max(primes, 1);
+  std::vector<Prepared> P((size_t)count * pl->primes);
+  for (int i = 0; i < count * pl->primes; ++i) {
+    const int prec = primes ? (WG_PREC_MOD0 + i / count) | (precision & WG_PREC_TERMS) : precision;
+    int rc = prepare(v[i % count], prec, P[i]);
+    if (rc) return fail(rc, "instance %d: %s", i % count, g_err.c_str());
   }
+  if (primes) precision = WG_PREC_MOD0;
   return finalize_plan(P, precision, opt, pl, nullptr, nullptr);
 }
 
@@ -758,7 +770,8 @@ static double tree_mac_clocks(int stype) {
 
 // Groups the tree members of a plan into launches (one scalar type each, as many instances as share
 // a workspace budget), makes their programs and lays out their partial slots.  Returns the
-// workspace bytes; the launches run one after another and share it.
+// workspace bytes; the launches run one after another and share it, or (an exact sum's primes) side
+// by side.
 static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) {
   // A level's byte budget: larger levels are walked in blocks.  A launch's: beyond it the
   // instances go to the next launch.  Both keep the workspace within what the device's pool keeps.
@@ -775,6 +788,14 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     return P[a].stype != P[b].stype ? P[a].stype < P[b].stype : lev[a].bytes > lev[b].bytes;
   });
+  // Several primes side by side when their levels, of which two at a time are in use, keep to the L2:
+  // graph counts modulo three, n = 36 (75 MB each) 886 us one after another and 723 side by side,
+  // n = 38 (160 MB each) 1,508 and 1,642.
+  constexpr double kSideBytes = 250e6;
+  long long first = 0;
+  for (size_t k = 0; k < order.size() && P[order[k]].stype == P[order[0]].stype; ++k) first += lev[order[k]].bytes;
+  pl->side_trees = pl->primes > 1 && !order.empty() && (double)first * pl->primes <= kSideBytes;
+  const int sms = pl->side_trees ? g_num_sms / pl->primes : g_num_sms;
   long long ws = 0;
   for (size_t k = 0; k < order.size();) {
     TreeLaunch G;
@@ -795,7 +816,7 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
     TreeProgram prog;
     std::vector<int> base, cnt;
     const double clk = tree_mac_clocks(G.stype);
-    G.ctas = tree_one_cta(insts, levels, clk, g_num_sms) ? 1 : g_num_sms;
+    G.ctas = tree_one_cta(insts, levels, clk, sms) ? 1 : sms;
     tree_program(insts, levels, sb, tile, G.ctas * TREE_THREADS, nparts, base, cnt, prog);
     for (size_t j = 0; j < insts.size(); ++j) {
       InstDev& d = P[order[k0 + j]].d;
@@ -825,7 +846,8 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
       G.sm_ws = G.smem;
       G.smem += (int)prog.ws_bytes;
     } else {
-      ws = std::max(ws, prog.ws_bytes);
+      G.ws_off = pl->side_trees ? ws : 0;
+      ws = std::max(ws, G.ws_off + al(prog.ws_bytes));
     }
     pl->trees.push_back(G);
   }
@@ -835,19 +857,16 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
 // whether the plan is one tree launch, which then also reduces (tree_finish): few enough outputs
 // for one CTA
 static bool plan_single(const wg_plan* pl) {
-  return pl->groups.empty() && pl->trees.size() == 1 && pl->total_out <= 64;
+  return pl->groups.empty() && (pl->trees.size() == 1 || pl->side_trees) && pl->total_out <= 64 * pl->primes;
 }
 static int plan_counters(const wg_plan* pl) {
-  return (int)(pl->groups.size() + pl->trees.size()) + 1;  // and tree_finish's
-}
-static unsigned int plan_prime(const wg_plan* pl) {
-  return prec_mod(pl->precision) ? MOD_PRIMES[pl->precision - WG_PREC_MOD0] : 0u;
+  return (int)(pl->groups.size() + 2 * pl->trees.size());  // a tree launch's barrier and its tree_finish
 }
 // warps that sum an output's partials, of the `nw` of a block: one, as the per-term launches
 // always had, unless a tree left several hundred
 static int plan_wpo(const wg_plan* pl, int nw) {
   int w = 1;
-  while (w < nw && w * 64 < pl->tree_parts && w * pl->total_out < nw) w *= 2;
+  while (w < nw && w * 64 < pl->tree_parts && w * (pl->total_out / pl->primes) < nw) w *= 2;
   return w;
 }
 
@@ -1035,7 +1054,10 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   const size_t b_mag = al(sizeof(double) * std::max(out, 1));
   const size_t ncnt = (size_t)plan_counters(pl);
   int counter = (int)pl->groups.size();
-  for (TreeLaunch& g : pl->trees) g.counter = counter++;
+  for (TreeLaunch& g : pl->trees) {
+    g.counter = counter;
+    counter += 2;
+  }
   const size_t b_cnt = al(sizeof(unsigned int) * std::max<size_t>(ncnt, 1));
   const size_t b_tree = al(std::max<size_t>(pl->tree_prog.size(), 1));
   const size_t b_ws = al((size_t)ws_bytes);
@@ -1137,28 +1159,15 @@ static int terms_plan(wg_plan* pl, wg_plan** out) {
 }
 
 static int launch_trees(wg_plan* pl, cudaStream_t st) {
-  TreeParams p;
-  memset(&p, 0, sizeof(p));
-  p.pool = pl->d_pool;
-  p.partials = pl->d_partials;
-  p.ws = pl->d_ws;
-  p.err = pl->d_err;
-  if (plan_single(pl)) {
-    p.fin.inst = pl->d_inst;
-    p.fin.ninst = (int)pl->inst.size();
-    p.fin.partials = pl->d_partials;
-    p.fin.scales = pl->d_scales;
-    p.fin.out = pl->d_out;
-    p.fin.mags = pl->d_mag;
-    p.fin.err = pl->d_err;
-    p.fin.counters = pl->d_counters;
-    p.fin.ncounters = plan_counters(pl);
-    p.fin.done = pl->d_counters + plan_counters(pl) - 1;
-    p.fin.total_out = pl->total_out;
-    p.fin.wpo = plan_wpo(pl, TREE_THREADS / 32);
-    p.fin.modp = plan_prime(pl);
-  }
+  TreeMods side;
+  side.n = 0;
   for (const TreeLaunch& G : pl->trees) {
+    TreeParams p;
+    memset(&p, 0, sizeof(p));
+    p.pool = pl->d_pool;
+    p.partials = pl->d_partials;
+    p.ws = pl->d_ws + G.ws_off;
+    p.err = pl->d_err;
     p.ninst = G.ninst;
     p.nrounds = G.nrounds;
     p.nsegs = G.nsegs;
@@ -1170,7 +1179,29 @@ static int launch_trees(wg_plan* pl, cudaStream_t st) {
     p.sm_cache = G.sm_cache;
     p.sm_ws = G.sm_ws;
     p.bar = pl->d_counters + G.counter;
-    const cudaError_t e = tree_launch(G.stype, p, G.ctas, G.smem, st);
+    if (plan_single(pl)) {
+      p.fin.inst = pl->d_inst;
+      p.fin.ninst = (int)pl->inst.size();
+      p.fin.partials = pl->d_partials;
+      p.fin.scales = pl->d_scales;
+      p.fin.out = pl->d_out;
+      p.fin.mags = pl->d_mag;
+      p.fin.err = pl->d_err;
+      p.fin.counters = pl->d_counters + G.counter;
+      p.fin.ncounters = 2;
+      p.fin.done = p.fin.counters + 1;
+      const int each = pl->total_out / pl->primes, g = side.n;
+      p.fin.first_out = g * each;
+      p.fin.end_out = (g + 1) * each;
+      p.fin.wpo = plan_wpo(pl, TREE_THREADS / 32);
+    }
+    if (pl->side_trees) {
+      side.prime[side.n] = G.stype - ST_MOD0;
+      side.p[side.n++] = p;  // the primes' programs are alike: G.ctas and G.smem too
+      if (side.n < (int)pl->trees.size()) continue;
+    }
+    const cudaError_t e = pl->side_trees ? tree_launch_mods(side, G.ctas * side.n, G.smem, st)
+                                         : tree_launch(G.stype, p, G.ctas, G.smem, st);
     if (e != cudaSuccess) return fail(WG_ECUDA, "tree launch: %s", cudaGetErrorString(e));
   }
   return WG_OK;
@@ -1226,7 +1257,7 @@ static int launch_plan(wg_plan* pl, cudaStream_t st) {
     const int per = threads / 32 / wpo, blocks = (pl->total_out + per - 1) / per;
     reduce_kernel<<<std::max(blocks, 1), threads, 0, st>>>(pl->d_inst, ninst, pl->d_partials, pl->d_scales, pl->d_out,
                                                            pl->d_counters, plan_counters(pl), pl->total_out, wpo,
-                                                           plan_prime(pl), pl->d_mag, pl->d_err);
+                                                           pl->d_mag, pl->d_err);
     CK(cudaGetLastError());
   }
   return WG_OK;
@@ -1399,7 +1430,8 @@ int wg_plan_outputs(const wg_plan* plan) { return plan ? plan->total_out : fail(
 
 int wg_plan_kernel_launches(const wg_plan* plan) {
   if (!plan) return fail(WG_EINVAL, "plan is NULL");
-  return (int)(plan->groups.size() + plan->trees.size()) + (plan->inst.empty() || plan_single(plan) ? 0 : 1);
+  const size_t trees = plan->side_trees ? 1 : plan->trees.size();
+  return (int)(plan->groups.size() + trees) + (plan->inst.empty() || plan_single(plan) ? 0 : 1);
 }
 
 int wg_plan_partials(wg_plan* plan, double* out, int capacity, void* stream) {

@@ -62,6 +62,7 @@ struct InstDev {
   int mag_off;     // slot offset of the term magnitudes (0: none)
   int out_base;    // first output slot
   int scale_base;  // first output scale
+  unsigned int modp;  // residues: the prime (0: numbers)
 };
 
 struct ChunkDev {
@@ -1243,13 +1244,13 @@ __device__ __forceinline__ const InstDev& reduce_instance(const InstDev* inst, i
 // The final scale (0.5^(N/2-1) etc., and the undoing of any input prescaling); NaN when a launch gave
 // up waiting for its own blocks (*err).
 __device__ __forceinline__ void reduce_write(const InstDev& I, int gw, const RSum& s, const double* scales, double2* out,
-                                             unsigned int modp, double* mags, const int* err) {
+                                             double* mags, const int* err) {
   const double sc = scales[I.scale_base + gw - I.out_base];
   if (err && *err) {
     out[gw] = make_double2(nan(""), nan(""));
-  } else if (modp) {  // residues (< 2^31) summed exactly in FP64 (fewer than 2^22 chunks), then mod p
-    const unsigned long long r = (unsigned long long)(s.sr + s.cr) % modp;
-    out[gw] = make_double2((double)(r * (unsigned long long)sc % modp), 0.0);
+  } else if (I.modp) {  // residues (< 2^31) summed exactly in FP64 (fewer than 2^22 chunks), then mod p
+    const unsigned long long r = (unsigned long long)(s.sr + s.cr) % I.modp;
+    out[gw] = make_double2((double)(r * (unsigned long long)sc % I.modp), 0.0);
   } else {
     out[gw] = make_double2((s.sr + s.cr) * sc, (s.si + s.ci) * sc);
   }
@@ -1260,7 +1261,7 @@ __device__ __forceinline__ void reduce_write(const InstDev& I, int gw, const RSu
 // warp order), so that one output of many partials is not one warp's serial sum.
 __device__ __forceinline__ void reduce_block(const InstDev* inst, int ninst, const double2* partials,
                                              const double* scales, double2* out, int first, int step, int total_out,
-                                             int wpo, unsigned int modp, double* mags, const int* err) {
+                                             int wpo, double* mags, const int* err) {
   __shared__ RSum s_part[32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = warp % wpo, per = (blockDim.x >> 5) / wpo;
   for (int g0 = first; g0 < total_out; g0 += step) {
@@ -1275,7 +1276,7 @@ __device__ __forceinline__ void reduce_block(const InstDev* inst, int ninst, con
     __syncthreads();
     if (live && sub == 0 && lane == 0) {
       for (int w = 1; w < wpo; ++w) rsum_merge(s, s_part[warp + w]);
-      reduce_write(reduce_instance(inst, ninst, gw), gw, s, scales, out, modp, mags, err);
+      reduce_write(reduce_instance(inst, ninst, gw), gw, s, scales, out, mags, err);
     }
     __syncthreads();
   }
@@ -1285,10 +1286,10 @@ __device__ __forceinline__ void reduce_block(const InstDev* inst, int ninst, con
 // execution.
 static __global__ void reduce_kernel(const InstDev* __restrict__ inst, int ninst, const double2* __restrict__ partials,
                                      const double* __restrict__ scales, double2* __restrict__ out,
-                                     unsigned int* counters, int ncounters, int total_out, int wpo, unsigned int modp,
+                                     unsigned int* counters, int ncounters, int total_out, int wpo,
                                      double* __restrict__ mags, const int* __restrict__ err) {
   const int per = (blockDim.x >> 5) / wpo;
-  reduce_block(inst, ninst, partials, scales, out, blockIdx.x * per, gridDim.x * per, total_out, wpo, modp, mags, err);
+  reduce_block(inst, ninst, partials, scales, out, blockIdx.x * per, gridDim.x * per, total_out, wpo, mags, err);
   if (blockIdx.x == 0 && threadIdx.x == 0)
     for (int i = 0; i < ncounters; ++i) counters[i] = 0u;
 }

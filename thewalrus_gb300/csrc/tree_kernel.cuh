@@ -111,8 +111,7 @@ struct TreeFinish {
   double* mags;
   int* err;
   unsigned int *done, *counters;
-  int ninst, total_out, ncounters, wpo;  // wpo: warps per output
-  unsigned int modp;
+  int ninst, first_out, end_out, ncounters, wpo;  // wpo: warps per output
 };
 
 struct TreeParams {
@@ -129,6 +128,13 @@ struct TreeParams {
   unsigned int* bar;
   int* err;
   TreeFinish fin;
+};
+
+// trees modulo several primes side by side in one launch, whose CTAs they share in equal parts
+struct TreeMods {
+  int n;
+  int prime[MOD_N];  // indices
+  TreeParams p[MOD_N];
 };
 
 __host__ __device__ __forceinline__ int tree_width(int X, int E, int q) { return X + 2 * (E - q); }
@@ -194,7 +200,6 @@ struct RealAcc<ddr> {
   }
   __device__ __forceinline__ ddr sum() const { return dd_two_sum(hi, lo); }
 };
-
 // Complex nodes carry re + im beside the parts, so that a product of series takes three real products
 // a term instead of four (re = P1 - P2, im = P3 - P1 - P2 with P1 = sum re re, P2 = sum im im, P3 = sum
 // (re + im)(re + im)); its rounding is relative to |a| |b|, as the four products' is.  C: the matrix
@@ -1231,18 +1236,19 @@ __device__ __forceinline__ void tree_store(const TreeInst& T, S sum, long long s
   }
 }
 
-// Barrier of all CTAs of a cooperative launch (one CTA: a block barrier).  The wait is bounded: after
-// about 3 s of polling a CTA gives up, its later barriers do not wait, and the error flag makes the
-// outputs NaN.
+// Barrier of the `ctas` CTAs of a cooperative launch that share trees (one CTA: a block barrier).  The
+// wait is bounded: after about 3 s of polling a CTA gives up, its later barriers do not wait, and the
+// error flag makes the outputs NaN.
 struct TreeSync {
   unsigned int* bar;
   int* err;
+  unsigned int ctas;
   unsigned int target = 0;
   bool ok = true;  // thread 0's
   __device__ __forceinline__ void operator()() {
     __syncthreads();
-    if (gridDim.x == 1) return;
-    target += gridDim.x;
+    if (ctas == 1) return;
+    target += ctas;
     if (threadIdx.x == 0) {
       __threadfence();
       atomicAdd(bar, 1u);
@@ -1262,19 +1268,19 @@ struct TreeSync {
 
 // The plan's only launch also reduces: the CTA that finishes last sums the partials of every
 // output, as reduce_kernel does, and re-arms the counters.
-__device__ __forceinline__ void tree_finish(const TreeFinish& F) {
+__device__ __forceinline__ void tree_finish(const TreeFinish& F, unsigned int ctas) {
   if (!F.done) return;
   __shared__ int s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    s_last = gridDim.x == 1 || atomicAdd(F.done, 1u) == gridDim.x - 1;
+    s_last = ctas == 1 || atomicAdd(F.done, 1u) == ctas - 1;
     __threadfence();
   }
   __syncthreads();
   if (!s_last) return;
   const int nw = blockDim.x >> 5;
-  reduce_block(F.inst, F.ninst, F.partials, F.scales, F.out, 0, nw / F.wpo, F.total_out, F.wpo, F.modp, F.mags, F.err);
+  reduce_block(F.inst, F.ninst, F.partials, F.scales, F.out, F.first_out, nw / F.wpo, F.end_out, F.wpo, F.mags, F.err);
   for (int i = threadIdx.x; i < F.ncounters; i += blockDim.x) F.counters[i] = 0u;
 }
 
@@ -1282,8 +1288,9 @@ __device__ __forceinline__ void tree_finish(const TreeFinish& F) {
 // the launch after it.  Consecutive warps of a round lie on different SMs, so that a narrow level
 // still uses every FP64 pipe.  Levels live in the workspace (L2 resident; a single CTA's in shared
 // memory).
+// `cta` of the `ctas` CTAs that share P's trees.
 template <class S>
-static __global__ void __launch_bounds__(TREE_THREADS, 1) tree_kernel(const TreeParams P) {
+__device__ __forceinline__ void tree_body(const TreeParams& P, const int cta, const int ctas) {
   extern __shared__ __align__(16) unsigned char smem[];
   using A = Ar<S>;
   constexpr int TL = tree_tile<S>();
@@ -1305,11 +1312,11 @@ static __global__ void __launch_bounds__(TREE_THREADS, 1) tree_kernel(const Tree
   }
   unsigned char* ws = P.sm_ws ? smem + P.sm_ws : P.ws;
   const int lane = threadIdx.x & 31;
-  const int gn = gridDim.x * (blockDim.x >> 5);
+  const int gn = ctas * (blockDim.x >> 5);
   __shared__ int s_next[2];
   if (threadIdx.x == 0) s_next[0] = 0;
   __syncthreads();
-  TreeSync sync{P.bar, P.err};
+  TreeSync sync{P.bar, P.err, (unsigned int)ctas};
   for (int r = 0; r < P.nrounds; ++r) {
     const TreeRound R = rounds[r];
     // A round's warps go to the CTAs in turn.  Where that is more than one a warp, the CTA's warps take
@@ -1323,7 +1330,7 @@ static __global__ void __launch_bounds__(TREE_THREADS, 1) tree_kernel(const Tree
         if (lane == 0) turn = atomicAdd(&s_next[r & 1], 1);
         turn = __shfl_sync(0xffffffffu, turn, 0);
       }
-      const int vw = turn * (int)gridDim.x + (int)blockIdx.x;
+      const int vw = turn * ctas + cta;
       if (vw >= R.nwarps) break;
       int lo = R.seg0, hi = R.seg0 + R.nseg - 1;
       while (lo < hi) {
@@ -1405,10 +1412,15 @@ static __global__ void __launch_bounds__(TREE_THREADS, 1) tree_kernel(const Tree
       if (T.nout == 1) s = warp_sum(lane < nw ? sm[lane] : s);
       else if (lane < T.nout)
         for (int w = 0; w < nw; ++w) s = A::add(s, sm[w * T.nout + lane]);
-      tree_store<S>(T, s, segs[P.nsegs - 1].part + (long long)blockIdx.x * T.pstride, P.partials);
+      tree_store<S>(T, s, segs[P.nsegs - 1].part + (long long)cta * T.pstride, P.partials);
     }
   }
-  tree_finish(P.fin);
+  tree_finish(P.fin, ctas);
+}
+
+template <class S>
+static __global__ void __launch_bounds__(TREE_THREADS, 1) tree_kernel(const TreeParams P) {
+  tree_body<S>(P, blockIdx.x, gridDim.x);
 }
 
 }  // namespace wg
