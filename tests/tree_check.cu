@@ -96,8 +96,11 @@ static void phase(const TreeInst& T, const TreeSeg& G, const unsigned char* pool
   switch (G.phase) {
     case TP_ROOT: tree_root<hc>(T, pool, chi, tid, nthr); break;
     case TP_FIRST: tree_first<hc>(T, pool, chi, tid, nthr); break;
-    case TP_M: tree_m<hc, TL>(T, G.q, par, G.pstride, G.np, scr, tid, nthr); break;
-    case TP_UNIT: tree_unit<hc, TL>(T, G.q, par, G.pstride, G.np, G.fused ? nullptr : scr, chi, tid, nthr); break;
+    case TP_M: tree_m<hc, TL>(T, G.q, par, G.pstride, G.np, tree_m_of(T, scr, G.q), tid, nthr); break;
+    case TP_UNIT: case TP_G:
+      tree_unit<hc, TL>(T, G.q, par, G.pstride, G.np, tree_m_of(T, scr, G.q), chi, tree_unit_begin(T, G.phase),
+                        tree_unit_end(T, G.phase, G.q), tid, nthr);
+      break;
     case TP_G2:
       tree_g2<hc>(T, G.q, par, G.pstride, G.np, scr + (2ll * tree_width(T.X, T.E, G.q + 1)) * (T.deg[G.q] + 1) * G.np, chi,
                   sm, smn, tid, nthr);
@@ -109,7 +112,7 @@ static void phase(const TreeInst& T, const TreeSeg& G, const unsigned char* pool
     case TP_MULTI: tree_multi<hc, TL>(T, G.q, par, G.pstride, G.np, y, chi, tid, nthr); break;
     case TP_GLOOP: tree_gloop<hc>(T, G.q, par, G.pstride, G.np, scr, y, chi, sm, smn, tid, nthr); break;
     default: {
-      const hc s = tree_leaf<hc, TL>(T, par, G.pstride, G.np, scr, sm, smn, tid, nthr);
+      const hc s = tree_leaf<hc, TL>(T, par, G.pstride, G.np, tree_m_of(T, scr, G.q), sm, smn, tid, nthr);
       if (T.pB < 0) out[0] = Ar<hc>::add(out[0], s);
       else
         for (int k = 0; k < T.nout; ++k) out[k] = Ar<hc>::add(out[k], sm[k]);
@@ -161,7 +164,9 @@ int main() {
   for (int k = 0; k < count; ++k) out[k].assign(P.insts[k].nout, hc{0, 0});
   unsigned char* w = reinterpret_cast<unsigned char*>(ws.data());
   for (const TreeRound& R : P.rounds)
-    for (int g = R.seg0; g < R.seg0 + R.nseg; ++g) {
+    for (int k = 0; k < R.nseg; ++k) {
+      // a round's segments run side by side: last to first here for one tile size, first to last for the others
+      const int g = tile == 1 ? R.seg0 + R.nseg - 1 - k : R.seg0 + k;
       const TreeSeg& G = P.segs[g];
       const TreeInst& T = P.insts[G.inst];
       const TreeLevels& L = levels[G.inst];

@@ -86,13 +86,16 @@ static inline int tree_bytes(int stype) {
   }
 }
 
-// elements of a node, and of the scratch of step q (np parents)
+// elements of a node, of m in step q (np parents), and of its other scratch
 static inline long long tree_node_elems(const TreeInst& T, int q) {
   return (long long)tree_entries(tree_width(T.X, T.E, q), T.diag) * (T.deg[q] + 1);
 }
+static inline long long tree_m_elems(const TreeInst& T, int q, long long np) {
+  const bool has = q == T.steps ? T.pO >= 0 && T.steps < T.E : T.reps[q] == 1 && T.pL >= 0;
+  return has ? np * (T.deg[q] + 1) : 0;
+}
 static inline long long tree_scratch_elems(const TreeInst& T, int q, long long np) {
-  if (q == T.steps) return T.pO >= 0 && T.steps < T.E ? np * (T.deg[q] + 1) : 0;
-  if (T.reps[q] == 1) return T.pL >= 0 ? np * (T.deg[q] + 1) : 0;
+  if (q == T.steps || T.reps[q] == 1) return 0;
   if (T.reps[q] == 2) return np * (T.deg[q] + 1) * (8 + 2ll * tree_width(T.X, T.E, q + 1));
   return np * T.radix[q] * (T.deg[q + 1] + 1) * (6 + 2ll * tree_width(T.X, T.E, q + 1));
 }
@@ -103,7 +106,7 @@ struct TreeLevels {
   long long cap[MAX_EDGES + 2] = {0};    // nodes of level q's buffer
   long long chunk[MAX_EDGES + 2] = {0};  // parents of step q per block
   long long off[MAX_EDGES + 2] = {0};    // byte offsets
-  long long scr_off = 0, bytes = 0;
+  long long scr_off = 0, m_elems = 0, bytes = 0;  // m_elems: of one step
   double phases = 0;                     // about, of one execution
 };
 
@@ -117,14 +120,16 @@ static inline void tree_levels(const TreeInst& T, int sb, double budget, TreeLev
     const int R = q ? T.radix[q - 1] : 1;
     long long cap = std::max<long long>((long long)(budget / (double)nb), std::max(R, 64));
     if (q) {  // a block's children and its scratch
-      const long long se = std::max<long long>(tree_scratch_elems(T, q - 1, 1) * sb, 1);
+      const long long se =
+          std::max<long long>((tree_scratch_elems(T, q - 1, 1) + 2 * tree_m_elems(T, q - 1, 1)) * sb, 1);
       long long c = std::min(std::max<long long>(cap / R, 1), std::max<long long>((long long)(budget / (double)se), 1));
       c = std::min(c, g.cap[q - 1]);
       g.chunk[q - 1] = c;
       cap = c * R;
       scr = std::max(scr, tree_scratch_elems(T, q - 1, c) * sb);
+      g.m_elems = std::max(g.m_elems, tree_m_elems(T, q - 1, c));
       walks *= (double)((g.cap[q - 1] + c - 1) / c);
-      g.phases += walks * (T.reps[q - 1] == 1 ? (T.pL >= 0 ? 2 : 1) : (T.reps[q - 1] == 2 ? 2 : 4));
+      g.phases += walks * (T.reps[q - 1] == 1 ? 1 : (T.reps[q - 1] == 2 ? 2 : 4));
     }
     if (nodes < (double)cap) cap = (long long)nodes;
     g.cap[q] = cap;
@@ -132,21 +137,26 @@ static inline void tree_levels(const TreeInst& T, int sb, double budget, TreeLev
     off += al(cap * nb);
     if (q < T.steps) nodes *= T.radix[q];
   }
-  g.phases += walks * (T.pO >= 0 ? 2 : 1);
-  scr = std::max(scr, tree_scratch_elems(T, T.steps, g.cap[T.steps]) * sb);
+  g.phases += walks * (T.pL >= 0 ? 2 : 1);
+  g.m_elems = std::max(g.m_elems, tree_m_elems(T, T.steps, g.cap[T.steps]));
+  scr = std::max(scr, 2 * g.m_elems * sb);  // multiple edges come first: their scratch is free by then
   g.scr_off = off;
   g.bytes = off + al(std::max<long long>(scr, 16));
 }
 
-// A loop kind's simple edge needs m = C_ij + v_i v_j as a series first (TP_M); a level of so few
-// coefficients that four threads each do not fill `threads` sums it inside the step instead.
-static inline bool tree_fused(const TreeInst& T, int q, double np, double threads) {
-  return 4.0 * np * (T.deg[q] + 1) * tree_entries(tree_width(T.X, T.E, q + 1), T.diag) <= threads;
+// Whether a phase stands in the round of the one before it: a double edge's g beside its rows; of a
+// loop kind's simple edge the g of the step before, m and the other entries.
+static inline bool tree_same_round(int before, int phase) {
+  return (before == TP_W2 && phase == TP_G2) || (before == TP_G && phase == TP_M) || (before == TP_M && phase == TP_UNIT);
 }
 
-// the phases of an instance in order, each once for every block: f(phase, q, p0, np, level's nodes)
+// The phases of an instance in order, each once for every block: f(phase, q, p0, np, level's nodes).
+// `late`, a parents' block [late0, late0 + late) of a level of `lateps` nodes: step q - 1's TP_G, due in
+// this step's first round.
 template <class F>
-static void tree_walk(const TreeInst& T, const TreeLevels& g, int q, int np, double threads, F& f) {
+static void tree_walk(const TreeInst& T, const TreeLevels& g, int q, int np, F& f, int late0 = 0, int late = 0,
+                      int lateps = 0) {
+  if (late) f(TP_G, q - 1, late0, late, lateps);
   if (q == T.steps) {
     if (T.pO >= 0 && T.steps < T.E) f(TP_M, q, 0, np, np);
     f(TP_LEAF, q, 0, np, np);
@@ -156,8 +166,12 @@ static void tree_walk(const TreeInst& T, const TreeLevels& g, int q, int np, dou
   for (int p0 = 0; p0 < np; p0 += per) {
     const int c = std::min(per, np - p0);
     if (T.reps[q] == 1) {
-      if (T.pL >= 0 && !tree_fused(T, q, c, threads)) f(TP_M, q, p0, c, np);
+      if (T.pL >= 0) f(TP_M, q, p0, c, np);
       f(TP_UNIT, q, p0, c, np);
+      if (T.pL >= 0) {
+        tree_walk(T, g, q + 1, c * R, f, p0, c, np);
+        continue;
+      }
     } else if (T.reps[q] == 2) {
       const bool rows = tree_width(T.X, T.E, q + 1) > 0;
       if (rows) f(TP_W2, q, p0, c, np);
@@ -171,7 +185,7 @@ static void tree_walk(const TreeInst& T, const TreeLevels& g, int q, int np, dou
         if (T.pL >= 0) f(TP_GLOOP, q, p0, c, np);
       }
     }
-    tree_walk(T, g, q + 1, c * R, threads, f);
+    tree_walk(T, g, q + 1, c * R, f);
   }
 }
 
@@ -189,7 +203,8 @@ static inline double tree_items(const TreeInst& T, int phase, int q, double np, 
     case TP_ROOT: return tree_entries(tree_width(T.X, T.E, 0), T.diag);
     case TP_FIRST: return tree_entries(W, T.diag);
     case TP_M: return np * tree_tiles(Lp, tile);
-    case TP_UNIT: return np * tree_tiles(Lp, tile) * tree_entries(W, T.diag);
+    case TP_UNIT: case TP_G:
+      return np * tree_tiles(Lp, tile) * (tree_unit_end(T, phase, q) - tree_unit_begin(T, phase));
     case TP_PREP: case TP_GLOOP: return 32 * nc;
     case TP_G2: return 32 * np;
     case TP_W2: return np * 2 * W * tree_tiles(Lp, tile);
@@ -205,8 +220,8 @@ static inline double tree_macs(const TreeInst& T, int phase, int q, double np) {
   switch (phase) {
     case TP_ROOT: return 0;
     case TP_FIRST: return 2 * tree_entries((int)W, T.diag);
-    case TP_M: return np * tp;
-    case TP_UNIT: return np * tp * (2 * tree_entries((int)W, T.diag) - 1);
+    case TP_M: case TP_G: return np * tp;
+    case TP_UNIT: return np * tp * (2 * tree_entries((int)W, T.diag) - (T.pL >= 0 ? 2 : 1));
     case TP_PREP: return nc * 12 * tc * std::max(1.0, 32 / Lc);
     case TP_GLOOP: return nc * 5 * tc * std::max(1.0, 32 / Lc);
     case TP_G2: return np * 8 * tp * std::max(1.0, 10 / Lp);
@@ -262,8 +277,8 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
     TreeInst& T = insts[k];
     const TreeLevels& g = levels[k];
     T.scr_off = P.ws_bytes + g.scr_off;
+    T.m_odd = (int)g.m_elems;
     P.smem = std::max(P.smem, tree_warp_elems(T, sb));
-    const double fuse_threads = chip_threads / (double)insts.size();
     size_t r = 0;
     int last = -1;
     auto add = [&](int phase, int q, int p0, int np, int ps) {
@@ -277,18 +292,17 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
       s.pstride = ps;
       s.phase = (unsigned char)phase;
       s.q = (unsigned char)q;
-      s.fused = phase == TP_UNIT && T.pL >= 0 && tree_fused(T, q, np, fuse_threads);
-      if (phase == TP_G2 && last == TP_W2) --r;
+      if (tree_same_round(last, phase)) --r;
       last = phase;
       if (rounds.size() <= r) rounds.emplace_back();
       rounds[r++].push_back(s);
     };
     if (T.steps > 0 && T.reps[0] == 1) {
       add(TP_FIRST, 0, 0, 1, 1);
-      tree_walk(T, g, 1, 1, fuse_threads, add);
+      tree_walk(T, g, 1, 1, add);
     } else {
       add(TP_ROOT, 0, 0, 1, 1);
-      tree_walk(T, g, 0, 1, fuse_threads, add);
+      tree_walk(T, g, 0, 1, add);
     }
     P.ws_bytes += g.bytes;
   }
@@ -311,7 +325,7 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
     });
     for (TreeSeg& s : R) {
       const TreeInst& T = insts[s.inst];
-      s.tile = (unsigned char)(s.fused ? 0 : (use == 1 && (s.phase == TP_W2 || s.phase == TP_MULTI2) ? tile : use));
+      s.tile = (unsigned char)(use == 1 && (s.phase == TP_W2 || s.phase == TP_MULTI2) ? tile : use);
       long long warps = (long long)((tree_items(T, s.phase, s.q, s.np, s.tile) + 31) / 32);
       // leaves: at most the chip's warps, each with a partial for the reduction; the CTAs of a
       // single instance keep their sums over all leaf rounds and leave one partial each
@@ -343,12 +357,14 @@ static inline bool tree_one_cta(const std::vector<TreeInst>& insts, const std::v
   for (size_t k = 0; k < insts.size(); ++k) {
     const TreeInst& T = insts[k];
     double n = 0;
+    int last = -1;
     auto add = [&](int phase, int q, int, int np, int) {
       macs += tree_macs(T, phase, q, np);
-      n += 1;
+      n += !tree_same_round(last, phase);
+      last = phase;
     };
     if (levels[k].phases > 200) return false;
-    tree_walk(T, levels[k], 0, 1, 1e30, add);
+    tree_walk(T, levels[k], 0, 1, add);
     rounds = std::max(rounds, n);
   }
   return 1.5 * macs * clk + 2500.0 * rounds <= macs * clk / sms + 8000.0 * rounds;

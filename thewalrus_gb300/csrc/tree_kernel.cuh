@@ -76,6 +76,7 @@ struct alignas(16) TreeInst {
   int steps;                 // edges eliminated by steps: E, E - 1 or E - 2 (tree_leaf's closed forms)
   int nout;
   int pstride, comp_off;     // partial slots of a leaf warp (as InstDev's)
+  int m_odd;                 // loop kinds: scratch element from which odd steps keep m (even ones: 0)
   c64 oddloop;               // entry (pO, pL) when the unpaired vertex is not a vertex of A
   short row[TREE_MAX_POS], col[TREE_MAX_POS];  // position -> row and column of the extended matrix
   unsigned char reps[MAX_EDGES], radix[MAX_EDGES];
@@ -85,15 +86,18 @@ struct alignas(16) TreeInst {
 // The program of a launch: rounds of segments, with a barrier of the whole launch after each round.
 // A segment is one phase of one step of one instance over a block of parents [p0, p0 + np) of a
 // level of pstride nodes, by the round's warps [warp0, next segment's warp0).
-enum TreePhase : int { TP_ROOT = 0, TP_FIRST, TP_M, TP_UNIT, TP_PREP, TP_Y, TP_MULTI, TP_GLOOP, TP_W2, TP_G2, TP_MULTI2, TP_LEAF };
+// A loop kind's simple edge needs m = C_ij + v_i v_j as a series (TP_M) before its children's g (TP_G),
+// which nothing reads before the next step's TP_G: so that TP_M stands in the round of the other
+// entries (TP_UNIT) and TP_G in the round after it, beside the next step.  (A round of its own for
+// TP_M: loop n = 27 160 us, 131 so; n = 21 93 and 81.)
+enum TreePhase : int { TP_ROOT = 0, TP_FIRST, TP_M, TP_UNIT, TP_G, TP_PREP, TP_Y, TP_MULTI, TP_GLOOP, TP_W2, TP_G2, TP_MULTI2, TP_LEAF };
 struct alignas(16) TreeSeg {
   long long par, chi;        // workspace byte offsets of the parents' and the children's level
   int inst, warp0;
   int np, p0, pstride;
   int part;                  // leaf: the first warp's partial slot (one instance: the first CTA's)
   unsigned char phase, q, tile;  // tile: coefficients a thread, 0: four threads a coefficient
-  unsigned char fused;       // TP_UNIT without a TP_M before it
-  unsigned char pad[4];
+  unsigned char pad[5];
 };
 struct alignas(16) TreeRound {
   int seg0, nseg, nwarps, pad;
@@ -148,6 +152,13 @@ __host__ __device__ __forceinline__ int tree_ent(int a, int b, int diag) {
 __host__ __device__ __forceinline__ int tree_ent2(int a, int b, int diag) {
   return a > b ? tree_ent(a, b, diag) : tree_ent(b, a, diag);
 }
+// the entries of a segment TP_UNIT or TP_G, and where step q keeps its m
+__host__ __device__ __forceinline__ int tree_unit_begin(const TreeInst& T, int phase) { return phase == TP_UNIT && T.pL >= 0; }
+__host__ __device__ __forceinline__ int tree_unit_end(const TreeInst& T, int phase, int q) {
+  return phase == TP_G ? 1 : tree_entries(tree_width(T.X, T.E, q + 1), T.diag);
+}
+template <class S>
+__host__ __device__ __forceinline__ S* tree_m_of(const TreeInst& T, S* scr, int q) { return scr + (q & 1 ? T.m_odd : 0); }
 __host__ __device__ __forceinline__ void tree_decode(int e, int diag, int& a, int& b) {
   const int x = e - 1;
   int r = (int)((sqrtf(8.0f * (float)x + 1.0f) - 1.0f) * 0.5f);
@@ -532,15 +543,15 @@ __host__ __device__ void tree_m(const TreeInst& T, int q, const S* par, long lon
   }
 }
 
-// ---- a simple edge: children delta = +1 (nodes 0 .. np-1) and -1 (np .. 2 np - 1) from the same
-// products.  The weight -1 of the second joins g.
+// ---- a simple edge's entries [e0, e1): children delta = +1 (nodes 0 .. np-1) and -1 (np .. 2 np - 1)
+// from the same products.  The weight -1 of the second joins g.
 #pragma nv_exec_check_disable
 template <class S, int TL>
 __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long long ps, int np,
-                          const S* m, S* chi, int tid, int nthr) {
+                          const S* m, S* chi, int e0, int e1, int tid, int nthr) {
   using A = Ar<S>;
   const int i = T.X + 2 * (T.E - 1 - q), j = i + 1, dg = T.diag;
-  const int ne = tree_entries(i, dg), Lp = T.deg[q] + 1, Lc = Lp + 1;
+  const int ne = e1 - e0, Lp = T.deg[q] + 1, Lc = Lp + 1;
   const int nd = T.radix[q];  // 1: the root, which takes +1 only
   const long long cs = (long long)np * nd;
   if constexpr (TL == 0) {
@@ -548,7 +559,7 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
     const int sub = tid % WG_TREE_SPLIT;
     for (unsigned x0 = 0; x0 < total; x0 += step) {
       const unsigned x = x0 + tid / WG_TREE_SPLIT, r = x / np;
-      const int p = x - r * np, e = r % ne, t = Lp - 1 - (int)(r / ne);
+      const int p = x - r * np, e = e0 + r % ne, t = Lp - 1 - (int)(r / ne);
       int a = 0, b = 0;
       if (e) tree_decode(e, dg, a, b);
       const bool live = x < total && (e == 0 || tree_need(T, a, b));
@@ -563,14 +574,10 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
         if (e) {
           conv_part2(acc, pp + tree_ent(i, a, dg) * st, pp + tree_ent(j, b, dg) * st, pp + tree_ent(j, a, dg) * st,
                      pp + tree_ent(i, b, dg) * st, ps, Lp, ps, t, sub);
-        } else if (T.pL >= 0 && m) {
+        } else if (T.pL >= 0) {
           conv_part(acc, pp, ps, Lp, m + p, (long long)np, t, sub);
         } else {
           conv_part(acc, pp, ps, Lp, pp + tree_ent(j, i, dg) * st, ps, t, sub);
-          if (T.pL >= 0)  // m not formed beforehand: a round less, where rounds are the time
-            for (int s = sub; s <= t; s += WG_TREE_SPLIT)
-              acc.fma(tld(pp + s * ps), conv_one(pp + tree_ent(i, T.pL, dg) * st, ps, Lp,
-                                                 pp + tree_ent(j, T.pL, dg) * st, ps, Lp, t - s));
         }
       }
       using CA = ConvAcc<S>;
@@ -592,7 +599,7 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
   const unsigned total = (unsigned)nt * ne * np;
   for (unsigned x = tid; x < total; x += nthr) {
     const unsigned r = x / np;
-    const int p = x - r * np, e = r % ne, t0 = Lp - TT * ((int)(r / ne) + 1);
+    const int p = x - r * np, e = e0 + r % ne, t0 = Lp - TT * ((int)(r / ne) + 1);
     const S* pp = par + p;
     ConvAcc<S> acc[TT];
 #pragma unroll
@@ -1344,24 +1351,28 @@ __device__ __forceinline__ void tree_body(const TreeParams& P, const int cta, co
       const S* par = reinterpret_cast<const S*>(ws + G.par) + G.p0;
       S* chi = reinterpret_cast<S*>(ws + G.chi);
       S* scr = reinterpret_cast<S*>(ws + T.scr_off);
+      S* ms = tree_m_of(T, scr, G.q);
       switch (G.phase) {
         case TP_ROOT: tree_root<S>(T, P.pool, chi, tid, nthr); break;
         case TP_FIRST: tree_first<S>(T, P.pool, chi, tid, nthr); break;
         case TP_M:
-          if (G.tile == 0) tree_m<S, 0>(T, G.q, par, G.pstride, G.np, scr, tid, nthr);
-          else if (G.tile == 1) tree_m<S, 1>(T, G.q, par, G.pstride, G.np, scr, tid, nthr);
-          else tree_m<S, TL>(T, G.q, par, G.pstride, G.np, scr, tid, nthr);
+          if (G.tile == 0) tree_m<S, 0>(T, G.q, par, G.pstride, G.np, ms, tid, nthr);
+          else if (G.tile == 1) tree_m<S, 1>(T, G.q, par, G.pstride, G.np, ms, tid, nthr);
+          else tree_m<S, TL>(T, G.q, par, G.pstride, G.np, ms, tid, nthr);
           break;
         case TP_UNIT:
-          if (G.tile == 0) tree_unit<S, 0>(T, G.q, par, G.pstride, G.np, G.fused ? nullptr : scr, chi, tid, nthr);
-          else if (G.tile == 1) tree_unit<S, 1>(T, G.q, par, G.pstride, G.np, scr, chi, tid, nthr);
-          else tree_unit<S, TL>(T, G.q, par, G.pstride, G.np, scr, chi, tid, nthr);
+        case TP_G: {
+          const int e0 = tree_unit_begin(T, G.phase), e1 = tree_unit_end(T, G.phase, G.q);
+          if (G.tile == 0) tree_unit<S, 0>(T, G.q, par, G.pstride, G.np, ms, chi, e0, e1, tid, nthr);
+          else if (G.tile == 1) tree_unit<S, 1>(T, G.q, par, G.pstride, G.np, ms, chi, e0, e1, tid, nthr);
+          else tree_unit<S, TL>(T, G.q, par, G.pstride, G.np, ms, chi, e0, e1, tid, nthr);
           break;
+        }
         case TP_PREP: tree_prep<S>(T, G.q, par, G.pstride, G.np, scr, chi, smw, P.sm_warp, tid, nthr); break;
         case TP_LEAF: {
-          const S sum = G.tile == 0   ? tree_leaf<S, 0>(T, par, G.pstride, G.np, scr, smw, P.sm_warp, tid, nthr)
-                        : G.tile == 1 ? tree_leaf<S, 1>(T, par, G.pstride, G.np, scr, smw, P.sm_warp, tid, nthr)
-                                      : tree_leaf<S, TL>(T, par, G.pstride, G.np, scr, smw, P.sm_warp, tid, nthr);
+          const S sum = G.tile == 0   ? tree_leaf<S, 0>(T, par, G.pstride, G.np, ms, smw, P.sm_warp, tid, nthr)
+                        : G.tile == 1 ? tree_leaf<S, 1>(T, par, G.pstride, G.np, ms, smw, P.sm_warp, tid, nthr)
+                                      : tree_leaf<S, TL>(T, par, G.pstride, G.np, ms, smw, P.sm_warp, tid, nthr);
           if (P.ninst == 1) {  // all leaves are one instance's: one partial per CTA, below
             total = A::add(total, T.pB < 0 ? sum : tree_warp_share<S>(T, sum, smw));
           } else {
