@@ -854,10 +854,11 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
   return ws;
 }
 
-// whether the plan is one tree launch, which then also reduces (tree_finish): few enough outputs
-// for one CTA
+// whether the plan is one tree launch, which then also reduces (tree_finish): an output a warp of the
+// last CTA (64 photon patterns, whose partials one CTA sums in 150 us: 631 -> 518 us by a launch of
+// its own; one hafnian's launch 4 us)
 static bool plan_single(const wg_plan* pl) {
-  return pl->groups.empty() && (pl->trees.size() == 1 || pl->side_trees) && pl->total_out <= 64 * pl->primes;
+  return pl->groups.empty() && (pl->trees.size() == 1 || pl->side_trees) && pl->total_out <= TREE_THREADS / 32 * pl->primes;
 }
 static int plan_counters(const wg_plan* pl) {
   return (int)(pl->groups.size() + 2 * pl->trees.size());  // a tree launch's barrier and its tree_finish
