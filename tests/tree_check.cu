@@ -97,10 +97,8 @@ static void phase(const TreeInst& T, const TreeSeg& G, const unsigned char* pool
     case TP_ROOT: tree_root<hc>(T, pool, chi, tid, nthr); break;
     case TP_FIRST: tree_first<hc>(T, pool, chi, tid, nthr); break;
     case TP_M: tree_m<hc, TL>(T, G.q, par, G.pstride, G.np, tree_m_of(T, scr, G.q), tid, nthr); break;
-    case TP_UNIT: case TP_G:
-      tree_unit<hc, TL>(T, G.q, par, G.pstride, G.np, tree_m_of(T, scr, G.q), chi, tree_unit_begin(T, G.phase),
-                        tree_unit_end(T, G.phase, G.q), tid, nthr);
-      break;
+    case TP_UNIT: tree_unit<hc, TL>(T, G.q, par, G.pstride, G.np, chi, tid, nthr); break;
+    case TP_G: tree_g<hc, TL>(T, G.q, par, G.pstride, G.np, tree_m_of(T, scr, G.q), chi, tid, nthr); break;
     case TP_G2:
       tree_g2<hc>(T, G.q, par, G.pstride, G.np, scr + (2ll * tree_width(T.X, T.E, G.q + 1)) * (T.deg[G.q] + 1) * G.np, chi,
                   sm, smn, tid, nthr);

@@ -202,9 +202,8 @@ static inline double tree_items(const TreeInst& T, int phase, int q, double np, 
   switch (phase) {
     case TP_ROOT: return tree_entries(tree_width(T.X, T.E, 0), T.diag);
     case TP_FIRST: return tree_entries(W, T.diag);
-    case TP_M: return np * tree_tiles(Lp, tile);
-    case TP_UNIT: case TP_G:
-      return np * tree_tiles(Lp, tile) * (tree_unit_end(T, phase, q) - tree_unit_begin(T, phase));
+    case TP_M: case TP_G: return np * tree_tiles(Lp, tile);
+    case TP_UNIT: return np * tree_tiles(Lp, tile) * (tree_entries(W, T.diag) - (T.pL >= 0));
     case TP_PREP: case TP_GLOOP: return 32 * nc;
     case TP_G2: return 32 * np;
     case TP_W2: return np * 2 * W * tree_tiles(Lp, tile);

@@ -152,11 +152,7 @@ __host__ __device__ __forceinline__ int tree_ent(int a, int b, int diag) {
 __host__ __device__ __forceinline__ int tree_ent2(int a, int b, int diag) {
   return a > b ? tree_ent(a, b, diag) : tree_ent(b, a, diag);
 }
-// the entries of a segment TP_UNIT or TP_G, and where step q keeps its m
-__host__ __device__ __forceinline__ int tree_unit_begin(const TreeInst& T, int phase) { return phase == TP_UNIT && T.pL >= 0; }
-__host__ __device__ __forceinline__ int tree_unit_end(const TreeInst& T, int phase, int q) {
-  return phase == TP_G ? 1 : tree_entries(tree_width(T.X, T.E, q + 1), T.diag);
-}
+// where step q keeps its m
 template <class S>
 __host__ __device__ __forceinline__ S* tree_m_of(const TreeInst& T, S* scr, int q) { return scr + (q & 1 ? T.m_odd : 0); }
 __host__ __device__ __forceinline__ void tree_decode(int e, int diag, int& a, int& b) {
@@ -543,15 +539,15 @@ __host__ __device__ void tree_m(const TreeInst& T, int q, const S* par, long lon
   }
 }
 
-// ---- a simple edge's entries [e0, e1): children delta = +1 (nodes 0 .. np-1) and -1 (np .. 2 np - 1)
-// from the same products.  The weight -1 of the second joins g.
+// ---- a simple edge: children delta = +1 (nodes 0 .. np-1) and -1 (np .. 2 np - 1) from the same
+// products.  The weight -1 of the second joins g (loop kinds: tree_g).
 #pragma nv_exec_check_disable
 template <class S, int TL>
 __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long long ps, int np,
-                          const S* m, S* chi, int e0, int e1, int tid, int nthr) {
+                          S* chi, int tid, int nthr) {
   using A = Ar<S>;
   const int i = T.X + 2 * (T.E - 1 - q), j = i + 1, dg = T.diag;
-  const int ne = e1 - e0, Lp = T.deg[q] + 1, Lc = Lp + 1;
+  const int e0 = T.pL >= 0, ne = tree_entries(i, dg) - e0, Lp = T.deg[q] + 1, Lc = Lp + 1;
   const int nd = T.radix[q];  // 1: the root, which takes +1 only
   const long long cs = (long long)np * nd;
   if constexpr (TL == 0) {
@@ -574,8 +570,6 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
         if (e) {
           conv_part2(acc, pp + tree_ent(i, a, dg) * st, pp + tree_ent(j, b, dg) * st, pp + tree_ent(j, a, dg) * st,
                      pp + tree_ent(i, b, dg) * st, ps, Lp, ps, t, sub);
-        } else if (T.pL >= 0) {
-          conv_part(acc, pp, ps, Lp, m + p, (long long)np, t, sub);
         } else {
           conv_part(acc, pp, ps, Lp, pp + tree_ent(j, i, dg) * st, ps, t, sub);
         }
@@ -605,8 +599,7 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
 #pragma unroll
     for (int k = 0; k < TT; ++k) acc[k] = ConvAcc<S>::of(A::zero());
     if (e == 0) {
-      if (T.pL >= 0) conv_tile<S, TT>(acc, pp, ps, Lp, m + p, np, t0);
-      else conv_tile<S, TT>(acc, pp, ps, Lp, pp + (long long)tree_ent(j, i, dg) * Lp * ps, ps, t0);
+      conv_tile<S, TT>(acc, pp, ps, Lp, pp + (long long)tree_ent(j, i, dg) * Lp * ps, ps, t0);
     } else {
       int a, b;
       tree_decode(e, dg, a, b);
@@ -636,6 +629,57 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
           }
         }
       }
+    }
+  }
+}
+
+// ---- a loop kind's simple edge: the children's g = g (1 + delta eta m), of delta = -1 negative
+#pragma nv_exec_check_disable
+template <class S, int TL>
+__host__ __device__ void tree_g(const TreeInst& T, int q, const S* par, long long ps, int np, const S* m, S* chi, int tid,
+                                int nthr) {
+  using A = Ar<S>;
+  const int Lp = T.deg[q] + 1;
+  const long long cs = 2ll * np;
+  if constexpr (TL == 0) {
+    const int total = Lp * np, sub = tid % WG_TREE_SPLIT, step = nthr / WG_TREE_SPLIT;
+    for (int x0 = 0; x0 < total; x0 += step) {
+      const int x = x0 + tid / WG_TREE_SPLIT, p = x % np, t = Lp - 1 - x / np;
+      ConvAcc<S> acc = ConvAcc<S>::of(A::zero());
+      if (x < total) conv_part(acc, par + p, ps, Lp, m + p, (long long)np, t, sub);
+      const S u = split_sum(acc.sum());
+      if (x < total && sub == 0) {
+        const S c = t + 1 < Lp ? tld(par + p + (t + 1) * ps) : A::zero();
+        S* o = chi + p + (t + 1) * cs;
+        tst(o, A::add(c, u));
+        tst(o + np, A::sub(u, c));
+        if (t == 0) {
+          tst(chi + p, tld(par + p));
+          tst(chi + p + np, A::neg(tld(par + p)));
+        }
+      }
+    }
+    return;
+  }
+  constexpr int TT = TL ? TL : 1;
+  const int nt = (Lp + TT - 1) / TT;
+  for (int x = tid; x < nt * np; x += nthr) {
+    const int p = x % np, t0 = Lp - TT * (x / np + 1);
+    ConvAcc<S> acc[TT];
+#pragma unroll
+    for (int k = 0; k < TT; ++k) acc[k] = ConvAcc<S>::of(A::zero());
+    conv_tile<S, TT>(acc, par + p, ps, Lp, m + p, (long long)np, t0);
+#pragma unroll
+    for (int k = 0; k < TT; ++k) {
+      const int t = t0 + k;
+      if (t < 0) continue;
+      const S c = t + 1 < Lp ? tld(par + p + (t + 1) * ps) : A::zero(), u = acc[k].sum();
+      tst(chi + p + (t + 1) * cs, A::add(c, u));
+      tst(chi + p + np + (t + 1) * cs, A::sub(u, c));
+    }
+    if (t0 <= 0) {
+      tst(chi + p, tld(par + p));
+      tst(chi + p + np, A::neg(tld(par + p)));
     }
   }
 }
@@ -1361,13 +1405,15 @@ __device__ __forceinline__ void tree_body(const TreeParams& P, const int cta, co
           else tree_m<S, TL>(T, G.q, par, G.pstride, G.np, ms, tid, nthr);
           break;
         case TP_UNIT:
-        case TP_G: {
-          const int e0 = tree_unit_begin(T, G.phase), e1 = tree_unit_end(T, G.phase, G.q);
-          if (G.tile == 0) tree_unit<S, 0>(T, G.q, par, G.pstride, G.np, ms, chi, e0, e1, tid, nthr);
-          else if (G.tile == 1) tree_unit<S, 1>(T, G.q, par, G.pstride, G.np, ms, chi, e0, e1, tid, nthr);
-          else tree_unit<S, TL>(T, G.q, par, G.pstride, G.np, ms, chi, e0, e1, tid, nthr);
+          if (G.tile == 0) tree_unit<S, 0>(T, G.q, par, G.pstride, G.np, chi, tid, nthr);
+          else if (G.tile == 1) tree_unit<S, 1>(T, G.q, par, G.pstride, G.np, chi, tid, nthr);
+          else tree_unit<S, TL>(T, G.q, par, G.pstride, G.np, chi, tid, nthr);
           break;
-        }
+        case TP_G:
+          if (G.tile == 0) tree_g<S, 0>(T, G.q, par, G.pstride, G.np, ms, chi, tid, nthr);
+          else if (G.tile == 1) tree_g<S, 1>(T, G.q, par, G.pstride, G.np, ms, chi, tid, nthr);
+          else tree_g<S, TL>(T, G.q, par, G.pstride, G.np, ms, chi, tid, nthr);
+          break;
         case TP_PREP: tree_prep<S>(T, G.q, par, G.pstride, G.np, scr, chi, smw, P.sm_warp, tid, nthr); break;
         case TP_LEAF: {
           const S sum = G.tile == 0   ? tree_leaf<S, 0>(T, par, G.pstride, G.np, ms, smw, P.sm_warp, tid, nthr)
