@@ -30,7 +30,7 @@ def exe(tmp_path_factory):
     return path
 
 
-def evaluate(exe, insts, budget, chip):
+def evaluate(exe, insts, budget, chip, split=False):
     words = [len(insts), budget, 4, chip]
 
     def put(x, count):
@@ -45,7 +45,7 @@ def evaluate(exe, insts, budget, chip):
         put(inst.D, n)
         put(inst.oddV, n)
         words.extend([repr(s.oddloop[0]), repr(s.oddloop[1])])
-    run = subprocess.run([exe], input=" ".join(str(w) for w in words).encode(), stdout=subprocess.PIPE,
+    run = subprocess.run([exe] + ["split"] * split, input=" ".join(str(w) for w in words).encode(), stdout=subprocess.PIPE,
                          stderr=subprocess.STDOUT, timeout=120)
     assert run.returncode == 0, run.stdout.decode()
     v = np.array([[float(x) for x in line.split()] for line in run.stdout.decode().split("\n") if line])
@@ -57,8 +57,9 @@ def check(exe, inst, want):
     # Whole levels; blocks of nodes; one coefficient a thread everywhere and tiles everywhere
     want = np.atleast_1d(np.asarray(want, dtype=complex))
     for budget, chip in ((1e9, 77824), (3e4, 64), (2e3, 32)):
-        got = evaluate(exe, [inst], budget, chip)
-        assert np.max(np.abs(got - want)) <= 1e-11 * np.max(np.abs(want)), (budget, chip, got, want)
+        for split in (False, True):  # multiple edges as simple ones
+            got = evaluate(exe, [inst], budget, chip, split)
+            assert np.max(np.abs(got - want)) <= 1e-11 * np.max(np.abs(want)), (budget, chip, split, got, want)
 
 
 @pytest.mark.parametrize("n", [2, 4, 6, 8, 10, 14, 18])

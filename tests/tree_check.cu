@@ -118,7 +118,7 @@ static void phase(const TreeInst& T, const TreeSeg& G, const unsigned char* pool
   }
 }
 
-int main() {
+int main(int argc, char**) {  // with an argument: multiple edges as simple ones
   const int count = (int)rd();
   const double budget = rd();
   const int tile = (int)rd(), chip = (int)rd();  // as tree_program's
@@ -148,7 +148,7 @@ int main() {
     for (int i = 0; i < n; ++i) { const double re = rd(); at(n + 1, i) = {re, rd()}; }
     d.oddloop.re = rd();
     d.oddloop.im = rd();
-    if (!tree_build(d, insts[k])) { std::printf("FAIL no tree\n"); return 1; }
+    if (!(argc > 1 && tree_build(d, insts[k], true)) && !tree_build(d, insts[k])) { std::printf("FAIL no tree\n"); return 1; }
     insts[k].pstride = insts[k].nout;
     tree_levels(insts[k], sizeof(hc), budget, levels[k]);
   }
@@ -163,8 +163,8 @@ int main() {
   unsigned char* w = reinterpret_cast<unsigned char*>(ws.data());
   for (const TreeRound& R : P.rounds)
     for (int k = 0; k < R.nseg; ++k) {
-      // a round's segments run side by side: last to first here for one tile size, first to last for the others
-      const int g = tile == 1 ? R.seg0 + R.nseg - 1 - k : R.seg0 + k;
+      // a round's segments run side by side: last to first here for one of the sizes
+      const int g = chip == 64 ? R.seg0 + R.nseg - 1 - k : R.seg0 + k;
       const TreeSeg& G = P.segs[g];
       const TreeInst& T = P.insts[G.inst];
       const TreeLevels& L = levels[G.inst];

@@ -186,7 +186,9 @@ struct Prepared {
   long long t_lo = 0, t_hi = 0;  // sieve terms [t_lo, t_hi) of this instance
   bool tree = false;             // evaluated as an elimination tree
   TreeInst T;
-  std::vector<double> tscales;   // output scales of the tree's sum
+  std::vector<double> ascale;    // the input prescale's share of each output
+  int precision;
+  std::vector<double> tscales() const;  // output scales of the tree's sum
 };
 
 struct Group {
@@ -329,30 +331,41 @@ static inline double tree_asymmetry(int precision) {
 
 static MatrixForm matrix_form(const void* A, int dtype, size_t n, double tol) {
   MatrixForm f;
-  double big = 0, diff = 0, re, im, re2, im2;
-  bool pos = false, neg = false;
+  const int nc = dtype == WG_COMPLEX128 ? 2 : 1;
+  const double* M = (const double*)A;
+  double big = 0, diff = 0;
+  bool pos = false, neg = false, finite = true;
   std::vector<int> comp(n);
   for (size_t i = 0; i < n; ++i) comp[i] = (int)i;
+  size_t parts = n;
   auto root = [&](int x) {
     while (comp[x] != x) x = comp[x] = comp[comp[x]];
     return x;
   };
   for (size_t i = 0; i < n; ++i)
     for (size_t j = 0; j <= i; ++j) {
-      get_val(A, dtype, i * n + j, re, im);
-      get_val(A, dtype, j * n + i, re2, im2);
-      if (!(std::isfinite(re) && std::isfinite(im) && std::isfinite(re2) && std::isfinite(im2))) return f;
-      big = std::max(big, std::max(std::fabs(re), std::fabs(im)));
-      diff = std::max(diff, std::max(std::fabs(re - re2), std::fabs(im - im2)));
+      const double *x = M + (i * n + j) * nc, *y = M + (j * n + i) * nc;
+      bool zero = true;
+      for (int c = 0; c < nc; ++c) {
+        finite = finite && std::isfinite(x[c]) && std::isfinite(y[c]);
+        big = std::max(big, std::fabs(x[c]));
+        diff = std::max(diff, std::fabs(x[c] - y[c]));
+        zero = zero && x[c] == 0;
+      }
       if (i != j) {
-        pos = pos || re > 0;
-        neg = neg || re < 0;
-        if (re != 0 || im != 0) comp[root((int)i)] = root((int)j);
+        pos = pos || x[0] > 0;
+        neg = neg || x[0] < 0;
+        if (!zero && parts > 1 && comp[i] != comp[j]) {
+          const int a = root((int)i), b = root((int)j);
+          parts -= a != b;
+          comp[a] = b;
+        }
       }
     }
+  if (!finite) return f;
   f.symmetric = diff <= tol * big;
   f.signs = pos && neg;
-  for (size_t i = 1; i < n; ++i) f.blocks = f.blocks || root((int)i) != root(0);
+  f.blocks = parts > 1;
   return f;
 }
 
@@ -376,15 +389,21 @@ static bool keeps_terms(int stype, int kind, int K, const MatrixForm& f) {
   return false;  // residues are exact, double-double results agree to the last bits
 }
 
-// takes the tree when the instance has one; `ascale`: the input prescale's share of each output
+std::vector<double> Prepared::tscales() const {
+  std::vector<double> s;
+  for (double a : ascale) s.push_back(pow2_scale(tree_scale_exp(T), precision) * a);
+  return s;
+}
+
+// takes the tree when the instance has one
 static void take_tree(Prepared& P, int precision, const std::vector<double>& ascale, const MatrixForm& f) {
   P.tree = f.symmetric && tree_build(P.d, P.T) && tree_fits(P.T, tree_bytes(P.stype)) &&
            !keeps_terms(P.stype, P.d.kind, P.T.K, f);
   if (!P.tree) return;
   P.T.comp_off = stype_dd(P.stype) ? P.d.nout : 0;
   P.T.pstride = (stype_dd(P.stype) ? 2 : 1) * P.d.nout;
-  P.tscales.clear();
-  for (double a : ascale) P.tscales.push_back(pow2_scale(tree_scale_exp(P.T), precision) * a);
+  P.ascale = ascale;
+  P.precision = precision;
 }
 
 static int prepare(const wg_instance& in, int precision, Prepared& P) {
@@ -768,6 +787,11 @@ static double tree_mac_clocks(int stype) {
   }
 }
 
+// and of one edge of a term's latency (tree_latency's unit)
+static double tree_edge_clocks(int stype) {
+  return stype == ST_CPLXDD ? 80000 : stype == ST_REALDD ? 32000 : 16000;
+}
+
 // Groups the tree members of a plan into launches (one scalar type each, as many instances as share
 // a workspace budget), makes their programs and lays out their partial slots.  Returns the
 // workspace bytes; the launches run one after another and share it, or (an exact sum's primes) side
@@ -871,6 +895,40 @@ static int plan_wpo(const wg_plan* pl, int nw) {
   return w;
 }
 
+// Few photon pairs: a multiple edge as simple ones costs more nodes but fewer and shorter rounds, where
+// those are the time.  us before and after (FP64): loops [1, 1, 1, 2, 2, 2] 93 and 80, [1 x 8, 2, 2] 132
+// and 115, batches [1, 2, 2, 3] 167 and 133; over 1064 calls of 1 to 12 edges 14 % less.  Not in a batch of
+// at most five pairs in simple and double edges, whose leaves, a warp a node, are the time (batch [1, 2, 2]
+// 92 us, split 104).
+static void split_edges(std::vector<Prepared>& P) {
+  constexpr int kSplitPairs = 16;
+  std::vector<TreeInst> alt(P.size());
+  double lat = 0, lat1 = 0, work = 0, work1 = 0;
+  bool any = false;
+  for (size_t i = 0; i < P.size(); ++i) {
+    if (!P[i].tree) continue;
+    const TreeInst& T = P[i].T;
+    const int sb = tree_bytes(P[i].stype);
+    const double clk = tree_mac_clocks(P[i].stype) / g_num_sms;
+    const bool leaves = T.pB >= 0 && T.K <= 5 && *std::max_element(T.reps, T.reps + T.E) <= 2;
+    const bool split = T.K > T.E && T.K <= kSplitPairs && !leaves && tree_build(P[i].d, alt[i], true);
+    any = any || split;
+    const double unit = tree_edge_clocks(P[i].stype), w = tree_work(T, sb) * clk;
+    lat = std::max(lat, unit * tree_latency(T));
+    lat1 = std::max(lat1, unit * tree_latency(split ? alt[i] : T));
+    work += w;
+    work1 += split ? tree_work(alt[i], sb) * clk : w;
+    if (!split) alt[i].E = 0;
+  }
+  if (!any || lat1 + work1 >= lat + work) return;
+  for (size_t i = 0; i < P.size(); ++i)
+    if (P[i].tree && alt[i].E) {
+      alt[i].comp_off = P[i].T.comp_off;
+      alt[i].pstride = P[i].T.pstride;
+      P[i].T = alt[i];
+    }
+}
+
 // Whether the terms of a plan's trees are summed sooner one by one.  The terms run side by side, so
 // that their latency grows with the edges alone, and a tree's with its rounds: 0.7 of a term's edge for
 // a simple one, 2 for a double edge, 4 for one of three photons or more (its root and exponential
@@ -878,27 +936,26 @@ static int plan_wpo(const wg_plan* pl, int nw) {
 // their number, a tree's time hardly.  One unit is 6.5 to 12.5 us (FP64 plain to batches; double-double
 // 17 to 108); the weights are fitted to 2261 measured calls of 1 to 12 edges, multiplicities 1 to 12,
 // 1 to 10^4 terms, all scalar types.  us by tree and by terms (complex FP64, plain): [1 x 8] 57 and 97,
-// [3, 3, 3, 3] 136 and 76, [1, 2, 3] 68 and 57, [1 x 4, 2, 2, 3] 105 and 107, [1 x 6, 2, 2, 3] 118 and 203;
-// the rule takes the slower side by more than 10 % in 9 calls (1.27 at most) for the tree.
+// [3, 3, 3, 3] 136 and 76, [8, 8] 89 and 54, [1 x 6, 2, 2, 3] 118 and 203; of 1064 calls it takes the
+// tree in 7 where that is slower by more than 10 % (double-double [1, 2, 2, 3, 3, 3] 645 and 390 us the worst).
 static bool terms_sooner(const std::vector<Prepared>& P) {
   double tree = 0, terms = 0, work = 0;
   for (const Prepared& p : P) {
     if (!p.tree) continue;
     if (!tile_rows_ok(p.stype, p.rows_max)) return false;
-    const TreeInst& T = p.T;
-    double rounds = 0, t = 1;
-    int big = 0;
-    for (int q = 0; q < T.E; ++q) {
-      rounds += T.reps[q] == 1 ? 0.7 : (T.reps[q] == 2 ? 2.0 : 4.0);
-      big += T.reps[q] > 2;
-      t *= T.radix[q];
+    int E = 0, big = 0;
+    double t = 0.5;
+    for (int e = p.d.kind == KIND_BATCH_EVEN ? 1 : (p.d.kind == KIND_BATCH_ODD ? 2 : 0); e < p.d.E; ++e) {
+      E += p.d.reps[e] > 0;
+      big += p.d.reps[e] > 2;
+      t *= p.d.reps[e] + 1;
     }
     const bool dd = stype_dd(p.stype);
     // per-term work against a tree's: no less of it where all edges are multiple, a batch has its outputs'
-    const double share = p.d.nout > 1 ? 1.2 * p.d.nout : (T.E - big) / (double)std::max(T.E, 1);
-    tree = std::max(tree, rounds);
-    terms = std::max(terms, (dd ? 0.9 : 2.0) + T.E);
-    work += (dd ? 3.75e-5 : 1.5e-5) * share * t * ((double)T.E * T.E * T.E + (double)T.K * T.K);
+    const double share = p.d.nout > 1 ? 1.2 * p.d.nout : (E - big) / (double)std::max(E, 1);
+    tree = std::max(tree, tree_latency(p.T));
+    terms = std::max(terms, (dd ? 0.9 : 2.0) + E);
+    work += (dd ? 3.75e-5 : 1.5e-5) * share * t * ((double)E * E * E + (double)p.T.K * p.T.K);
   }
   return tree > terms + work;
 }
@@ -914,6 +971,7 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   pl->serial_groups = opt.serial_groups != 0;
   pl->precision = precision;
   pl->device = g_device;
+  split_edges(P);
   if (terms_sooner(P))
     for (Prepared& p : P) p.tree = false;
   // outputs and scales in instance order
@@ -923,7 +981,7 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
     P[i].d.out_base = out;
     P[i].d.scale_base = (int)scales.size();
     out += P[i].d.nout;
-    const std::vector<double>& sc = P[i].tree ? P[i].tscales : P[i].scales;
+    const std::vector<double> sc = P[i].tree ? P[i].tscales() : P[i].scales;
     scales.insert(scales.end(), sc.begin(), sc.end());
   }
   pl->total_out = out;

@@ -13,8 +13,10 @@ namespace wg {
 constexpr long long TREE_SMEM_BYTES = 200 << 10;  // dynamic shared memory of a CTA, at most
 
 // The tree of a prepared instance (whole sum, finite-difference signs); false when it does not
-// take one: more than TREE_MAX_K photon pairs, or inclusion/exclusion signs.
-static inline bool tree_build(const InstDev& d, TreeInst& T) {
+// take one: more than TREE_MAX_K photon pairs, or inclusion/exclusion signs.  `simple_only`: an edge of
+// multiplicity r as r simple edges on copies of its vertices (the same sum: r signs add up to each
+// delta binomially often), for at most MAX_EDGES pairs.
+static inline bool tree_build(const InstDev& d, TreeInst& T, bool simple_only = false) {
   memset(&T, 0, sizeof(T));
   const bool batch = d.kind >= KIND_BATCH_EVEN;
   const int nbe = d.kind == KIND_BATCH_EVEN ? 1 : (d.kind == KIND_BATCH_ODD ? 2 : 0);
@@ -39,11 +41,11 @@ static inline bool tree_build(const InstDev& d, TreeInst& T) {
   // edges by multiplicity, the other simple edges (cheapest per child, so at the wide bottom)
   std::vector<int> simple, multi, order;
   for (int e = nbe; e < d.E; ++e) {
-    if (d.reps[e] == 1) simple.push_back(e);
+    if (d.reps[e] == 1 || simple_only) simple.insert(simple.end(), d.reps[e], e);
     else if (d.reps[e] > 1) multi.push_back(e);
     T.K += d.reps[e];
   }
-  if (T.K > TREE_MAX_K) return false;
+  if (T.K > (simple_only ? MAX_EDGES : TREE_MAX_K)) return false;
   std::stable_sort(multi.begin(), multi.end(), [&](int a, int b) { return d.reps[a] < d.reps[b]; });
   size_t s0 = 0;
   if (!simple.empty()) order.push_back(simple[s0++]);
@@ -56,19 +58,19 @@ static inline bool tree_build(const InstDev& d, TreeInst& T) {
   // closed forms of the last simple edges
   int rem = 0;
   if (!batch)
-    while (rem < (T.pL < 0 ? 2 : 1) && rem < T.E && d.reps[order[T.E - 1 - rem]] == 1) ++rem;
+    while (rem < (T.pL < 0 ? 2 : 1) && rem < T.E && (simple_only || d.reps[order[T.E - 1 - rem]] == 1)) ++rem;
   T.steps = T.E - rem;
   T.diag = batch || !multi.empty();
   T.dpos = TREE_MAX_POS;
   for (int q = 0; q < T.E; ++q) {
-    const int e = order[q], i = T.X + 2 * (T.E - 1 - q);
+    const int e = order[q], i = T.X + 2 * (T.E - 1 - q), r = simple_only ? 1 : d.reps[e];
     T.row[i] = T.col[i] = (short)e;
     T.row[i + 1] = T.col[i + 1] = (short)(d.E + e);
-    T.reps[q] = (unsigned char)d.reps[e];
-    T.radix[q] = (unsigned char)(d.reps[e] + 1);
-    if (q == 0) T.radix[q] = (unsigned char)((d.reps[e] + 1 + (d.reps[e] % 2 == 0)) / 2);
-    if (d.reps[e] > 1) T.dpos = i;
-    T.deg[q + 1] = (unsigned char)(T.deg[q] + d.reps[e]);
+    T.reps[q] = (unsigned char)r;
+    T.radix[q] = (unsigned char)(r + 1);
+    if (q == 0) T.radix[q] = (unsigned char)((r + 1 + (r % 2 == 0)) / 2);
+    if (r > 1) T.dpos = i;
+    T.deg[q + 1] = (unsigned char)(T.deg[q] + r);
   }
   return true;
 }
@@ -349,6 +351,24 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
   for (TreeSeg& s : P.segs)
     if (s.phase == TP_LEAF) s.part = part_base[s.inst] + s.part * insts[s.inst].pstride;
   P.insts = insts;
+}
+
+// Latency of a tree's rounds in edges of the per-term evaluation (8.4 us for plain FP64): a simple edge's
+// one round, a double edge's two, the four of more photons with their root and exponential recurrences,
+// chains of FP64 latencies.
+static inline double tree_latency(const TreeInst& T) {
+  double lat = 0;
+  for (int q = 0; q < T.E; ++q) lat += T.reps[q] == 1 ? 0.7 : (T.reps[q] == 2 ? 2.0 : 4.0);
+  return lat;
+}
+// a tree's multiply-adds
+static inline double tree_work(const TreeInst& T, int sb) {
+  TreeLevels g;
+  tree_levels(T, sb, 1e18, g);
+  double macs = 0;
+  auto add = [&](int phase, int q, int, int np, int) { macs += tree_macs(T, phase, q, np); };
+  tree_walk(T, g, 0, 1, add);
+  return macs;
 }
 
 // Whether one CTA does a launch's work sooner than the whole chip: the multiply-adds against the
