@@ -218,6 +218,7 @@ struct wg_plan {
   int precision = 0;
   int primes = 1;           // > 1: every instance modulo so many primes, all instances of one first
   bool side_trees = false;  // the primes' trees run side by side in one launch
+  bool fork_trees = false;  // the scalar types' on side streams, each on its share of the SMs
   void* dmem = nullptr;
   wg::InstDev* d_inst = nullptr;
   wg::ChunkDev* d_chunks = nullptr;
@@ -819,7 +820,21 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
   long long first = 0;
   for (size_t k = 0; k < order.size() && P[order[k]].stype == P[order[0]].stype; ++k) first += lev[order[k]].bytes;
   pl->side_trees = pl->primes > 1 && !order.empty() && (double)first * pl->primes <= kSideBytes;
-  const int sms = pl->side_trees ? g_num_sms / pl->primes : g_num_sms;
+  // The launches of several scalar types side by side, each with SMs by its work and at least 30 % of an
+  // even share: one's narrow rounds and barriers no longer wait for the other's.  us in turn and so, plans of
+  // complex and real matrices: 8 of n = 8 to 12 72 and 55, 64 to n = 18 112 and 77, 160 to n = 28 833 and
+  // 769 (even shares: 985), 40 to n = 32 853 and 746.  Not beyond a launch's workspace, where they evict one
+  // another's levels from the L2 (250 to n = 30: 1,778 and 1,954).
+  std::map<int, double> works;  // SM clocks of a scalar type
+  double total = 0, work = 0;
+  for (int i : order) {
+    const double w = tree_work(P[i].T, lev[i]) * tree_mac_clocks(P[i].stype);
+    works[P[i].stype] += w;
+    work += w;
+    total += lev[i].bytes;
+  }
+  pl->fork_trees = !pl->side_trees && !pl->serial_groups && works.size() > 1 && total <= kLaunchBytes;
+  const double least = 0.3 / works.size();
   long long ws = 0;
   for (size_t k = 0; k < order.size();) {
     TreeLaunch G;
@@ -840,6 +855,9 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
     TreeProgram prog;
     std::vector<int> base, cnt;
     const double clk = tree_mac_clocks(G.stype);
+    const double share = pl->side_trees ? 1.0 / pl->primes
+                         : pl->fork_trees ? least + (1 - least * works.size()) * works[G.stype] / work : 1.0;
+    const int sms = std::max((int)(g_num_sms * share), 1);
     G.ctas = tree_one_cta(insts, levels, clk, sms) ? 1 : sms;
     tree_program(insts, levels, sb, tile, G.ctas * TREE_THREADS, nparts, base, cnt, prog);
     for (size_t j = 0; j < insts.size(); ++j) {
@@ -870,7 +888,7 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
       G.sm_ws = G.smem;
       G.smem += (int)prog.ws_bytes;
     } else {
-      G.ws_off = pl->side_trees ? ws : 0;
+      G.ws_off = pl->side_trees || pl->fork_trees ? ws : 0;
       ws = std::max(ws, G.ws_off + al(prog.ws_bytes));
     }
     pl->trees.push_back(G);
@@ -908,16 +926,20 @@ static void split_edges(std::vector<Prepared>& P) {
   for (size_t i = 0; i < P.size(); ++i) {
     if (!P[i].tree) continue;
     const TreeInst& T = P[i].T;
-    const int sb = tree_bytes(P[i].stype);
+    auto work_of = [&](const TreeInst& t) {
+      TreeLevels g;
+      tree_levels(t, tree_bytes(P[i].stype), 1e18, g);
+      return tree_work(t, g);
+    };
     const double clk = tree_mac_clocks(P[i].stype) / g_num_sms;
     const bool leaves = T.pB >= 0 && T.K <= 5 && *std::max_element(T.reps, T.reps + T.E) <= 2;
     const bool split = T.K > T.E && T.K <= kSplitPairs && !leaves && tree_build(P[i].d, alt[i], true);
     any = any || split;
-    const double unit = tree_edge_clocks(P[i].stype), w = tree_work(T, sb) * clk;
+    const double unit = tree_edge_clocks(P[i].stype), w = work_of(T) * clk;
     lat = std::max(lat, unit * tree_latency(T));
     lat1 = std::max(lat1, unit * tree_latency(split ? alt[i] : T));
     work += w;
-    work1 += split ? tree_work(alt[i], sb) * clk : w;
+    work1 += split ? work_of(alt[i]) * clk : w;
     if (!split) alt[i].E = 0;
   }
   if (!any || lat1 + work1 >= lat + work) return;
@@ -1217,10 +1239,37 @@ static int terms_plan(wg_plan* pl, wg_plan** out) {
   return WG_OK;
 }
 
+// `n` side streams that start where `st` stands
+static int fork_side(wg_plan* pl, cudaStream_t st, size_t n) {
+  if (!pl->fork) CK(cudaEventCreateWithFlags(&pl->fork, cudaEventDisableTiming));
+  while (pl->side.size() < n) {
+    cudaStream_t s2;
+    cudaEvent_t e2;
+    CK(cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&e2, cudaEventDisableTiming));
+    pl->side.push_back(s2);
+    pl->side_done.push_back(e2);
+  }
+  CK(cudaEventRecord(pl->fork, st));
+  for (size_t g = 0; g < n; ++g) CK(cudaStreamWaitEvent(pl->side[g], pl->fork, 0));
+  return WG_OK;
+}
+static int join_side(wg_plan* pl, cudaStream_t st, size_t g) {
+  CK(cudaEventRecord(pl->side_done[g], pl->side[g]));
+  CK(cudaStreamWaitEvent(st, pl->side_done[g], 0));
+  return WG_OK;
+}
+
 static int launch_trees(wg_plan* pl, cudaStream_t st) {
   TreeMods side;
   side.n = 0;
-  for (const TreeLaunch& G : pl->trees) {
+  if (pl->fork_trees) {
+    const int rc = fork_side(pl, st, pl->trees.size() - 1);
+    if (rc) return rc;
+  }
+  for (size_t i = 0; i < pl->trees.size(); ++i) {
+    const TreeLaunch& G = pl->trees[i];
+    const bool forked = pl->fork_trees && i > 0;
     TreeParams p;
     memset(&p, 0, sizeof(p));
     p.pool = pl->d_pool;
@@ -1260,8 +1309,12 @@ static int launch_trees(wg_plan* pl, cudaStream_t st) {
       if (side.n < (int)pl->trees.size()) continue;
     }
     const cudaError_t e = pl->side_trees ? tree_launch_mods(side, G.ctas * side.n, G.smem, st)
-                                         : tree_launch(G.stype, p, G.ctas, G.smem, st);
+                                         : tree_launch(G.stype, p, G.ctas, G.smem, forked ? pl->side[i - 1] : st);
     if (e != cudaSuccess) return fail(WG_ECUDA, "tree launch: %s", cudaGetErrorString(e));
+    if (forked) {
+      const int rc = join_side(pl, st, i - 1);
+      if (rc) return rc;
+    }
   }
   return WG_OK;
 }
@@ -1272,19 +1325,8 @@ static int launch_plan(wg_plan* pl, cudaStream_t st) {
   const size_t ng = pl->groups.size();
   const bool side = ng > 1 && !pl->serial_groups;
   if (side) {
-    if (pl->side.size() < ng - 1) {
-      if (!pl->fork) CK(cudaEventCreateWithFlags(&pl->fork, cudaEventDisableTiming));
-      while (pl->side.size() < ng - 1) {
-        cudaStream_t s2;
-        cudaEvent_t e2;
-        CK(cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&e2, cudaEventDisableTiming));
-        pl->side.push_back(s2);
-        pl->side_done.push_back(e2);
-      }
-    }
-    CK(cudaEventRecord(pl->fork, st));
-    for (size_t g = 1; g < ng; ++g) CK(cudaStreamWaitEvent(pl->side[g - 1], pl->fork, 0));
+    const int rc = fork_side(pl, st, ng - 1);
+    if (rc) return rc;
   }
   for (size_t g = 0; g < ng; ++g) {
     const Group& G = pl->groups[g];
@@ -1306,8 +1348,8 @@ static int launch_plan(wg_plan* pl, cudaStream_t st) {
     const cudaError_t e = sieve_launch(G.stype, p, G.ctas, G.wpc, gs);
     if (e != cudaSuccess) return fail(WG_ECUDA, "sieve launch: %s", cudaGetErrorString(e));
     if (g > 0 && side) {
-      CK(cudaEventRecord(pl->side_done[g - 1], gs));
-      CK(cudaStreamWaitEvent(st, pl->side_done[g - 1], 0));
+      const int rc = join_side(pl, st, g - 1);
+      if (rc) return rc;
     }
   }
   const int ninst = (int)pl->inst.size();

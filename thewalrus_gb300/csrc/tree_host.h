@@ -362,9 +362,7 @@ static inline double tree_latency(const TreeInst& T) {
   return lat;
 }
 // a tree's multiply-adds
-static inline double tree_work(const TreeInst& T, int sb) {
-  TreeLevels g;
-  tree_levels(T, sb, 1e18, g);
+static inline double tree_work(const TreeInst& T, const TreeLevels& g) {
   double macs = 0;
   auto add = [&](int phase, int q, int, int np, int) { macs += tree_macs(T, phase, q, np); };
   tree_walk(T, g, 0, 1, add);
