@@ -10,7 +10,7 @@ value    : hafnians/s with the input resident in HBM (device time of the sieve +
            over ranks (each rank runs its own shard of hafnians: weak scaling).
 e2e      : the same metric through the public API thewalrus_gb300.hafnian(A) from host NumPy
            input: host preparation, host->device upload, kernels, device->host result.
-roofline : algorithmic flops of the sieve (thewalrus_gb300.costmodel) / mean device time,
+roofline : algorithmic flops of the sieve's tree (thewalrus_gb300.costmodel) / mean device time,
            against the FP64 (or, for df, FP32) FMA-pipe peak measured in the same run.
 cpu_baseline : the CPU oracle (a C restatement of the reference algorithm: mixed-radix term
            order, power traces by repeated matrix products) on all host cores, timed on a
@@ -50,6 +50,12 @@ def workload(n=N_MATRIX, matrix="complex"):
     from thewalrus_gb300 import workloads as wl
 
     return wl.complex_symmetric(n, seed=0) if matrix == "complex" else wl.real_signed(n, seed=0)
+
+
+def by_call(precision):
+    """The ``precision`` argument of a call whose plan ran in ``precision``: FP64 is the default there
+    (asked for by name it is the per-term evaluation)."""
+    return None if precision == "fp64" else precision
 
 
 def dist_env():
@@ -249,11 +255,11 @@ def run_gpu(args, rank, world, local):
 
     # end to end through the public API: host prep + upload + kernels + result download
     for _ in range(min(args.warmup, 2)):
-        tw.hafnian(A, precision=args.precision)
+        tw.hafnian(A, precision=by_call(args.precision))
     torch.cuda.synchronize()
     t0 = time.perf_counter()
     for _ in range(args.steps):
-        r = tw.hafnian(A, precision=args.precision)
+        r = tw.hafnian(A, precision=by_call(args.precision))
     e2e_s = time.perf_counter() - t0
     if world > 1:
         t = torch.tensor([e2e_s], device="cuda", dtype=torch.float64)
@@ -262,7 +268,10 @@ def run_gpu(args, rank, world, local):
     e2e_value = world * args.steps / e2e_s
     h2d, d2h = plan.transfer_bytes()
 
-    flops = costmodel.plain_hafnian_flops(n, complex_input=args.matrix == "complex")
+    # a hafnian by its tree is one launch, its reduction included; by terms two
+    by_tree = plan.kernel_launches == 1
+    flops = (costmodel.tree_hafnian_flops if by_tree else costmodel.plain_hafnian_flops)(
+        n, complex_input=args.matrix == "complex")
     mean_s = total_ms / args.steps * 1e-3
     achieved = flops / mean_s / 1e12
     peak = fp32_peak if args.precision == "df" else fp64_peak  # double-double runs on the FP64 pipe
@@ -286,7 +295,7 @@ def run_gpu(args, rank, world, local):
                      "frac": achieved / peak, "traffic": None,
                      "traffic_note": "DRAM bytes need an ncu capture, not taken inside the bench",
                      "peak_source": "FMA-pipe microbenchmark (wg_measure_fp_peaks) in this run",
-                     "flops_per_launch": flops},
+                     "flops_per_launch": flops, "evaluation": "tree" if by_tree else "terms"},
         "gpu_launches": args.steps * plan.kernel_launches,
         "clocks": {"sm_mhz": clk["sm_mhz"], "sm_max_mhz": clk["sm_max_mhz"], "reasons": clk["reasons"]},
         "result": [float(np.real(result)), float(np.imag(result))],
@@ -355,8 +364,8 @@ def batch_summary(args):
     plan.close()
     outputs = len(mats) + sum(int(c) + 1 for _, _, _, c in calls)
     t0 = time.perf_counter()
-    per = [tw.hafnian(A, precision="fp64") for A in mats]
-    per_b = [tw.loop_hafnian_batch(B, D, list(f), c, precision="fp64") for B, D, f, c in calls]
+    per = [tw.hafnian(A) for A in mats]
+    per_b = [tw.loop_hafnian_batch(B, D, list(f), c) for B, D, f, c in calls]
     per_call_s = time.perf_counter() - t0
     diff = max(abs(per[i] - got[i]) / abs(per[i]) for i in range(len(mats)))
     off = len(mats)
@@ -549,7 +558,7 @@ def run_batch(args):
     # per-call plain launches on a deterministic sample (every 32nd instance), same accuracy
     sample = list(range(0, len(mats), 32))
     t0 = time.perf_counter()
-    per = [tw.hafnian(mats[i], precision=args.precision) for i in sample]
+    per = [tw.hafnian(mats[i], precision=by_call(args.precision)) for i in sample]
     per_call_s = time.perf_counter() - t0
     idx_sum = 0
     err = 0.0
@@ -579,7 +588,7 @@ def run_batch(args):
     sgot = splan.read(s.cuda_stream)
     ssample = list(range(0, len(small), 16))
     t0 = time.perf_counter()
-    sper = [tw.hafnian(small[i], precision=args.precision) for i in ssample]
+    sper = [tw.hafnian(small[i], precision=by_call(args.precision)) for i in ssample]
     small_per_call_s = (time.perf_counter() - t0) / len(ssample)
     small_err = max(abs(sper[k] - sgot[i]) / abs(sper[k]) for k, i in enumerate(ssample))
     print(json.dumps({

@@ -110,3 +110,11 @@ def test_several_instances(exe):
         got = evaluate(exe, insts, budget, chip)
         want = np.concatenate([evaluate(exe, [i], 1e9, 77824) for i in insts])
         assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
+
+
+def test_tree_macs():
+    """The cost model's count against a walk over the levels by hand: n = 6, 3 edges, one step."""
+    from thewalrus_gb300 import costmodel
+
+    assert costmodel.tree_hafnian_macs(6) == 2 * 7 + 3 * 3  # entries of 4 vertices; three products to order 1
+    assert costmodel.tree_hafnian_flops(40) == 6 * costmodel.tree_hafnian_macs(40) == 3 * costmodel.tree_hafnian_flops(40, False)

@@ -120,10 +120,7 @@ def matched_reps(reps):
     itself ``r // 2`` times, otherwise it is paired with the second as often as the second
     allows.  Returns ``(x, edge_reps, oddmode)`` with vertex ``x[i]`` matched to ``x[i + E]``.
     """
-    arr = np.asarray(reps)
-    if arr.ndim != 1 or arr.dtype.kind not in "iu":
-        arr = np.array([int(r) for r in reps], dtype=np.int64)
-    return nat.matched_reps(np.ascontiguousarray(arr, dtype=np.int64))
+    return nat.matched_reps(reps.tolist() if isinstance(reps, np.ndarray) else list(reps))
 
 
 def _cast(x, dt):

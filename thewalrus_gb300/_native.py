@@ -160,7 +160,7 @@ def load(build_if_needed=True):
     lib.wg_loop_hafnian.argtypes = [vp, vp, i32, i32, ip, i32, i32, dp, vp, i32, i32, dp, vp]
     lib.wg_loop_hafnian_batch.argtypes = [vp, vp, i32, i32, ip, i32, i32, i32, i32, i32, i32, dp, vp]
     lib.wg_hafnian_direct.argtypes = [vp, i32, i32, i32, ctypes.c_double, ctypes.c_double, dp, ctypes.POINTER(i32)]
-    lib.wg_matched_reps.argtypes = [vp, i32, vp, vp, ctypes.POINTER(i32), ctypes.POINTER(i32)]
+    lib.wg_matched_reps.argtypes = [vp, i32, vp, vp, vp, vp]
     lib.wg_plan_create.argtypes = [ctypes.POINTER(WgInstance), i32, i32, ctypes.c_double,
                                    ctypes.POINTER(vp)]
     lib.wg_plan_create_ex.argtypes = [ctypes.POINTER(WgInstance), i32, i32, ctypes.POINTER(WgPlanOptions),
@@ -466,14 +466,19 @@ def hafnian_direct(A, loop, rtol, atol):
 
 
 def matched_reps(reps):
-    """Pairing of the repetition counts (an int64 array): (x, edge_reps, oddmode or None)."""
+    """Pairing of the repetition counts (a list of ints): (x, edge_reps, oddmode or None).  One block
+    holds the counts, both results' room and the two scalars: the call is ~2 us, most of it ctypes."""
     n = len(reps)
-    buf = np.empty(6 * n + 1, dtype=np.int64)
-    p = buf.__array_interface__["data"][0]
-    E, odd = ctypes.c_int(), ctypes.c_int()
-    check(load().wg_matched_reps(reps.__array_interface__["data"][0], n, p, p + 32 * n, ctypes.byref(E),
-                                 ctypes.byref(odd)))
-    return buf[:2 * E.value], buf[4 * n:4 * n + E.value], None if odd.value < 0 else odd.value
+    buf = (ctypes.c_int64 * (7 * n + 2))()
+    try:
+        buf[:n] = reps
+    except TypeError:  # numbers of other types
+        buf[:n] = [int(r) for r in reps]
+    p = ctypes.addressof(buf)
+    check((_lib or load()).wg_matched_reps(p, n, p + 8 * n, p + 40 * n, p + 56 * n, p + 56 * n + 8))
+    E, odd = buf[7 * n], buf[7 * n + 1]  # 32-bit stores into zeros
+    res = np.frombuffer(buf, dtype=np.int64)
+    return res[n:n + 2 * E], res[5 * n:5 * n + E], None if odd == 0xFFFFFFFF else odd
 
 
 def check_arith(op, x, x_lo=None, y=None, y_lo=None):

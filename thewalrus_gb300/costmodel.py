@@ -13,12 +13,17 @@ Per sieve term with an m x m term matrix (mb = m + border, rows = mb + odd-mode 
   (1 + odd-mode rows) sum_{t=1..K} (min(t, Kc) + min(t-1, Kc)) (numerator, division by P), and
   the exp series K^2/2 (+ N^2/2 odd)
 
+The elimination tree, with E edges, q of them eliminated: 2^(q-1) nodes, whose 1 + W(W-1)/2 entries
+(W = 2 (E - q - 1)) each take two truncated series products of q + 1 coefficients in the next step (g
+one), and three at the leaves, two edges from the end.  A complex MAC is three real ones there.
+
 ``reference_term_macs`` is the reference's own per-term work (charpoly.powertrace by repeated
 matrix products, (K-1) * m^3 MACs), reported beside, never mixed into, the roofline.
 """
 import numpy as np
 
-__all__ = ["term_macs", "instance_flops", "plain_hafnian_flops", "reference_term_macs"]
+__all__ = ["term_macs", "instance_flops", "plain_hafnian_flops", "tree_hafnian_macs", "tree_hafnian_flops",
+           "reference_term_macs"]
 
 
 def term_macs(m, K, border=0, extra_rows=0, loop=False, odd_N=0):
@@ -76,6 +81,21 @@ def instance_flops(edge_reps, complex_input=True, kind="plain", glynn=True, odd=
 def plain_hafnian_flops(n, complex_input=True):
     """Flops of one plain Glynn hafnian of an n x n matrix (all repetitions 1)."""
     return instance_flops([1] * (n // 2), complex_input)
+
+
+def tree_hafnian_macs(n):
+    """Series multiply-adds of the elimination tree of a plain n x n hafnian (n >= 6, simple edges)."""
+    E = n // 2
+    entries = [1 + W * (W - 1) // 2 for W in range(2 * (E - 1), 2, -2)]  # after step 0, 1, ..., E - 3
+    macs = 2 * entries[0]
+    for q in range(1, E - 2):
+        macs += 2 ** (q - 1) * ((q + 1) * (q + 2) // 2) * (2 * entries[q] - 1)
+    return macs + 2 ** (E - 3) * 3 * ((E - 1) * E // 2)
+
+
+def tree_hafnian_flops(n, complex_input=True):
+    """Real flops of ``tree_hafnian_macs``: a complex MAC as the three real ones that are run."""
+    return tree_hafnian_macs(n) * (6 if complex_input else 2)
 
 
 def reference_term_macs(m, K):

@@ -920,9 +920,14 @@ static int plan_wpo(const wg_plan* pl, int nw) {
 // 92 us, split 104).
 static void split_edges(std::vector<Prepared>& P) {
   constexpr int kSplitPairs = 16;
+  auto splits = [](const Prepared& p) {
+    const TreeInst& T = p.T;
+    if (!p.tree || T.K == T.E || T.K > kSplitPairs) return false;
+    return T.pB < 0 || T.K > 5 || *std::max_element(T.reps, T.reps + T.E) > 2;
+  };
+  if (std::none_of(P.begin(), P.end(), splits)) return;
   std::vector<TreeInst> alt(P.size());
   double lat = 0, lat1 = 0, work = 0, work1 = 0;
-  bool any = false;
   for (size_t i = 0; i < P.size(); ++i) {
     if (!P[i].tree) continue;
     const TreeInst& T = P[i].T;
@@ -932,9 +937,7 @@ static void split_edges(std::vector<Prepared>& P) {
       return tree_work(t, g);
     };
     const double clk = tree_mac_clocks(P[i].stype) / g_num_sms;
-    const bool leaves = T.pB >= 0 && T.K <= 5 && *std::max_element(T.reps, T.reps + T.E) <= 2;
-    const bool split = T.K > T.E && T.K <= kSplitPairs && !leaves && tree_build(P[i].d, alt[i], true);
-    any = any || split;
+    const bool split = splits(P[i]) && tree_build(P[i].d, alt[i], true);
     const double unit = tree_edge_clocks(P[i].stype), w = work_of(T) * clk;
     lat = std::max(lat, unit * tree_latency(T));
     lat1 = std::max(lat1, unit * tree_latency(split ? alt[i] : T));
@@ -942,7 +945,7 @@ static void split_edges(std::vector<Prepared>& P) {
     work1 += split ? work_of(alt[i]) * clk : w;
     if (!split) alt[i].E = 0;
   }
-  if (!any || lat1 + work1 >= lat + work) return;
+  if (lat1 + work1 >= lat + work) return;
   for (size_t i = 0; i < P.size(); ++i)
     if (P[i].tree && alt[i].E) {
       alt[i].comp_off = P[i].T.comp_off;

@@ -2,6 +2,7 @@
 // and the program (rounds of segments) that a launch of the tree kernel runs.
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -26,8 +27,8 @@ static inline bool tree_build(const InstDev& d, TreeInst& T, bool simple_only = 
   T.pL = T.pO = T.pB = -1;
   T.a_off = d.a_off;
   auto extra = [&](int row, int col) {
-    T.row[T.X] = (short)row;
-    T.col[T.X] = (short)col;
+    T.row[T.X] = (signed char)row;
+    T.col[T.X] = (signed char)col;
     return T.X++;
   };
   if (d.kind != KIND_PLAIN) T.pL = extra(d.n, d.n);
@@ -64,8 +65,8 @@ static inline bool tree_build(const InstDev& d, TreeInst& T, bool simple_only = 
   T.dpos = TREE_MAX_POS;
   for (int q = 0; q < T.E; ++q) {
     const int e = order[q], i = T.X + 2 * (T.E - 1 - q), r = simple_only ? 1 : d.reps[e];
-    T.row[i] = T.col[i] = (short)e;
-    T.row[i + 1] = T.col[i + 1] = (short)(d.E + e);
+    T.row[i] = T.col[i] = (signed char)e;
+    T.row[i + 1] = T.col[i + 1] = (signed char)(d.E + e);
     T.reps[q] = (unsigned char)r;
     T.radix[q] = (unsigned char)(r + 1);
     if (q == 0) T.radix[q] = (unsigned char)((r + 1 + (r % 2 == 0)) / 2);
@@ -295,7 +296,10 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
       s.q = (unsigned char)q;
       if (tree_same_round(last, phase)) --r;
       last = phase;
-      if (rounds.size() <= r) rounds.emplace_back();
+      if (rounds.size() <= r) {
+        rounds.emplace_back();
+        rounds.back().reserve(insts.size());
+      }
       rounds[r++].push_back(s);
     };
     if (T.steps > 0 && T.reps[0] == 1) {
@@ -308,6 +312,11 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
     P.ws_bytes += g.bytes;
   }
   const bool dd = !insts.empty() && insts[0].comp_off > 0;
+  std::vector<unsigned char> key;
+  std::vector<int> order;
+  size_t nsegs = 0;
+  for (const auto& R : rounds) nsegs += R.size();
+  P.segs.reserve(nsegs);
   // partial slots instance by instance, so that an instance's are contiguous
   for (auto& R : rounds) {
     // whole tiles when those fill the chip, else one coefficient a thread, else four threads each
@@ -323,11 +332,22 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
     memset(&rr, 0, sizeof(rr));
     rr.seg0 = (int)P.segs.size();
     rr.nseg = (int)R.size();
-    // the costly segments' warps first
-    std::stable_sort(R.begin(), R.end(), [&](const TreeSeg& a, const TreeSeg& b) {
-      return tree_macs(insts[a.inst], a.phase, a.q, a.np) > tree_macs(insts[b.inst], b.phase, b.q, b.np);
-    });
-    for (TreeSeg& s : R) {
+    // the costly segments' warps first, by the exponent of their multiply-adds
+    key.resize(R.size());
+    order.resize(R.size());
+    int at[64] = {0};
+    for (size_t i = 0; i < R.size(); ++i) {
+      const TreeSeg& s = R[i];
+      ++at[key[i] = (unsigned char)(63 - std::min(std::ilogb(tree_macs(insts[s.inst], s.phase, s.q, s.np) + 1), 63))];
+    }
+    for (int b = 0, sum = 0; b < 64; ++b) {
+      const int c = at[b];
+      at[b] = sum;
+      sum += c;
+    }
+    for (size_t i = 0; i < R.size(); ++i) order[at[key[i]]++] = (int)i;
+    for (int i : order) {
+      TreeSeg& s = R[i];
       const TreeInst& T = insts[s.inst];
       s.tile = (unsigned char)(use == 1 && (s.phase == TP_W2 || s.phase == TP_MULTI2) ? tile : use);
       long long warps = (long long)((tree_items(T, s.phase, s.q, s.np, s.tile) + 31) / 32);

@@ -78,7 +78,7 @@ struct alignas(16) TreeInst {
   int pstride, comp_off;     // partial slots of a leaf warp (as InstDev's)
   int m_odd;                 // loop kinds: scratch element from which odd steps keep m (even ones: 0)
   c64 oddloop;               // entry (pO, pL) when the unpaired vertex is not a vertex of A
-  short row[TREE_MAX_POS], col[TREE_MAX_POS];  // position -> row and column of the extended matrix
+  signed char row[TREE_MAX_POS], col[TREE_MAX_POS];  // position -> row and column of the extended matrix
   unsigned char reps[MAX_EDGES], radix[MAX_EDGES];
   unsigned char deg[MAX_EDGES + 4];  // degree of the series after q steps
 };
