@@ -12,8 +12,9 @@ Same names, arguments, return conventions and errors as the reference's public f
 * ``loop_hafnian_batch`` thewalrus/loop_hafnian_batch.py:260-304
 
 The host keeps validation, the closed forms for tiny matrices, edge pairing and reordering;
-every sieve runs on the GPU (no CPU fallback).  Extra keyword ``precision`` selects "fp64"
-(default), "df" (FP32 double-float term arithmetic), "dd" (FP64 double-double terms, for sums
+every sieve runs on the GPU (no CPU fallback).  Extra keyword ``precision``: None (exact for
+integer inputs, else FP64, the sum taken as an elimination tree where one exists), "fp64" (the
+per-term FP64 evaluation, whose rounding the term magnitudes bound), "df" (FP32 double-float term arithmetic), "dd" (FP64 double-double terms, for sums
 that cancel beyond FP64's reach), "auto" (FP64, and double-double again for the instances whose
 term magnitudes say FP64 may miss 1e-10) or "exact" (integer inputs).  Sieve results come back as
 ``numpy.complex128`` also for real input, as in the reference.
@@ -393,8 +394,9 @@ def hafnian(A, loop=False, rtol=1e-05, atol=1e-08, approx=False, num_samples=100
 
     Args and results as ``thewalrus.hafnian``; ``method`` is "glynn" or "inclexcl" (the loop
     hafnian always uses the finite-difference sieve, as in the reference).  ``precision``:
-    None (exact for integer-valued real inputs, FP64 otherwise), "fp64", "df" (double-float
-    terms), "dd" (double-double terms: ~14x the FP64 time, for sieve sums whose terms cancel by
+    None (exact for integer-valued real inputs, FP64 otherwise), "fp64" (FP64 term by term: 50x
+    the default's time at n = 40), "df" (double-float),
+    "dd" (double-double: ~6 to 12x the FP64 time, for sieve sums whose terms cancel by
     more than ~1e6, e.g. the loop hafnians of many-photon Gaussian-state patterns), "auto"
     (FP64, re-run in double-double when the sum of the terms' magnitudes says FP64 may miss
     1e-10) or "exact" (integer inputs only).

@@ -5,11 +5,12 @@
 //     converted to the kernel's scalar type,
 //   * a chunk queue: every instance's term range split into chunks whose cost is balanced
 //     against the number of resident warps, largest instances first,
-//   * the elimination tree of every instance that takes one (tree_kernel.cuh): small trees as one
-//     launch per scalar type over a task queue, large ones level by level,
+//   * the elimination tree of every instance that takes one (tree_kernel.cuh): one cooperative launch
+//     per scalar type and workspace budget, whose rounds hold the levels of all its trees,
 //   * for the others (term ranges, inclusion/exclusion, per-term precisions, matrices that are not
 //     symmetric) one persistent sieve launch per (scalar type, resident warps per SM) group,
-//   * one reduction launch that sums the partials in a fixed order (bitwise reproducible results).
+//   * one reduction launch that sums the partials in a fixed order (bitwise reproducible results);
+//     a plan of a single tree launch and few outputs reduces in it.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -775,7 +776,7 @@ static int build_plan(const wg_instance* v, int count, int precision, const wg_p
   return finalize_plan(P, precision, opt, pl, nullptr, nullptr);
 }
 
-// Per scalar type: SM clocks per multiply-add of a tree (measured at the grid kernel's rate)
+// Per scalar type: SM clocks per multiply-add of a tree, measured over launches that fill the chip
 static double tree_mac_clocks(int stype) {
   switch (stype) {
     case ST_REAL64: return 0.5;

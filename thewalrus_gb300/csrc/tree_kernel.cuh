@@ -25,11 +25,13 @@
 // What bounds it: the FP64 pipe (2 multiply-adds per clock and SM), i.e. the number of FP64 warp
 // instructions; loads are a few bytes per clock even from L2.  So lanes are nodes (p fastest: the
 // same entry and coefficients of 32 nodes, no idle lanes below the top few levels) and every
-// thread forms tree_tile() consecutive coefficients of one entry in registers.  Measured against the
-// per-term kernel (us a call): complex n = 24 568 -> 248, n = 40 244,700 -> 6,580; real n = 44
-// (positive) 380,900 -> 9,010; 96 matrices of n = 8 .. 32 in a plan 61,850 -> 2,560; complex n = 28
-// in double-double 22,330 -> 1,910, n = 34 in double-float 12,420 -> 520; a graph of 32 vertices
-// modulo the primes of its exact count 9,090 -> 600.
+// thread forms tree_tile() consecutive coefficients of one entry in registers.  The levels are rounds
+// of one cooperative launch with a barrier after each (2,400 clocks): the narrow ones, a few thousand
+// clocks of FP64 and L2 latency, bound trees of up to ~14 pairs, the FP64 pipe (77 % busy at n = 34)
+// the larger ones.  Measured against the per-term kernel (us a call): complex n = 24 576 -> 102, n = 40
+// 244,600 -> 4,820; real n = 44 (positive) 380,900 -> 7,980; loops n = 27 2,330 -> 148; 96 matrices of
+// n = 8 .. 32 in a plan 61,850 -> 1,720; complex n = 28 in double-double 22,450 -> 756, n = 34 in
+// double-float 12,410 -> 448; the exact count of a graph of 32 vertices 9,110 -> 360.
 // (The reference's tree for unit edges is thewalrus/_hafnian.py recursive_hafnian's squeeze; this
 // one sums the finite-difference signs of _calc_hafnian / _calc_loop_hafnian, :443-577, and of
 // loop_hafnian_batch.py:50-208.)
