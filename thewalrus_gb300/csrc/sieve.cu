@@ -841,7 +841,9 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
     TreeLaunch G;
     memset(&G, 0, sizeof(G));
     G.stype = P[order[k]].stype;
-    const int sb = tree_bytes(G.stype), tile = G.stype == ST_CPLXDD ? tree_tile<cdd>() : tree_tile<c64>();
+    const int sb = tree_bytes(G.stype);
+    const int tile = stype_mod(G.stype) ? tree_tile<modp<MOD_PRIMES[0]>>()
+                                        : (G.stype == ST_CPLXDD ? tree_tile<cdd>() : tree_tile<c64>());
     std::vector<TreeInst> insts;
     std::vector<TreeLevels> levels;
     const size_t k0 = k;

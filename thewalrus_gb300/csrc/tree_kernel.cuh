@@ -59,9 +59,10 @@ constexpr int TREE_THREADS = 512;  // one CTA per SM
 // Coefficients a thread forms in registers (TL below): more of them share a load, but a level with
 // fewer tiles than threads leaves the chip idle, so narrower levels take one coefficient a thread and
 // the narrowest four threads a coefficient (TL = 0), whose chain of loads and FP64 instructions is the
-// level's time.
+// level's time.  Residues, one register each, take four (n = 40 999 -> 878 us, n = 36 257 -> 244, n = 32 as with
+// three); four or more cost the others: double-float n = 34 316 -> 331 us, real n = 32 144 -> 149 (five).
 template <class S>
-__host__ __device__ constexpr int tree_tile() { return Ar<S>::dd && Ar<S>::cplx ? 2 : 3; }
+__host__ __device__ constexpr int tree_tile() { return Ar<S>::modular ? 4 : (Ar<S>::dd && Ar<S>::cplx ? 2 : 3); }
 __host__ __device__ __forceinline__ int tree_tiles(int L, int TL) { return (L + TL - 1) / TL; }
 
 // One instance's tree.  Positions 0 .. X-1 are the rows that are never eliminated (pL: the loop
