@@ -187,7 +187,7 @@ int main(int argc, char**) {  // with an argument: multiple edges as simple ones
       const bool wide = G.phase == TP_PREP || G.phase == TP_GLOOP || G.phase == TP_G2 || (G.phase == TP_LEAF && T.pB >= 0);
       const int nthr = wide ? warps : warps * 32;
       for (int t = 0; t < nthr; ++t) {
-        if (G.tile == 0) phase<0>(T, G, pool, par, chi, scr, sm.data(), smn, t, nthr, out[G.inst].data());
+        if (G.tile == 0 || G.tile == TREE_PAIRS) phase<0>(T, G, pool, par, chi, scr, sm.data(), smn, t, nthr, out[G.inst].data());
         else if (G.tile == 1) phase<1>(T, G, pool, par, chi, scr, sm.data(), smn, t, nthr, out[G.inst].data());
         else phase<4>(T, G, pool, par, chi, scr, sm.data(), smn, t, nthr, out[G.inst].data());
       }

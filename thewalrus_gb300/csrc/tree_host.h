@@ -195,6 +195,7 @@ static void tree_walk(const TreeInst& T, const TreeLevels& g, int q, int np, F& 
 // threads of a phase with `tile` coefficients a thread (0: four threads a coefficient), and its
 // multiply-adds
 static inline double tree_items(const TreeInst& T, int phase, int q, double np, int tile) {
+  if (tile == TREE_PAIRS) return 2 * tree_items(T, phase, q, np, 1);
   if (tile == 0) {
     const bool whole = phase == TP_ROOT || phase == TP_FIRST || phase == TP_PREP || phase == TP_GLOOP || phase == TP_G2 ||
                        (phase == TP_LEAF && (T.pB >= 0 || T.steps == T.E));
@@ -319,7 +320,10 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
   P.segs.reserve(nsegs);
   // partial slots instance by instance, so that an instance's are contiguous
   for (auto& R : rounds) {
-    // whole tiles when those fill the chip, else one coefficient a thread, else four threads each
+    // whole tiles when those fill the chip, else one coefficient a thread, else four threads each, or two
+    // (a step's entries, when four would be more than a warp a sub-partition: fewer warps pay the sum over
+    // the threads and the children's; double-double n = 24 305 -> 265 us, FP64 n = 24 84 -> 81, others within
+    // 1 %; from a quarter of the chip on FP64 n = 22 72 -> 75)
     double whole = 0, split = 0;
     for (const TreeSeg& s : R) {
       whole += tree_items(insts[s.inst], s.phase, s.q, s.np, tile);
@@ -349,7 +353,9 @@ static inline void tree_program(std::vector<TreeInst>& insts, const std::vector<
     for (int i : order) {
       TreeSeg& s = R[i];
       const TreeInst& T = insts[s.inst];
-      s.tile = (unsigned char)(use == 1 && (s.phase == TP_W2 || s.phase == TP_MULTI2) ? tile : use);
+      s.tile = (unsigned char)use;
+      if (use == 1 && (s.phase == TP_W2 || s.phase == TP_MULTI2)) s.tile = (unsigned char)tile;
+      if (use == 0 && s.phase == TP_UNIT && split > 0.35 * chip_threads) s.tile = TREE_PAIRS;
       long long warps = (long long)((tree_items(T, s.phase, s.q, s.np, s.tile) + 31) / 32);
       // leaves: at most the chip's warps, each with a partial for the reduction; the CTAs of a
       // single instance keep their sums over all leaf rounds and leave one partial each

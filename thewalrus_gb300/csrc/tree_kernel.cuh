@@ -28,9 +28,9 @@
 // thread forms tree_tile() consecutive coefficients of one entry in registers.  The levels are rounds
 // of one cooperative launch with a barrier after each (2,400 clocks): the narrow ones, a few thousand
 // clocks of FP64 and L2 latency, bound trees of up to ~14 pairs, the FP64 pipe (77 % busy at n = 34)
-// the larger ones.  Measured against the per-term kernel (us a call): complex n = 24 576 -> 99, n = 40
-// 244,600 -> 4,820; real n = 44 (positive) 380,900 -> 7,980; loops n = 27 2,320 -> 145; 96 matrices of
-// n = 8 .. 32 in a plan 61,850 -> 1,720; complex n = 28 in double-double 22,250 -> 741, n = 34 in
+// the larger ones.  Measured against the per-term kernel (us a call): complex n = 24 576 -> 96, n = 40
+// 244,600 -> 4,820; real n = 44 (positive) 380,900 -> 7,980; loops n = 27 2,320 -> 144; 96 matrices of
+// n = 8 .. 32 in a plan 61,850 -> 1,720; complex n = 28 in double-double 22,300 -> 731, n = 34 in
 // double-float 12,380 -> 436; the exact count of a graph of 32 vertices 9,100 -> 342.
 // (The reference's tree for unit edges is thewalrus/_hafnian.py recursive_hafnian's squeeze; this
 // one sums the finite-difference signs of _calc_hafnian / _calc_loop_hafnian, :443-577, and of
@@ -85,6 +85,8 @@ struct alignas(16) TreeInst {
   unsigned char reps[MAX_EDGES], radix[MAX_EDGES];
   unsigned char deg[MAX_EDGES + 4];  // degree of the series after q steps
 };
+
+constexpr int TREE_PAIRS = 255;  // a segment's tile: two threads a coefficient (TP_UNIT)
 
 // The program of a launch: rounds of segments, with a barrier of the whole launch after each round.
 // A segment is one phase of one step of one instance over a block of parents [p0, p0 + np) of a
@@ -400,36 +402,36 @@ __host__ __device__ __forceinline__ S conv_one(const S* a, long long sa, int la,
   return r.sum();
 }
 
-// the terms s = sub, sub + WG_TREE_SPLIT, ... of coefficient t of a product
+// the terms s = sub, sub + SP, ... of coefficient t of a product
 #pragma nv_exec_check_disable
-template <class S>
+template <int SP = WG_TREE_SPLIT, class S>
 __host__ __device__ __forceinline__ void conv_part(ConvAcc<S>& acc, const S* a, long long sa, int la, const S* b, long long sb,
                                                    int t, int sub) {
   const int n = t < la - 1 ? t : la - 1;
 #pragma unroll 4
-  for (int s = sub; s <= n; s += WG_TREE_SPLIT) acc.fma(tld(a + s * sa), tld(b + (t - s) * sb));
+  for (int s = sub; s <= n; s += SP) acc.fma(tld(a + s * sa), tld(b + (t - s) * sb));
 }
 // the same of two products at once: their loads overlap
 #pragma nv_exec_check_disable
-template <class S>
+template <int SP = WG_TREE_SPLIT, class S>
 __host__ __device__ __forceinline__ void conv_part2(ConvAcc<S>& acc, const S* a, const S* b, const S* c, const S* d, long long sa,
                                                     int la, long long sb, int t, int sub) {
   const int n = t < la - 1 ? t : la - 1;
 #pragma unroll 2
-  for (int s = sub; s <= n; s += WG_TREE_SPLIT) {
+  for (int s = sub; s <= n; s += SP) {
     const S x = tld(a + s * sa), y = tld(b + (t - s) * sb), z = tld(c + s * sa), w = tld(d + (t - s) * sb);
     acc.fma(x, y);
     acc.fma(z, w);
   }
 }
-// the sum over the four threads of a coefficient, in each of them
+// the sum over the SP threads of a coefficient, in each of them
 #pragma nv_exec_check_disable
-template <class S>
+template <int SP = WG_TREE_SPLIT, class S>
 __host__ __device__ __forceinline__ S split_sum(S v) {
 #ifdef __CUDA_ARCH__
   using A = Ar<S>;
 #pragma unroll
-  for (int off = 1; off < WG_TREE_SPLIT; off *= 2) {
+  for (int off = 1; off < SP; off *= 2) {
 #pragma unroll
     for (int c = 0; c < A::NC; ++c) {
       const typename A::Comp x = A::comp(v, c);
@@ -553,11 +555,12 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
   const int e0 = T.pL >= 0, ne = tree_entries(i, dg) - e0, Lp = T.deg[q] + 1, Lc = Lp + 1;
   const int nd = T.radix[q];  // 1: the root, which takes +1 only
   const long long cs = (long long)np * nd;
-  if constexpr (TL == 0) {
-    const unsigned total = (unsigned)Lp * ne * np, step = nthr / WG_TREE_SPLIT;
-    const int sub = tid % WG_TREE_SPLIT;
+  if constexpr (TL <= 0) {  // TL < 0: two threads a coefficient
+    constexpr int SP = TL < 0 ? (WG_TREE_SPLIT + 1) / 2 : WG_TREE_SPLIT;
+    const unsigned total = (unsigned)Lp * ne * np, step = nthr / SP;
+    const int sub = tid % SP;
     for (unsigned x0 = 0; x0 < total; x0 += step) {
-      const unsigned x = x0 + tid / WG_TREE_SPLIT, r = x / np;
+      const unsigned x = x0 + tid / SP, r = x / np;
       const int p = x - r * np, e = e0 + r % ne, t = Lp - 1 - (int)(r / ne);
       int a = 0, b = 0;
       if (e) tree_decode(e, dg, a, b);
@@ -571,17 +574,17 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
         if (sub < 2 && t + 1 < Lp) c = tld(base + (t + 1) * ps);
         if (sub < 2 && t == 0) c0 = tld(base);
         if (e) {
-          conv_part2(acc, pp + tree_ent(i, a, dg) * st, pp + tree_ent(j, b, dg) * st, pp + tree_ent(j, a, dg) * st,
+          conv_part2<SP>(acc, pp + tree_ent(i, a, dg) * st, pp + tree_ent(j, b, dg) * st, pp + tree_ent(j, a, dg) * st,
                      pp + tree_ent(i, b, dg) * st, ps, Lp, ps, t, sub);
         } else {
-          conv_part(acc, pp, ps, Lp, pp + tree_ent(j, i, dg) * st, ps, t, sub);
+          conv_part<SP>(acc, pp, ps, Lp, pp + tree_ent(j, i, dg) * st, ps, t, sub);
         }
       }
       using CA = ConvAcc<S>;
-      const typename CA::U u = split_sum(acc.parts());
+      const typename CA::U u = split_sum<SP>(acc.parts());
       if (live && sub < 2) {  // thread 0 stores the +1 child, thread 1 the -1 child, in the same instructions
         S* o = chi + (long long)e * Lc * cs + p;
-        for (int h = sub; h < (WG_TREE_SPLIT > 1 ? sub + 1 : 2) && h < nd; ++h) {
+        for (int h = sub; h < (SP > 1 ? sub + 1 : 2) && h < nd; ++h) {
           const S v = CA::plus(c, h ? Ar<typename CA::U>::neg(u) : u);
           const bool flip = h == 1 && e == 0;
           tst(o + h * np + (t + 1) * cs, flip ? A::neg(v) : v);
@@ -591,7 +594,7 @@ __host__ __device__ void tree_unit(const TreeInst& T, int q, const S* par, long 
     }
     return;
   }
-  constexpr int TT = TL ? TL : 1;
+  constexpr int TT = TL > 0 ? TL : 1;
   const int nt = (Lp + TT - 1) / TT;
   const unsigned total = (unsigned)nt * ne * np;
   for (unsigned x = tid; x < total; x += nthr) {
@@ -1408,6 +1411,7 @@ __device__ __forceinline__ void tree_body(const TreeParams& P, const int cta, co
           break;
         case TP_UNIT:
           if (G.tile == 0) tree_unit<S, 0>(T, G.q, par, G.pstride, G.np, chi, tid, nthr);
+          else if (G.tile == TREE_PAIRS) tree_unit<S, -1>(T, G.q, par, G.pstride, G.np, chi, tid, nthr);
           else if (G.tile == 1) tree_unit<S, 1>(T, G.q, par, G.pstride, G.np, chi, tid, nthr);
           else tree_unit<S, TL>(T, G.q, par, G.pstride, G.np, chi, tid, nthr);
           break;
