@@ -65,14 +65,21 @@ static inline int sieve_occupancy(int stype, int wpc, int smem) {
   }
 }
 
-static inline cudaError_t tree_launch(int stype, const TreeParams& p, int ctas, int smem, cudaStream_t st) {
+// The node type of a tree: the matrix's scalar class; complex ones with re + im beside the parts
+// (three products a term) unless TREE_PARTS is added (four).
+constexpr int TREE_PARTS = 16;
+static inline int tree_stype(int ttype) { return ttype & ~TREE_PARTS; }
+
+static inline cudaError_t tree_launch(int ttype, const TreeParams& p, int ctas, int smem, cudaStream_t st) {
+  const int stype = tree_stype(ttype);
+  const bool parts = ttype != stype;
   switch (stype) {
-    case ST_CPLX64: return tree_launch_c64(p, ctas, smem, st);
-    case ST_CPLXDF: return tree_launch_cdf(p, ctas, smem, st);
-    case ST_REAL64: return tree_launch_f64(p, ctas, smem, st);
-    case ST_REALDF: return tree_launch_fdf(p, ctas, smem, st);
-    case ST_REALDD: return tree_launch_fdd(p, ctas, smem, st);
-    case ST_CPLXDD: return tree_launch_cdd(p, ctas, smem, st);
+    case ST_CPLX64: return tree_launch_c64(p, parts, ctas, smem, st);
+    case ST_CPLXDF: return tree_launch_cdf(p, parts, ctas, smem, st);
+    case ST_REAL64: return tree_launch_f64(p, parts, ctas, smem, st);
+    case ST_REALDF: return tree_launch_fdf(p, parts, ctas, smem, st);
+    case ST_REALDD: return tree_launch_fdd(p, parts, ctas, smem, st);
+    case ST_CPLXDD: return tree_launch_cdd(p, parts, ctas, smem, st);
     default: {
       TreeMods m;
       m.n = 1;

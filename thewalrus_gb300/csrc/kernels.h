@@ -29,7 +29,8 @@ WG_KERNEL_UNIT_DECL(mod2)
 WG_KERNEL_UNIT_DECL(mod3)
 WG_KERNEL_UNIT_DECL(mod4)
 #undef WG_KERNEL_UNIT_DECL
-#define WG_TREE_UNIT_DECL(T) cudaError_t tree_launch_##T(const TreeParams& p, int ctas, int smem, cudaStream_t st);
+#define WG_TREE_UNIT_DECL(T) \
+  cudaError_t tree_launch_##T(const TreeParams& p, bool parts, int ctas, int smem, cudaStream_t st);
 WG_TREE_UNIT_DECL(c64)
 WG_TREE_UNIT_DECL(cdf)
 WG_TREE_UNIT_DECL(f64)

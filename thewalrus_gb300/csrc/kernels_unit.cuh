@@ -25,7 +25,8 @@ int WG_CAT(sieve_occupancy_, WG_UNIT_NAME)(int wpc, int smem) {
 }
 
 #ifndef WG_UNIT_PRIME  // (residues: kernels_mods.cu)
-cudaError_t WG_CAT(tree_launch_, WG_UNIT_NAME)(const TreeParams& p, int ctas, int smem, cudaStream_t st) {
+cudaError_t WG_CAT(tree_launch_, WG_UNIT_NAME)(const TreeParams& p, bool parts, int ctas, int smem, cudaStream_t st) {
+  if (parts) return tree_launch_kernel(tree_kernel<WG_UNIT_SCALAR>, p, ctas, ctas, smem, st);
   return tree_launch_kernel(tree_kernel<typename TreeScalar<WG_UNIT_SCALAR>::T>, p, ctas, ctas, smem, st);
 }
 #endif

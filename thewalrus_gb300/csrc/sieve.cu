@@ -173,6 +173,19 @@ static int ensure_init(int device) {
 // entries of both signs, indices that fall into uncoupled blocks (zero entries between them).
 struct MatrixForm {
   bool symmetric = false, signs = false, blocks = false;
+  bool mixed = false;  // complex entries have parts of like size (mixed_rows)
+};
+
+// sums over entries of the smaller and of the larger part (mixed_rows)
+struct PartSums {
+  double low = 0, high = 0;
+  void add(double re, double im) {
+    const double x = std::fabs(re), y = std::fabs(im);
+    low += std::min(x, y);
+    high += std::max(x, y);
+  }
+  void add(c64 a, c64 b) { add(a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re); }
+  bool mixed() const { return low >= 0.125 * high; }
 };
 
 struct Prepared {
@@ -189,7 +202,12 @@ struct Prepared {
   TreeInst T;
   std::vector<double> ascale;    // the input prescale's share of each output
   int precision;
+  bool mixed = false;            // (MatrixForm)
   std::vector<double> tscales() const;  // output scales of the tree's sum
+  int ttype() const {            // the tree's node type
+    const bool cplx = stype == ST_CPLX64 || stype == ST_CPLXDF || stype == ST_CPLXDD;
+    return cplx && !mixed ? stype | TREE_PARTS : stype;
+  }
 };
 
 struct Group {
@@ -201,7 +219,7 @@ struct Group {
 
 // One launch of the tree kernel: trees of one scalar type and the program that walks them.
 struct TreeLaunch {
-  int stype, ctas, smem, sm_warp, sm_cache, sm_ws, cached, counter;
+  int ttype, ctas, smem, sm_warp, sm_cache, sm_ws, cached, counter;
   int ninst, nrounds, nsegs;
   size_t prog_off;  // of the instances, rounds and segments in the plan's program bytes
   long long ws_off;
@@ -260,7 +278,9 @@ struct wg_state {
   int M = 0;
   wg::c64* d_B = nullptr;
   wg::c64* d_gamma = nullptr;
-  std::vector<wg::c64> gamma;  // host copy: self-loop weights of unpaired modes
+  std::vector<wg::c64> gamma;  // host copies: self-loop weights of unpaired modes, requests' forms
+  std::vector<wg::c64> B;
+  std::vector<wg::PartSums> parts;
   double alpha = 1.0;          // double-float prescale (power of two, from ||B||_inf)
   wg::MatrixForm form;         // of B, whose blocks and symmetry every request's matrix inherits
 };
@@ -331,6 +351,40 @@ static inline double tree_asymmetry(int precision) {
   return prec_mod(precision) ? 0.0 : std::ldexp(1.0, precision == WG_PREC_DD ? -52 : -48);
 }
 
+// Whether the parts of a complex matrix's entries are of like size.  A product of three real ones
+// rounds a part relative to the whole, so that an imaginary part 1e-8 of the real one keeps 8 digits
+// fewer than by four.  Every matching takes an entry of every row, A_ij or with loops D_i and another
+// row's: where sum min(|re|, |im|) >= sum max(|re|, |im|) / 8 over a row's A_ij and D_i D_j, the rounding of
+// those entries alone moves either part of the sum relative to the whole, and three products lose nothing.
+// At least half of the rows have to say so (random phases: ratios of 0.41, and all but a few rows of two or
+// three entries do; rows of purely real and purely imaginary entries have 0).
+// of an instance's rows: `diag` with the diagonal, which edges of one pair each do not read
+static bool mixed_rows(const wg_instance& in, bool loops, bool odd, bool diag) {
+  if (in.dtype != WG_COMPLEX128) return false;
+  const c64 *A = (const c64*)in.A, *D = (const c64*)in.D, *V = (const c64*)in.oddV;
+  const c64 o = {in.oddloop[0], in.oddloop[1]};
+  const int n = in.n;
+  int rows = 0;
+  PartSums last;  // the unpaired vertex's row
+  for (int i = 0; i < n; ++i) {
+    PartSums s;
+    for (int j = 0; j < n; ++j)
+      if (j != i || diag) {
+        s.add(A[(size_t)i * n + j].re, A[(size_t)i * n + j].im);
+        if (loops) s.add(D[i], D[j]);
+      }
+    if (odd) {
+      s.add(V[i].re, V[i].im);
+      s.add(D[i], o);
+      last.add(V[i].re, V[i].im);
+      last.add(D[i], o);
+    }
+    rows += s.mixed();
+  }
+  if (odd) rows += last.mixed();
+  return 2 * rows >= n + odd;
+}
+
 static MatrixForm matrix_form(const void* A, int dtype, size_t n, double tol) {
   MatrixForm f;
   const int nc = dtype == WG_COMPLEX128 ? 2 : 1;
@@ -399,7 +453,8 @@ std::vector<double> Prepared::tscales() const {
 
 // takes the tree when the instance has one
 static void take_tree(Prepared& P, int precision, const std::vector<double>& ascale, const MatrixForm& f) {
-  P.tree = f.symmetric && tree_build(P.d, P.T) && tree_fits(P.T, tree_bytes(P.stype)) &&
+  P.mixed = f.mixed;
+  P.tree = f.symmetric && tree_build(P.d, P.T) && tree_fits(P.T, tree_bytes(P.ttype())) &&
            !keeps_terms(P.stype, P.d.kind, P.T.K, f);
   if (!P.tree) return;
   P.T.comp_off = stype_dd(P.stype) ? P.d.nout : 0;
@@ -619,8 +674,11 @@ static int prepare(const wg_instance& in, int precision, Prepared& P) {
         put_scalar(at(n + 2, i), P.stype, re * alpha, im * alpha);
       }
   }
-  if (!terms_only && in.term_begin == 0 && in.term_end == 0)
-    take_tree(P, precision, ascale, matrix_form(in.A, in.dtype, (size_t)n, tree_asymmetry(precision)));
+  if (!terms_only && in.term_begin == 0 && in.term_end == 0) {
+    MatrixForm f = matrix_form(in.A, in.dtype, (size_t)n, tree_asymmetry(precision));
+    f.mixed = mixed_rows(in, nb > 0, kind == KIND_LOOP_ODD, maxr > 1 || kind >= KIND_BATCH_EVEN);
+    take_tree(P, precision, ascale, f);
+  }
   return WG_OK;
 }
 
@@ -671,6 +729,48 @@ static __global__ void gather_kernel(const GatherDev* __restrict__ gd, const int
       reinterpret_cast<cdf*>(dst)[e] = {{hr, __double2float_rn(re - (double)hr)}, {hi, __double2float_rn(im - (double)hi)}};
     }
   }
+}
+
+// What mixed_rows adds up, of every entry of the state's matrix
+static void state_parts(wg_state& st) {
+  const int M = st.M;
+  st.parts.assign((size_t)M * M, PartSums());
+  for (int i = 0; i < M; ++i)
+    for (int j = 0; j < M; ++j) {
+      PartSums& s = st.parts[(size_t)i * M + j];
+      s.add(st.B[(size_t)i * M + j].re, st.B[(size_t)i * M + j].im);
+      s.add(st.gamma[i], st.gamma[j]);
+    }
+}
+// mixed_rows of a request's matrix, over its modes (the unpaired one among them) with the times it has
+// them: a few ns an entry, and half of the rows are enough
+static bool request_mixed(const wg_request& r, const wg_state& st, bool diag) {
+  int modes[2 * MAX_EDGES + 1], times[2 * MAX_EDGES + 1], n = 0;
+  int all = 2 * r.E;
+  std::copy(r.x, r.x + all, modes);
+  if (r.oddmode >= 0) modes[all++] = r.oddmode;
+  std::sort(modes, modes + all);
+  for (int k = 0; k < all; ++k) {
+    if (n && modes[n - 1] == modes[k]) {
+      ++times[n - 1];
+    } else {
+      modes[n] = modes[k];
+      times[n++] = 1;
+    }
+  }
+  int rows = 0;
+  for (int i = 0; i < n && 2 * rows < all; ++i) {
+    const PartSums* row = &st.parts[(size_t)modes[i] * st.M];
+    PartSums s;
+    for (int j = 0; j < n; ++j) {
+      const PartSums& e = row[modes[j]];
+      const double t = times[j] - (j == i && !diag);
+      s.low += t * e.low;
+      s.high += t * e.high;
+    }
+    rows += s.mixed() ? times[i] : 0;
+  }
+  return 2 * rows >= all;
 }
 
 // Loop-hafnian instance of one serving request (the host part of prepare() for WG_KIND_LOOP,
@@ -747,7 +847,11 @@ static int prepare_request(const wg_request& r, const wg_state& st, int precisio
   g.alpha = alpha;
   g.salpha = salpha;
   for (int i = 0; i < 2 * r.E; ++i) idx.push_back(r.x[i]);
-  if (!terms_only) take_tree(P, precision, {ascale}, st.form);
+  if (!terms_only) {
+    MatrixForm f = st.form;
+    f.mixed = request_mixed(r, st, maxr > 1);
+    take_tree(P, precision, {ascale}, f);
+  }
   return WG_OK;
 }
 
@@ -776,8 +880,11 @@ static int build_plan(const wg_instance* v, int count, int precision, const wg_p
   return finalize_plan(P, precision, opt, pl, nullptr, nullptr);
 }
 
-// Per scalar type: SM clocks per multiply-add of a tree, measured over launches that fill the chip
-static double tree_mac_clocks(int stype) {
+// Per node type: SM clocks per multiply-add of a tree, measured over launches that fill the chip (four
+// products instead of three: in proportion)
+static double tree_mac_clocks(int ttype) {
+  const int stype = tree_stype(ttype);
+  if (ttype != stype) return 4.0 / 3.0 * tree_mac_clocks(stype);
   switch (stype) {
     case ST_REAL64: return 0.5;
     case ST_CPLX64: return 2.0;
@@ -808,29 +915,29 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
   std::vector<int> order;
   for (int i = 0; i < count; ++i)
     if (P[i].tree) {
-      tree_levels(P[i].T, tree_bytes(P[i].stype), kLevelBytes, lev[i]);
+      tree_levels(P[i].T, tree_bytes(P[i].ttype()), kLevelBytes, lev[i]);
       order.push_back(i);
     }
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-    return P[a].stype != P[b].stype ? P[a].stype < P[b].stype : lev[a].bytes > lev[b].bytes;
+    return P[a].ttype() != P[b].ttype() ? P[a].ttype() < P[b].ttype() : lev[a].bytes > lev[b].bytes;
   });
   // Several primes side by side when their levels, of which two at a time are in use, keep to the L2:
   // graph counts modulo three, n = 36 (75 MB each) 886 us one after another and 723 side by side,
   // n = 38 (160 MB each) 1,508 and 1,642.
   constexpr double kSideBytes = 250e6;
   long long first = 0;
-  for (size_t k = 0; k < order.size() && P[order[k]].stype == P[order[0]].stype; ++k) first += lev[order[k]].bytes;
+  for (size_t k = 0; k < order.size() && P[order[k]].ttype() == P[order[0]].ttype(); ++k) first += lev[order[k]].bytes;
   pl->side_trees = pl->primes > 1 && !order.empty() && (double)first * pl->primes <= kSideBytes;
   // The launches of several scalar types side by side, each with SMs by its work and at least 30 % of an
   // even share: one's narrow rounds and barriers no longer wait for the other's.  us in turn and so, plans of
   // complex and real matrices: 8 of n = 8 to 12 72 and 55, 64 to n = 18 112 and 77, 160 to n = 28 833 and
   // 769 (even shares: 985), 40 to n = 32 853 and 746.  Not beyond a launch's workspace, where they evict one
   // another's levels from the L2 (250 to n = 30: 1,778 and 1,954).
-  std::map<int, double> works;  // SM clocks of a scalar type
+  std::map<int, double> works;  // SM clocks of a node type
   double total = 0, work = 0;
   for (int i : order) {
-    const double w = tree_work(P[i].T, lev[i]) * tree_mac_clocks(P[i].stype);
-    works[P[i].stype] += w;
+    const double w = tree_work(P[i].T, lev[i]) * tree_mac_clocks(P[i].ttype());
+    works[P[i].ttype()] += w;
     work += w;
     total += lev[i].bytes;
   }
@@ -840,15 +947,15 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
   for (size_t k = 0; k < order.size();) {
     TreeLaunch G;
     memset(&G, 0, sizeof(G));
-    G.stype = P[order[k]].stype;
-    const int sb = tree_bytes(G.stype);
-    const int tile = stype_mod(G.stype) ? tree_tile<modp<MOD_PRIMES[0]>>()
-                                        : (G.stype == ST_CPLXDD ? tree_tile<cdd>() : tree_tile<c64>());
+    G.ttype = P[order[k]].ttype();
+    const int sb = tree_bytes(G.ttype);
+    const int tile = stype_mod(G.ttype) ? tree_tile<modp<MOD_PRIMES[0]>>()
+                                        : (tree_stype(G.ttype) == ST_CPLXDD ? tree_tile<cdd>() : tree_tile<c64>());
     std::vector<TreeInst> insts;
     std::vector<TreeLevels> levels;
     const size_t k0 = k;
     long long bytes = 0;
-    for (; k < order.size() && P[order[k]].stype == G.stype; ++k) {
+    for (; k < order.size() && P[order[k]].ttype() == G.ttype; ++k) {
       if (k > k0 && (double)(bytes + lev[order[k]].bytes) > kLaunchBytes) break;
       bytes += lev[order[k]].bytes;
       insts.push_back(P[order[k]].T);
@@ -857,9 +964,9 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
     }
     TreeProgram prog;
     std::vector<int> base, cnt;
-    const double clk = tree_mac_clocks(G.stype);
+    const double clk = tree_mac_clocks(G.ttype);
     const double share = pl->side_trees ? 1.0 / pl->primes
-                         : pl->fork_trees ? least + (1 - least * works.size()) * works[G.stype] / work : 1.0;
+                         : pl->fork_trees ? least + (1 - least * works.size()) * works[G.ttype] / work : 1.0;
     const int sms = std::max((int)(g_num_sms * share), 1);
     G.ctas = tree_one_cta(insts, levels, clk, sms) ? 1 : sms;
     tree_program(insts, levels, sb, tile, G.ctas * TREE_THREADS, nparts, base, cnt, prog);
@@ -936,10 +1043,10 @@ static void split_edges(std::vector<Prepared>& P) {
     const TreeInst& T = P[i].T;
     auto work_of = [&](const TreeInst& t) {
       TreeLevels g;
-      tree_levels(t, tree_bytes(P[i].stype), 1e18, g);
+      tree_levels(t, tree_bytes(P[i].ttype()), 1e18, g);
       return tree_work(t, g);
     };
-    const double clk = tree_mac_clocks(P[i].stype) / g_num_sms;
+    const double clk = tree_mac_clocks(P[i].ttype()) / g_num_sms;
     const bool split = splits(P[i]) && tree_build(P[i].d, alt[i], true);
     const double unit = tree_edge_clocks(P[i].stype), w = work_of(T) * clk;
     lat = std::max(lat, unit * tree_latency(T));
@@ -1310,12 +1417,12 @@ static int launch_trees(wg_plan* pl, cudaStream_t st) {
       p.fin.wpo = plan_wpo(pl, TREE_THREADS / 32);
     }
     if (pl->side_trees) {
-      side.prime[side.n] = G.stype - ST_MOD0;
+      side.prime[side.n] = G.ttype - ST_MOD0;
       side.p[side.n++] = p;  // the primes' programs are alike: G.ctas and G.smem too
       if (side.n < (int)pl->trees.size()) continue;
     }
     const cudaError_t e = pl->side_trees ? tree_launch_mods(side, G.ctas * side.n, G.smem, st)
-                                         : tree_launch(G.stype, p, G.ctas, G.smem, forked ? pl->side[i - 1] : st);
+                                         : tree_launch(G.ttype, p, G.ctas, G.smem, forked ? pl->side[i - 1] : st);
     if (e != cudaSuccess) return fail(WG_ECUDA, "tree launch: %s", cudaGetErrorString(e));
     if (forked) {
       const int rc = join_side(pl, st, i - 1);
@@ -1598,6 +1705,9 @@ int wg_state_create(const double* B, const double* gamma, int M, wg_state** stat
   CK(cudaMemcpy(st->d_B, B, sizeof(c64) * (size_t)M * M, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(st->d_gamma, gamma, sizeof(c64) * M, cudaMemcpyHostToDevice));
   st->form = matrix_form(B, WG_COMPLEX128, (size_t)M, tree_asymmetry(WG_PREC_FP64));
+  st->B.resize((size_t)M * M);
+  memcpy(st->B.data(), B, sizeof(c64) * st->B.size());
+  state_parts(*st);
   *state = st;
   return WG_OK;
 }
@@ -1650,12 +1760,11 @@ int wg_state_create_from_cov(const double* cov, const double* mu, int M, double 
   if (B_out && cudaMemcpy(B_out, st->d_B, sizeof(c64) * (size_t)M * M, cudaMemcpyDeviceToHost) != cudaSuccess)
     return abandon(WG_ECUDA, "state readback failed");
   if (gamma_out) memcpy(gamma_out, st->gamma.data(), sizeof(c64) * M);
-  {
-    std::vector<c64> B((size_t)M * M);
-    if (cudaMemcpy(B.data(), st->d_B, sizeof(c64) * B.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
-      return abandon(WG_ECUDA, "state readback failed");
-    st->form = matrix_form(B.data(), WG_COMPLEX128, (size_t)M, tree_asymmetry(WG_PREC_FP64));
-  }
+  st->B.resize((size_t)M * M);
+  if (cudaMemcpy(st->B.data(), st->d_B, sizeof(c64) * st->B.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
+    return abandon(WG_ECUDA, "state readback failed");
+  st->form = matrix_form(st->B.data(), WG_COMPLEX128, (size_t)M, tree_asymmetry(WG_PREC_FP64));
+  state_parts(*st);
   release();
   const double rs = out[3];
   if (rs > 0 && std::isfinite(rs)) st->alpha = std::exp2(-std::round(std::log2(rs)));

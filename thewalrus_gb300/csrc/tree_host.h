@@ -80,12 +80,12 @@ static inline bool tree_build(const InstDev& d, TreeInst& T, bool simple_only = 
 static inline int tree_scale_exp(const TreeInst& T) { return T.deg[T.steps] - (T.steps > 0 ? 1 : 0); }
 
 // bytes of a node element
-static inline int tree_bytes(int stype) {
-  switch (stype) {
+static inline int tree_bytes(int ttype) {
+  switch (ttype) {
     case ST_CPLX64: return (int)sizeof(TreeScalar<c64>::T);
     case ST_CPLXDF: return (int)sizeof(TreeScalar<cdf>::T);
     case ST_CPLXDD: return (int)sizeof(TreeScalar<cdd>::T);
-    default: return (int)stype_bytes(stype);
+    default: return (int)stype_bytes(tree_stype(ttype));
   }
 }
 

@@ -212,10 +212,33 @@ struct RealAcc<ddr> {
   }
   __device__ __forceinline__ ddr sum() const { return dd_two_sum(hi, lo); }
 };
-// Complex nodes carry re + im beside the parts, so that a product of series takes three real products
-// a term instead of four (re = P1 - P2, im = P3 - P1 - P2 with P1 = sum re re, P2 = sum im im, P3 = sum
-// (re + im)(re + im)); its rounding is relative to |a| |b|, as the four products' is.  C: the matrix
-// scalar, R: its real one.  FP64 n = 40: 5,836 -> 5,405 us, n = 36: 1,212 -> 1,147 us.
+// Complex nodes as the matrix's own scalar: four real products a term, each part rounded relative to
+// its own terms.
+template <class R, class C>
+struct RealAccParts {
+  RealAcc<R> re, im;
+  __device__ __forceinline__ void fma(C a, C b) {
+    re.fma(a.re, b.re);
+    re.fma(Ar<R>::neg(a.im), b.im);
+    im.fma(a.re, b.im);
+    im.fma(a.im, b.re);
+  }
+  __device__ __forceinline__ C sum() const { return {re.sum(), im.sum()}; }
+};
+template <>
+struct RealAcc<cdf> : RealAccParts<dfr, cdf> {
+  __device__ static __forceinline__ RealAcc of(cdf x) { return {{RealAcc<dfr>::of(x.re), RealAcc<dfr>::of(x.im)}}; }
+};
+template <>
+struct RealAcc<cdd> : RealAccParts<ddr, cdd> {
+  __device__ static __forceinline__ RealAcc of(cdd x) { return {{RealAcc<ddr>::of(x.re), RealAcc<ddr>::of(x.im)}}; }
+};
+// Or with re + im beside the parts, so that a product of series takes three real products a term
+// instead of four (re = P1 - P2, im = P3 - P1 - P2 with P1 = sum re re, P2 = sum im im, P3 = sum
+// (re + im)(re + im)).  Its rounding is relative to |a| |b|: each part keeps its accuracy only where the
+// parts are of like size, so that the host takes it for matrices whose rows say so (mixed_rows,
+// sieve.cu) and the four products for the others.  C: the matrix scalar, R: its real one.  FP64 n = 40:
+// 5,836 -> 5,405 us, n = 36: 1,212 -> 1,147 us.
 template <class R, class C>
 struct c3 {
   R re, im, s;
