@@ -936,7 +936,7 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
   std::map<int, double> works;  // SM clocks of a node type
   double total = 0, work = 0;
   for (int i : order) {
-    const double w = tree_work(P[i].T, lev[i]) * tree_mac_clocks(P[i].ttype());
+    const double w = tree_work(P[i].T) * tree_mac_clocks(P[i].ttype());
     works[P[i].ttype()] += w;
     work += w;
     total += lev[i].bytes;
@@ -1041,18 +1041,13 @@ static void split_edges(std::vector<Prepared>& P) {
   for (size_t i = 0; i < P.size(); ++i) {
     if (!P[i].tree) continue;
     const TreeInst& T = P[i].T;
-    auto work_of = [&](const TreeInst& t) {
-      TreeLevels g;
-      tree_levels(t, tree_bytes(P[i].ttype()), 1e18, g);
-      return tree_work(t, g);
-    };
     const double clk = tree_mac_clocks(P[i].ttype()) / g_num_sms;
     const bool split = splits(P[i]) && tree_build(P[i].d, alt[i], true);
-    const double unit = tree_edge_clocks(P[i].stype), w = work_of(T) * clk;
+    const double unit = tree_edge_clocks(P[i].stype), w = tree_work(T) * clk;
     lat = std::max(lat, unit * tree_latency(T));
     lat1 = std::max(lat1, unit * tree_latency(split ? alt[i] : T));
     work += w;
-    work1 += split ? work_of(alt[i]) * clk : w;
+    work1 += split ? tree_work(alt[i]) * clk : w;
     if (!split) alt[i].E = 0;
   }
   if (lat1 + work1 >= lat + work) return;

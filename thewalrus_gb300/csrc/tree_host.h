@@ -153,6 +153,31 @@ static inline bool tree_same_round(int before, int phase) {
   return (before == TP_W2 && phase == TP_G2) || (before == TP_G && phase == TP_M) || (before == TP_M && phase == TP_UNIT);
 }
 
+// The phases of step q (the last: of the leaves) in order: f(phase).  A loop kind's TP_G is not among
+// them, see tree_walk.
+template <class F>
+static void tree_step(const TreeInst& T, int q, F f) {
+  if (q == T.steps) {
+    if (T.pO >= 0 && T.steps < T.E) f(TP_M);
+    f(TP_LEAF);
+  } else if (T.reps[q] == 1) {
+    if (T.pL >= 0) f(TP_M);
+    f(TP_UNIT);
+  } else if (T.reps[q] == 2) {
+    const bool rows = tree_width(T.X, T.E, q + 1) > 0;
+    if (rows) f(TP_W2);
+    f(TP_G2);  // beside TP_W2, in the same round
+    if (rows) f(TP_MULTI2);
+  } else {
+    f(TP_PREP);
+    if (tree_width(T.X, T.E, q + 1) > 0) {
+      f(TP_Y);
+      f(TP_MULTI);
+      if (T.pL >= 0) f(TP_GLOOP);
+    }
+  }
+}
+
 // The phases of an instance in order, each once for every block: f(phase, q, p0, np, level's nodes).
 // `late`, a parents' block [late0, late0 + late) of a level of `lateps` nodes: step q - 1's TP_G, due in
 // this step's first round.
@@ -161,34 +186,16 @@ static void tree_walk(const TreeInst& T, const TreeLevels& g, int q, int np, F& 
                       int lateps = 0) {
   if (late) f(TP_G, q - 1, late0, late, lateps);
   if (q == T.steps) {
-    if (T.pO >= 0 && T.steps < T.E) f(TP_M, q, 0, np, np);
-    f(TP_LEAF, q, 0, np, np);
+    tree_step(T, q, [&](int phase) { f(phase, q, 0, np, np); });
     return;
   }
   const int R = T.radix[q], blocks = (int)((np + g.chunk[q] - 1) / g.chunk[q]), per = (np + blocks - 1) / blocks;
+  const bool loop = T.reps[q] == 1 && T.pL >= 0;
   for (int p0 = 0; p0 < np; p0 += per) {
     const int c = std::min(per, np - p0);
-    if (T.reps[q] == 1) {
-      if (T.pL >= 0) f(TP_M, q, p0, c, np);
-      f(TP_UNIT, q, p0, c, np);
-      if (T.pL >= 0) {
-        tree_walk(T, g, q + 1, c * R, f, p0, c, np);
-        continue;
-      }
-    } else if (T.reps[q] == 2) {
-      const bool rows = tree_width(T.X, T.E, q + 1) > 0;
-      if (rows) f(TP_W2, q, p0, c, np);
-      f(TP_G2, q, p0, c, np);  // beside TP_W2, in the same round
-      if (rows) f(TP_MULTI2, q, p0, c, np);
-    } else {
-      f(TP_PREP, q, p0, c, np);
-      if (tree_width(T.X, T.E, q + 1) > 0) {
-        f(TP_Y, q, p0, c, np);
-        f(TP_MULTI, q, p0, c, np);
-        if (T.pL >= 0) f(TP_GLOOP, q, p0, c, np);
-      }
-    }
-    tree_walk(T, g, q + 1, c * R, f);
+    tree_step(T, q, [&](int phase) { f(phase, q, p0, c, np); });
+    if (loop) tree_walk(T, g, q + 1, c * R, f, p0, c, np);
+    else tree_walk(T, g, q + 1, c * R, f);
   }
 }
 
@@ -387,11 +394,16 @@ static inline double tree_latency(const TreeInst& T) {
   for (int q = 0; q < T.E; ++q) lat += T.reps[q] == 1 ? 0.7 : (T.reps[q] == 2 ? 2.0 : 4.0);
   return lat;
 }
-// a tree's multiply-adds
-static inline double tree_work(const TreeInst& T, const TreeLevels& g) {
-  double macs = 0;
-  auto add = [&](int phase, int q, int, int np, int) { macs += tree_macs(T, phase, q, np); };
-  tree_walk(T, g, 0, 1, add);
+// a tree's multiply-adds, level by level (the blocks that large levels are walked in add up to the same;
+// a level may have more nodes than an int holds)
+static inline double tree_work(const TreeInst& T) {
+  double macs = 0, nodes = 1;
+  for (int q = 0; q <= T.steps; ++q) {
+    tree_step(T, q, [&](int phase) { macs += tree_macs(T, phase, q, nodes); });
+    if (q == T.steps) break;
+    if (T.reps[q] == 1 && T.pL >= 0) macs += tree_macs(T, TP_G, q, nodes);
+    nodes *= T.radix[q];
+  }
   return macs;
 }
 
