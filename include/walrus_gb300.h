@@ -148,6 +148,10 @@ typedef struct wg_plan_options {
   int32_t serial_groups; /* 1: launch the groups one after another on the caller's stream (default:
                             groups after the first on side streams, overlapping their tails) */
   void* stream;
+  int64_t max_workspace; /* device bytes that the elimination trees' levels and programs may take (0: what
+                            they use best, up to a few GB each).  Within it larger levels are walked in smaller blocks; a
+                            tree that does not fit is summed term by term.  A plan whose allocation fails is
+                            made again with less. */
 } wg_plan_options;
 int wg_plan_create_ex(const wg_instance* inst, int count, int precision, const wg_plan_options* options,
                       wg_plan** plan);

@@ -1,0 +1,77 @@
+"""The device memory of the elimination trees' levels.
+
+A tree within less memory walks smaller blocks, so that its sum is taken in another order: equal to
+1e-12, a hundred roundings of these sums; one that does not fit is the per-term sum, bit for bit."""
+import numpy as np
+import pytest
+
+import thewalrus_gb300 as tw
+from thewalrus_gb300 import _native as nat
+from thewalrus_gb300 import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+
+def run(insts, precision="fp64", **options):
+    plan = nat.Plan(insts, precision=precision, **options)
+    plan.execute()
+    got, size = plan.read(), plan.device_bytes()
+    plan.close()
+    return got, size
+
+
+@pytest.mark.parametrize("limit", [100e6, 20e6, 4e6])
+def test_blocks_within_a_limit(limit):
+    A, g, rpt = wl.gaussian_state_loop(modes=12, seed=2, photons=20, max_rep=3)
+    insts = [tw.prepare_hafnian(wl.complex_symmetric(32, seed=1)), tw.prepare_hafnian(wl.real_nonneg(30, seed=1)),
+             tw.prepare_hafnian(wl.complex_symmetric(20, seed=2)), tw.prepare_loop_hafnian(A, g, list(rpt)),
+             tw.prepare_loop_hafnian(wl.complex_symmetric(25, seed=3), wl.complex_symmetric(25, seed=4)[0])]
+    want, most = run(insts)
+    got, size = run(insts, max_workspace=limit)
+    assert most > limit and size < limit + 8e6  # programs, matrices and partials beside the levels
+    assert np.all(np.abs(got - want) <= 1e-12 * np.abs(want))
+
+
+def test_no_room_is_the_per_term_sum():
+    insts = [tw.prepare_hafnian(wl.complex_symmetric(22, seed=1)), tw.prepare_hafnian(wl.real_nonneg(24, seed=1))]
+    got, size = run(insts, max_workspace=1)
+    assert size < 8e6 and np.array_equal(got, run(insts, "fp64-terms")[0])
+
+
+@pytest.fixture
+def small_pool():
+    """A function that makes the device's stream-ordered allocations come from a pool of so many bytes."""
+    import ctypes
+
+    class Props(ctypes.Structure):  # CUmemPoolProps
+        _fields_ = [("alloc_type", ctypes.c_int), ("handle_types", ctypes.c_int), ("location_type", ctypes.c_int),
+                    ("location_id", ctypes.c_int), ("security", ctypes.c_void_p), ("max_size", ctypes.c_size_t),
+                    ("usage", ctypes.c_ushort), ("reserved", ctypes.c_ubyte * 54)]
+
+    nat.run([tw.prepare_hafnian(wl.real_nonneg(4, seed=1))])  # the library's context
+    cuda = ctypes.CDLL("libcuda.so.1")
+    dev, default, made = ctypes.c_int(), ctypes.c_void_p(), []
+    assert cuda.cuCtxGetDevice(ctypes.byref(dev)) == 0
+    assert cuda.cuDeviceGetDefaultMemPool(ctypes.byref(default), dev) == 0
+
+    def use(size):
+        pool, props = ctypes.c_void_p(), Props(1, 0, 1, dev.value, None, int(size))  # pinned, on the device
+        if cuda.cuMemPoolCreate(ctypes.byref(pool), ctypes.byref(props)) != 0:
+            pytest.skip("no memory pool of a bounded size")
+        made.append(pool)
+        assert cuda.cuDeviceSetMemPool(dev, pool) == 0
+
+    yield use
+    assert cuda.cuDeviceSetMemPool(dev, default) == 0
+    for pool in made:
+        cuda.cuMemPoolDestroy(pool)
+
+
+def test_allocation_that_fails_is_tried_with_less(small_pool):
+    insts = [tw.prepare_hafnian(wl.complex_symmetric(34, seed=1)), tw.prepare_hafnian(wl.complex_symmetric(20, seed=2))]
+    want = nat.run(insts)
+    small_pool(256e6)  # smaller blocks
+    assert np.all(np.abs(nat.run(insts) - want) <= 1e-12 * np.abs(want))
+    last = [tw.prepare_hafnian(wl.complex_symmetric(30, seed=3))]
+    small_pool(32e6)  # no tree
+    assert np.array_equal(nat.run(last), nat.run(last, "fp64-terms"))

@@ -1,9 +1,10 @@
-// Host check of the elimination tree's estimates (tree_host.h): for instances read from standard input,
-// their multiply-adds as estimated and as a walk in blocks adds them up.  Built and run by
-// tests/test_tree_limits.py.
+// Host check of the elimination tree's estimates and sizes (tree_host.h), for instances read from standard
+// input.  Built and run by tests/test_tree_limits.py.
 //
+// Arguments: walk-bytes limit node-bytes.
 // Input: instances; per instance kind (InstDev's) E edge_reps.
-// Output per instance: estimate, sum of the walk with `walk-bytes` a level (0: not walked).
+// Output per instance: multiply-adds as estimated and as a walk in levels of walk-bytes adds them up
+// (0: not walked); whether its levels fit the limit, and their bytes.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -19,7 +20,8 @@ static int rd() {
 }
 
 int main(int, char** argv) {
-  const double walk = std::atof(argv[1]);
+  const double walk = std::atof(argv[1]), limit = std::atof(argv[2]);
+  const int sb = std::atoi(argv[3]);
   for (int k = rd(); k > 0; --k) {
     InstDev d;
     memset(&d, 0, sizeof(d));
@@ -37,7 +39,9 @@ int main(int, char** argv) {
       auto add = [&](int phase, int q, int, int np, int) { sum += tree_macs(T, phase, q, np); };
       tree_walk(T, g, 0, 1, add);
     }
-    std::printf("%.17g %.17g\n", tree_work(T), sum);
+    TreeLevels g;
+    const bool fits = tree_levels_within(T, sb, limit, g);
+    std::printf("%.17g %.17g %d %.17g\n", tree_work(T), sum, fits, (double)g.bytes);
   }
   return 0;
 }

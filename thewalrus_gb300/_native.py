@@ -286,6 +286,7 @@ class WgPlanOptions(ctypes.Structure):
         ("use_graph", ctypes.c_int32),
         ("serial_groups", ctypes.c_int32),
         ("stream", ctypes.c_void_p),
+        ("max_workspace", ctypes.c_int64),
     ]
 
 
@@ -293,12 +294,13 @@ class Plan:
     """Device-resident batch of instances: create once, execute many times, read results.
 
     ``chunk_scale`` (term-chunk size), ``max_warps_per_cta``, ``merge_classes`` (one persistent
-    launch per scalar type), ``use_graph`` (CUDA-graph replay) and ``serial_groups`` (launch the
-    groups one after another on the caller's stream) map to ``wg_plan_options``.
+    launch per scalar type), ``use_graph`` (CUDA-graph replay), ``serial_groups`` (launch the
+    groups one after another on the caller's stream) and ``max_workspace`` (device bytes for the
+    trees' levels, 0: what they use best) map to ``wg_plan_options``.
     """
 
     def __init__(self, instances, precision="fp64", chunk_scale=1.0, max_warps_per_cta=0,
-                 merge_classes=False, use_graph=False, serial_groups=False):
+                 merge_classes=False, use_graph=False, serial_groups=False, max_workspace=0):
         self.lib = load()
         self.instances = list(instances)
         arr = (WgInstance * max(len(self.instances), 1))()
@@ -306,7 +308,7 @@ class Plan:
             arr[i] = inst.struct
         self._arr = arr
         opt = WgPlanOptions(float(chunk_scale), int(max_warps_per_cta), int(bool(merge_classes)),
-                            int(bool(use_graph)), int(bool(serial_groups)), None)
+                            int(bool(use_graph)), int(bool(serial_groups)), None, int(max_workspace))
         h = ctypes.c_void_p()
         check(self.lib.wg_plan_create_ex(arr, len(self.instances), PRECISIONS[precision],
                                          ctypes.byref(opt), ctypes.byref(h)))
@@ -333,7 +335,8 @@ class Plan:
         self._keep, self._arr = (xa, ra), arr
         opt = WgPlanOptions(float(options.get("chunk_scale", 1.0)), int(options.get("max_warps_per_cta", 0)),
                             int(bool(options.get("merge_classes", False))), int(bool(options.get("use_graph", False))),
-                            int(bool(options.get("serial_groups", False))), options.get("stream"))
+                            int(bool(options.get("serial_groups", False))), options.get("stream"),
+                            int(options.get("max_workspace", 0)))
         h = ctypes.c_void_p()
         check(self.lib.wg_plan_create_requests(state.handle, arr, len(requests), PRECISIONS[precision],
                                                ctypes.byref(opt), ctypes.byref(h)))

@@ -901,23 +901,40 @@ static double tree_edge_clocks(int stype) {
   return stype == ST_CPLXDD ? 80000 : stype == ST_REALDD ? 32000 : 16000;
 }
 
-// Groups the tree members of a plan into launches (one scalar type each, as many instances as share
+// The levels of a plan's trees, each within what `limit` bytes leave beside the trees' programs (about
+// as many rounds and segments as phases); those that do not fit are summed by terms.  `limit` becomes
+// what is left for the levels of a launch.
+static std::vector<TreeLevels> place_trees(std::vector<Prepared>& P, double& limit) {
+  std::vector<TreeLevels> lev(P.size());
+  double programs = 0;
+  for (size_t i = 0; i < P.size(); ++i) {
+    if (!P[i].tree) continue;
+    P[i].tree = tree_levels_within(P[i].T, tree_bytes(P[i].ttype()), limit, lev[i]);
+    if (P[i].tree) programs += sizeof(TreeInst) + 512 + lev[i].phases * (sizeof(TreeRound) + sizeof(TreeSeg));
+  }
+  const double left = limit - programs;
+  for (size_t i = 0; i < P.size(); ++i)
+    if (P[i].tree && (double)lev[i].bytes > left)
+      P[i].tree = tree_levels_within(P[i].T, tree_bytes(P[i].ttype()), left, lev[i]);
+  limit = left;
+  return lev;
+}
+
+// Groups the tree members of a plan into launches (one node type each, as many instances as share
 // a workspace budget), makes their programs and lays out their partial slots.  Returns the
 // workspace bytes; the launches run one after another and share it, or (an exact sum's primes) side
 // by side.
-static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) {
-  // A level's byte budget: larger levels are walked in blocks.  A launch's: beyond it the
-  // instances go to the next launch.  Both keep the workspace within what the device's pool keeps.
-  constexpr double kLevelBytes = 200e6, kLaunchBytes = 600e6;
+static long long plan_trees(std::vector<Prepared>& P, const std::vector<TreeLevels>& lev, double limit, wg_plan* pl,
+                            int& nparts) {
+  // A launch's levels: beyond this the instances go to the next launch, which uses the same workspace.
+  // (One instance alone may take more, up to place_trees' limit: complex FP64 1.3 GB at n = 40, 1.9 at 44,
+  // 4.2 at 64.)
+  const double kLaunchBytes = std::min(600e6, limit);
   const int count = (int)P.size();
   auto al = [](long long x) { return (x + 255) & ~255ll; };
-  std::vector<TreeLevels> lev(count);
   std::vector<int> order;
   for (int i = 0; i < count; ++i)
-    if (P[i].tree) {
-      tree_levels(P[i].T, tree_bytes(P[i].ttype()), kLevelBytes, lev[i]);
-      order.push_back(i);
-    }
+    if (P[i].tree) order.push_back(i);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     return P[a].ttype() != P[b].ttype() ? P[a].ttype() < P[b].ttype() : lev[a].bytes > lev[b].bytes;
   });
@@ -927,7 +944,7 @@ static long long plan_trees(std::vector<Prepared>& P, wg_plan* pl, int& nparts) 
   constexpr double kSideBytes = 250e6;
   long long first = 0;
   for (size_t k = 0; k < order.size() && P[order[k]].ttype() == P[order[0]].ttype(); ++k) first += lev[order[k]].bytes;
-  pl->side_trees = pl->primes > 1 && !order.empty() && (double)first * pl->primes <= kSideBytes;
+  pl->side_trees = pl->primes > 1 && !order.empty() && (double)first * pl->primes <= std::min(kSideBytes, limit);
   // The launches of several scalar types side by side, each with SMs by its work and at least 30 % of an
   // even share: one's narrow rounds and barriers no longer wait for the other's.  us in turn and so, plans of
   // complex and real matrices: 8 of n = 8 to 12 72 and 55, 64 to n = 18 112 and 77, 160 to n = 28 833 and
@@ -1090,6 +1107,9 @@ static bool terms_sooner(const std::vector<Prepared>& P) {
   return tree > terms + work;
 }
 
+// What a plan whose allocation failed asks for next
+constexpr double kLeastWorkspace = 64e6;
+
 // ext_pool: the instances' matrices are on the device already, at their a_off
 static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_options& opt, wg_plan* pl,
                          GatherSpec* gs, unsigned char* ext_pool) {
@@ -1104,6 +1124,9 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   split_edges(P);
   if (terms_sooner(P))
     for (Prepared& p : P) p.tree = false;
+  const bool roomy = opt.max_workspace <= 0 || opt.max_workspace > kLeastWorkspace;
+  double limit = opt.max_workspace > 0 ? (double)opt.max_workspace : 1e18;
+  const std::vector<TreeLevels> lev = place_trees(P, limit);
   // outputs and scales in instance order
   int out = 0;
   std::vector<double> scales;
@@ -1155,7 +1178,7 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   if (gs)
     for (int i = 0; i < count; ++i) gs->desc[i].a_off = P[i].d.a_off;
   int nparts = 0;
-  const long long ws_bytes = plan_trees(P, pl, nparts);
+  const long long ws_bytes = plan_trees(P, lev, limit, pl, nparts);
   for (size_t g = 0; g < keys.size(); ++g) {
     Group G;
     G.stype = keys[g].st;
@@ -1264,6 +1287,15 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   const cudaError_t ae = pl->async_alloc ? cudaMallocAsync(&pl->dmem, total, cs) : cudaMalloc(&pl->dmem, total);
   if (ae != cudaSuccess) {
     cudaGetLastError();
+    if (!pl->trees.empty()) {  // with less workspace, then by terms
+      wg_plan fresh;
+      fresh.pinned = pl->pinned;
+      fresh.primes = pl->primes;
+      *pl = std::move(fresh);
+      wg_plan_options less = opt;
+      less.max_workspace = roomy ? (long long)kLeastWorkspace : 1;
+      return finalize_plan(P, precision, less, pl, gs, ext_pool);
+    }
     pl->dmem = nullptr;
     return fail(WG_ENOMEM, "device allocation of %zu bytes failed", total);
   }
