@@ -1,4 +1,4 @@
-"""The device memory of the elimination trees' levels.
+"""The device memory of the elimination trees' levels: a plan's option, the server's budget.
 
 A tree within less memory walks smaller blocks, so that its sum is taken in another order: equal to
 1e-12, a hundred roundings of these sums; one that does not fit is the per-term sum, bit for bit."""
@@ -36,6 +36,52 @@ def test_no_room_is_the_per_term_sum():
     insts = [tw.prepare_hafnian(wl.complex_symmetric(22, seed=1)), tw.prepare_hafnian(wl.real_nonneg(24, seed=1))]
     got, size = run(insts, max_workspace=1)
     assert size < 8e6 and np.array_equal(got, run(insts, "fp64-terms")[0])
+
+
+@pytest.mark.parametrize("budget", [2e6, 30e6, 300e6])
+def test_served_within_the_budget(budget, monkeypatch):
+    """All plans that a server holds at a time, their trees included, stay within its budget."""
+    pytest.importorskip("torch")
+    from thewalrus_gb300.serving import GaussianState, ProbabilityServer, poisson_requests
+
+    held = {"now": 0, "most": 0}
+
+    class Counted(nat.Plan):
+        @classmethod
+        def from_requests(cls, *args, **options):
+            plan = super().from_requests(*args, **options)
+            held["now"] += plan.device_bytes()
+            held["most"] = max(held["most"], held["now"])
+            return plan
+
+        def close(self):
+            if self.handle:
+                held["now"] -= self.device_bytes()
+            super().close()
+
+    states = [GaussianState.synthetic(modes=32, seed=3)]
+    reqs = poisson_requests(states, rate=1e6, count=24, photons=(8, 28), seed=1, max_rep=1)
+    want = [r["amplitude"] for r in ProbabilityServer(states).serve(reqs)]
+    monkeypatch.setattr(nat, "Plan", Counted)
+    got = [r["amplitude"] for r in ProbabilityServer(states, mem_budget=budget).serve(reqs)]
+    assert 0 < held["most"] <= budget and held["now"] == 0
+    assert np.all(np.abs(np.array(got) - want) <= 1e-10 * np.abs(want))
+
+
+def test_estimate_of_a_request():
+    """What the server counts for a request is at least what its per-term plan takes."""
+    pytest.importorskip("torch")
+    from thewalrus_gb300.serving import GaussianState, ProbabilityServer
+
+    state = GaussianState.synthetic(modes=48, seed=3).to_device()
+    for photons in (2, 5, 10, 16, 24, 27, 28, 33, 36, 40, 44, 47):
+        for rep in (1, 2, 4):
+            p = np.zeros(48, dtype=np.int64)
+            p[:-(-photons // rep)] = rep
+            p[0] -= p.sum() - photons
+            plan = nat.Plan.from_requests(state, [tw.matched_reps(p)], "fp64-terms")
+            assert plan.device_bytes() <= ProbabilityServer.estimate_bytes(photons), (photons, rep)
+            plan.close()
 
 
 @pytest.fixture

@@ -10,7 +10,8 @@ det(Q)^(-1/4) written as det(I - B B^*)^(1/4) for a pure state.
 Serving loop (``ProbabilityServer.serve``):
 * requests arrive at their timestamps (Poisson streams in the benchmark);
 * a batch is formed from the pending requests of one state as long as a stream slot is free and
-  the batch's device memory fits the budget (admission by device memory).  With
+  the batch's device memory fits the budget (admission by device memory; its trees' workspace keeps
+  to what is left).  With
   ``order="cost"`` (the default) pending requests are taken cheapest first -- the cost of a
   request is its sieve term count times (m + 1)^3 for its largest term matrix, known from the
   pattern before any work -- and a batch closes once its summed cost passes ``batch_cost``
@@ -181,9 +182,13 @@ class ProbabilityServer:
 
     @staticmethod
     def estimate_bytes(N):
-        """Upper estimate of one request's plan memory (pool + partials + bookkeeping)."""
+        """Upper estimate of one request's plan memory (pool, chunks, partials and bookkeeping; up to
+        12,000 chunks of 64 bytes for the resident warps, and one for every 6.4e7 of a sum's work),
+        without the workspace that a plan's trees share: a batch's takes what the budget has left."""
         n = N + (N % 2)
-        return (n + 3) * (n + 1) * 16 + 8192 * 16 + 2048
+        terms = 2.0 ** (N // 2 - 1 + N % 2)
+        chunks = min(terms, 12000 + terms * (n + 2.0) ** 3 / 6.4e7)
+        return (n + 3) * (n + 1) * 16 + max(8192 * 16, int(64 * chunks)) + 2048
 
     def serve(self, requests, time_scale=1.0, timeout=600.0):
         """Serve ``requests`` = [(arrival_s, state_index, pattern)] (sorted by arrival) in real time.
@@ -265,7 +270,8 @@ class ProbabilityServer:
                     stream = self.streams[slot]
                     triples = [info[j][1] for j in batch]
                     plan = nat.Plan.from_requests(self.states[sidx].device, triples, self.precision,
-                                                  chunk_scale=self.chunk_scale, stream=stream.cuda_stream)
+                                                  chunk_scale=self.chunk_scale, stream=stream.cuda_stream,
+                                                  max_workspace=max(self.mem_budget - mem_used - est, 1))
                     plan.execute(stream.cuda_stream)
                     ev = torch.cuda.Event()
                     ev.record(stream)
