@@ -19,6 +19,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -267,11 +268,15 @@ struct wg_plan {
   int tree_parts = 0;  // most partials of a tree's output
   unsigned char* d_prog = nullptr;
   unsigned char* d_ws = nullptr;
+  long long executions = 0;
   // a plan with trees answers the per-term queries (magnitudes, chunks, partials) by a plan over
-  // the same device matrices that evaluates term by term, made when first asked
+  // the same device matrices that evaluates term by term, made when first asked and run once for every
+  // execution that is asked about; one query at a time (terms_mu)
   std::vector<wg::Prepared> prep;
   wg_plan_options opt{};
-  wg_plan* terms = nullptr;
+  std::unique_ptr<std::mutex> terms_mu{new std::mutex};
+  mutable wg_plan* terms = nullptr;
+  mutable long long terms_of = -1;  // the execution that `terms` has run for
 };
 
 struct wg_state {
@@ -1360,23 +1365,37 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
 }
 
 // The per-term plan of a plan with trees, made on first use over the same device matrices: its
-// magnitudes, chunks and partials are those of the sieve's terms.
+// magnitudes, chunks and partials are those of the sieve's terms.  What the caller's streams have in
+// flight may still write those matrices, and the query may come on any stream: the device is waited
+// for, and the plan's own memory is allocated and filled synchronously.
 static void destroy_plan(wg_plan* pl);
-static int terms_plan(wg_plan* pl, wg_plan** out) {
+static int terms_plan(const wg_plan* pl, const wg_plan** out) {
   *out = pl;
   if (pl->prep.empty()) return WG_OK;
   if (!pl->terms) {
     int rc = ensure_init(pl->device);
     if (rc) return rc;
+    CK(cudaDeviceSynchronize());
     std::vector<Prepared> P = pl->prep;
     for (Prepared& p : P) p.tree = false;
+    wg_plan_options opt = pl->opt;
+    opt.stream = nullptr;
     wg_plan* t = new wg_plan();
-    rc = finalize_plan(P, pl->precision, pl->opt, t, nullptr, pl->d_pool);
+    rc = finalize_plan(P, pl->precision, opt, t, nullptr, pl->d_pool);
     if (rc) { destroy_plan(t); return rc; }
     pl->terms = t;
   }
   *out = pl->terms;
   return WG_OK;
+}
+static int launch_plan(wg_plan* pl, cudaStream_t st);
+// The same, run for the plan's last execution
+static int terms_run(const wg_plan* pl, cudaStream_t st, const wg_plan** out) {
+  const int rc = terms_plan(pl, out);
+  if (rc || *out == pl || pl->terms_of == pl->executions) return rc;
+  const int rc2 = launch_plan(pl->terms, st);
+  if (!rc2) pl->terms_of = pl->executions;
+  return rc2;
 }
 
 // `n` side streams that start where `st` stands
@@ -1507,6 +1526,7 @@ static int launch_plan(wg_plan* pl, cudaStream_t st) {
 // Direct launches, or -- with use_graph -- one CUDA graph captured on first use (the launch
 // attributes are set by a direct execution first) and replayed on the caller's stream.
 static int execute_plan(wg_plan* pl, cudaStream_t st) {
+  ++pl->executions;
   if (!pl->use_graph) return launch_plan(pl, st);
   if (!pl->graph_exec) {
     int rc = launch_plan(pl, st);  // sets the kernels' shared-memory attributes, warms up
@@ -1654,13 +1674,10 @@ int wg_plan_read(wg_plan* plan, double* out, void* stream) {
 int wg_plan_read_magnitudes(wg_plan* plan, double* out, void* stream) {
   if (!plan || (!out && plan->total_out > 0)) return fail(WG_EINVAL, "NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
-  wg_plan* terms = nullptr;
-  const int rc = terms_plan(plan, &terms);
+  std::lock_guard<std::mutex> lk(*plan->terms_mu);
+  const wg_plan* terms = nullptr;
+  const int rc = terms_run(plan, st, &terms);
   if (rc) return rc;
-  if (terms != plan) {
-    const int rc2 = launch_plan(terms, st);
-    if (rc2) return rc2;
-  }
   if (plan->total_out > 0)
     CK(cudaMemcpyAsync(out, terms->d_mag, sizeof(double) * plan->total_out, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -1677,15 +1694,14 @@ int wg_plan_kernel_launches(const wg_plan* plan) {
 
 int wg_plan_partials(wg_plan* plan, double* out, int capacity, void* stream) {
   if (!plan) return fail(WG_EINVAL, "plan is NULL");
-  wg_plan* terms = nullptr;
-  const int rc = terms_plan(plan, &terms);
+  cudaStream_t st = (cudaStream_t)stream;
+  std::lock_guard<std::mutex> lk(*plan->terms_mu);
+  const wg_plan* terms = nullptr;
+  int rc = terms_plan(plan, &terms);
   if (rc) return rc;
   if (!out || capacity < terms->nparts) return terms->nparts;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (terms != plan) {
-    const int rc2 = launch_plan(terms, st);
-    if (rc2) return rc2;
-  }
+  rc = terms_run(plan, st, &terms);
+  if (rc) return rc;
   if (terms->nparts > 0)
     CK(cudaMemcpyAsync(out, terms->d_partials, sizeof(double2) * terms->nparts, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -1694,8 +1710,9 @@ int wg_plan_partials(wg_plan* plan, double* out, int capacity, void* stream) {
 
 int wg_plan_chunk(const wg_plan* plan, int chunk, int* inst, int* part, long long* t0, long long* t1) {
   if (!plan) return fail(WG_EINVAL, "bad chunk index");
-  wg_plan* terms = nullptr;
-  const int rc = terms_plan(const_cast<wg_plan*>(plan), &terms);
+  std::lock_guard<std::mutex> lk(*plan->terms_mu);
+  const wg_plan* terms = nullptr;
+  const int rc = terms_plan(plan, &terms);
   if (rc) return rc;
   if (chunk < 0 || chunk >= (int)terms->chunks.size()) return fail(WG_EINVAL, "bad chunk index");
   const ChunkDev& c = terms->chunks[chunk];
