@@ -156,7 +156,12 @@ typedef struct wg_plan_options {
 int wg_plan_create_ex(const wg_instance* inst, int count, int precision, const wg_plan_options* options,
                       wg_plan** plan);
 int wg_plan_execute(wg_plan* plan, void* stream);
+/* Waits for the stream and copies the outputs.  WG_ECUDA when a tree launch since the last read gave up
+ * waiting for its own blocks (about 3 s of polling); the next execution starts afresh. */
 int wg_plan_read(wg_plan* plan, double* out, void* stream);
+/* Polls of a barrier before a tree launch gives up (0: the default, 2^22); not of a graph captured
+ * before. */
+int wg_plan_barrier_polls(wg_plan* plan, unsigned int polls);
 /* Per output of the last execution: the sum over sieve terms of |prefactor x term| (real plus
  * imaginary magnitude) times the output's final scale, i.e. the size of the terms the result
  * cancels from.  magnitude / |result| is the sum's condition number: the result's rounding error

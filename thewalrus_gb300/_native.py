@@ -125,6 +125,7 @@ EXPORTS = [
     "wg_measure_fp_peaks", "wg_hafnian_noalloc", "wg_state_create", "wg_state_destroy",
     "wg_plan_create_requests", "wg_plan_device_bytes", "wg_instance_terms", "wg_state_create_from_cov",
     "wg_check_arith", "wg_plan_read_magnitudes", "wg_hafnian_direct", "wg_matched_reps",
+    "wg_plan_barrier_polls",
 ]
 
 
@@ -168,6 +169,7 @@ def load(build_if_needed=True):
     lib.wg_plan_execute.argtypes = [vp, vp]
     lib.wg_plan_read.argtypes = [vp, dp, vp]
     lib.wg_plan_read_magnitudes.argtypes = [vp, dp, vp]
+    lib.wg_plan_barrier_polls.argtypes = [vp, ctypes.c_uint]
     lib.wg_plan_outputs.argtypes = [vp]
     lib.wg_plan_kernel_launches.argtypes = [vp]
     lib.wg_plan_transfer_bytes.argtypes = [vp, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong)]

@@ -268,6 +268,7 @@ struct wg_plan {
   int tree_parts = 0;  // most partials of a tree's output
   unsigned char* d_prog = nullptr;
   unsigned char* d_ws = nullptr;
+  unsigned int polls = wg::TREE_POLLS;
   long long executions = 0;
   // a plan with trees answers the per-term queries (magnitudes, chunks, partials) by a plan over
   // the same device matrices that evaluates term by term, made when first asked and run once for every
@@ -1434,6 +1435,7 @@ static int launch_trees(wg_plan* pl, cudaStream_t st) {
     p.pool = pl->d_pool;
     p.partials = pl->d_partials;
     p.ws = pl->d_ws + G.ws_off;
+    p.polls = pl->polls;
     p.err = pl->d_err;
     p.ninst = G.ninst;
     p.nrounds = G.nrounds;
@@ -1551,6 +1553,21 @@ static int execute_plan(wg_plan* pl, cudaStream_t st) {
   return WG_OK;
 }
 
+// The outputs, when `st` has come to them (written into pinned memory by the kernels, or copied).  An
+// execution whose launch gave up is an error, reported once: the flag is cleared for the next one.
+static int read_outputs(wg_plan* pl, double* out, cudaStream_t st) {
+  const size_t bytes = sizeof(double2) * pl->total_out;
+  if (bytes && !pl->h_out) CK(cudaMemcpyAsync(out, pl->d_out, bytes, cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (bytes && pl->h_out) memcpy(out, pl->h_out, bytes);
+  for (int i = 0; i < pl->total_out; ++i) {
+    if (memcmp(out + 2 * i, &GAVE_UP, sizeof(GAVE_UP))) continue;
+    CK(cudaMemsetAsync(pl->d_err, 0, sizeof(int), st));
+    return fail(WG_ECUDA, "a tree launch gave up waiting for its own blocks");
+  }
+  return WG_OK;
+}
+
 static void destroy_plan(wg_plan* pl) {
   if (!pl) return;
   destroy_plan(pl->terms);
@@ -1664,10 +1681,12 @@ int wg_plan_execute(wg_plan* plan, void* stream) {
 
 int wg_plan_read(wg_plan* plan, double* out, void* stream) {
   if (!plan || (!out && plan->total_out > 0)) return fail(WG_EINVAL, "NULL argument");
-  cudaStream_t st = (cudaStream_t)stream;
-  if (plan->total_out > 0)
-    CK(cudaMemcpyAsync(out, plan->d_out, sizeof(double2) * plan->total_out, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  return read_outputs(plan, out, (cudaStream_t)stream);
+}
+
+int wg_plan_barrier_polls(wg_plan* plan, unsigned int polls) {
+  if (!plan) return fail(WG_EINVAL, "plan is NULL");
+  plan->polls = polls ? polls : TREE_POLLS;
   return WG_OK;
 }
 
@@ -1888,13 +1907,7 @@ int wg_run(const wg_instance* inst, int count, int precision, double* out, void*
   rc = build_plan(inst, count, precision, opt, pl);
   if (!rc) rc = execute_plan(pl, st);
   if (!rc && !out && pl->total_out > 0) rc = fail(WG_EINVAL, "NULL argument");
-  if (!rc && pl->h_out) {
-    const cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) rc = fail(WG_ECUDA, "one-shot run: %s", cudaGetErrorString(e));
-    else memcpy(out, pl->h_out, sizeof(double2) * pl->total_out);
-  } else if (!rc) {
-    rc = wg_plan_read(pl, out, st);
-  }
+  if (!rc) rc = read_outputs(pl, out, st);
   // nothing in flight may still read or write the block that the next call takes
   if (rc) cudaStreamSynchronize(st);
   pinned_give(pl->pinned);

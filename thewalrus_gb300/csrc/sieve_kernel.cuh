@@ -1241,13 +1241,17 @@ __device__ __forceinline__ const InstDev& reduce_instance(const InstDev* inst, i
   return inst[lo];
 }
 
-// The final scale (0.5^(N/2-1) etc., and the undoing of any input prescaling); NaN when a launch gave
-// up waiting for its own blocks (*err).
+// Both parts of the outputs of an execution whose launch gave up waiting for its own blocks: a quiet NaN
+// that no arithmetic makes.
+constexpr unsigned long long GAVE_UP = 0x7ff8776169742121ull;
+__device__ __forceinline__ double gave_up() { return __longlong_as_double((long long)GAVE_UP); }
+
+// The final scale (0.5^(N/2-1) etc., and the undoing of any input prescaling), unless *err.
 __device__ __forceinline__ void reduce_write(const InstDev& I, int gw, const RSum& s, const double* scales, double2* out,
                                              double* mags, const int* err) {
   const double sc = scales[I.scale_base + gw - I.out_base];
   if (err && *err) {
-    out[gw] = make_double2(nan(""), nan(""));
+    out[gw] = make_double2(gave_up(), gave_up());
   } else if (I.modp) {  // residues (< 2^31) summed exactly in FP64 (fewer than 2^22 chunks), then mod p
     const unsigned long long r = (unsigned long long)(s.sr + s.cr) % I.modp;
     out[gw] = make_double2((double)(r * (unsigned long long)sc % I.modp), 0.0);

@@ -135,6 +135,7 @@ struct TreeParams {
   unsigned char* ws;
   double2* partials;
   unsigned int* bar;
+  unsigned int polls;        // of a barrier before a CTA gives up
   int* err;
   TreeFinish fin;
 };
@@ -1317,12 +1318,13 @@ __device__ __forceinline__ void tree_store(const TreeInst& T, S sum, long long s
 }
 
 // Barrier of the `ctas` CTAs of a cooperative launch that share trees (one CTA: a block barrier).  The
-// wait is bounded: after about 3 s of polling a CTA gives up, its later barriers do not wait, and the
-// error flag makes the outputs NaN.
+// wait is bounded: after TREE_POLLS polls, about 3 s, a CTA gives up, its later barriers do not wait, and
+// the error flag makes the outputs gave_up(), which the host reports and clears (read_outputs, sieve.cu).
+constexpr unsigned int TREE_POLLS = 1u << 22;
 struct TreeSync {
   unsigned int* bar;
   int* err;
-  unsigned int ctas;
+  unsigned int ctas, polls;
   unsigned int target = 0;
   bool ok = true;  // thread 0's
   __device__ __forceinline__ void operator()() {
@@ -1336,7 +1338,7 @@ struct TreeSync {
         unsigned int v, n = 0;
         do {
           asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-        } while (v < target && ++n < (1u << 22));
+        } while (v < target && ++n < polls);
         ok = v >= target;
         if (!ok) atomicExch(err, 1);
       }
@@ -1395,7 +1397,7 @@ __device__ __forceinline__ void tree_body(const TreeParams& P, const int cta, co
   __shared__ int s_next[2];
   if (threadIdx.x == 0) s_next[0] = 0;
   __syncthreads();
-  TreeSync sync{P.bar, P.err, (unsigned int)ctas};
+  TreeSync sync{P.bar, P.err, (unsigned int)ctas, P.polls};
   for (int r = 0; r < P.nrounds; ++r) {
     const TreeRound R = rounds[r];
     // A round's warps go to the CTAs in turn.  Where that is more than one a warp, the CTA's warps take
