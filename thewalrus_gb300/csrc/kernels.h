@@ -7,6 +7,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "sieve_kernel.cuh"
 #include "tree_kernel.cuh"
 
@@ -41,22 +43,36 @@ WG_TREE_UNIT_DECL(fdd)
 cudaError_t tree_launch_mods(const TreeMods& m, int ctas, int smem, cudaStream_t st);
 cudaError_t sieve_tables_mods(const double* binom, const double* inv);
 
+// Lets a kernel's launches on the current device ask for all the dynamic shared memory there is beside
+// its static part.  Once and always the same: launches of several threads, each with its own size, would
+// otherwise lower it for one another between setting it and launching.
+template <auto K>
+static inline cudaError_t allow_shared() {
+  static std::atomic<unsigned long long> done{0};  // a bit per device
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (dev < 64 && (done.load() >> dev & 1))) return e;
+  cudaFuncAttributes a;
+  e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, K);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+  if (e == cudaSuccess && dev < 64) done |= 1ull << dev;
+  return e;
+}
+
 // A launch of `ctas` CTAs whose trees are shared by `group` of them: these wait for one another, so
 // that more than one are launched cooperatively.
-template <class Params>
-static inline cudaError_t tree_launch_kernel(void (*k)(Params), const Params& p, int ctas, int group, int smem,
-                                             cudaStream_t st) {
-  if (smem > 32 * 1024) {  // with the kernel's static shared memory it may pass 48 KB, which needs the attribute
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
+template <auto K, class Params>
+static inline cudaError_t tree_launch_kernel(const Params& p, int ctas, int group, int smem, cudaStream_t st) {
+  const cudaError_t e = allow_shared<K>();
+  if (e != cudaSuccess) return e;
   if (group == 1) {
-    k<<<ctas, TREE_THREADS, smem, st>>>(p);
+    K<<<ctas, TREE_THREADS, smem, st>>>(p);
     return cudaGetLastError();
   }
   Params arg = p;
   void* args[] = {&arg};
-  return cudaLaunchCooperativeKernel((const void*)k, dim3(ctas), dim3(TREE_THREADS), args, (size_t)smem, st);
+  return cudaLaunchCooperativeKernel((const void*)K, dim3(ctas), dim3(TREE_THREADS), args, (size_t)smem, st);
 }
 
 // 1/k modulo a prime in Montgomery form, k < 256, by k * inv(k) = 1: inv(k) = -(p / k) inv(p mod k)

@@ -98,7 +98,7 @@ static __global__ void __launch_bounds__(TREE_THREADS, 1) tree_mods_kernel(const
 }
 
 cudaError_t tree_launch_mods(const TreeMods& m, int ctas, int smem, cudaStream_t st) {
-  return tree_launch_kernel(tree_mods_kernel, m, ctas, ctas / m.n, smem, st);
+  return tree_launch_kernel<tree_mods_kernel>(m, ctas, ctas / m.n, smem, st);
 }
 
 cudaError_t sieve_tables_mods(const double* binom, const double* inv) {

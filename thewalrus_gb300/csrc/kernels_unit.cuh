@@ -8,26 +8,24 @@ namespace wg {
 #define WG_CAT(a, b) WG_CAT2(a, b)
 
 cudaError_t WG_CAT(sieve_launch_, WG_UNIT_NAME)(const SieveParams& p, int ctas, int wpc, cudaStream_t st) {
-  auto k = sieve_kernel<WG_UNIT_SCALAR>;
-  const int smem = wpc * p.L.bytes;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t e = allow_shared<sieve_kernel<WG_UNIT_SCALAR>>();
   if (e != cudaSuccess) return e;
-  k<<<ctas, 32 * wpc, smem, st>>>(p);
+  sieve_kernel<WG_UNIT_SCALAR><<<ctas, 32 * wpc, wpc * p.L.bytes, st>>>(p);
   return cudaGetLastError();
 }
 
 int WG_CAT(sieve_occupancy_, WG_UNIT_NAME)(int wpc, int smem) {
   int nb = 0;
-  auto k = sieve_kernel<WG_UNIT_SCALAR>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 32 * wpc, smem) != cudaSuccess) return 0;
+  if (allow_shared<sieve_kernel<WG_UNIT_SCALAR>>() != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sieve_kernel<WG_UNIT_SCALAR>, 32 * wpc, smem) != cudaSuccess)
+    return 0;
   return nb;
 }
 
 #ifndef WG_UNIT_PRIME  // (residues: kernels_mods.cu)
 cudaError_t WG_CAT(tree_launch_, WG_UNIT_NAME)(const TreeParams& p, bool parts, int ctas, int smem, cudaStream_t st) {
-  if (parts) return tree_launch_kernel(tree_kernel<WG_UNIT_SCALAR>, p, ctas, ctas, smem, st);
-  return tree_launch_kernel(tree_kernel<typename TreeScalar<WG_UNIT_SCALAR>::T>, p, ctas, ctas, smem, st);
+  if (parts) return tree_launch_kernel<tree_kernel<WG_UNIT_SCALAR>>(p, ctas, ctas, smem, st);
+  return tree_launch_kernel<tree_kernel<typename TreeScalar<WG_UNIT_SCALAR>::T>>(p, ctas, ctas, smem, st);
 }
 #endif
 
