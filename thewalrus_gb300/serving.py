@@ -186,9 +186,11 @@ class ProbabilityServer:
         12,000 chunks of 64 bytes for the resident warps, and one for every 6.4e7 of a sum's work),
         without the workspace that a plan's trees share: a batch's takes what the budget has left."""
         n = N + (N % 2)
-        terms = 2.0 ** (N // 2 - 1 + N % 2)
-        chunks = min(terms, 12000 + terms * (n + 2.0) ** 3 / 6.4e7)
-        return (n + 3) * (n + 1) * 16 + max(8192 * 16, int(64 * chunks)) + 2048
+        chunks = 2048
+        if N > 24:  # more than 2,048 terms
+            terms = 2 ** (N // 2 - 1 + N % 2)
+            chunks = min(terms, int(12000 + terms * (n + 2.0) ** 3 / 6.4e7))
+        return (n + 3) * (n + 1) * 16 + 64 * chunks + 2048
 
     def serve(self, requests, time_scale=1.0, timeout=600.0):
         """Serve ``requests`` = [(arrival_s, state_index, pattern)] (sorted by arrival) in real time.
