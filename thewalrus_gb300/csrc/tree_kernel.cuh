@@ -335,6 +335,58 @@ struct ConvAcc<c3<R, C>> {
   }
 };
 
+// Sums over leaves.  Within a phase a thread adds its few (a level's 200 MB over the chip's threads: at
+// most 20) in the node's scalar, as a term's coefficients are.  Beyond it FP64 and double-float leaves are
+// added in FP64, a warp's phases with Neumaier's compensation, as the per-term kernel adds its terms;
+// double-double and residue sums stay in their own scalar.  V: what is added up and stored.
+template <class S>
+struct Leaf {
+  using V = S;
+  static constexpr bool compensated = false;
+  __device__ static __forceinline__ V of(S x) { return x; }
+};
+template <class S, class Val>
+struct LeafFp {
+  using V = Val;
+  static constexpr bool compensated = true;
+  __device__ static __forceinline__ V of(S x) {
+    if constexpr (Ar<S>::cplx) return Ar<S>::to_c64(x);
+    else return Ar<S>::to_c64(x).re;
+  }
+};
+template <> struct Leaf<double> : LeafFp<double, double> {};
+template <> struct Leaf<dfr> : LeafFp<dfr, double> {};
+template <> struct Leaf<c64> : LeafFp<c64, c64> {};
+template <> struct Leaf<cdf> : LeafFp<cdf, c64> {};
+template <> struct Leaf<c3<double, c64>> : LeafFp<c3<double, c64>, c64> {};
+template <> struct Leaf<c3<dfr, cdf>> : LeafFp<c3<dfr, cdf>, c64> {};
+
+// The sums of a single instance's leaves, output k of a warp at [warp][k], in shared memory: they are
+// touched once a leaf phase, and registers kept for them through all the others cost spills.
+template <class S>
+struct LeafSums {
+  using V = typename Leaf<S>::V;
+  V s[TREE_THREADS / 32][32], c[Leaf<S>::compensated ? TREE_THREADS / 32 : 1][32];
+  __device__ __forceinline__ void begin(int w, int k, V x) {
+    s[w][k] = x;
+    if constexpr (Leaf<S>::compensated) c[w][k] = Ar<V>::zero();
+  }
+  __device__ __forceinline__ void add(int w, int k, V x) {
+    if constexpr (!Leaf<S>::compensated) {
+      s[w][k] = Ar<V>::add(s[w][k], x);
+    } else if constexpr (Ar<V>::cplx) {
+      neumaier(s[w][k].re, c[w][k].re, x.re);
+      neumaier(s[w][k].im, c[w][k].im, x.im);
+    } else {
+      neumaier(s[w][k], c[w][k], x);
+    }
+  }
+  __device__ __forceinline__ V value(int w, int k) const {
+    if constexpr (Leaf<S>::compensated) return Ar<V>::add(s[w][k], c[w][k]);
+    else return s[w][k];
+  }
+};
+
 // loads and stores of node elements (the host check counts them)
 template <class S>
 __host__ __device__ __forceinline__ S tld(const S* p) { return *p; }
@@ -1153,11 +1205,10 @@ __host__ __device__ void tree_gloop(const TreeInst& T, int q, const S* par, long
   }
 }
 
-// ---- leaves: this thread's share of the output (batch: the sums of the warp, left in sm) over nodes [0, np) of a buffer of stride ps
+// ---- leaves without a batch mode: this thread's share of the output over nodes [0, np) of a buffer of stride ps
 #pragma nv_exec_check_disable
 template <class S, int TL>
-__host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, int np, const S* m, S* sm, int smn,
-                                int tid, int nthr) {
+__host__ __device__ S tree_leaf_sum(const TreeInst& T, const S* par, long long ps, int np, const S* m, int tid, int nthr) {
   using A = Ar<S>;
   const int L = T.deg[T.steps] + 1, D = L - 1, dg = T.diag;
   const long long st = (long long)L * ps;
@@ -1209,7 +1260,7 @@ __host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, i
       for (int k = 0; k < TT; ++k)
         if (t0 + k >= 0) sum = A::fma(tld(pp + (D - t0 - k) * ps), acc[k].sum(), sum);
     }
-  } else if (T.pB < 0) {
+  } else {
     for (int p = tid; p < np; p += nthr) {
       if (T.pO < 0) {
         sum = A::add(sum, tld(par + D * ps + p));
@@ -1218,91 +1269,100 @@ __host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, i
         for (int s = 0; s <= D; ++s) sum = A::fma(tld(par + p + (D - s) * ps), tld(vo + s * ps), sum);
       }
     }
-  } else {
-    // batch mode b with loop series v and pair series c: k photons give H_k = v H_(k-1) +
-    // (k-1) c H_(k-2); with an unpaired vertex o: v_o H_k + k c_ob H_(k-1).  One warp per node, the
-    // series and the output sums in its shared memory.  An FP64 instruction takes its 64 clocks
-    // however few lanes it has, so the lanes split: four to a coefficient, then four to an output
-    // (12 modes, cutoff 6: 53,000 clocks with a lane per coefficient and a warp sum per output).
-    const int lane = tid & (WG_TREE_LANES - 1), nw = nthr / WG_TREE_LANES;
-    const int sub = lane % WG_TREE_SPLIT, grp = lane / WG_TREE_SPLIT;
-    constexpr int NG = WG_TREE_LANES / WG_TREE_SPLIT;
-    const bool staged = smn >= 32 + (T.nout + 4) * L;  // every H_k kept, and copies of v and c
-    const int rows = staged ? T.nout : 3;
-    S *const o = sm, *const h = sm + 32, *gv = h + rows * L, *gc = gv + L;
-    for (int k = lane; k < T.nout; k += WG_TREE_LANES) o[k] = A::zero();
-    WG_TREE_SYNCWARP();
-    for (int p = tid / WG_TREE_LANES; p < np; p += nw) {
-      const S* pp = par + p;
-      TreeSer<S> v = {const_cast<S*>(pp + (long long)tree_ent2(T.pB, T.pL, dg) * st), ps};
-      TreeSer<S> c = {const_cast<S*>(pp + (long long)tree_ent(T.pB, T.pB, 1) * st), ps};
-      if (staged) {
-        v = ser_stage<S>(v.p, ps, L, gc + L, lane);
-        c = ser_stage<S>(c.p, ps, L, gc + 2 * L, lane);
-      }
-      for (int t = lane; t < L; t += WG_TREE_LANES) {
-        h[t] = t == 0 ? A::one() : A::zero();
-        if (T.pO >= 0) {
-          gv[t] = conv_one(pp, ps, L, pp + (long long)tree_ent2(T.pO, T.pL, dg) * st, ps, L, t);
-          gc[t] = conv_one(pp, ps, L, pp + (long long)tree_ent2(T.pO, T.pB, dg) * st, ps, L, t);
-        } else {
-          gv[t] = tld(pp + t * ps);
-        }
-      }
-      WG_TREE_SYNCWARP();
-      // the dots of outputs k0 .. k1 - 1
-      auto dots = [&](int k0, int k1) {
-        for (int kb = k0; kb < k1; kb += NG) {
-          const int k = kb + grp;
-          ConvAcc<S> x = ConvAcc<S>::of(A::zero()), y = x;
-          if (k < k1) {
-            const S *hk = h + (k % rows) * L, *hl = h + ((k + rows - 1) % rows) * L;
-            for (int t = sub; t < L; t += WG_TREE_SPLIT) {
-              x.fma(gv[D - t], hk[t]);
-              if (k && T.pO >= 0) y.fma(gc[D - t], hl[t]);
-            }
-          }
-          S r = x.sum();
-          if (T.pO >= 0) r = A::add(r, tree_times(y.sum(), k));
-          r = split_sum(r);
-          if (k < k1 && sub == 0) o[k] = A::add(o[k], r);
-        }
-        WG_TREE_SYNCWARP();
-      };
-      for (int k = 1; k < T.nout; ++k) {
-        S* hn = h + (k % rows) * L;
-        const S *h1 = h + ((k - 1) % rows) * L, *h2 = h + ((k + rows - 2) % rows) * L;
-        if (!staged) dots(k - 1, k);
-        for (int tb = 0; tb < L; tb += NG) {
-          const int t = tb + grp;
-          ConvAcc<S> x = ConvAcc<S>::of(A::zero()), y = x;
-          if (t < L) {
-            conv_part(x, (const S*)v.p, v.st, L, h1, 1ll, t, sub);
-            if (k > 1) conv_part(y, (const S*)c.p, c.st, L, h2, 1ll, t, sub);
-          }
-          S n = x.sum();
-          if (k > 1) n = A::add(n, tree_times(y.sum(), k - 1));
-          n = split_sum(n);
-          if (t < L && sub == 0) hn[t] = n;
-        }
-        WG_TREE_SYNCWARP();
-      }
-      dots(staged ? 0 : T.nout - 1, T.nout);
-    }
   }
   return sum;
 }
 
-// a warp's leaf share: lane k < nout returns output k's (batch: from the warp's part of sm)
+// ---- leaves with a batch mode: the sums of the warp's nodes, left in sm
+#pragma nv_exec_check_disable
 template <class S>
-__device__ __forceinline__ S tree_warp_share(const TreeInst& T, S sum, const S* sm) {
-  const int lane = threadIdx.x & 31;
-  if (T.pB < 0) return warp_sum(sum);
-  __syncwarp();
-  if (lane < T.nout) sum = sm[lane];
-  __syncwarp();
-  return sum;
+__host__ __device__ void tree_leaf_batch(const TreeInst& T, const S* par, long long ps, int np, S* sm, int smn, int tid,
+                                         int nthr) {
+  using A = Ar<S>;
+  const int L = T.deg[T.steps] + 1, D = L - 1, dg = T.diag;
+  const long long st = (long long)L * ps;
+  // batch mode b with loop series v and pair series c: k photons give H_k = v H_(k-1) +
+  // (k-1) c H_(k-2); with an unpaired vertex o: v_o H_k + k c_ob H_(k-1).  One warp per node, the
+  // series and the output sums in its shared memory.  An FP64 instruction takes its 64 clocks
+  // however few lanes it has, so the lanes split: four to a coefficient, then four to an output
+  // (12 modes, cutoff 6: 53,000 clocks with a lane per coefficient and a warp sum per output).
+  const int lane = tid & (WG_TREE_LANES - 1), nw = nthr / WG_TREE_LANES;
+  const int sub = lane % WG_TREE_SPLIT, grp = lane / WG_TREE_SPLIT;
+  constexpr int NG = WG_TREE_LANES / WG_TREE_SPLIT;
+  const bool staged = smn >= 32 + (T.nout + 4) * L;  // every H_k kept, and copies of v and c
+  const int rows = staged ? T.nout : 3;
+  S *const o = sm, *const h = sm + 32, *gv = h + rows * L, *gc = gv + L;
+  for (int k = lane; k < T.nout; k += WG_TREE_LANES) o[k] = A::zero();
+  WG_TREE_SYNCWARP();
+  for (int p = tid / WG_TREE_LANES; p < np; p += nw) {
+    const S* pp = par + p;
+    TreeSer<S> v = {const_cast<S*>(pp + (long long)tree_ent2(T.pB, T.pL, dg) * st), ps};
+    TreeSer<S> c = {const_cast<S*>(pp + (long long)tree_ent(T.pB, T.pB, 1) * st), ps};
+    if (staged) {
+      v = ser_stage<S>(v.p, ps, L, gc + L, lane);
+      c = ser_stage<S>(c.p, ps, L, gc + 2 * L, lane);
+    }
+    for (int t = lane; t < L; t += WG_TREE_LANES) {
+      h[t] = t == 0 ? A::one() : A::zero();
+      if (T.pO >= 0) {
+        gv[t] = conv_one(pp, ps, L, pp + (long long)tree_ent2(T.pO, T.pL, dg) * st, ps, L, t);
+        gc[t] = conv_one(pp, ps, L, pp + (long long)tree_ent2(T.pO, T.pB, dg) * st, ps, L, t);
+      } else {
+        gv[t] = tld(pp + t * ps);
+      }
+    }
+    WG_TREE_SYNCWARP();
+    // the dots of outputs k0 .. k1 - 1
+    auto dots = [&](int k0, int k1) {
+      for (int kb = k0; kb < k1; kb += NG) {
+        const int k = kb + grp;
+        ConvAcc<S> x = ConvAcc<S>::of(A::zero()), y = x;
+        if (k < k1) {
+          const S *hk = h + (k % rows) * L, *hl = h + ((k + rows - 1) % rows) * L;
+          for (int t = sub; t < L; t += WG_TREE_SPLIT) {
+            x.fma(gv[D - t], hk[t]);
+            if (k && T.pO >= 0) y.fma(gc[D - t], hl[t]);
+          }
+        }
+        S r = x.sum();
+        if (T.pO >= 0) r = A::add(r, tree_times(y.sum(), k));
+        r = split_sum(r);
+        if (k < k1 && sub == 0) o[k] = A::add(o[k], r);
+      }
+      WG_TREE_SYNCWARP();
+    };
+    for (int k = 1; k < T.nout; ++k) {
+      S* hn = h + (k % rows) * L;
+      const S *h1 = h + ((k - 1) % rows) * L, *h2 = h + ((k + rows - 2) % rows) * L;
+      if (!staged) dots(k - 1, k);
+      for (int tb = 0; tb < L; tb += NG) {
+        const int t = tb + grp;
+        ConvAcc<S> x = ConvAcc<S>::of(A::zero()), y = x;
+        if (t < L) {
+          conv_part(x, (const S*)v.p, v.st, L, h1, 1ll, t, sub);
+          if (k > 1) conv_part(y, (const S*)c.p, c.st, L, h2, 1ll, t, sub);
+        }
+        S n = x.sum();
+        if (k > 1) n = A::add(n, tree_times(y.sum(), k - 1));
+        n = split_sum(n);
+        if (t < L && sub == 0) hn[t] = n;
+      }
+      WG_TREE_SYNCWARP();
+    }
+    dots(staged ? 0 : T.nout - 1, T.nout);
+  }
 }
+
+// either
+#pragma nv_exec_check_disable
+template <class S, int TL>
+__host__ __device__ S tree_leaf(const TreeInst& T, const S* par, long long ps, int np, const S* m, S* sm, int smn,
+                                int tid, int nthr) {
+  if (T.pB < 0) return tree_leaf_sum<S, TL>(T, par, ps, np, m, tid, nthr);
+  tree_leaf_batch<S>(T, par, ps, np, sm, smn, tid, nthr);
+  return Ar<S>::zero();
+}
+
 template <class S>
 __device__ __forceinline__ void tree_store(const TreeInst& T, S sum, long long slot, double2* partials) {
   using A = Ar<S>;
@@ -1377,7 +1437,9 @@ __device__ __forceinline__ void tree_body(const TreeParams& P, const int cta, co
   constexpr int TL = tree_tile<S>();
   S* sm = reinterpret_cast<S*>(smem);
   S* smw = sm + (threadIdx.x >> 5) * P.sm_warp;
-  S total = A::zero();
+  using V = typename Leaf<S>::V;
+  __shared__ LeafSums<S> sums;
+  bool some = false;  // this warp has leaves in `sums`
   const TreeInst* insts = P.inst;
   const TreeRound* rounds = P.rounds;
   const TreeSeg* segs = P.segs;
@@ -1447,14 +1509,25 @@ __device__ __forceinline__ void tree_body(const TreeParams& P, const int cta, co
           break;
         case TP_PREP: tree_prep<S>(T, G.q, par, G.pstride, G.np, scr, chi, smw, P.sm_warp, tid, nthr); break;
         case TP_LEAF: {
-          const S sum = G.tile == 0   ? tree_leaf<S, 0>(T, par, G.pstride, G.np, ms, smw, P.sm_warp, tid, nthr)
-                        : G.tile == 1 ? tree_leaf<S, 1>(T, par, G.pstride, G.np, ms, smw, P.sm_warp, tid, nthr)
-                                      : tree_leaf<S, TL>(T, par, G.pstride, G.np, ms, smw, P.sm_warp, tid, nthr);
-          if (P.ninst == 1) {  // all leaves are one instance's: one partial per CTA, below
-            total = A::add(total, T.pB < 0 ? sum : tree_warp_share<S>(T, sum, smw));
+          V share;
+          if (T.pB >= 0) {  // output k's to lane k
+            tree_leaf_batch<S>(T, par, G.pstride, G.np, smw, P.sm_warp, tid, nthr);
+            __syncwarp();
+            share = Leaf<S>::of(lane < T.nout ? smw[lane] : A::zero());
+            __syncwarp();
           } else {
-            tree_store<S>(T, tree_warp_share<S>(T, sum, smw), G.part + (long long)(vw - G.warp0) * T.pstride, P.partials);
+            const S sum = G.tile == 0   ? tree_leaf_sum<S, 0>(T, par, G.pstride, G.np, ms, tid, nthr)
+                          : G.tile == 1 ? tree_leaf_sum<S, 1>(T, par, G.pstride, G.np, ms, tid, nthr)
+                                        : tree_leaf_sum<S, TL>(T, par, G.pstride, G.np, ms, tid, nthr);
+            share = warp_sum(Leaf<S>::of(sum));
           }
+          if (P.ninst > 1) {
+            tree_store<V>(T, share, G.part + (long long)(vw - G.warp0) * T.pstride, P.partials);
+          } else if (lane < T.nout) {  // all leaves are one instance's: one partial per CTA, below
+            if (some) sums.add(threadIdx.x >> 5, lane, share);
+            else sums.begin(threadIdx.x >> 5, lane, share);
+          }
+          some = true;
           break;
         }
         case TP_G2: {
@@ -1490,17 +1563,15 @@ __device__ __forceinline__ void tree_body(const TreeParams& P, const int cta, co
   }
   if (P.ninst == 1) {
     const TreeInst& T = insts[0];
-    if (T.pB < 0) total = warp_sum(total);
-    __syncthreads();  // sm's leaf part is free now
-    if (lane < T.nout) sm[(threadIdx.x >> 5) * T.nout + lane] = total;
+    if (!some && lane < T.nout) sums.begin(threadIdx.x >> 5, lane, Ar<V>::zero());
     __syncthreads();
     if (threadIdx.x < 32) {
       const int nw = blockDim.x >> 5;
-      S s = A::zero();
-      if (T.nout == 1) s = warp_sum(lane < nw ? sm[lane] : s);
+      V v = Ar<V>::zero();
+      if (T.nout == 1) v = warp_sum(lane < nw ? sums.value(lane, 0) : v);
       else if (lane < T.nout)
-        for (int w = 0; w < nw; ++w) s = A::add(s, sm[w * T.nout + lane]);
-      tree_store<S>(T, s, segs[P.nsegs - 1].part + (long long)cta * T.pstride, P.partials);
+        for (int w = 0; w < nw; ++w) v = Ar<V>::add(v, sums.value(w, lane));
+      tree_store<V>(T, v, segs[P.nsegs - 1].part + (long long)cta * T.pstride, P.partials);
     }
   }
   tree_finish(P.fin, ctas);
