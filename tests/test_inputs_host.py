@@ -17,3 +17,20 @@ def test_negative_counts_are_refused():
         with pytest.raises(ValueError):
             state.norm(pattern)
     assert abs(state.norm([2, 0, 3, 1]) - state.vacuum / np.sqrt(12)) <= 1e-15 * abs(state.vacuum)
+
+
+def test_pairing_of_counts_of_any_size():
+    """Counts up to the largest of 64 bits pair as smaller ones do; larger ones are refused, not cut."""
+    big = 2 ** 63 - 1
+    for reps in ([big, big], [big, 2 ** 62], [2 ** 62, 2 ** 62 + 1, 3], [big, 1, 1], [big]):
+        x, m, odd = tw.matched_reps(reps)
+        used = np.zeros(len(reps), dtype=object)
+        for e, r in enumerate(m.tolist()):
+            used[x[e]] += r
+            used[x[e + len(m)]] += r
+        if odd is not None:
+            used[odd] += 1
+        assert used.tolist() == reps
+    for reps in ([2 ** 64], [2 ** 64 + 2, 1, 1], [1, 2 ** 70], np.array([2 ** 64 - 1], dtype=np.uint64)):
+        with pytest.raises(OverflowError):
+            tw.matched_reps(reps)

@@ -3,6 +3,7 @@
 The library is compiled in-tree into ``thewalrus_gb300/_build/`` with nvcc.  There is no CPU
 fallback: every computing entry point fails with ``RuntimeError`` when no GPU is usable.
 """
+import array
 import ctypes
 import os
 import subprocess
@@ -472,18 +473,19 @@ def hafnian_direct(A, loop, rtol, atol):
 
 def matched_reps(reps):
     """Pairing of the repetition counts (a list of ints): (x, edge_reps, oddmode or None).  One block
-    holds the counts, both results' room and the two scalars: the call is ~2 us, most of it ctypes."""
+    holds both results' room and the two scalars: the call is ~2 us, most of it ctypes.  The counts are
+    an ``array``, which refuses (OverflowError) what 64 bits do not hold and a ctypes block would cut."""
     n = len(reps)
-    buf = (ctypes.c_int64 * (7 * n + 2))()
     try:
-        buf[:n] = reps
+        counts = array.array("q", reps)
     except TypeError:  # numbers of other types
-        buf[:n] = [int(r) for r in reps]
+        counts = array.array("q", [int(r) for r in reps])
+    buf = (ctypes.c_int64 * (6 * n + 2))()
     p = ctypes.addressof(buf)
-    check((_lib or load()).wg_matched_reps(p, n, p + 8 * n, p + 40 * n, p + 56 * n, p + 56 * n + 8))
-    E, odd = buf[7 * n], buf[7 * n + 1]  # 32-bit stores into zeros
+    check((_lib or load()).wg_matched_reps(counts.buffer_info()[0], n, p, p + 32 * n, p + 48 * n, p + 48 * n + 8))
+    E, odd = buf[6 * n], buf[6 * n + 1]  # 32-bit stores into zeros
     res = np.frombuffer(buf, dtype=np.int64)
-    return res[n:n + 2 * E], res[5 * n:5 * n + E], None if odd == 0xFFFFFFFF else odd
+    return res[:2 * E], res[4 * n:4 * n + E], None if odd == 0xFFFFFFFF else odd
 
 
 def check_arith(op, x, x_lo=None, y=None, y_lo=None):

@@ -2026,7 +2026,7 @@ int wg_matched_reps(const int64_t* reps, int n, int64_t* x, int64_t* mult, int* 
   if ((n > 0 && (!reps || !x || !mult)) || n < 0 || !E || !odd) return fail(WG_EINVAL, "bad pairing arguments");
   *E = 0;
   *odd = -1;
-  int64_t sum = 0;
+  __int128 sum = 0;
   std::vector<std::pair<int64_t, int>> pool;  // a heap by count, then index
   for (int i = 0; i < n; ++i) {
     sum += reps[i];
@@ -2048,7 +2048,7 @@ int wg_matched_reps(const int64_t* reps, int n, int64_t* x, int64_t* mult, int* 
   int e = 0;
   while (pool.size() > 1 || (pool.size() == 1 && pool.front().first > 1)) {
     const auto top = pop();
-    if (pool.empty() || top.first > 2 * pool.front().first) {
+    if (pool.empty() || top.first - pool.front().first > pool.front().first) {
       x[e] = top.second;
       right.push_back(top.second);
       mult[e++] = top.first / 2;
