@@ -34,3 +34,28 @@ def test_pairing_of_counts_of_any_size():
     for reps in ([2 ** 64], [2 ** 64 + 2, 1, 1], [1, 2 ** 70], np.array([2 ** 64 - 1], dtype=np.uint64)):
         with pytest.raises(OverflowError):
             tw.matched_reps(reps)
+
+
+def test_direct_route_leaves_balancing_and_copies_to_the_general_one(monkeypatch):
+    """Rows that balancing would scale although the unpaired vertex's entries hide it, and arrays whose numbers
+    do not lie on their own boundaries, are not the direct route's."""
+    seen = []
+    monkeypatch.setattr(nat, "run", lambda insts, precision="fp64", stream=0: seen.append(insts[0]) or np.zeros(1))
+    rng = np.random.default_rng(3)
+    S = rng.normal(size=(7, 7))
+    S = S + S.T
+    d = np.array([1, 1e3, 1, 1e3, 1, 1e3, 1])  # pairs (6, 5), (4, 3), (2, 1), and 0 left over
+    A = S * np.outer(d, d)
+    A[0, 1:] = A[1:, 0] = 1e9
+    assert H._pair_balance(H._sub(A, tw.matched_reps([1] * 7)[0])) is not None
+    assert nat.hafnian_direct(A, True, 1e-5, 1e-8) is None
+    raw = np.zeros(8 * 36 + 1, dtype=np.uint8)
+    U = raw[1:].view(np.float64).reshape(6, 6)
+    U[:] = S[:6, :6]
+    assert not U.flags.aligned and U.flags.c_contiguous
+    called = []
+    monkeypatch.setattr(nat, "hafnian_direct", lambda *a: called.append(a))
+    tw.hafnian(U)
+    assert not called and len(seen) == 1
+    tw.hafnian(U.copy())
+    assert len(called) == 1

@@ -403,7 +403,7 @@ def hafnian(A, loop=False, rtol=1e-05, atol=1e-08, approx=False, num_samples=100
     """
     if (precision is None and not approx and (loop or method == "glynn") and type(A) is np.ndarray
             and A.ndim == 2 and A.shape[0] == A.shape[1] >= 5 and A.dtype.char in "dD" and A.dtype.isnative
-            and A.flags.c_contiguous and isinstance(rtol, float) and isinstance(atol, float)):
+            and A.flags.c_contiguous and A.flags.aligned and isinstance(rtol, float) and isinstance(atol, float)):
         value = nat.hafnian_direct(A, loop, rtol, atol)  # the usual input: one native call
         if value is not None:
             return value

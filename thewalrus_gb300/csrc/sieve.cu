@@ -1963,7 +1963,7 @@ int wg_hafnian_direct(const void* A, int n, int dtype, int loop, double rtol, do
   for (int i = 0; i < n; ++i)
     for (int j = 0; j < n; ++j) {
       const double m = mod(i, j);
-      rows[i] += m;
+      if (n % 2 == 0 || j) rows[i] += m;  // of the paired vertices, as _pair_balance's
       if (i == j) {
         if (loop) rows[i] += m;
         continue;
