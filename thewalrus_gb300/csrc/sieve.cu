@@ -1663,6 +1663,7 @@ int wg_plan_create_ex(const wg_instance* inst, int count, int precision, const w
                       wg_plan** plan) {
   if (!plan) return fail(WG_EINVAL, "plan is NULL");
   *plan = nullptr;
+  if (!known_precision(precision)) return fail(WG_EINVAL, "unknown precision %d", precision);
   int rc = ensure_init(-1);
   if (rc) return rc;
   wg_plan_options opt;
