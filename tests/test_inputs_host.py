@@ -65,7 +65,7 @@ def test_plans_take_one_precision():
     """Several primes at once are wg_run's; a plan refuses them as it does any other unknown precision."""
     lib = nat.load()
     opt = nat.WgPlanOptions()
-    for code in [nat.WG_PREC_PRIMES + k for k in range(1, 6)] + [nat.WG_PREC_PRIMES + 3 | nat.WG_PREC_TERMS, 7, 99, -1]:
+    for code in [nat.WG_PREC_PRIMES + k for k in range(1, 6)] + [nat.WG_PREC_PRIMES + 3 | nat.WG_PREC_TERMS, 8, 99, -1]:
         h = ctypes.c_void_p()
         arr = (nat.WgInstance * 1)()
         assert lib.wg_plan_create_ex(arr, 0, code, ctypes.byref(opt), ctypes.byref(h)) == -1  # WG_EINVAL
