@@ -53,6 +53,10 @@ extern "C" {
  * whose term magnitudes, chunks and partials the plan reports (a plan with trees runs it when they
  * are asked for). */
 #define WG_PREC_TERMS 64
+/* Added to a precision: the elimination tree for every instance that has one, its multiple edges as they
+ * are, also where the terms are taken because that is sooner or what results were before.  For checks of
+ * the trees; what has none is evaluated term by term. */
+#define WG_PREC_TREE 128
 #define WG_MOD_PRIME_0 2147483647u
 #define WG_MOD_PRIME_1 2147483629u
 #define WG_MOD_PRIME_2 2147483587u
@@ -169,6 +173,8 @@ int wg_plan_barrier_polls(wg_plan* plan, unsigned int polls);
 int wg_plan_read_magnitudes(wg_plan* plan, double* out, void* stream);
 int wg_plan_outputs(const wg_plan* plan);
 int wg_plan_kernel_launches(const wg_plan* plan);
+/* Number of the plan's instances that are evaluated by an elimination tree. */
+int wg_plan_trees(const wg_plan* plan);
 /* Diagnostics for chunk-level checks.  wg_plan_partials copies the unscaled per-chunk partial
  * sums (complex interleaved, nout per chunk) of the last execution when capacity (in complex
  * values) suffices and returns their count.  wg_plan_chunk describes chunk `chunk`: its

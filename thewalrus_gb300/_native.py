@@ -34,7 +34,8 @@ PRECISIONS.update({"mod%d" % k: v for k, v in enumerate(WG_PREC_MOD)})
 # the same, evaluated term by term (WG_PREC_TERMS): the evaluation behind the term magnitudes
 WG_PREC_TERMS = 64
 WG_PREC_PRIMES = 16  # + k: modulo each of the first k primes
-PRECISIONS.update({k + "-terms": v | WG_PREC_TERMS for k, v in list(PRECISIONS.items())})
+WG_PREC_TREE = 128  # by tree wherever there is one
+PRECISIONS.update({k + s: v | f for k, v in list(PRECISIONS.items()) for s, f in (("-terms", WG_PREC_TERMS), ("-tree", WG_PREC_TREE))})
 
 _lock = threading.Lock()
 _lib = None
@@ -126,7 +127,7 @@ EXPORTS = [
     "wg_measure_fp_peaks", "wg_hafnian_noalloc", "wg_state_create", "wg_state_destroy",
     "wg_plan_create_requests", "wg_plan_device_bytes", "wg_instance_terms", "wg_state_create_from_cov",
     "wg_check_arith", "wg_plan_read_magnitudes", "wg_hafnian_direct", "wg_matched_reps",
-    "wg_plan_barrier_polls",
+    "wg_plan_barrier_polls", "wg_plan_trees",
 ]
 
 
@@ -170,6 +171,7 @@ def load(build_if_needed=True):
     lib.wg_plan_execute.argtypes = [vp, vp]
     lib.wg_plan_read.argtypes = [vp, dp, vp]
     lib.wg_plan_read_magnitudes.argtypes = [vp, dp, vp]
+    lib.wg_plan_trees.argtypes = [vp]
     lib.wg_plan_barrier_polls.argtypes = [vp, ctypes.c_uint]
     lib.wg_plan_outputs.argtypes = [vp]
     lib.wg_plan_kernel_launches.argtypes = [vp]
@@ -350,6 +352,10 @@ class Plan:
 
     def device_bytes(self):
         return int(self.lib.wg_plan_device_bytes(self.handle))
+
+    def trees(self):
+        """How many of the instances are evaluated by an elimination tree."""
+        return int(self.lib.wg_plan_trees(self.handle))
 
     def transfer_bytes(self):
         h, d = ctypes.c_longlong(), ctypes.c_longlong()

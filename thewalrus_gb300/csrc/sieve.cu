@@ -206,6 +206,7 @@ struct Prepared {
   std::vector<double> ascale;    // the input prescale's share of each output
   int precision;
   bool mixed = false;            // (MatrixForm)
+  bool forced = false;           // WG_PREC_TREE
   std::vector<double> tscales() const;  // output scales of the tree's sum
   int ttype() const {            // the tree's node type
     const bool cplx = stype == ST_CPLX64 || stype == ST_CPLXDF || stype == ST_CPLXDD;
@@ -219,6 +220,9 @@ struct Group {
   int wpc, ctas;
   int chunk_begin, chunk_count;
 };
+
+// the evaluations that may be added to a precision
+constexpr int kEvaluations = WG_PREC_TERMS | WG_PREC_TREE;
 
 // One launch of the tree kernel: trees of one scalar type and the program that walks them.
 struct TreeLaunch {
@@ -267,6 +271,7 @@ struct wg_plan {
   bool serial_groups = false;
   std::vector<wg::TreeLaunch> trees;
   std::vector<unsigned char> tree_prog;
+  int ntrees = 0;          // instances
   int tree_parts = 0;  // most partials of a tree's output
   unsigned char* d_prog = nullptr;
   unsigned char* d_ws = nullptr;
@@ -466,7 +471,7 @@ std::vector<double> Prepared::tscales() const {
 static void take_tree(Prepared& P, int precision, const std::vector<double>& ascale, const MatrixForm& f) {
   P.mixed = f.mixed;
   P.tree = f.symmetric && tree_build(P.d, P.T) && tree_fits(P.T, tree_bytes(P.ttype())) &&
-           !keeps_terms(P.stype, P.d.kind, P.T.K, f);
+           (P.forced || !keeps_terms(P.stype, P.d.kind, P.T.K, f));
   if (!P.tree) return;
   P.T.comp_off = stype_dd(P.stype) ? P.d.nout : 0;
   P.T.pstride = (stype_dd(P.stype) ? 2 : 1) * P.d.nout;
@@ -476,7 +481,8 @@ static void take_tree(Prepared& P, int precision, const std::vector<double>& asc
 
 static int prepare(const wg_instance& in, int precision, Prepared& P) {
   const bool terms_only = (precision & WG_PREC_TERMS) != 0;
-  precision &= ~WG_PREC_TERMS;
+  P.forced = (precision & WG_PREC_TREE) != 0;
+  precision &= ~kEvaluations;
   memset(&P.d, 0, sizeof(P.d));
   InstDev& d = P.d;
   if (in.dtype != WG_FLOAT64 && in.dtype != WG_COMPLEX128) return fail(WG_EINVAL, "dtype must be WG_FLOAT64 or WG_COMPLEX128");
@@ -795,7 +801,8 @@ static MatrixForm request_form(const wg_request& r, const wg_state& st) {
 static int prepare_request(const wg_request& r, const wg_state& st, int precision, Prepared& P, GatherDev& g,
                            std::vector<int>& idx) {
   const bool terms_only = (precision & WG_PREC_TERMS) != 0;
-  precision &= ~WG_PREC_TERMS;
+  P.forced = (precision & WG_PREC_TREE) != 0;
+  precision &= ~kEvaluations;
   memset(&P.d, 0, sizeof(P.d));
   InstDev& d = P.d;
   if (r.E < 1 || r.E > MAX_EDGES || !r.x || !r.edge_reps) return fail(WG_EINVAL, "request needs 1..32 edges");
@@ -873,12 +880,12 @@ static int prepare_request(const wg_request& r, const wg_state& st, int precisio
 }
 
 static bool known_precision(int precision) {
-  const int p = precision & ~WG_PREC_TERMS;
+  const int p = precision & ~kEvaluations;
   return p == WG_PREC_FP64 || p == WG_PREC_DF || p == WG_PREC_DD || prec_mod(p);
 }
 // the primes of WG_PREC_PRIMES(k) (0: another precision)
 static int prec_primes(int precision) {
-  const int k = (precision & ~WG_PREC_TERMS) - WG_PREC_PRIMES(0);
+  const int k = (precision & ~kEvaluations) - WG_PREC_PRIMES(0);
   return k >= 1 && k <= MOD_N ? k : 0;
 }
 
@@ -889,7 +896,7 @@ static int build_plan(const wg_instance* v, int count, int precision, const wg_p
   pl->primes = std::max(primes, 1);
   std::vector<Prepared> P((size_t)count * pl->primes);
   for (int i = 0; i < count * pl->primes; ++i) {
-    const int prec = primes ? (WG_PREC_MOD0 + i / count) | (precision & WG_PREC_TERMS) : precision;
+    const int prec = primes ? (WG_PREC_MOD0 + i / count) | (precision & kEvaluations) : precision;
     int rc = prepare(v[i % count], prec, P[i]);
     if (rc) return fail(rc, "instance %d: %s", i % count, g_err.c_str());
   }
@@ -952,6 +959,7 @@ static long long plan_trees(std::vector<Prepared>& P, const std::vector<TreeLeve
   std::vector<int> order;
   for (int i = 0; i < count; ++i)
     if (P[i].tree) order.push_back(i);
+  pl->ntrees = (int)order.size();
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     return P[a].ttype() != P[b].ttype() ? P[a].ttype() < P[b].ttype() : lev[a].bytes > lev[b].bytes;
   });
@@ -1130,7 +1138,7 @@ constexpr double kLeastWorkspace = 64e6;
 // ext_pool: the instances' matrices are on the device already, at their a_off
 static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_options& opt, wg_plan* pl,
                          GatherSpec* gs, unsigned char* ext_pool) {
-  precision &= ~WG_PREC_TERMS;
+  precision &= ~kEvaluations;
   const int count = (int)P.size();
   const double chunk_scale = opt.chunk_scale > 0 ? opt.chunk_scale : 1.0;
   const int wpc_cap = opt.max_warps_per_cta > 0 ? std::min(opt.max_warps_per_cta, 8) : kDefaultWarpsPerCta;
@@ -1138,9 +1146,11 @@ static int finalize_plan(std::vector<Prepared>& P, int precision, const wg_plan_
   pl->serial_groups = opt.serial_groups != 0;
   pl->precision = precision;
   pl->device = g_device;
-  split_edges(P);
-  if (terms_sooner(P))
-    for (Prepared& p : P) p.tree = false;
+  if (P.empty() || !P[0].forced) {
+    split_edges(P);
+    if (terms_sooner(P))
+      for (Prepared& p : P) p.tree = false;
+  }
   const bool roomy = opt.max_workspace <= 0 || opt.max_workspace > kLeastWorkspace;
   double limit = opt.max_workspace > 0 ? (double)opt.max_workspace : 1e18;
   const std::vector<TreeLevels> lev = place_trees(P, limit);
@@ -1717,6 +1727,8 @@ int wg_plan_read_magnitudes(wg_plan* plan, double* out, void* stream) {
 
 int wg_plan_outputs(const wg_plan* plan) { return plan ? plan->total_out : fail(WG_EINVAL, "plan is NULL"); }
 
+int wg_plan_trees(const wg_plan* plan) { return plan ? plan->ntrees : fail(WG_EINVAL, "plan is NULL"); }
+
 int wg_plan_kernel_launches(const wg_plan* plan) {
   if (!plan) return fail(WG_EINVAL, "plan is NULL");
   const size_t trees = plan->side_trees ? 1 : plan->trees.size();
@@ -1863,7 +1875,7 @@ int wg_plan_create_requests(const wg_state* state, const wg_request* req, int co
                             const wg_plan_options* options, wg_plan** plan) {
   if (!plan || !state || count < 0 || (count > 0 && !req)) return fail(WG_EINVAL, "bad request list");
   *plan = nullptr;
-  if ((precision & ~WG_PREC_TERMS) != WG_PREC_FP64 && (precision & ~WG_PREC_TERMS) != WG_PREC_DF)
+  if ((precision & ~kEvaluations) != WG_PREC_FP64 && (precision & ~kEvaluations) != WG_PREC_DF)
     return fail(WG_EINVAL, "unknown precision %d", precision);
   int rc = ensure_init(-1);
   if (rc) return rc;
