@@ -105,7 +105,7 @@ class GaussianState:
     def norm(self, pattern):
         """<0|psi> / sqrt(prod n_i!) for the pattern."""
         counts = pattern.tolist() if isinstance(pattern, np.ndarray) else pattern
-        return self.vacuum / math.sqrt(float(math.prod([math.factorial(int(k)) for k in counts if k > 1 or k < 0])))
+        return self.vacuum / math.sqrt(float(math.prod([math.factorial(int(k)) for k in counts if k and k != 1])))
 
     def trivial_loop_hafnian(self, pattern):
         """The loop hafnian for patterns with at most one photon (no sieve needed), else None."""
