@@ -298,6 +298,9 @@ class WgPlanOptions(ctypes.Structure):
 class Plan:
     """Device-resident batch of instances: create once, execute many times, read results.
 
+    ``precision``: "fp64", "df", "dd" or "mod0" to "mod4", evaluated as the default is (trees where
+    one exists); with "-terms" appended term by term, with "-tree" by tree wherever there is one.
+
     ``chunk_scale`` (term-chunk size), ``max_warps_per_cta``, ``merge_classes`` (one persistent
     launch per scalar type), ``use_graph`` (CUDA-graph replay), ``serial_groups`` (launch the
     groups one after another on the caller's stream) and ``max_workspace`` (device bytes for the

@@ -450,7 +450,8 @@ static MatrixForm matrix_form(const void* A, int dtype, size_t n, double tol) {
 //   n = 21 to 33), none (complex); Gaussian states and generic matrices with multiple edges none of
 //   200 for K <= 14, 1 % at K = 18; uncoupled blocks (a state and its conjugate, whose pairing
 //   couples what the matrix does not) 0.6 % at K = 12, 8 to 23 % at 16, 70 % at 20;
-//   double-float (roundoff 2^5 larger): complex n = 34 none of 100 (largest 8.5e-10), n = 40 15 %;
+//   double-float (roundoff 2^5 larger): complex n = 34 none of 140 (largest 8.5e-10), n = 36 none of 40 (9.0e-10),
+//   n = 38 one of 40, n = 40 15 %;
 //   real of both signs none at n = 14, 3 % at 20, 18 % at 32.
 static bool keeps_terms(int stype, int kind, int K, const MatrixForm& f) {
   const bool real = stype == ST_REAL64 || stype == ST_REALDF, loops = kind != KIND_PLAIN;

@@ -29,9 +29,9 @@
 // of one cooperative launch with a barrier after each (2,400 clocks): the narrow ones, a few thousand
 // clocks of FP64 and L2 latency, bound trees of up to ~14 pairs, the FP64 pipe (77 % busy at n = 34)
 // the larger ones.  Measured against the per-term kernel (us a call): complex n = 24 576 -> 96, n = 40
-// 244,600 -> 4,820; real n = 44 (positive) 380,900 -> 7,980; loops n = 27 2,320 -> 144; 96 matrices of
-// n = 8 .. 32 in a plan 61,850 -> 1,720; complex n = 28 in double-double 22,300 -> 731, n = 34 in
-// double-float 12,380 -> 436; the exact count of a graph of 32 vertices 9,100 -> 342.
+// 244,600 -> 4,840; real n = 44 (positive) 380,900 -> 7,980; loops n = 27 2,320 -> 145; 96 matrices of
+// n = 8 .. 32 in a plan 61,850 -> 1,720; complex n = 28 in double-double 22,300 -> 716, n = 34 in
+// double-float 12,380 -> 443; the exact count of a graph of 32 vertices 9,100 -> 338.
 // (The reference's tree for unit edges is thewalrus/_hafnian.py recursive_hafnian's squeeze; this
 // one sums the finite-difference signs of _calc_hafnian / _calc_loop_hafnian, :443-577, and of
 // loop_hafnian_batch.py:50-208.)
