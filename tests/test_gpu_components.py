@@ -75,3 +75,19 @@ def test_served_requests(pattern):
         plan = nat.Plan.from_requests(state, [tw.matched_reps(p)] * 2)
         plan.execute()
         close_by_component(plan.read(), nat.run([tw.prepare_loop_hafnian(A, gamma, p)] * 2, "dd-terms"), "fp64")
+
+
+@pytest.mark.parametrize("h", [1e-4, 1e-9])
+@pytest.mark.parametrize("fixed", [[1, 1], [1, 1, 1], [2, 1, 1], [2, 2, 1, 1, 1, 1]])
+def test_batches_whose_mode_alone_is_complex(fixed, h):
+    """Modes that are nearly real beside a batch mode of any phase: output 0 does not know the batch mode."""
+    m = len(fixed) + 1
+    A = wl.real_nonneg(m, seed=m) + 1j * h * wl.real_nonneg(m, seed=m + 1)
+    D = A[0] * 0.5
+    A[-1] = A[:, -1] = wl.complex_symmetric(m, seed=2)[0] * 3
+    D[-1] = 2 + 1j
+    inst = tw.prepare_loop_hafnian_batch(A, D, fixed, 4)
+    for precision in ("fp64", "df", "dd"):
+        got, want = nat.run([inst], precision), nat.run([inst], "dd-terms")
+        close_by_component(got[:1], want[:1], precision)
+        assert np.all(np.abs(got - want) <= TOL[precision] * np.abs(want))

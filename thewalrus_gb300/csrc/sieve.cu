@@ -371,18 +371,24 @@ static inline double tree_asymmetry(int precision) {
 // those entries alone moves either part of the sum relative to the whole, and three products lose nothing.
 // At least half of the rows have to say so (random phases: ratios of 0.41, and all but a few rows of two or
 // three entries do; rows of purely real and purely imaginary entries have 0).
-// of an instance's rows: `diag` with the diagonal, which edges of one pair each do not read
-static bool mixed_rows(const wg_instance& in, bool loops, bool odd, bool diag) {
+// of an instance's rows: `diag` with the diagonal, which edges of one pair each do not read; `fixed` without
+// a batch's own mode, on which output 0 does not depend
+static bool mixed_rows(const wg_instance& in, bool loops, bool odd, bool diag, bool fixed) {
   if (in.dtype != WG_COMPLEX128) return false;
+  auto batch = [&](int i) {  // the vertices of the batch's edge, and the one that its odd mode is matched to
+    return fixed && (i == 0 || i == in.n / 2 || (in.kind == WG_KIND_BATCH_ODD && i == in.n / 2 + 1));
+  };
   const c64 *A = (const c64*)in.A, *D = (const c64*)in.D, *V = (const c64*)in.oddV;
   const c64 o = {in.oddloop[0], in.oddloop[1]};
   const int n = in.n;
-  int rows = 0;
+  int rows = 0, all = odd;
   PartSums last;  // the unpaired vertex's row
   for (int i = 0; i < n; ++i) {
+    if (batch(i)) continue;
+    ++all;
     PartSums s;
     for (int j = 0; j < n; ++j)
-      if (j != i || diag) {
+      if ((j != i || diag) && !batch(j)) {
         s.add(A[(size_t)i * n + j].re, A[(size_t)i * n + j].im);
         if (loops) s.add(D[i], D[j]);
       }
@@ -395,7 +401,7 @@ static bool mixed_rows(const wg_instance& in, bool loops, bool odd, bool diag) {
     rows += s.mixed();
   }
   if (odd) rows += last.mixed();
-  return 2 * rows >= n + odd;
+  return 2 * rows >= all;
 }
 
 static MatrixForm matrix_form(const void* A, int dtype, size_t n, double tol) {
@@ -694,7 +700,9 @@ static int prepare(const wg_instance& in, int precision, Prepared& P) {
   }
   if (!terms_only && in.term_begin == 0 && in.term_end == 0) {
     MatrixForm f = matrix_form(in.A, in.dtype, (size_t)n, tree_asymmetry(precision));
-    f.mixed = mixed_rows(in, nb > 0, kind == KIND_LOOP_ODD, maxr > 1 || kind >= KIND_BATCH_EVEN);
+    const bool batch = kind >= KIND_BATCH_EVEN;
+    f.mixed = mixed_rows(in, nb > 0, kind == KIND_LOOP_ODD, maxr > 1 || batch, false) &&
+              (!batch || mixed_rows(in, true, false, true, true));
     take_tree(P, precision, ascale, f);
   }
   return WG_OK;
