@@ -91,3 +91,18 @@ def test_batches_whose_mode_alone_is_complex(fixed, h):
         got, want = nat.run([inst], precision), nat.run([inst], "dd-terms")
         close_by_component(got[:1], want[:1], precision)
         assert np.all(np.abs(got - want) <= TOL[precision] * np.abs(want))
+
+
+@pytest.mark.parametrize("options", [{"use_graph": True}, {"serial_groups": True}, {"max_workspace": 3e6}])
+def test_plan_of_both_nodes(options):
+    """The launches of both sorts of nodes side by side, replayed from a graph, one after another, in blocks."""
+    near = [wl.real_nonneg(n, seed=n) + 1e-9j * wl.real_nonneg(n, seed=n + 1) for n in (8, 20)]
+    insts = [tw.prepare_hafnian(M) for M in (near[0], wl.complex_symmetric(22, seed=2), near[1], wl.real_nonneg(18, seed=9))]
+    want = nat.run(insts, "dd-terms")
+    plan = nat.Plan(insts, **options)
+    assert plan.trees() == 4
+    for _ in range(3):
+        plan.execute()
+        got = plan.read()
+        close_by_component(got[[0, 2]], want[[0, 2]], "fp64")
+        assert np.all(np.abs(got - want) <= TOL["fp64"] * np.abs(want))

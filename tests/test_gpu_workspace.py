@@ -121,3 +121,13 @@ def test_allocation_that_fails_is_tried_with_less(small_pool):
     last = [tw.prepare_hafnian(wl.complex_symmetric(30, seed=3))]
     small_pool(32e6)  # no tree
     assert np.array_equal(nat.run(last), nat.run(last, "fp64-terms"))
+
+
+@pytest.mark.parametrize("reps", [[2] * 21, [1] + [2] * 20, [3] * 14, [1] * 30])
+def test_plan_of_a_small_and_a_huge_member(reps):
+    """A member of hours beside one whose multiple edge may be taken as copies: the plan is made (its estimates
+    had divided by zero) and not run."""
+    huge = nat.Instance(nat.WG_KIND_PLAIN, wl.real_nonneg(2 * len(reps), seed=1) * 0.1, np.array(reps, dtype=np.int64))
+    plan = nat.Plan([tw.prepare_hafnian(wl.real_nonneg(2, seed=1), [2, 2]), huge])
+    assert plan.total_out == 2
+    plan.close()
